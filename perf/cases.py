@@ -265,3 +265,65 @@ def tolerance(case):
         return {"rel": 1.7e-3}
     out = "bf16" if kind == "step" else case.get("x", "fp32")
     return {"rel": {"bf16": 7e-3, "fp16": 1.4e-3, "fp32": 1.1e-3}[out]}
+
+
+# ---- the same results in 64 bits, plain torch ----------------------------------------------------------------------
+E2M1_VALUES = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0, -0.0, -0.5, -1.0, -1.5, -2.0, -3.0, -4.0, -6.0)
+
+
+def _dense64(pw):
+    """The weight matrix that the packed tensors stand for: value or codebook entry, times the scale of its group."""
+    byte = pw.qweight.long()
+    code = torch.stack([byte & 15, byte >> 4], dim=2).reshape(pw.N, -1)[:, :pw.K]
+    if pw.spec.fmt == "e2m1":
+        w = torch.tensor(E2M1_VALUES, dtype=torch.float64, device=DEVICE)[code]
+    else:
+        w = torch.gather(pw.codebook.double(), 1, code)
+    if pw.scales is not None:
+        w.view(pw.N, -1, pw.spec.group_size).mul_(pw.scales.double()[:, :, None])
+    return w
+
+
+def _hadamard64(n):
+    h = torch.ones(1, 1, dtype=torch.float64, device=DEVICE)
+    while h.shape[0] < n:
+        h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)], 0)
+    return h / n ** 0.5
+
+
+def _linear64(x, pw, bias=None):
+    x = x.double()
+    if pw.spec.had_block:
+        b = pw.spec.had_block
+        x = (x.reshape(-1, pw.K // b, b) @ _hadamard64(b)).reshape(-1, pw.K)
+    y = x @ _dense64(pw).t()
+    return y if bias is None else y + bias.double()
+
+
+def exact(case, seed):
+    """Quantising has no value besides the one that the format defines; everything else is a product in 64 bits."""
+    kind = case["kind"]
+    if kind == "pack":
+        return None
+    s = prepare(case, seed)
+    if kind == "dequant":
+        return _dense64(s["pw"])
+    if kind == "layer":
+        return _linear64(s["x"], s["pw"], s["bias"])
+    if kind == "step":
+        grp = s["grp"]
+        y = torch.zeros(grp.y_arena.numel() // 2, dtype=torch.float64, device=DEVICE)
+        for x, w, o in zip(grp.xs, grp.weights, grp.y_offsets):
+            y[o // 2:o // 2 + case["rows"] * w.N] = _linear64(x, w).reshape(-1)
+        return y
+    if kind == "conv":
+        m, x = s["model"], s["x"]
+        w = _dense64(m.packed).reshape(m.out_channels, m.in_channels, *m.kernel_size)
+        return torch.nn.functional.conv2d(x.double(), w, m.bias.double(), m.stride, m.padding)
+    x = s["x"].double()
+    for m in s["model"]:
+        if isinstance(m, torch.nn.Linear):
+            x = _linear64(x, m.packed, m.bias)
+        elif isinstance(m, torch.nn.ReLU):
+            x = x.relu()
+    return x
