@@ -30,6 +30,11 @@ class jq_problem(ctypes.Structure):
     ]
 
 
+class jq_conv(ctypes.Structure):
+    _fields_ = [(n, c_int32) for n in ("batch", "channels", "height", "width", "kernel_h", "kernel_w", "stride_h", "stride_w",
+                                       "pad_h", "pad_w", "dilation_h", "dilation_w")] + [("stride_x", ctypes.c_int64 * 4)]
+
+
 _SIGNATURES = {
     "jq_version": (c_int, []),
     "jq_strerror": (c_char_p, [c_int]),
@@ -48,6 +53,11 @@ _SIGNATURES = {
     "jq_gemm_ta_grouped": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
     "jq_gemm_ta": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                            c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
+    "jq_gemm_rows_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "jq_gemm_rows": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                             c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p]),
+    "jq_conv_rows": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                             c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p]),
     "jq_ta_status": (c_int, [c_void_p, c_int, c_void_p]),
     "jq_selftest_bounded_wait": (c_int, [c_void_p, ctypes.c_uint, c_void_p]),
     "jq_grouped_plan_bytes": (c_size_t, [c_int]),

@@ -5,10 +5,10 @@ Mirrors the reference's ``QuantConv2d`` surface
 built from an ``nn.Conv2d`` with ``(conv_module, bitwidth=4, mask=None)``,
 ``forward`` = ``F.conv2d(x, W_hat, bias, stride, padding, dilation, groups)``,
 ``commit()``.  The weight ``[O, I, kh, kw]`` is packed as the matrix
-``[O, I*kh*kw]`` and the convolution runs as an implicit GEMM: ``F.unfold``
-lays out the receptive fields (plumbing), the fused packed kernels do the
-multiply (the tensor-core path when the batch of output positions is large
-and the format is E2M1 g32).  groups must be 1.
+``[O, I*kh*kw]`` and the convolution runs as an implicit GEMM: the many-row
+kernel's preparation step gathers the receptive fields from the image.  With a
+rotation, or for a handful of output positions, ``F.unfold`` lays the fields
+out and the linear operator does the multiply.  groups must be 1.
 """
 from __future__ import annotations
 
@@ -81,9 +81,14 @@ class JenksQuantConv2d(nn.Conv2d):
         kh, kw = self.kernel_size
         ho = (H + 2 * self.padding[0] - self.dilation[0] * (kh - 1) - 1) // self.stride[0] + 1
         wo = (W + 2 * self.padding[1] - self.dilation[1] * (kw - 1) - 1) // self.stride[1] + 1
+        packed = self.packed
+        if (x.is_cuda and x.dtype in ops._DT and packed.spec.had_block == 0 and ho > 0 and wo > 0
+                and ops.many_rows(packed.spec.fmt_id, packed.K, packed.spec.group_size, B * ho * wo)
+                and not torch.compiler.is_compiling()):
+            return ops.conv2d(x, packed, self.bias, self.kernel_size, self.stride, self.padding, self.dilation, (ho, wo))
         cols = F.unfold(x, self.kernel_size, self.dilation, self.padding, self.stride)   # [B, I*kh*kw, L]
         rows = cols.transpose(1, 2).reshape(B * ho * wo, -1).contiguous()
-        y = ops.linear(rows, self.packed, self.bias)                                       # [B*L, O]
+        y = ops.linear(rows, packed, self.bias)                                       # [B*L, O]
         return y.reshape(B, ho * wo, self.out_channels).transpose(1, 2).reshape(B, self.out_channels, ho, wo)
 
     def commit(self) -> None:

@@ -31,9 +31,7 @@
 // Every wait on an mbarrier is bounded: on expiry the CTA raises a status word
 // in the workspace, all roles leave their loops, tensor memory is freed and
 // the kernel returns.  Nothing traps or spins without a limit.
-#include "common.cuh"
-#include <cuda.h>
-#include <mutex>
+#include "tc.cuh"
 #include <string.h>
 
 namespace jqta {
@@ -43,7 +41,6 @@ constexpr int kTileM = 128;
 constexpr int kWStage = 32 * 128;            // bytes of a weight stage: 32 rows x 128 bytes (256 codes), swizzled by TMA
 constexpr int kXMaxStages = 8;               // stages of an MMA issuer's activation ring, at most
 constexpr int kTabBytes = 4 * 256 * 128;     // GF4: 256 entries x 32 lanes x 4 bytes per 32-row quarter
-constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr int kHeaderBytes = 1024;           // workspace: int status
 
 struct TaProblem {
@@ -66,123 +63,6 @@ struct PeerInfo {
     int n;
     long long delta[8];
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("{ .reg .b64 t; mbarrier.arrive.shared::cta.b64 t, [%0]; }" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("{ .reg .b64 t; mbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1; }" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Bounded wait: false (and the CTA-wide error flag raised) when it gives up, after kSpinLimit polls or
-// about 0.25 s of SM clock, whichever comes first; also false as soon as another thread has raised the flag.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *err) {
-    if (mbar_try(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        if (mbar_try(bar, parity)) return true;
-        if (*err) return false;
-        if (i > 8192) {
-            __nanosleep(64);
-            if (clock64() - t0 > 500000000LL) break;
-        }
-    }
-    *err = JQ_ERR_TIMEOUT;
-    return false;
-}
-// global -> shared bulk copy (16-byte aligned, a multiple of 16 bytes); its bytes are counted on the mbarrier
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-// 2-D tiled TMA load: box at (x bytes, y rows) of the tensor map -> shared memory; x must be a multiple of 16
-__device__ __forceinline__ void tma_2d_g2s(uint32_t dst, const void *tmap, int x, int y, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void tma_2d_prefetch_l2(const void *tmap, int x, int y) {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// K-major operand in shared memory without swizzle: 8 rows x 16 bytes are contiguous; lbo = bytes between
-// the two 16-byte K chunks of one MMA, sbo = bytes between 8-row groups (bits 46-47 = 1: sm_100 descriptor).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3fffu);
-    d |= (uint64_t)((lbo >> 4) & 0x3fffu) << 16;
-    d |= (uint64_t)((sbo >> 4) & 0x3fffu) << 32;
-    d |= (uint64_t)1 << 46;
-    return d;
-}
-// kind::f16 instruction descriptor: D = fp32, A = B = fp16, both K-major
-__host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
-    return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-// D[128 x N] (+)= A[128 x 16] (tensor memory) . B[N x 16]^T (shared memory)
-__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                 "  tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint32_t dp4a_u(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-
-// Programmatic dependent launch: the main kernels are launched while the activation preparation in front of them
-// is still running; everything they do before pdl_wait() (barrier set-up, problem look-ups, the first weight boxes)
-// overlaps it, everything that reads the prepared activation comes after.  Without the launch attribute both are
-// no-ops.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// e with amax * 2^-e below 2^15 after the rotation's worst-case growth (the rule of the GEMV kernels)
-__device__ __forceinline__ int act_exponent(float amax, bool had) {
-    uint32_t bits = __float_as_uint(amax);
-    int field = (bits >> 23) & 0xff;
-    if (field == 0xff || (bits & 0x7fffffffu) == 0) return 0;
-    int e = field - 127 - (had ? 10 : 14);
-    return max(-100, min(100, e));
-}
 
 // ---- activation preparation -----------------------------------------------------
 // One block per (problem, batch row): x -> (x 2^-e) -> block Hadamard -> fp16, written as
@@ -1127,24 +1007,6 @@ static size_t ta_align(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // Tensor map over the packed rows of one matrix: bytes [N rows][ldw], boxes of 32 rows x 128 bytes with the
 // 128-byte swizzle; rows past N read as zeros.  The driver entry point is looked up once (no link-time
 // dependency on the driver library).
-typedef CUresult (*ta_encode_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static ta_encode_fn ta_encoder() {
-    static ta_encode_fn fn = nullptr;
-    static bool tried = false;
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lk(mu);
-    if (!tried) {
-        tried = true;
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qr) == cudaSuccess &&
-            qr == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<ta_encode_fn>(p);
-    }
-    return fn;
-}
 static int ta_encode_map(CUtensorMap *out, const void *qw, int N, int ldw) {
     ta_encode_fn enc = ta_encoder();
     if (!enc) return JQ_ERR_UNSUPPORTED;

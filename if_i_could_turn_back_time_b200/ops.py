@@ -93,6 +93,18 @@ def _ta_aligned(*tensors) -> bool:
     return all(t is None or t.data_ptr() % 16 == 0 for t in tensors)
 
 
+MAX_ROWS_SCRATCH = 256 << 20      # bytes of prepared activation a many-row call holds at once; longer inputs go in parts
+
+
+def many_rows(fmt_id: int, K: int, g: int, batch: int) -> bool:
+    """Calls that the many-row kernel takes: more rows than one pass of the kernels for small batches.  Those read the
+    weights once per pass (16 rows for GF4, 64 for E2M1 in 32-code groups, 8 for the shapes that only the row loops
+    take), the many-row kernel decodes them once per 256 rows."""
+    if fmt_id == _lib.JQ_FMT_E2M1 and ta_eligible(fmt_id, K, g, batch):
+        return batch > ta_max_batch(fmt_id)
+    return batch > 16
+
+
 _tls = threading.local()   # every host thread has its own scratch buffers: calls from different threads never share one
 _checked = False
 
@@ -175,6 +187,64 @@ def _linear_rows_ta(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y
     return y
 
 
+def _rows_scratch(device, nbytes: int):
+    """(scratch pointer, size, status word) of a many-row call: the thread's "ta" buffer when the prepared activation
+    fits into it as it is, an allocation of the call's own otherwise.  The status word is the buffer's."""
+    ws = _workspace(device, 1024, "ta")
+    if ws.numel() >= 1024 + nbytes:
+        return None, ctypes.c_void_p(ws.data_ptr() + 1024), ws.numel() - 1024, _ptr(ws)
+    own = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    return own, _ptr(own), nbytes, _ptr(ws)
+
+
+def _linear_many_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y):
+    lib = _lib.load()
+    rows = x2.shape[0]
+    part = max(256, MAX_ROWS_SCRATCH // ((K + 127) // 128 * 256) // 256 * 256)
+    with _on(x2.device):
+        for b0 in range(0, rows, part):
+            b1 = min(rows, b0 + part)
+            xs, ys = (x2, y) if rows <= part else (x2[b0:b1], y[b0:b1])
+            own, scratch, size, status = _rows_scratch(x2.device, lib.jq_gemm_rows_scratch_bytes(fmt_id, N, K, b1 - b0, g))
+            st = lib.jq_gemm_rows(fmt_id, _ptr(qweight), _ptr(scales), _ptr(codebook), _ptr(xs), _ptr(bias), _ptr(ys), N, K,
+                                  b1 - b0, g, had, _DT[x2.dtype], _DT[y.dtype], scratch, size, status, _stream())
+            _lib.check(st, "jq_gemm_rows")
+            del own
+    if _checked:
+        check_status()
+    return y
+
+
+def conv2d(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor], kernel_size, stride, padding, dilation,
+           out_hw) -> torch.Tensor:
+    """The receptive fields of x [B, C, H, W] times the packed [O, C*kh*kw] matrix -> [B, O, ho, wo] (channels-last
+    strides): the fields are gathered by the preparation kernel, there is no unfolded copy."""
+    lib = _lib.load()
+    _need_cuda(x, pw.qweight, pw.scales, pw.codebook, bias)
+    if bias is not None and bias.dtype != torch.float32:
+        bias = bias.float()
+    B, C, H, W = x.shape
+    L = out_hw[0] * out_hw[1]
+    y = torch.empty((B * L, pw.N), dtype=x.dtype, device=x.device)
+    geo = [int(v) for pair in (kernel_size, stride, padding, dilation) for v in pair]
+    part = max(1, MAX_ROWS_SCRATCH // ((pw.K + 127) // 128 * 256) // L)          # images at once
+    with _on(x.device):
+        for b0 in range(0, B, part):
+            b1 = min(B, b0 + part)
+            xs, ys = x[b0:b1], y[b0 * L:b1 * L]
+            c = _lib.jq_conv(b1 - b0, C, H, W, *geo, (ctypes.c_int64 * 4)(*x.stride()))
+            own, scratch, size, status = _rows_scratch(
+                x.device, lib.jq_gemm_rows_scratch_bytes(pw.spec.fmt_id, pw.N, pw.K, (b1 - b0) * L, pw.spec.group_size))
+            st = lib.jq_conv_rows(pw.spec.fmt_id, _ptr(pw.qweight), _ptr(pw.scales), _ptr(pw.codebook), _ptr(xs), _ptr(bias),
+                                  _ptr(ys), ctypes.byref(c), pw.N, pw.spec.group_size, _DT[x.dtype], _DT[y.dtype], scratch, size,
+                                  status, _stream())
+            _lib.check(st, "jq_conv_rows")
+            del own
+    if _checked:
+        check_status()
+    return y.view(B, out_hw[0], out_hw[1], pw.N).permute(0, 3, 1, 2)
+
+
 _wsb_cache = {}
 
 
@@ -198,6 +268,8 @@ def _linear_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, out_
     lib = _lib.load()
     Bt = x2.shape[0]
     y = torch.empty((Bt, N), dtype=_OUT[out_id] or x2.dtype, device=x2.device)
+    if many_rows(fmt_id, K, g, Bt):
+        return _linear_many_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y)
     if ta_eligible(fmt_id, K, g, Bt) and _ta_aligned(qweight, scales, codebook):
         return _linear_rows_ta(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y)
     xd, yd = _DT[x2.dtype], _DT[y.dtype]

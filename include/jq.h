@@ -259,6 +259,33 @@ int jq_gemm_ta(int fmt, const void *qweight, const void *scales, const void *cod
                jq_stream_t stream);
 int jq_ta_status(void *workspace, int clear, jq_stream_t stream);
 
+/* Many activation rows (prompts, evaluation batches): the same operator as jq_gemv_* / jq_gemm_ta for any B >= 1 and
+ * every K, g and alignment of the formats above, the F.linear(x, W_bar, bias) of
+ * Quantization_Experiments/layers.py:38.  The weights are decoded once per tile of up to 256 rows and multiplied on the
+ * tensor cores (tcgen05, fp16 operands, fp32 accumulation).  Scales are applied in fp32 to the sums of their group
+ * (weights and scales exact); E2M1 with g = 32, K % 256 == 0, K >= 512 and 16-byte aligned scales folds them into fp16
+ * weights, as jq_gemm_ta does.  scratch (256-byte aligned, jq_gemm_rows_scratch_bytes) holds the prepared activation
+ * and may be overwritten as soon as the call's kernels have run; status_dev is a device int that must be zero before its
+ * first use and is raised to JQ_ERR_TIMEOUT like the status word of jq_gemm_ta's workspace (whose first word may be
+ * given).  Two launches. */
+size_t jq_gemm_rows_scratch_bytes(int fmt, int N, int K, int B, int g);
+int jq_gemm_rows(int fmt, const void *qweight, const void *scales_or_null, const void *codebook_or_null, const void *x,
+                 const float *bias_or_null, void *y, int N, int K, int B, int g, int had_block, int x_dtype,
+                 int y_dtype, void *scratch, size_t scratch_bytes, int *status_dev, jq_stream_t stream);
+
+/* A convolution as the same product: the packed matrix is [O, channels * kernel_h * kernel_w], the activation rows are
+ * the receptive fields of the output positions, gathered from the image x (zeros outside it) by the preparation
+ * kernel without an unfolded copy; y is [batch * out_h * out_w, O] row-major.  Replaces the F.conv2d of
+ * Quantization_Experiments/layers.py:48-97 (groups = 1).  Scratch as for jq_gemm_rows with B = batch * out_h * out_w. */
+typedef struct jq_conv {
+    int32_t batch, channels, height, width;
+    int32_t kernel_h, kernel_w, stride_h, stride_w, pad_h, pad_w, dilation_h, dilation_w;
+    int64_t stride_x[4];   /* elements between images, channels, rows and columns of x */
+} jq_conv;
+int jq_conv_rows(int fmt, const void *qweight, const void *scales_or_null, const void *codebook_or_null, const void *x,
+                 const float *bias_or_null, void *y, const jq_conv *conv, int O, int g, int x_dtype, int y_dtype,
+                 void *scratch, size_t scratch_bytes, int *status_dev, jq_stream_t stream);
+
 /* Bytes of caller-provided device scratch an op needs for these sizes. */
 size_t jq_workspace_bytes(int op, int N, int K, int B);
 

@@ -1,0 +1,98 @@
+"""The many-row kernel (prompts, evaluation batches, convolutions) against the oracle: edges of its 128-row tiles, of the
+token tiles (32 to 256, one or two accumulators), of the 128-code groups, of the K split over a cluster, and every way
+of folding scales (128, 64 and 32 codes at once, none, folded into fp16 weights)."""
+import numpy as np
+import pytest
+import torch
+
+import if_i_could_turn_back_time_b200 as jq
+from if_i_could_turn_back_time_b200 import ops
+from oracle import formats
+from test_gpu_parity import DEV, TOL, _check_gemv, _weights
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("fmt,N,K,g,had,rows,dtype", [
+    ("gf4", 10, 100, 0, 0, 17, torch.float32),          # one ragged group, odd row count
+    ("gf4", 300, 784, 0, 0, 64, torch.float32),         # seven groups, the last one an eighth full
+    ("gf4", 129, 333, 0, 0, 130, torch.float16),        # odd K; two token halves
+    ("gf4", 128, 640, 128, 128, 129, torch.bfloat16),   # K % 256 != 0: an odd number of groups
+    ("gf4", 257, 1024, 64, 0, 256, torch.bfloat16),     # 64-code scales, a full token tile
+    ("gf4", 70, 960, 32, 0, 257, torch.float32),        # 32-code scales, two token tiles
+    ("gf4", 200, 1024, 256, 128, 33, torch.float16),    # one scale for two groups
+    ("gf4", 64, 11008, 128, 128, 40, torch.bfloat16),   # K split eight ways
+    ("gf4", 1100, 512, 128, 0, 700, torch.bfloat16),
+    ("e2m1", 33, 256, 32, 128, 24, torch.bfloat16),     # too short for the folded weights: exact
+    ("e2m1", 130, 1152, 32, 0, 100, torch.float32),     # K % 256 != 0: exact
+    ("e2m1", 96, 1024, 64, 0, 300, torch.float16),
+    ("e2m1", 140, 384, 96, 0, 20, torch.bfloat16),      # a group that is not a power of two
+    ("e2m1", 256, 2048, 128, 128, 65, torch.bfloat16),
+    ("e2m1", 300, 4096, 32, 0, 65, torch.bfloat16),     # folded
+    ("e2m1", 129, 512, 32, 128, 513, torch.float32),    # folded, three token tiles
+])
+def test_many_rows_against_the_oracle(fmt, N, K, g, had, rows, dtype):
+    spec = jq.QuantSpec(fmt, g, had)
+    assert ops.many_rows(spec.fmt_id, K, g, rows)
+    pw = jq.pack_weight(_weights(N, K, N + K), spec)
+    gen = torch.Generator("cpu").manual_seed(rows)
+    x = (torch.randn(rows, K, generator=gen) * torch.logspace(-2, 2, rows)[:, None]).to(dtype)
+    _check_gemv(pw, x / 100, torch.randn(N, generator=gen))
+    y32 = ops.linear(x.to(DEV), pw.to(DEV), out_dtype=torch.float32)
+    assert torch.equal(ops.linear(x.to(DEV), pw.to(DEV)), y32.to(dtype))      # rounded once
+
+
+def test_many_rows_unit_vectors_read_back_columns_and_misaligned_rows():
+    """x = e_k is exact: every output is an entry of the dequantised matrix, bit for bit; also from an activation that
+    starts 2 bytes off a vector boundary."""
+    pw = jq.pack_weight(_weights(150, 700, 5), jq.QuantSpec("gf4", 0, 0)).to(DEV)
+    ks = [0, 1, 7, 8, 127, 128, 511, 512, 640, 698, 699] * 3
+    raw = torch.zeros(len(ks) * 700 + 1, dtype=torch.float16, device=DEV)
+    x = raw[1:].view(len(ks), 700)
+    for i, k in enumerate(ks):
+        x[i, k] = 1.0
+    y = ops.linear(x, pw, out_dtype=torch.float32)
+    assert torch.equal(y, ops.dequantize(pw)[:, ks].t())
+    assert ops.check_status(raise_on_error=False) == 0
+
+
+def test_many_rows_in_parts_and_from_a_cuda_graph(monkeypatch):
+    pw = jq.pack_weight(_weights(130, 512, 6), jq.QuantSpec("gf4", 128, 128)).to(DEV)
+    x = torch.randn(600, 512, generator=torch.Generator("cpu").manual_seed(1)).bfloat16().to(DEV)
+    whole = ops.linear(x, pw, out_dtype=torch.float32)
+    monkeypatch.setattr(ops, "MAX_ROWS_SCRATCH", 256 * 512 * 2)               # 256 rows at a time
+    parts = ops.linear(x, pw, out_dtype=torch.float32)
+    assert formats.rel_err(parts.cpu().numpy(), whole.cpu().numpy()) <= 2e-6  # fp32 summation order (K split) may differ
+    monkeypatch.undo()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ops.linear(x, pw)
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y = ops.linear(x, pw)
+    x2 = torch.randn(600, 512, generator=torch.Generator("cpu").manual_seed(2)).bfloat16().to(DEV)
+    x.copy_(x2)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, ops.linear(x2, pw))
+
+
+@pytest.mark.parametrize("cin,cout,k,stride,pad,dilation,hw,batch,dtype", [
+    (3, 8, 3, 1, 1, 1, (9, 11), 2, torch.float32), (16, 130, 5, 2, 2, 1, (17, 8), 3, torch.float16),
+    (48, 24, 1, 1, 0, 1, (7, 7), 5, torch.bfloat16), (20, 40, (3, 2), (2, 1), (0, 3), (2, 3), (14, 13), 2, torch.float32)])
+def test_convolution_gathers_receptive_fields(cin, cout, k, stride, pad, dilation, hw, batch, dtype):
+    """Against float64 conv2d on the dequantised weight; contiguous, channels-last and sliced images give the same bits."""
+    torch.manual_seed(cin)
+    q = jq.JenksQuantConv2d(torch.nn.Conv2d(cin, cout, k, stride, pad, dilation), 4).to(DEV)
+    x = torch.randn(batch, cin, *hw, device=DEV).to(dtype)
+    y = q(x)
+    ref = torch.nn.functional.conv2d(x.double(), q.dequantized_weight().double(), q.bias.double(), stride, pad, dilation)
+    assert y.shape == ref.shape and y.dtype == dtype
+    limit = TOL + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11 if dtype == torch.float16 else 0)
+    assert np.abs(y.double().cpu().numpy() - ref.cpu().numpy()).max() <= limit * ref.abs().max().item()
+    assert torch.equal(q(x.to(memory_format=torch.channels_last)), y)
+    wide = torch.zeros(batch, cin + 1, hw[0] + 2, hw[1] + 3, device=DEV, dtype=dtype)
+    wide[:, 1:, 1:-1, 2:-1] = x
+    assert torch.equal(q(wide[:, 1:, 1:-1, 2:-1]), y)
+    assert ops.check_status(raise_on_error=False) == 0
