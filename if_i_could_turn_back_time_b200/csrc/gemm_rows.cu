@@ -76,13 +76,15 @@ __device__ __forceinline__ void store_tile(const Args &p, const float (&acc)[128
     }
 }
 
+template <int N> struct Slices { static constexpr int n = N; };
+
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const __grid_constant__ Args p,
                                                                 const __grid_constant__ CUtensorMap wmap) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint32_t s_tmem;
     __shared__ int s_err;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wg = warp >> 2;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), wg = warp >> 2;   // (uniform for the compiler)
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t xring = sbase, wring0 = sbase + kXRingBytes, bars = wring0 + 4 * kSW * kWStage;
     auto wbar = [&](int w, int s) { return bars + 8u * (w * kSW + s); };                      // weight box landed
@@ -112,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
     // this CTA's tiles and its part of every tile's K range, in 256-code steps
     const int rank = p.split > 1 ? (int)(blockIdx.x % p.split) : 0;
@@ -327,50 +329,63 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const __grid_con
         }
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
-        if (warp == 12 && lane == 0) {
+        if (warp == 12) {
             // =============================== MMA issuer ===============================
+            // (the warp runs converged, see mma_f16_ts)
+            const uint32_t elected = elect_one();
+            auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)); };
             const int cols = p.halves == 2 ? p.HN : p.NT;
             const uint32_t idesc = idesc_f16(kTileM, cols);
             const uint32_t lbo = (uint32_t)p.NT * 16;
             const uint32_t kstep = (2 * lbo) >> 4;             // descriptor address units per K = 16 slice
-            const int per_unit = p.unit >> 4;                  // K slices per fold
+            // Only the address field of a descriptor changes, by constants, and the slices of a fold are unrolled (forming
+            // a descriptor per MMA in a loop took 340 clocks per MMA; 2048 rows: 583 us).
+            const uint64_t desc0 = smem_desc(xring, lbo, 128);
+            const uint32_t stage_units = xstage >> 4, half_units = (uint32_t)p.HN;
             int a_slot = 0, buf = 0, xs = 0;
             uint32_t a_par = 0, d_par = 1, x_par = 0;          // (the first wait on a free accumulator passes at once)
             bool ok = true;
             for (int tile = tile_lo; tile < p.tiles && ok; tile += tile_stride)
                 for (int g = g_lo; g < g_hi && ok; ++g) {
-                    if (!(ok = mbar_wait(afull(a_slot), a_par, err))) break;
+                    if (!(ok = wait(afull(a_slot), a_par))) break;
                     const int xs0 = xs;
                     const uint32_t par0 = x_par;
                     if (++xs == nxs) { xs = 0; x_par ^= 1; }
                     const int xs1 = xs;
                     const uint32_t par1 = x_par;
                     if (++xs == nxs) { xs = 0; x_par ^= 1; }
-                    if (!(ok = mbar_wait(xfull(xs0), par0, err))) break;
+                    if (!(ok = wait(xfull(xs0), par0))) break;
                     tc_fence_after();
-                    bool second = false;
                     const uint32_t a_t = tmem + kA0 + a_slot * 64;
-                    for (int i0 = 0; i0 < 8 && ok; i0 += per_unit)
-                        for (int h = 0; h < p.halves; ++h) {
-                            if (!(ok = mbar_wait(dfree(buf), d_par, err))) break;
-                            tc_fence_after();
-                            for (int i = i0; i < i0 + per_unit; ++i) {
-                                if (i >= 4 && !second) {
-                                    if (!(ok = mbar_wait(xfull(xs1), par1, err))) break;
-                                    second = true;
-                                }
-                                const uint64_t desc = smem_desc(xring + (i < 4 ? xs0 : xs1) * xstage + h * p.HN * 16, lbo, 128) +
-                                                      (uint64_t)((i & 3) * kstep);
-                                mma_f16_ts(tmem + buf * kD, a_t + 8 * i, desc, idesc, i > i0);
-                            }
-                            if (!ok) break;
-                            mma_commit(dfull(buf));
-                            if (++buf == kDBufs) { buf = 0; d_par ^= 1; }
-                        }
+                    const uint64_t lo = desc0 + xs0 * stage_units, hi = desc0 + xs1 * stage_units;
+                    auto fold_unit = [&](auto slices, int i0, uint64_t d0, uint64_t d1) -> bool {   // d0, d1: slices 0-3, 4-7 of the group
+                        if (!wait(dfree(buf), d_par)) return false;
+                        tc_fence_after();
+                        const uint32_t d_t = tmem + buf * kD;
+#pragma unroll
+                        for (int i = 0; i < decltype(slices)::n; ++i)
+                            mma_f16_ts(elected, d_t, a_t + 8 * (i0 + i), (i < 4 ? d0 : d1) + (uint64_t)((i & 3) * kstep), idesc, i > 0);
+                        mma_commit(elected, dfull(buf));
+                        if (++buf == kDBufs) { buf = 0; d_par ^= 1; }
+                        return true;
+                    };
+                    if (p.unit == 128) {
+                        if (!(ok = wait(xfull(xs1), par1))) break;
+                        for (int h = 0; h < p.halves && ok; ++h) ok = fold_unit(Slices<8>{}, 0, lo + h * half_units, hi + h * half_units);
+                    } else if (p.unit == 64) {
+                        for (int h = 0; h < p.halves && ok; ++h) ok = fold_unit(Slices<4>{}, 0, lo + h * half_units, 0);
+                        if (!ok || !(ok = wait(xfull(xs1), par1))) break;
+                        for (int h = 0; h < p.halves && ok; ++h) ok = fold_unit(Slices<4>{}, 4, hi + h * half_units, 0);
+                    } else {
+                        if (!(ok = wait(xfull(xs1), par1))) break;
+                        for (int i0 = 0; i0 < 8 && ok; i0 += 2)
+                            for (int h = 0; h < p.halves && ok; ++h)
+                                ok = fold_unit(Slices<2>{}, i0, (i0 < 4 ? lo : hi) + h * half_units + (uint64_t)((i0 & 3) * kstep), 0);
+                    }
                     if (!ok) break;
-                    mma_commit(xfree(xs0));
-                    mma_commit(xfree(xs1));
-                    mma_commit(afree(a_slot));
+                    mma_commit(elected, xfree(xs0));
+                    mma_commit(elected, xfree(xs1));
+                    mma_commit(elected, afree(a_slot));
                     if (++a_slot == 2) { a_slot = 0; a_par ^= 1; }
                 }
         } else if (warp == 13 && lane == 0) {

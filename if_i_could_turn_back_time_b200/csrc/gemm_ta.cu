@@ -40,7 +40,7 @@ constexpr int kDecodeWarps = 8;              // warps 0-3: first half of the ste
 constexpr int kTileM = 128;
 constexpr int kWStage = 32 * 128;            // bytes of a weight stage: 32 rows x 128 bytes (256 codes), swizzled by TMA
 constexpr int kXMaxStages = 8;               // stages of an MMA issuer's activation ring, at most
-constexpr int kTabBytes = 4 * 256 * 128;     // GF4: 256 entries x 32 lanes x 4 bytes per 32-row quarter
+constexpr int kTabBytes = 4 * 256 * 128;     // GF4, up to 16 rows: 256 entries x 32 lanes x 4 bytes per 32-row quarter
 constexpr int kHeaderBytes = 1024;           // workspace: int status
 
 struct TaProblem {
@@ -115,130 +115,131 @@ __global__ void __launch_bounds__(kPrepThreads) ta_prepare_kernel(const TaProble
 }
 
 // ---- main kernel --------------------------------------------------------------------
-// Roles of a CTA (12 warps): warps 0-7 decode (warp = 32-row quarter q of the tile x half h of the 256-code
-// steps of a row: step sg belongs to half sg & 1); lane 0 of warps 8-11 issues MMAs (two issuers per half:
-// a thread cannot issue a tcgen05.mma more often than every 50 clocks, threads of different warps can) and
-// streams the prepared activation of its own groups; warp 11 also owns the tensor-memory allocation.  The
-// two halves are independent pipelines that meet at the end of a tile.
+// Roles of a CTA (16 warps): warps 0-7 decode (warp = 32-row quarter q of the tile x half h of the 256-code
+// steps of a row: step sg belongs to half sg & 1); warps 8-11 fold (thread = row): they read every 128-code group's
+// accumulator back, add it, times the group's scale, to the row's fp32 sums, and write the outputs; warps
+// 12-15 issue MMAs (two issuers per half: a thread cannot issue a tcgen05.mma more often than every 50 clocks, threads
+// of different warps can) and stream the prepared activation of their own groups; warp 15 also owns the tensor-memory
+// allocation.
 //
-// Tensor-memory columns: kRing slots per half of 64 columns each for the A operand (one 128-code group);
-// GF4 adds NB accumulator columns to every slot (one accumulator per group: the group's fp16 scale is
-// applied in fp32 after tcgen05.ld), E2M1 has one accumulator of NB columns per issuer for the whole row
-// (its scales are folded into the fp16 weights).  The second half's sums reach the first half's threads at
-// the end of a tile through NB more columns (GF4) or through shared memory (E2M1, which needs all 512
-// columns at 32 and 64 rows).
+// Tensor-memory columns: kRing slots per half of 64 columns each for the A operand (one 128-code group) and kAccBufs
+// accumulators of NB columns per issuer.
 //
-// Where the time goes (clock64 counters per role, 11008 x 4096 GF4 and 8192 x 8192 E2M1, 16 batch rows): the
-// decode threads are busy decoding for about 60 % of a tile (GF4: the shared-memory pipe, 80 wavefronts per
-// 128 codes of 32 rows, is 3/4 full while they do; E2M1: about 230 instructions per 128 codes and thread),
-// the rest goes to the table build, the accumulator read-back and the end of the tile; neither the weight
-// ring nor the activation rings are waited for (deepening the weight ring to four stages changed nothing).
-// The MMA issuers are single lanes running dependent scalar code beside two decode warps: while they still
-// divided their ring positions out of counters they were the bottleneck of E2M1 (busy 89 % of the time, half
-// of it bookkeeping; with the MMAs left out the kernel ran 17 % faster); with the positions carried along
-// E2M1 runs at that decode bound, and GF4's issuers idle 3/4 of the time.
-constexpr int kTaThreads = 12 * 32;
+// The decode threads bound the kernel, so everything else is kept off them.  (When they also folded the accumulators,
+// exchanged the halves' sums and wrote the outputs, they were decoding for 60 % of a tile.)  GF4 up to 16 rows: the
+// shared-memory pipe takes 5 wavefronts per 8 codes of 32 rows with every byte looked up in the pair table; one word of
+// four goes through byte permutes on the ALU instead (tc.cuh, Codebook), which has room.  From 17 rows on there is no
+// shared memory for tables beside the activation rings and all words go through the permutes.
+//
+// A row's sum is formed in four parts of K (one, for short rows and for 33 rows and more), each in group order, added in
+// part order.  A single call with few tiles lets the CTAs of a cluster take the parts; the partial sums meet in
+// distributed shared memory and are added in the same order, so the result does not depend on the split.
+constexpr int kTaThreads = 16 * 32;
+constexpr int kPartMinSteps = 8;                                    // 256-code steps from which a row is summed in parts
 template <int FMT, int NB>
 struct Cols {
-    static constexpr bool kGf4 = FMT == JQ_FMT_GF4;
-    // MMA issuers per half.  One thread issues a tcgen05.mma every 50 clocks at best, whatever N up to 32 and
-    // whatever the accumulator; threads of different warps issue in parallel.  At N = 64 two issuers already
-    // saturate the pipe's arithmetic.
-    static constexpr int kIssuers = (!kGf4 && NB == 64) ? 1 : 2;
-    static constexpr int kRing = 3;                                // groups a half may have in flight
-    static constexpr int kSlot = 64 + (kGf4 ? NB : 0);
-    static constexpr int kAcc = 2 * kRing * kSlot;                 // E2M1: accumulator of (half h, issuer i) at kAcc + (h * kIssuers + i) * NB
-    // GF4 hands the second half's sums to the first half's threads through NB more columns; E2M1 needs all 512
-    // columns at 32 and 64 rows and uses shared memory for that (GF4 has none to spare)
-    static constexpr int kExchange = kAcc;
-    static_assert(kGf4 ? kExchange + NB <= 512 : kAcc + 2 * kIssuers * NB <= 512, "tensor memory");
+    static constexpr bool kTable = FMT == JQ_FMT_GF4 && NB == 16;   // pair tables in shared memory
+    static constexpr int kRing = NB == 16 ? 3 : 2;                  // groups a half may have in flight
+    static constexpr int kAccBufs = NB == 64 ? 1 : 2;               // accumulators of an issuer
+    static constexpr int kAcc = 2 * kRing * 64;                     // accumulator b of issuer i at kAcc + (i * kAccBufs + b) * NB
+    static constexpr int kParts = NB == 64 ? 1 : 4;
+    static_assert(kAcc + 4 * kAccBufs * NB <= 512, "tensor memory");
+    // one barrier per accumulator says that a group's MMAs are done, to the fold threads and to the decode threads that
+    // wait for the group's slot; before a slot's next group is written, no later group can have used the accumulator
+    static_assert(2 * kAccBufs >= kRing, "the barrier would be a phase ahead");
 };
 
-template <int FMT>
+template <bool TABLE>
 struct Smem {
-    static constexpr bool kGf4 = FMT == JQ_FMT_GF4;
     static constexpr int kTab = 0;
-    static constexpr int kWRing = kGf4 ? kTabBytes : 0;
+    static constexpr int kWRing = TABLE ? kTabBytes : 0;
     static constexpr int kSW = 2;       // stages of a decode warp's weight ring (four did not change anything: the ring is not what the decode threads wait for)
     static constexpr int kXRing = kWRing + kDecodeWarps * kSW * kWStage;
-    static constexpr int kXBytes = kGf4 ? 32 * 1024 : 96 * 1024;    // E2M1 has no tables: three stages of 64 batch rows per issuer
-    static constexpr int kExch = kXRing + kXBytes + 512;            // + what the MMA reads past the last chunk (rows >= B)
-    static constexpr int kExchBytes = kGf4 ? 0 : 2 * kTileM * 64 * 4;   // E2M1: second half's sums, [tile parity][batch row][tile row] fp32
-    static constexpr int kBars = kExch + kExchBytes;
-    static constexpr int kNumBars = kDecodeWarps * 4 + 4 * 3 + 2 * 4 * kXMaxStages + 4;   // weights, A full, MMAs done, x full/free per issuer, quarter sync
+    static constexpr int kXBytes = TABLE ? 32 * 1024 : 152 * 1024;  // without tables: two stages of 64 batch rows per issuer
+    static constexpr int kBars = kXRing + kXBytes + 512;            // + what the MMA reads past the last chunk (rows >= B)
+    static constexpr int kNumBars = kDecodeWarps * kSW + 6 + 2 * 8 + 4 * kXMaxStages + 4;   // weights, A full, accumulator full/free, x full per issuer, quarter sync
     static constexpr int kBytes = kBars + kNumBars * 8 + 1024;      // + slack for the 1 KB alignment of the base (TMA swizzle)
+    static constexpr int kExch = TABLE ? kTab : kXRing;             // K split: partial sums, once nothing else uses the region
+    static_assert(kBytes <= 227 * 1024, "shared memory");
 };
 
 // geometry of an issuer's activation ring for a batch of B rows: a stage is one group (128 codes), 256 B bytes
 struct XGeom {
-    int chunk, ring, nstages, lag;
+    int chunk, ring, nstages;
     __host__ __device__ XGeom(int B, int ring_bytes) {
         chunk = 256 * B;
         ring = ring_bytes;
         nstages = ring_bytes / chunk < kXMaxStages ? ring_bytes / chunk : kXMaxStages;
-        lag = nstages > 2 ? 2 : 1;      // a stage is refilled this many groups after the MMAs that read it were issued
     }
 };
+
+// first step of part i of a row of nsteps 256-code steps
+__host__ __device__ inline int part_step(int nsteps, int parts, int i) { return nsteps * i / parts; }
 
 template <int FMT, int NB>
 __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem *probs, const CUtensorMap *maps,
                                                                 const __grid_constant__ TaProblem single,
                                                                 const __grid_constant__ CUtensorMap single_map, int nprob,
                                                                 const int *tile_start, const int *cta_first,
-                                                                int B, int y_dtype, PeerInfo peers, int *status) {
+                                                                int B, int y_dtype, PeerInfo peers, int split, int *status) {
     using C = Cols<FMT, NB>;
-    using S = Smem<FMT>;
+    using S = Smem<C::kTable>;
     constexpr bool kGf4 = FMT == JQ_FMT_GF4;
     constexpr int kRing = C::kRing;
     constexpr int kSW = S::kSW;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint32_t s_tmem;
     __shared__ int s_err;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (uniform for the compiler)
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bars = sbase + S::kBars;
+    constexpr int kB0 = kDecodeWarps * kSW;
     auto wbar = [&](int w, int s) { return bars + 8u * (w * kSW + s); };
-    auto abar = [&](int h, int s) { return bars + 8u * (kDecodeWarps * kSW + h * 3 + s); };
-    auto dbar = [&](int h, int s) { return bars + 8u * (kDecodeWarps * kSW + 6 + h * 3 + s); };
-    auto xbar = [&](int iss, int s) { return bars + 8u * (kDecodeWarps * kSW + 12 + iss * kXMaxStages + s); };           // issuer's stage filled
-    auto xebar = [&](int iss, int s) { return bars + 8u * (kDecodeWarps * kSW + 12 + (4 + iss) * kXMaxStages + s); };    // its MMAs have read it
-    auto qbar = [&](int q) { return bars + 8u * (kDecodeWarps * kSW + 12 + 8 * kXMaxStages + q); };
+    auto abar = [&](int h, int s) { return bars + 8u * (kB0 + h * 3 + s); };                  // operand slot written
+    auto dbar = [&](int iss, int b) { return bars + 8u * (kB0 + 6 + iss * 2 + b); };          // accumulator complete: a group's MMAs are done
+    auto ebar = [&](int iss, int b) { return bars + 8u * (kB0 + 14 + iss * 2 + b); };         // accumulator folded
+    auto xbar = [&](int iss, int s) { return bars + 8u * (kB0 + 22 + iss * kXMaxStages + s); };   // issuer's stage filled
+    auto qbar = [&](int q) { return bars + 8u * (kB0 + 22 + 4 * kXMaxStages + q); };
     volatile int *err = &s_err;
-    const XGeom xg(B, S::kXBytes / (2 * C::kIssuers));
+    const XGeom xg(B, S::kXBytes / 4);
 
     if (tid == 0) {
         s_err = 0;
         for (int w = 0; w < kDecodeWarps; ++w)
             for (int s = 0; s < kSW; ++s) mbar_init(wbar(w, s), 1);     // one arrive.expect_tx per fill
         for (int h = 0; h < 2; ++h)
-            for (int s = 0; s < 3; ++s) {
-                mbar_init(abar(h, s), 128);                             // the 128 decode threads of the half
-                mbar_init(dbar(h, s), 1);                               // one tcgen05.commit
-            }
+            for (int s = 0; s < 3; ++s) mbar_init(abar(h, s), 128);     // the 128 decode threads of the half
         for (int i = 0; i < 4; ++i)
-            for (int s = 0; s < kXMaxStages; ++s) { mbar_init(xbar(i, s), 1); mbar_init(xebar(i, s), 1); }
+            for (int b = 0; b < 2; ++b) { mbar_init(dbar(i, b), 1); mbar_init(ebar(i, b), 128); }
+        for (int i = 0; i < 4; ++i)
+            for (int s = 0; s < kXMaxStages; ++s) mbar_init(xbar(i, s), 1);
         for (int q = 0; q < 4; ++q) mbar_init(qbar(q), 64);             // the two warps that share a quarter of the rows
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 11) {
+    if (warp == 15) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
     // this CTA's tiles
-    int tile_lo, tile_hi;
-    if (nprob == 0) {   // one problem, passed by value: an even split of its tiles
-        const int nt = (single.N + kTileM - 1) / kTileM;
-        tile_lo = (int)((long long)nt * blockIdx.x / gridDim.x);
-        tile_hi = (int)((long long)nt * (blockIdx.x + 1) / gridDim.x);
+    int tile_lo, tile_hi, rank = 0;
+    if (nprob == 0) {   // one problem, passed by value: an even split of its tiles; with a K split one tile per cluster
+        const int nt = (single.N + kTileM - 1) / kTileM, n_cl = gridDim.x / split, cl = blockIdx.x / split;
+        rank = blockIdx.x - cl * split;
+        tile_lo = (int)((long long)nt * cl / n_cl);
+        tile_hi = (int)((long long)nt * (cl + 1) / n_cl);
     } else {
         tile_lo = cta_first[blockIdx.x];
         tile_hi = cta_first[blockIdx.x + 1];
     }
+    // parts of a row's sum, and the steps [lo, hi) of a row that this CTA works on
+    auto parts_of = [&](int nsteps) { return nsteps >= kPartMinSteps ? C::kParts : 1; };
+    auto step_lo = [&](int nsteps) { return split > 1 ? part_step(nsteps, C::kParts, C::kParts / split * rank) : 0; };
+    auto step_hi = [&](int nsteps) { return split > 1 ? part_step(nsteps, C::kParts, C::kParts / split * (rank + 1)) : nsteps; };
     // Problems change rarely along a CTA's tile sequence: every walker keeps what it needs of its current
     // problem in registers and goes back to global memory only for a tile beyond that problem's last one.
     auto problem_at = [&](int &pi, int &t_end, int tile, TaProblem &p) {
@@ -261,28 +262,31 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
 
     if (warp < kDecodeWarps) {
         // =============================== decode threads ===============================
+        if constexpr (NB > 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");     // 256 x 112 + 128 x 184 + 128 x 96 of 65536 registers
         const int q = warp & 3, h = warp >> 2;
         const int r = q * 32 + lane;                       // row of the tile = tensor-memory lane
         const uint32_t lane_t = tmem + ((uint32_t)(q * 32) << 16);
-        const uint32_t tcol = sbase + S::kTab + q * (256 * 128) + lane * 4;   // GF4: entry e of this row at tcol + 128 e
+        const uint32_t tcol = sbase + S::kTab + q * (256 * 128) + lane * 4;   // pair table: entry e of this row at tcol + 128 e
         const uint32_t wring = sbase + S::kWRing + warp * (kSW * kWStage);     // + stage * kWStage; 1 KB aligned
         // 16-byte piece c of this lane's row sits at piece c ^ (lane & 7) of the row (128-byte swizzle)
         const uint32_t lrow = lane * 128, lkey = (lane & 7) << 4;
 
         // ---- producer side of the weight ring: the (tile, step) whose box is requested next
-        int i_tile = tile_lo, i_pi = 0, i_tend = -1, i_j = 0, i_n = 0, i_x = 0, i_y = 0, i_tile0 = 0, i_steps = 0, i_stage = 0;
+        int i_tile = tile_lo, i_pi = 0, i_tend = -1, i_j = 0, i_n = 0, i_x = 0, i_x0 = 0, i_y = 0, i_tile0 = 0, i_steps = 0, i_stage = 0;
         const void *i_map = nullptr;
         auto i_open = [&]() {
             while (i_tile < tile_hi) {
                 if (i_tile >= i_tend) {
                     TaProblem p;
                     problem_at(i_pi, i_tend, i_tile, p);
-                    i_steps = ((p.K >> 8) - h + 1) >> 1;
+                    const int ns = p.K >> 8, lo = step_lo(ns);
+                    i_steps = (step_hi(ns) - lo - h + 1) >> 1;
+                    i_x0 = (lo + h) * 128;
                     i_tile0 = p.tile0;
                     i_map = nprob ? &maps[i_pi] : &single_map;
                 }
                 i_n = i_steps;
-                i_x = h * 128;
+                i_x = i_x0;
                 i_y = (i_tile - i_tile0) * kTileM + q * 32;     // rows past N read as zeros
                 i_j = 0;
                 if (i_n > 0) return;
@@ -324,25 +328,16 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
         };
 
         // ---- consumer state
-        uint32_t wcount = 0;        // weight stages consumed so far
-        uint32_t t_h = 0;           // groups this half has handed to the MMA so far
-        uint32_t t_fold = 0;        // groups whose slot has been released (GF4: folded into acc) so far
-        uint32_t qcount = 0;        // quarter syncs so far
-        unsigned short raw_q[3] = {0, 0, 0};   // GF4: fp16 scales (bits) of the groups in flight, by slot
-        float acc[NB];
-        bool have_prev = false;     // a finished tile waiting for its last group and its outputs
-        float prev_bias = 0.f;
-        int prev_row = 0, prev_N = 0, prev_ldy = 0;
-        void *prev_y = nullptr;
-        float prev_xs[(NB + 31) / 32];   // lane l holds 2^e of batch rows l, l + 32 (loaded at the start of the tile)
-
-        uint32_t fin_count = 0;     // finished tiles so far (parity picks the E2M1 exchange buffer)
-        int pend_slot = -1;         // slot of the group whose tensor-memory stores are issued but not yet handed over
+        int w_stage = 0, slot = 0, pend_slot = -1;   // pend_slot: its tensor-memory stores are issued but not yet handed over
+        uint32_t w_par = 0;
+        uint32_t t_next = 0;                         // groups this half has decoded so far
+        uint32_t qcount = 0;                         // quarter syncs so far
+        Codebook book;
         auto hand_over = [&]() {
             if (pend_slot >= 0) {
                 tmem_wait_st();
                 tc_fence_before();
-                mbar_arrive(abar(h, (uint32_t)pend_slot));
+                mbar_arrive(abar(h, pend_slot));
                 pend_slot = -1;
             }
         };
@@ -352,128 +347,21 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             ++qcount;
             return ok;
         };
-        // release the oldest slot in flight: wait for its group's MMAs; GF4 folds the group's accumulator (scaled)
-        auto fold_one = [&]() -> bool {
-            const uint32_t s = t_fold % kRing;
-            const bool ok = __all_sync(0xffffffffu, mbar_wait(dbar(h, s), (t_fold / kRing) & 1, err));
-            if (!ok) return false;
-            if constexpr (kGf4) {
-                tc_fence_after();
-                unsigned short raw = raw_q[0];
-#pragma unroll
-                for (int i = 1; i < kRing; ++i) raw = (s == (uint32_t)i) ? raw_q[i] : raw;
-                const float sc = __half2float(__ushort_as_half(raw));
-#pragma unroll
-                for (int c = 0; c < NB; c += 16) {
-                    uint32_t d[16];
-                    tmem_ld16(lane_t + (h * kRing + s) * C::kSlot + 64 + c, d);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) acc[c + i] = fmaf(__uint_as_float(d[i]), sc, acc[c + i]);
-                }
-            }
-            ++t_fold;
-            return true;
-        };
-        // outputs of the finished tile: the second half hands its sums over through tensor memory
-        auto finish_prev = [&]() -> bool {
-            if (!have_prev) return true;
-            while (t_fold < t_h)
-                if (!fold_one()) return false;
-            if constexpr (!kGf4) {          // the accumulators of the half's issuers hold the whole row between them
-                tc_fence_after();
-#pragma unroll
-                for (int c = 0; c < NB; c += 16) {
-#pragma unroll
-                    for (int is = 0; is < C::kIssuers; ++is) {
-                        uint32_t d[16];
-                        tmem_ld16(lane_t + C::kAcc + (h * C::kIssuers + is) * NB + c, d);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) acc[c + i] = is ? acc[c + i] + __uint_as_float(d[i]) : __uint_as_float(d[i]);
-                    }
-                }
-            }
-            // E2M1: two buffers by tile parity, so that the second half (which does not meet the first again until
-            // the end of the next tile) never overwrites sums that are still to be read; column b of the buffer is
-            // 128 consecutive floats, one per tile row: conflict-free for a warp
-            float *exch = reinterpret_cast<float *>(smem_raw + (sbase - smem_u32(smem_raw)) + S::kExch) +
-                          (fin_count & 1) * (kTileM * 64) + r;
-            ++fin_count;
-            if (h == 1) {
-                if constexpr (kGf4) {
-#pragma unroll
-                    for (int c = 0; c < NB; c += 16) {
-                        uint32_t v[16];
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(acc[c + i]);
-                        tmem_st16(lane_t + C::kExchange + c, v);
-                    }
-                    tmem_wait_st();
-                } else {
-#pragma unroll
-                    for (int b = 0; b < NB; ++b)
-                        exch[b * kTileM] = acc[b];
-                }
-            }
-            tc_fence_before();
-            if (!quarter_sync()) return false;
-            if (h == 0) {
-                tc_fence_after();
-                const bool live = prev_row < prev_N;
-#pragma unroll
-                for (int c = 0; c < NB; c += 16) {
-                    uint32_t v[16];
-                    if constexpr (kGf4) {
-                        tmem_ld16(lane_t + C::kExchange + c, v);
-                        tmem_wait_ld();
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(exch[(c + i) * kTileM]);
-                    }
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int b = c + i;
-                        const float xs_b = __shfl_sync(0xffffffffu, prev_xs[b >> 5], b & 31);
-                        acc[b] = fmaf(acc[b] + __uint_as_float(v[i]), xs_b, prev_bias);
-                    }
-                }
-                if (live) {
-                    for (int cpy = 0; cpy < peers.n; ++cpy) {
-                        char *yb = reinterpret_cast<char *>(prev_y) + jq::peer_offset(peers.delta, cpy);
-#pragma unroll
-                        for (int b = 0; b < NB; ++b)
-                            if (b < B) jq::store_out(yb, (size_t)b * prev_ldy + prev_row, acc[b], y_dtype);
-                    }
-                }
-                tc_fence_before();
-            }
-            have_prev = false;
-            return true;
-        };
-
-        // scales of one 256-code step of a row: E2M1 eight fp16 (16 bytes), GF4 one fp16 per 128 * 2^k codes (.x, .y)
-        auto load_scales = [&](const unsigned short *srow, int sg, int gshift) -> uint4 {
-            if constexpr (kGf4)
-                return make_uint4(__ldg(srow + ((2 * sg) >> gshift)), __ldg(srow + ((2 * sg + 1) >> gshift)), 0, 0);
-            else
-                return __ldg(reinterpret_cast<const uint4 *>(srow + sg * 8));
-        };
 
         int c_pi = 0, c_tend = -1;
         TaProblem p = single;
         fetch_codebook(tile_lo);
-        pdl_wait();                 // from here on the prepared activation and its row factors are read
         bool ok = true;
         for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
             if (tile >= c_tend) problem_at(c_pi, c_tend, tile, p);
-            const int row_raw = (tile - p.tile0) * kTileM + r;
-            const int row = min(row_raw, p.N - 1);
-            const int nsteps = ((p.K >> 8) - h + 1) >> 1;
-            const unsigned short *srow = reinterpret_cast<const unsigned short *>(p.scales) + (size_t)row * p.lds;
-            const int gshift = kGf4 ? 31 - __clz(p.g >> 7) : 0;   // GF4: log2 of the 128-code groups per scale
-            uint4 sc_nxt = load_scales(srow, h, gshift);          // in flight during the table build / the previous tile's outputs
-            if constexpr (kGf4) {
+            const int s_lo = step_lo(p.K >> 8), s_hi = step_hi(p.K >> 8);
+            // E2M1: eight fp16 scales (16 bytes) per 256-code step of the row, a step ahead
+            const int row = min((tile - p.tile0) * kTileM + r, p.N - 1);
+            const uint4 *srow = reinterpret_cast<const uint4 *>(p.scales + (size_t)row * p.lds);
+            uint4 sc_nxt = make_uint4(0, 0, 0, 0);
+            if (!kGf4 && s_lo + h < s_hi) sc_nxt = __ldg(srow + s_lo + h);
+            if constexpr (kGf4) book.set(cb0, cb1);
+            if constexpr (C::kTable) {
                 // ---- the pair table of this row (this thread fills the entries whose second code is in its half)
                 if (!(ok = quarter_sync())) break;      // both warps are done with the previous tile's lookups
                 const uint32_t c[8] = {cb0.x, cb0.y, cb0.z, cb0.w, cb1.x, cb1.y, cb1.z, cb1.w};
@@ -489,51 +377,50 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                                                        ((lo & 1) ? 0x32u : 0x10u) | (((i & 1) ? 0x76u : 0x54u) << 8));
                         asm volatile("st.shared.u32 [%0], %1;" ::"r"(tb + (i * 16 + lo) * 128), "r"(e) : "memory");
                     }
-                fetch_codebook(tile + 1);
             }
-            // the previous tile's last groups have had the table build to finish; its sync also publishes the table
-            const bool had_prev = have_prev;
-            if (!(ok = finish_prev())) break;
-            if (kGf4 && !had_prev) { if (!(ok = quarter_sync())) break; }
-#pragma unroll
-            for (int b = 0; b < NB; ++b) acc[b] = 0.f;
-
-            float xs_next[(NB + 31) / 32];
-#pragma unroll
-            for (int i = 0; i < (NB + 31) / 32; ++i) xs_next[i] = (lane + 32 * i < B) ? p.xscale[lane + 32 * i] : 0.f;
-            for (int j = 0; j < nsteps && ok; ++j) {
-                const int stage = wcount % kSW;
-                ok = __all_sync(0xffffffffu, mbar_wait(wbar(warp, stage), (wcount / kSW) & 1, err));
+            fetch_codebook(tile + 1);
+            if constexpr (C::kTable) { if (!(ok = quarter_sync())) break; }
+            for (int sg = s_lo + h; sg < s_hi; sg += 2) {
+                ok = __all_sync(0xffffffffu, mbar_wait(wbar(warp, w_stage), w_par, err));
                 if (!ok) break;
-                ++wcount;
-                const uint32_t slot = wring + stage * kWStage + lrow;
-                // the step's scales were loaded a step ahead; the next step's start their way now
+                const uint32_t src = wring + w_stage * kWStage + lrow;
+                if (++w_stage == kSW) { w_stage = 0; w_par ^= 1; }
                 const uint4 sc_cur = sc_nxt;
-                if (j + 1 < nsteps) sc_nxt = load_scales(srow, 2 * (j + 1) + h, gshift);
+                if (!kGf4 && sg + 2 < s_hi) sc_nxt = __ldg(srow + sg + 2);
 #pragma unroll
                 for (int gi = 0; gi < 2; ++gi) {
-                    // this group's scales: GF4 one fp16 (per 128 * 2^k codes), E2M1 four (one per 32 codes)
-                    const unsigned short scale_raw = (unsigned short)(gi ? sc_cur.y : sc_cur.x);
                     const uint2 sc4 = gi ? make_uint2(sc_cur.z, sc_cur.w) : make_uint2(sc_cur.x, sc_cur.y);
-                    // slot t % kRing is free once group t - kRing has been released
-                    if (t_h - t_fold == (uint32_t)kRing && !(ok = fold_one())) break;
-                    const uint32_t t = t_h, s = t % kRing;
-                    const uint32_t a_t = lane_t + (h * kRing + s) * C::kSlot;
+                    // the slot is free once the MMAs of the group that used it last are done
+                    if (t_next >= (uint32_t)kRing) {
+                        const uint32_t t = t_next - kRing, n = t >> 1;     // group t was its issuer's n-th
+                        ok = __all_sync(0xffffffffu, mbar_wait(dbar(h + 2 * (t & 1), n % C::kAccBufs), (n / C::kAccBufs) & 1, err));
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
+                    ++t_next;
+                    const uint32_t a_t = lane_t + (h * kRing + slot) * 64;
                     uint4 w4[4];
 #pragma unroll
-                    for (int part = 0; part < 4; ++part) w4[part] = lds128(slot + (((gi * 4 + part) << 4) ^ lkey));
+                    for (int part = 0; part < 4; ++part) w4[part] = lds128(src + (((gi * 4 + part) << 4) ^ lkey));
                     // 32 codes (four words) -> 16 fp16 pairs
                     auto decode16 = [&](int part, uint32_t (&v)[16]) {
 #pragma unroll
                         for (int wi = 0; wi < 4; ++wi) {
                             const uint32_t w = wi == 0 ? w4[part].x : (wi == 1 ? w4[part].y : (wi == 2 ? w4[part].z : w4[part].w));
                             if constexpr (kGf4) {
+                                if (C::kTable && wi < 3) {
 #pragma unroll
-                                for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = lds32(dp4a_u(w, 0x80u << (8 * bj), tcol));
+                                    for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = lds32(dp4a_u(w, 0x80u << (8 * bj), tcol));
+                                } else {
+                                    uint32_t hh[4];
+                                    book.look_up8(w, hh);
+#pragma unroll
+                                    for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = hh[bj];
+                                }
                             } else {
                                 // E2M1: the group scale folded into the fp16 weight (one rounding per weight)
-                                const uint32_t sh = part == 0 ? (sc4.x & 0xffffu) : (part == 1 ? (sc4.x >> 16) : (part == 2 ? (sc4.y & 0xffffu) : (sc4.y >> 16)));
-                                const uint32_t s2 = sh * 0x00010001u;
+                                const uint32_t pr = part < 2 ? sc4.x : sc4.y;
+                                const uint32_t s2 = prmt(pr, pr, (part & 1) ? 0x3232 : 0x1010);
                                 uint32_t hh[4];
                                 asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %4;\n"
                                     "  cvt.rn.f16x2.e2m1x2 %0, b0; cvt.rn.f16x2.e2m1x2 %1, b1;\n"
@@ -558,10 +445,8 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                     decode16(3, vb);
                     tmem_st16(a_t + 32, va);
                     tmem_st16(a_t + 48, vb);
-                    pend_slot = (int)s;
-                    ++t_h;
-#pragma unroll
-                    for (int i = 0; i < kRing; ++i) raw_q[i] = (s == (uint32_t)i) ? scale_raw : raw_q[i];
+                    pend_slot = slot;
+                    if (++slot == kRing) slot = 0;
                 }
                 if (!ok) break;
                 __syncwarp();                           // every lane has read its row of the stage
@@ -569,57 +454,177 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                 issue();                                // refill the stage just read
             }
             hand_over();
-            have_prev = true;
-            prev_bias = (p.bias && row_raw < p.N) ? p.bias[row_raw] : 0.f;
-            prev_row = row_raw; prev_N = p.N; prev_ldy = p.ldy; prev_y = p.y;
-#pragma unroll
-            for (int i = 0; i < (NB + 31) / 32; ++i) prev_xs[i] = xs_next[i];
         }
-        if (ok) ok = finish_prev();
+        if (split > 1) { __syncwarp(); cluster_sync(); cluster_sync(); }
+    } else if (warp < 12) {
+        // =============================== fold threads ===============================
+        if constexpr (NB > 16) asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+        const int r = tid & 127;
+        const uint32_t lane_t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::kAcc;
+        uint32_t counts = 0;                        // steps of each half so far, modulo 4 (two bits each)
+        int c_pi = 0, c_tend = -1;
+        TaProblem p = single;
+        pdl_wait();                                 // the row factors of the prepared activation are read below
+        bool ok = true;
+        for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
+            if (tile >= c_tend) problem_at(c_pi, c_tend, tile, p);
+            const int row_raw = (tile - p.tile0) * kTileM + r, row = min(row_raw, p.N - 1);
+            const int nsteps = p.K >> 8, parts = parts_of(nsteps), s_lo = step_lo(nsteps), s_hi = step_hi(nsteps);
+            const unsigned short *srow = reinterpret_cast<const unsigned short *>(p.scales) + (size_t)row * p.lds;
+            const int gshift = kGf4 ? 31 - __clz(p.g >> 7) : 0;   // GF4: log2 of the 128-code groups per scale
+            float xs[(NB + 31) / 32];
+#pragma unroll
+            for (int i = 0; i < (NB + 31) / 32; ++i) xs[i] = (lane + 32 * i < B) ? p.xscale[lane + 32 * i] : 0.f;
+            const float bias = (p.bias && row_raw < p.N) ? p.bias[row_raw] : 0.f;
+            float acc[NB], total[C::kParts > 1 ? NB : 1];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) acc[b] = 0.f;
+            const uint32_t exch = sbase + S::kExch + r * 4;
+            int part = split > 1 ? C::kParts / split * rank : 0, part_end = part_step(nsteps, parts, part + 1);
+            bool first = true;
+            unsigned short raw0 = 0, raw1 = 0;
+            auto load_scales = [&](int sg) {
+                if (kGf4) { raw0 = __ldg(srow + ((2 * sg) >> gshift)); raw1 = __ldg(srow + ((2 * sg + 1) >> gshift)); }
+            };
+            load_scales(s_lo);
+            for (int sg = s_lo; sg < s_hi && ok; ++sg) {
+                const int h = (sg - s_lo) & 1;
+                const uint32_t cnt = (counts >> (2 * h)) & 3;
+                const uint32_t buf = C::kAccBufs == 2 ? cnt & 1 : 0, par = C::kAccBufs == 2 ? cnt >> 1 : cnt & 1;
+                const float sc[2] = {__half2float(__ushort_as_half(raw0)), __half2float(__ushort_as_half(raw1))};
+                if (sg + 1 < s_hi) load_scales(sg + 1);
+#pragma unroll
+                for (int gi = 0; gi < 2; ++gi) {
+                    const int iss = h + 2 * gi;
+                    ok = __all_sync(0xffffffffu, mbar_wait(dbar(iss, buf), par, err));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t d_t = lane_t + (iss * C::kAccBufs + buf) * NB;
+                    if constexpr (NB == 16) {
+                        uint32_t d[16];
+                        tmem_ld16(d_t, d);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 16; i += 2) fma2(acc[i], acc[i + 1], d[i], d[i + 1], kGf4 ? sc[gi] : 1.f);
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < NB; c += 32) {
+                            uint32_t d[32];
+                            tmem_ld32(d_t + c, d);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 32; i += 2) fma2(acc[c + i], acc[c + i + 1], d[i], d[i + 1], kGf4 ? sc[gi] : 1.f);
+                        }
+                    }
+                    tc_fence_before();
+                    mbar_arrive(ebar(iss, buf));
+                }
+                if (!ok) break;
+                counts = (counts & ~(3u << (2 * h))) | (((cnt + 1) & 3) << (2 * h));
+                if (C::kParts > 1 && sg + 1 == part_end) {      // a part of the row's sum is complete
+                    if (split > 1) {        // at most two per CTA: the first waits in `total`, the second stays in `acc`
+                        if (first) {
+#pragma unroll
+                            for (int b = 0; b < NB; ++b) { total[b] = acc[b]; acc[b] = 0.f; }
+                        }
+                    } else {
+#pragma unroll
+                        for (int b = 0; b < NB; ++b) {
+                            total[b] = first ? acc[b] : total[b] + acc[b];
+                            acc[b] = 0.f;
+                        }
+                    }
+                    first = false;
+                    ++part;
+                    part_end = part_step(nsteps, parts, part + 1);
+                }
+            }
+            if constexpr (C::kParts > 1) {
+                if (split > 1) {
+                    // every group of this CTA has been folded: nothing reads the tables or the activation rings any more.
+                    // Each CTA leaves its parts in its shared memory; rank k writes columns k, k + split, ...
+                    const int per = C::kParts / split;
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(exch + b * 512), "f"(total[b]) : "memory");
+                        if (per == 2) asm volatile("st.shared.f32 [%0], %1;" ::"r"(exch + (NB + b) * 512), "f"(acc[b]) : "memory");
+                    }
+                    cluster_sync();
+                    for (int b = rank; b < B; b += split) {
+                        float v = ld_cluster_f32(exch + b * 512, 0);
+                        for (int i = 1; i < C::kParts; ++i) v += ld_cluster_f32(exch + ((i % per) * NB + b) * 512, i / per);
+                        if (ok && row_raw < p.N) jq::store_out(p.y, (size_t)b * p.ldy + row_raw, fmaf(v, p.xscale[b], bias), y_dtype);
+                    }
+                    cluster_sync();
+                    break;
+                }
+            }
+            if (!ok) break;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const float xs_b = __shfl_sync(0xffffffffu, xs[b >> 5], b & 31);
+                const float v = C::kParts > 1 ? total[C::kParts > 1 ? b : 0] : acc[b];
+                acc[b] = fmaf(v, xs_b, bias);
+            }
+            if (row_raw < p.N) {
+                for (int cpy = 0; cpy < peers.n; ++cpy) {
+                    char *yb = reinterpret_cast<char *>(p.y) + jq::peer_offset(peers.delta, cpy);
+#pragma unroll
+                    for (int b = 0; b < NB; ++b)
+                        if (b < B) jq::store_out(yb, (size_t)b * p.ldy + row_raw, acc[b], y_dtype);
+                }
+            }
+        }
     } else {
         // =============================== MMA issuers ===============================
-        // Warps 8, 9: half 0, 1; warps 10, 11: a second issuer per half (kIssuers == 2).  With two issuers a half's
-        // groups alternate between them (the first group of every 256-code step to one, the second to the other).
+        // Warps 12, 13: half 0, 1; warps 14, 15: the second issuer per half.  A half's groups alternate between its
+        // issuers (the first group of every 256-code step to one, the second to the other).
         // Every issuer owns a ring of activation stages (one 128-code group each) that it fills itself, so the
-        // only thing it ever waits for besides the decode threads is its own earlier work.
-        const int h = (warp - 8) & 1, sub = (warp - 8) >> 1, iss = warp - 8;
-        if (lane == 0 && sub < C::kIssuers) {
+        // only things it ever waits for are the decode and fold threads and its own earlier work.
+        if constexpr (NB > 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+        const int h = (warp - 12) & 1, sub = (warp - 12) >> 1, iss = warp - 12;
+        // (the warps run converged, see mma_f16_ts)
+        {
+            const uint32_t elected = elect_one();
+            auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)); };
             constexpr uint32_t idesc = idesc_f16(kTileM, NB);
-            constexpr int kPer = 2 / C::kIssuers;       // groups of a step this issuer takes
             const uint32_t lbo = (uint32_t)B * 16;
             const uint32_t ring = sbase + S::kXRing + iss * xg.ring;
             // two walks over the same sequence of groups: the loads run ahead of the MMAs
-            struct Walk { int tile, pi, t_end, nsg, sg, k; const unsigned char *xp; };
+            struct Walk { int tile, pi, t_end, lo, hi, sg; const unsigned char *xp; };
             auto open_tile = [&](Walk &w) {
                 while (w.tile < tile_hi) {
                     if (w.tile >= w.t_end) {
                         TaProblem p;
                         problem_at(w.pi, w.t_end, w.tile, p);
-                        w.nsg = p.K >> 8;
+                        w.lo = step_lo(p.K >> 8);
+                        w.hi = step_hi(p.K >> 8);
                         w.xp = reinterpret_cast<const unsigned char *>(p.xprep);
                     }
-                    w.sg = h; w.k = 0;
-                    if (w.sg < w.nsg) return;
+                    w.sg = w.lo + h;
+                    if (w.sg < w.hi) return;
                     ++w.tile;
                 }
             };
             auto advance = [&](Walk &w) {
-                if (++w.k == kPer) { w.k = 0; w.sg += 2; }
-                if (w.sg >= w.nsg) { ++w.tile; open_tile(w); }
+                w.sg += 2;
+                if (w.sg >= w.hi) { ++w.tile; open_tile(w); }
             };
             Walk ld = {tile_lo, 0, -1, 0, 0, 0, nullptr};
             open_tile(ld);
             Walk mm = ld;
-            // The issuing thread is a single lane running dependent scalar code on a scheduler it shares with two
-            // decode warps, so every instruction of this loop costs several clocks: ring positions and parities
-            // are carried along instead of being divided out of counters, and the operand descriptor is formed
-            // once per group.
+            // An issuer shares its scheduler with two decode warps, so every instruction of this loop costs several clocks:
+            // ring positions and parities are carried along instead of being divided out of counters, and the operand
+            // descriptor is formed once per group.
             uint32_t ld_s = 0;                          // stage the next load goes to
             auto load_next = [&]() {
                 if (ld.tile < tile_hi) {
-                    const int G = 2 * ld.sg + (C::kIssuers == 2 ? sub : ld.k);
-                    mbar_expect_tx(xbar(iss, ld_s), xg.chunk);
-                    bulk_g2s(ring + ld_s * xg.chunk, ld.xp + (size_t)G * xg.chunk, xg.chunk, xbar(iss, ld_s));
+                    const int G = 2 * ld.sg + sub;
+                    if (elected) {
+                        mbar_expect_tx(xbar(iss, ld_s), xg.chunk);
+                        bulk_g2s(ring + ld_s * xg.chunk, ld.xp + (size_t)G * xg.chunk, xg.chunk, xbar(iss, ld_s));
+                    }
+                    __syncwarp();
                     advance(ld);
                 }
                 ld_s = (ld_s + 1 == (uint32_t)xg.nstages) ? 0 : ld_s + 1;
@@ -628,34 +633,37 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             for (int i = 0; i < xg.nstages; ++i) load_next();
             bool ok = true;
             uint32_t cs = 0, cpar = 0;                  // stage and phase parity of the group being multiplied
-            uint32_t rs = 0, rpar = 0;                  // stage and phase parity of the group whose stage is refilled next
-            uint32_t slot = (uint32_t)sub % kRing, spar = 0;   // A slot of this issuer's next group (the half's group count t = kIssuers n + sub)
+            uint32_t slot = (uint32_t)sub % kRing, spar = 0;   // A slot of this issuer's next group (the half's group count t = 2 n + sub)
+            uint32_t db = 0, dpar = 1;                  // accumulator (the first round finds it free)
+            const bool tight = xg.nstages <= C::kAccBufs;
             const uint32_t desc_step = (2 * lbo) >> 4;  // descriptor address field per K = 16 slice
             for (uint32_t n = 0; mm.tile < tile_hi && ok; ++n) {
-                // the stage whose MMAs were issued xg.lag groups ago is free by now: refill it
-                if (n >= (uint32_t)xg.lag) {
-                    if (!(ok = mbar_wait(xebar(iss, rs), rpar, err))) break;
+                // a ring with no more stages than accumulators refills the previous group's stage once its MMAs are done
+                if (tight && n > 0) {
+                    if (!(ok = wait(dbar(iss, (n - 1) % C::kAccBufs), ((n - 1) / C::kAccBufs) & 1))) break;
                     load_next();
-                    if (++rs == (uint32_t)xg.nstages) { rs = 0; rpar ^= 1; }
                 }
-                if (!(ok = mbar_wait(xbar(iss, cs), cpar, err))) break;
-                if (!(ok = mbar_wait(abar(h, slot), spar, err))) break;
+                // the accumulator's last group has been folded, so its MMAs have read their activation stage: refill that
+                if (!(ok = wait(ebar(iss, db), dpar))) break;
+                if (!tight && n >= (uint32_t)C::kAccBufs) load_next();
+                if (!(ok = wait(xbar(iss, cs), cpar))) break;
+                if (!(ok = wait(abar(h, slot), spar))) break;
                 tc_fence_after();
-                const uint32_t a_t = tmem + (h * kRing + slot) * C::kSlot;
-                const uint32_t d_t = kGf4 ? a_t + 64 : tmem + C::kAcc + (h * C::kIssuers + sub) * NB;
+                const uint32_t a_t = tmem + (h * kRing + slot) * 64;
+                const uint32_t d_t = tmem + C::kAcc + (iss * C::kAccBufs + db) * NB;
                 const uint64_t desc0 = smem_desc(ring + cs * xg.chunk, lbo, 128);
-                const bool first = mm.sg == h && mm.k == 0;                // E2M1: this issuer's first group of the tile
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    mma_f16_ts(d_t, a_t + 8 * i, desc0 + (uint64_t)(i * desc_step), idesc, kGf4 ? (i > 0) : (i > 0 || !first));
-                mma_commit(dbar(h, slot));
-                mma_commit(xebar(iss, cs));
+                    mma_f16_ts(elected, d_t, a_t + 8 * i, desc0 + (uint64_t)(i * desc_step), idesc, i > 0);
+                mma_commit(elected, dbar(iss, db));
                 if (++cs == (uint32_t)xg.nstages) { cs = 0; cpar ^= 1; }
-                slot += C::kIssuers;
+                if (++db == (uint32_t)C::kAccBufs) { db = 0; dpar ^= 1; }
+                slot += 2;
                 if (slot >= (uint32_t)kRing) { slot -= kRing; spar ^= 1; }
                 advance(mm);
             }
         }
+        if (split > 1) { __syncwarp(); cluster_sync(); cluster_sync(); }
     }
 
     // ---- teardown
@@ -665,7 +673,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
     tc_fence_before();
     __syncthreads();
     if (tid == 0 && s_err) atomicExch(status, s_err);
-    if (warp == 11) {
+    if (warp == 15) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }
@@ -994,12 +1002,8 @@ static const int kTaMagic = 0x4a515441;
 static const double kTileCost = 1408, kProblemCost = 6144;
 static const int kTaHeader = 12;
 
-// MMA N: GF4 keeps one accumulator per group and slot (up to 16 columns); E2M1 one per half (up to 64)
-static int ta_cols(int fmt, int B) {
-    if (B <= 16) return 16;
-    if (fmt == JQ_FMT_E2M1) return B <= 32 ? 32 : (B <= 64 ? 64 : 0);
-    return 0;
-}
+// MMA N
+static int ta_cols(int B) { return B <= 16 ? 16 : (B <= 32 ? 32 : (B <= 64 ? 64 : 0)); }
 
 static bool ta_use_lut(int B, int maxK);
 static size_t ta_align(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -1032,7 +1036,11 @@ static bool ta_shape_ok(int fmt, int N, int K, int g, int had) {
 
 // batch 1 runs on the CUDA cores when the prepared activation of one problem fits its shared-memory buffer
 // (K up to 12288); from two rows on the tensor-memory kernel is faster (decode7b: 1800 against 1090 tokens/s)
+#ifdef JQ_NO_LUT
+static bool ta_use_lut(int B, int maxK) { return false; }
+#else
 static bool ta_use_lut(int B, int maxK) { return B == 1 && (size_t)maxK * 2 <= (size_t)LutSmem::kXBytes; }
+#endif
 
 extern "C" size_t jq_ta_workspace_bytes(const jq_problem *ph, int n, int B) {
     if (!ph || n <= 0 || B < 1 || B > 64) return 0;
@@ -1076,7 +1084,7 @@ extern "C" int jq_ta_plan(int fmt, const jq_problem *ph, int n, int B, void *wor
                           void *plan_host, size_t plan_bytes) {
     if (!ph || !plan_host || !workspace_dev) return JQ_ERR_NULL_PTR;
     if (n <= 0 || B < 1) return JQ_ERR_BAD_SHAPE;
-    if ((fmt != JQ_FMT_GF4 && fmt != JQ_FMT_E2M1) || !ta_cols(fmt, B)) return JQ_ERR_UNSUPPORTED;
+    if ((fmt != JQ_FMT_GF4 && fmt != JQ_FMT_E2M1) || !ta_cols(B)) return JQ_ERR_UNSUPPORTED;
     if (plan_bytes < jq_ta_plan_bytes(n) || workspace_bytes < jq_ta_workspace_bytes(ph, n, B)) return JQ_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(workspace_dev) & 127u) return JQ_ERR_BAD_ALIGN;
     const int grid = jq_sm_count();
@@ -1118,21 +1126,26 @@ extern "C" int jq_ta_plan(int fmt, const jq_problem *ph, int n, int B, void *wor
             acc += c;
         }
     while (cta < grid) cta_first[++cta] = tile_start[n];
-    h[0] = kTaMagic; h[1] = n; h[2] = grid; h[3] = ta_cols(fmt, B); h[4] = (int)moff; h[5] = B; h[6] = fmt; h[7] = (int)poff;
+    h[0] = kTaMagic; h[1] = n; h[2] = grid; h[3] = ta_cols(B); h[4] = (int)moff; h[5] = B; h[6] = fmt; h[7] = (int)poff;
     h[8] = maxK; h[9] = h[10] = h[11] = 0;
     return JQ_OK;
 }
 
-// launch configuration of a main kernel: allowed to start while the preparation kernel in front of it still runs
-static void ta_pdl_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, int grid, int threads, int smem, cudaStream_t st) {
+// launch configuration of a main kernel: allowed to start while the preparation kernel in front of it still runs;
+// cluster: CTAs that share a tile
+static void ta_pdl_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2], int grid, int threads, int smem, int cluster,
+                          cudaStream_t st) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
 }
 
 template <int FMT, int NB>
@@ -1146,14 +1159,18 @@ static int ta_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, co
     int s = jq_launch_status();
     if (s) return s;
     auto kern = gemm_ta_kernel<FMT, NB>;
-    constexpr int smem = Smem<FMT>::kBytes;
-    static_assert(smem <= 227 * 1024, "shared memory");
+    using C = Cols<FMT, NB>;
+    constexpr int smem = Smem<C::kTable>::kBytes;
+    // A single matrix with few tiles: 4 or 2 CTAs take parts of every row (N = 4096 is 32 tiles for 148 SMs)
+    int split = 1;
+    if (!nprob && C::kParts == 4 && (single.K >> 8) >= kPartMinSteps)
+        split = grid * 4 <= jq_sm_count() ? 4 : (grid * 2 <= jq_sm_count() ? 2 : 1);
     JQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    ta_pdl_config(cfg, attr, grid, kTaThreads, smem, st);
+    cudaLaunchAttribute attr[2];
+    ta_pdl_config(cfg, attr, grid * split, kTaThreads, smem, split, st);
     JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, probs_dev, maps_dev, single, single_map, nprob, tile_start, cta_first, B, y_dtype,
-                                   peers, status));
+                                   peers, split, status));
     return jq_launch_status();
 }
 
@@ -1171,8 +1188,8 @@ static int lut2_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, 
     static_assert(smem <= 227 * 1024, "shared memory");
     JQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    ta_pdl_config(cfg, attr, grid, kLutThreads, smem, st);
+    cudaLaunchAttribute attr[2];
+    ta_pdl_config(cfg, attr, grid, kLutThreads, smem, 1, st);
     JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, probs_dev, maps_dev, single, single_map, nprob, tile_start, cta_first, y_dtype,
                                    peers, status));
     return jq_launch_status();
@@ -1188,6 +1205,8 @@ static int ta_dispatch(int fmt, int nb, int maxK, const TaProblem *probs_dev, co
             return lut2_launch<1>(probs_dev, maps_dev, single, single_map, nprob, tile_start, cta_first, grid, x_dtype, y_dtype, peers, status, st);
         }
         if (nb == 16) return ta_launch<JQ_FMT_GF4, 16>(JQ_TA_ARGS);
+        if (nb == 32) return ta_launch<JQ_FMT_GF4, 32>(JQ_TA_ARGS);
+        if (nb == 64) return ta_launch<JQ_FMT_GF4, 64>(JQ_TA_ARGS);
         return JQ_ERR_UNSUPPORTED;
     }
     if (nb == 16) return ta_launch<JQ_FMT_E2M1, 16>(JQ_TA_ARGS);
@@ -1223,7 +1242,7 @@ extern "C" int jq_gemm_ta(int fmt, const void *qweight, const void *scales, cons
                           int y_dtype, void *workspace, size_t workspace_bytes, jq_stream_t stream) {
     if (!workspace) return JQ_ERR_NULL_PTR;
     if (B < 1) return JQ_ERR_BAD_SHAPE;
-    if ((fmt != JQ_FMT_GF4 && fmt != JQ_FMT_E2M1) || !ta_cols(fmt, B)) return JQ_ERR_UNSUPPORTED;
+    if ((fmt != JQ_FMT_GF4 && fmt != JQ_FMT_E2M1) || !ta_cols(B)) return JQ_ERR_UNSUPPORTED;
     if (x_dtype < 0 || x_dtype > 2 || y_dtype < 0 || y_dtype > 2) return JQ_ERR_BAD_DTYPE;
     if (reinterpret_cast<uintptr_t>(workspace) & 127u) return JQ_ERR_BAD_ALIGN;
     jq_problem p{};
@@ -1244,7 +1263,7 @@ extern "C" int jq_gemm_ta(int fmt, const void *qweight, const void *scales, cons
     const int tile_m = (fmt == JQ_FMT_GF4 && ta_use_lut(B, K)) ? kLutTileM : kTileM;
     const int tiles = (N + tile_m - 1) / tile_m;
     if (grid > tiles) grid = tiles;
-    return ta_dispatch(fmt, ta_cols(fmt, B), K, nullptr, nullptr, t, tm, 0, nullptr, nullptr, grid, B, x_dtype, y_dtype, peers,
+    return ta_dispatch(fmt, ta_cols(B), K, nullptr, nullptr, t, tm, 0, nullptr, nullptr, grid, B, x_dtype, y_dtype, peers,
                        reinterpret_cast<int *>(workspace), reinterpret_cast<cudaStream_t>(stream));
 }
 

@@ -70,14 +70,24 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 __host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
     return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-// D[128 x N] (+)= A[128 x 16] (tensor memory) . B[N x 16]^T (shared memory)
-__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                 "  tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+// One lane of a converged warp.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t p;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(p));
+    return p;
 }
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+// D[128 x N] (+)= A[128 x 16] (tensor memory) . B[N x 16]^T (shared memory), issued by the elected lane.  The whole warp
+// runs the issuing loop and only the instruction itself is predicated: its operands have to be in uniform registers, and
+// in a loop that one lane runs alone every one of them is moved there for every MMA (150 clocks per MMA).
+__device__ __forceinline__ void mma_f16_ts(uint32_t elected, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                           uint32_t accumulate) {
+    asm volatile("{ .reg .pred p, q; setp.ne.b32 p, %4, 0; setp.ne.b32 q, %5, 0;\n"
+                 "  @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
+                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint32_t elected, uint32_t bar) {
+    asm volatile("{ .reg .pred q; setp.ne.b32 q, %1, 0;\n"
+                 "  @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0]; }" ::"r"(bar), "r"(elected) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }

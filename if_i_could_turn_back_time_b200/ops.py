@@ -68,16 +68,16 @@ _OUT = {-1: None, _lib.JQ_F32: torch.float32, _lib.JQ_F16: torch.float16, _lib.J
 
 def ta_max_batch(fmt_id: int) -> int:
     """Rows one pass of the pair-table / tensor-memory kernels takes."""
-    return 16 if fmt_id == _lib.JQ_FMT_GF4 else 64
+    return 64
 
 
 def ta_eligible(fmt_id: int, K: int, g: int, batch: int) -> bool:
     """Problems the TMA-fed kernels take.  GF4 (group size 128 * 2^k): every
     batch -- one row (while the prepared activation fits in shared memory, K
     up to 12288) on the CUDA-core pair-table loop, the rest on the
-    tensor-memory kernel, 16 rows per pass.  E2M1 g32: batches from 9 rows on
-    the tensor-memory kernel, 64 rows per pass (up to 8 rows the mma.sync row
-    loops are faster)."""
+    tensor-memory kernel.  E2M1 g32: batches from 9 rows on the tensor-memory
+    kernel (up to 8 rows the mma.sync row loops are faster).  64 rows per
+    pass."""
     if K % 256 or K < 512:
         return False
     if fmt_id == _lib.JQ_FMT_GF4:

@@ -209,14 +209,16 @@ int jq_gemv_grouped_peers(const jq_problem *problems_dev, const void *plan_host,
  * jq_gemv_e2m1, i.e. the F.linear(x, W_bar, bias) of
  * Quantization_Experiments/layers.py:38, for K % 256 == 0, K >= 512,
  * qweight / codebook / E2M1 scales 16-byte aligned, and
- *   fmt GF4,  group sizes of 128 * 2^k, 1 <= B <= 16;
+ *   fmt GF4,  group sizes of 128 * 2^k,
  *   fmt E2M1, group size 32,            1 <= B <= 64.
  * The packed rows arrive by 2-D tiled TMA (32-row x 128-byte boxes, 128-byte
  * swizzle), a decode thread owns one weight row of a 128-row tile.
  *   GF4: a byte of packed codes indexes a 256-entry table of fp16 pairs that is
  *        built per tile in shared memory, one bank column per weight row, so
- *        two codes cost one conflict-free lookup.  Every weight and every scale
- *        stays exact; only the fp32 summation order differs from jq_gemv_gf4.
+ *        two codes cost one conflict-free lookup (part of the codes, and all
+ *        of them for B > 16, are looked up in registers instead).  Every weight
+ *        and every scale stays exact; only the fp32 summation order differs
+ *        from jq_gemv_gf4.
  *        B == 1 (K <= 12288): the decode threads also multiply (fma.rn.f32.f16,
  *        fp32 accumulation), reading the prepared activation by broadcast
  *        shared-memory loads.  Otherwise the fp16 values go to tensor memory
@@ -228,8 +230,10 @@ int jq_gemv_grouped_peers(const jq_problem *problems_dev, const void *plan_host,
  *        jq_gemv_e2m1 does not have (its weights are exact): the results of the
  *        two entry points differ by up to about 2^-11 relative per weight, well
  *        inside the 1e-3 gate of the operator, and the dequantised matrix
- *        (jq_dequant_e2m1) remains the exact one.  The whole row accumulates in
- *        tensor memory (fp32).
+ *        (jq_dequant_e2m1) remains the exact one.
+ * Both: rows of 8 or more 256-code steps are summed in four parts of K (B <= 32)
+ * that are added in order; a single matrix with few tiles spreads the parts over
+ * a cluster of CTAs, with the same result.
  * A launch is preceded by a small kernel that rotates, normalises and rounds
  * the activation to fp16 once per problem (not once per CTA).  The workspace
  * (128-byte aligned, jq_ta_workspace_bytes) holds that prepared activation and

@@ -1,0 +1,41 @@
+"""The tensor-memory kernel's row sums: parts of K, folded group by group, spread over a cluster or not."""
+import pytest
+import torch
+
+import if_i_could_turn_back_time_b200 as jq
+from if_i_could_turn_back_time_b200 import ops
+from test_gpu_parity import DEV, _check_gemv, _weights
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N,K", [(40, 512), (129, 2048), (320, 2304), (130, 11008), (9600, 2048)])
+@pytest.mark.parametrize("fmt,g,B", [("gf4", 128, 2), ("gf4", 256, 16), ("gf4", 128, 17), ("gf4", 128, 33), ("gf4", 128, 64),
+                                     ("e2m1", 32, 9), ("e2m1", 32, 23), ("e2m1", 32, 48)])
+def test_single_calls_groups_and_row_shards_agree(fmt, g, B, N, K):
+    """Fewer than 8 steps (one part) and more (four parts of unequal length), clusters of 4, 2 and no cluster: against the
+    oracle, and the same bits from a grouped launch (never split) and from a row shard (split differently)."""
+    spec = jq.QuantSpec(fmt, g, 0)
+    pw = jq.pack_weight(_weights(N, K, N + K).to(DEV), spec)
+    # (a copy: rows of a shard whose scales start off a 16-byte boundary would be left to the row loops)
+
+    def half(i):
+        part, copy = pw.rows(i * (N // 2), (i + 1) * (N // 2)), lambda t: None if t is None else t.clone()
+        return jq.PackedWeight(spec, part.N, K, copy(part.qweight), copy(part.scales), copy(part.codebook))
+
+    gen = torch.Generator("cpu").manual_seed(B)
+    x = torch.randn(B, K, generator=gen).bfloat16()
+    if N < 1000:
+        _check_gemv(pw.to("cpu"), x, torch.randn(N, generator=gen))
+    grp = ops.GroupedGemv([pw, half(0)], B, torch.float32)
+    for gx in grp.xs:
+        gx.copy_(x)
+    grp.run()
+    assert grp.status() == 0 and grp._ta
+    assert torch.equal(grp.ys[1], grp.ys[0][:, :N // 2])
+    if not ops.many_rows(spec.fmt_id, K, g, B):
+        y = ops.linear(x.to(DEV).float(), pw)
+        assert torch.equal(y, grp.ys[0])
+        assert torch.equal(ops.linear(x.to(DEV).float(), half(1)), y[:, N // 2:2 * (N // 2)])
+    else:
+        assert (ops.linear(x.to(DEV).float(), pw) - grp.ys[0]).abs().max() <= 3e-6 * grp.ys[0].abs().max()
