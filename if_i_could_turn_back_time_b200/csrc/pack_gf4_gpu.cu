@@ -1,255 +1,408 @@
 // Device-side GF4 packer: per-row 16-class Jenks natural breaks on the GPU,
 // bit-identical to the host packer (pack_host.cpp) and to the CPU oracle.
 //
-// One CTA per row at a time (persistent CTAs stride over the rows):
-//   1. group scales (fp16_rn of the group absmax) and u = w / scale into shared memory;
-//   2. bitonic sort of u in shared memory (padded with +inf to a power of two);
-//   3. run-length compression to (distinct value, multiplicity);
-//   4. float64 prefix sums, sequential in index order (the summation order is
-//      part of the format contract: codebooks must come out bit-identical);
-//   5. the dynamic programme over 16 classes in its divide-and-conquer form
-//      (the left-most optimal split is monotone in the prefix length): the
-//      recursion is walked level by level, one warp per node, lanes striding
-//      over the node's candidate range, then a warp-wide (value, index) minimum
-//      with the smaller index winning ties -- the same candidates and the same
-//      tie rule as the host's depth-first walk;
-//   6. back-track, class means -> fp16 codebook, codes by comparing each u with
-//      the classes' upper bounds, nibbles packed 8 per thread.
+// Two kernels per chunk of rows:
+//   sort_rows_kernel, one small CTA per row, several per SM:
+//     1. group scales (fp16_rn of the group absmax) and u = w / scale into shared memory;
+//     2. bitonic sort of u (padded with +inf to a power of two);
+//     3. run-length compression to distinct values and their start indices (= the prefix sums of the multiplicities);
+//     4. float64 prefix sums, sequential in index order (the summation order is part of the format contract: codebooks
+//        must come out bit-identical).  A chain of K dependent additions by one thread: the other CTAs of the SM fill
+//        the time.
+//   jenks_rows_kernel, one CTA per SM:
+//     5. the dynamic programme over 16 classes in its divide-and-conquer form (the left-most optimal split is monotone
+//        in the prefix length), with the host's candidates and tie rule.  The recursion [lo, hi] -> mid,
+//        [lo, mid - 1], [mid + 1, hi] is a fixed tree, walked level by level: a node's range of candidates lies between
+//        the results next to its interval.  Groups of lanes take the nodes; ranges that are long for their group
+//        are cut in pieces that all warps share;
+//     6. back-track, class means -> fp16 codebook, codes by comparing each u with the classes' upper bounds.
 // The objective is the k-class form of the one the reference evaluates for two
 // classes (Python_Jenks_Test/Jenks_Tests/cuda_helpers.py:151-184).
+//
+// What bounds it: float64 arithmetic, 64 lanes per clock and SM, on about 15 x (log2(K) + 1) x K candidate splits of a
+// row.  A candidate's cost has a division (some 20 float64 operations); it is estimated with a table of reciprocals
+// first (6 operations), and only a thread's candidates within the estimate's error bound of its smallest are computed
+// exactly, normally one.  The ranges of a level add up to K, but one node's can be most of it (weights with outliers): left
+// to the node's own lanes, the longest range set the pace.  4096 x 4096: 92.7 ms with queues of nodes in global memory, one
+// warp per node; 26 ms with a static tree of warps and lanes; see jq_pack_gf4 for the present figure.
 #include "common.cuh"
 #include <cfloat>
 
 namespace jqg {
 
-constexpr int kThreads = 1024;
-constexpr int kWarps = kThreads / 32;
 constexpr int kClasses = 16;
+constexpr int kSortThreads = 256;
+constexpr int kRowsPerSm = 8;             // rows of a chunk per SM
 
-struct Node { int lo, hi, olo, ohi; };
+__host__ __device__ inline size_t up256(size_t v) { return (v + 255) / 256 * 256; }
 
-struct RowWs {            // per-CTA scratch in global memory, sized for mcap = padded K
-    double *uv;           // [mcap]   distinct values
-    int *cnt;             // [mcap]   multiplicities
-    double *P1, *P2, *C;  // [mcap+1] prefix sums
-    double *prev, *cur;   // [mcap+1]
-    int *arg;             // [17][mcap+1]
-    Node *nodes[2];       // [mcap + 2] each: the non-empty intervals of one recursion level
+// a chunk row's slice of the workspace, written by the first kernel
+struct RowData {
+    double2 *P;          // [K + 1] prefix sums of n v and n v^2 over the distinct values
+    int *C;              // [K + 1] prefix sums of n
+    float *uv;           // [K]     distinct values
+    int *m;              // how many
 };
-
-__host__ __device__ inline size_t ws_bytes_per_cta(int mcap) {
-    const size_t m1 = (size_t)mcap + 1;
-    const size_t raw = sizeof(double) * mcap + sizeof(int) * (size_t)mcap + 5 * sizeof(double) * m1 +
-                       sizeof(int) * 17 * m1 + 2 * sizeof(Node) * ((size_t)mcap + 2);
-    return (raw + 255) / 256 * 256;   // every CTA's slice starts 256-byte aligned (it begins with doubles)
+__host__ __device__ inline size_t row_bytes(int K) {
+    return up256(sizeof(double2) * ((size_t)K + 1)) + up256(sizeof(int) * ((size_t)K + 1)) + up256(sizeof(float) * (size_t)K + 8);
+}
+__device__ inline RowData row_data(unsigned char *base, int K) {
+    RowData r;
+    r.P = reinterpret_cast<double2 *>(base); base += up256(sizeof(double2) * ((size_t)K + 1));
+    r.C = reinterpret_cast<int *>(base); base += up256(sizeof(int) * ((size_t)K + 1));
+    r.m = reinterpret_cast<int *>(base);
+    r.uv = reinterpret_cast<float *>(base) + 2;
+    return r;
 }
 
-__device__ inline RowWs carve_ws(unsigned char *base, int mcap) {
-    RowWs w;
-    const size_t m1 = (size_t)mcap + 1;
-    unsigned char *p = base;
-    w.uv = reinterpret_cast<double *>(p); p += sizeof(double) * mcap;
-    w.P1 = reinterpret_cast<double *>(p); p += sizeof(double) * m1;
-    w.P2 = reinterpret_cast<double *>(p); p += sizeof(double) * m1;
-    w.C = reinterpret_cast<double *>(p); p += sizeof(double) * m1;
-    w.prev = reinterpret_cast<double *>(p); p += sizeof(double) * m1;
-    w.cur = reinterpret_cast<double *>(p); p += sizeof(double) * m1;
-    w.nodes[0] = reinterpret_cast<Node *>(p); p += sizeof(Node) * ((size_t)mcap + 2);
-    w.nodes[1] = reinterpret_cast<Node *>(p); p += sizeof(Node) * ((size_t)mcap + 2);
-    w.cnt = reinterpret_cast<int *>(p); p += sizeof(int) * (size_t)mcap;
-    w.arg = reinterpret_cast<int *>(p);
-    return w;
+// the second kernel's arrays: where they lie (shared memory as far as they fit, the CTA's slice of the workspace
+// otherwise), in the order of the traffic that a candidate causes
+enum { kP1 = 0, kP2, kPrev, kCur, kRecip, kArg, kCount, kArrays };
+struct Layout {
+    size_t off[kArrays];
+    unsigned shared;          // bit a: array a lies in shared memory
+    size_t shared_bytes, cta_bytes;
+};
+__host__ inline Layout make_layout(int K, size_t shared_limit) {
+    const size_t m1 = (size_t)K + 1, d = sizeof(double) * ((m1 + 15) / 16 * 16);     // (doubles are stored permuted in blocks of 16)
+    const size_t bytes[kArrays] = {d, d, d, d, d, sizeof(unsigned short) * m1, sizeof(int) * m1};
+    Layout L{};
+    L.cta_bytes = up256((kClasses + 1) * sizeof(unsigned short) * m1);    // the arguments of all classes, for the back-track
+    for (int a = 0; a < kArrays; ++a) {
+        const size_t b = (bytes[a] + 15) / 16 * 16;
+        if (L.shared_bytes + b <= shared_limit) { L.shared |= 1u << a; L.off[a] = L.shared_bytes; L.shared_bytes += b; }
+        else { L.off[a] = L.cta_bytes; L.cta_bytes += up256(b); }
+    }
+    return L;
 }
+constexpr size_t kSharedLimit = 200 * 1024;       // of the second kernel's CTAs on an SM together (besides their static arrays)
 
-__device__ __forceinline__ double seg_cost(const RowWs &w, int a, int b) {
-    const double d1 = __dsub_rn(w.P1[b], w.P1[a]);
-    const double d2 = __dsub_rn(w.P2[b], w.P2[a]);
-    const double c = __dsub_rn(w.C[b], w.C[a]);
-    const double sq = __dmul_rn(d1, d1);
-    const double q = __ddiv_rn(sq, c);
-    return __dsub_rn(d2, q);
-}
-
-__global__ void __launch_bounds__(kThreads, 1) pack_gf4_kernel(const float *__restrict__ W, int N, int K, int g,
-                                                                uint8_t *__restrict__ qw, __half *__restrict__ scales,
-                                                                __half *__restrict__ codebook, unsigned char *__restrict__ ws,
-                                                                int npad) {
+__global__ void __launch_bounds__(kSortThreads) sort_rows_kernel(const float *__restrict__ W, int row0, int N, int K, int g,
+                                                                 __half *__restrict__ scales, unsigned char *__restrict__ ws,
+                                                                 int npad) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float *sv = reinterpret_cast<float *>(smem_raw);   // npad floats: the row being sorted
-    __shared__ int s_m, s_ke, s_zero, s_breaks[kClasses + 1];
-    __shared__ float s_upper[kClasses];                // largest value of each class
+    constexpr int kWarps = kSortThreads / 32;
     __shared__ int s_scan[kWarps + 1];
-    __shared__ int s_nn[2];                            // node counts of the current and next recursion level
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const RowWs w = carve_ws(ws + (size_t)blockIdx.x * ws_bytes_per_cta(npad), npad);
+    const int row = row0 + blockIdx.x;
+    const RowData rd = row_data(ws + (size_t)blockIdx.x * row_bytes(K), K);
+    const int G = g ? K / g : 0;
+    const float *wr = W + (size_t)row * K;
+    // ---- 1. scales and normalised values
+    if (g) {
+        for (int gi = warp; gi < G; gi += kWarps) {
+            float amax = 0.f;
+            for (int k = lane; k < g; k += 32) amax = fmaxf(amax, fabsf(wr[gi * g + k]));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+            __half hs = __float2half_rn(amax);
+            float s = __half2float(hs);
+            if (amax == 0.f || s == 0.f || isinf(s) || isnan(s)) { hs = __float2half_rn(1.0f); s = 1.0f; }
+            if (lane == 0) scales[(size_t)row * G + gi] = hs;
+            for (int k = lane; k < g; k += 32) sv[gi * g + k] = __fdiv_rn(wr[gi * g + k], s);
+        }
+    } else {
+        for (int k = tid; k < K; k += kSortThreads) sv[k] = wr[k];
+    }
+    for (int k = K + tid; k < npad; k += kSortThreads) sv[k] = __int_as_float(0x7f800000);  // +inf padding sorts last
+    __syncthreads();
+    // ---- 2. bitonic sort, ascending
+    for (int size = 2; size <= npad; size <<= 1) {
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int i = tid; i < npad / 2; i += kSortThreads) {
+                const int lo = 2 * i - (i & (stride - 1));
+                const int hi = lo + stride;
+                const bool up = (lo & size) == 0;
+                const float a = sv[lo], b = sv[hi];
+                if ((a > b) == up) { sv[lo] = b; sv[hi] = a; }
+            }
+            __syncthreads();
+        }
+    }
+    // ---- 3. run-length compression of sv[0..K): a warp's 32 consecutive elements at a time
+    int base = 0;                                          // distinct values so far
+    for (int c0 = 0; c0 < K; c0 += kSortThreads) {
+        const int i = c0 + tid;
+        const bool head = i < K && (i == 0 || sv[i] != sv[i - 1]);
+        const unsigned mask = __ballot_sync(0xffffffffu, head);
+        if (lane == 0) s_scan[warp] = __popc(mask);
+        __syncthreads();
+        int before = base, all = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) { before += w < warp ? s_scan[w] : 0; all += s_scan[w]; }
+        if (head) {
+            const int t = before + __popc(mask & ((1u << lane) - 1u));
+            rd.uv[t] = sv[i] + 0.0f;                       // -0.0 and +0.0 are one value: +0.0
+            rd.C[t] = i;
+        }
+        base += all;
+        __syncthreads();
+    }
+    const int m = base;
+    if (tid == 0) { rd.C[m] = K; *rd.m = m; }
+    __syncthreads();
+    // ---- 4. the terms, then their sequential float64 prefix sums
+    for (int t = tid; t < m; t += kSortThreads) {
+        const double v = (double)rd.uv[t], n = (double)(rd.C[t + 1] - rd.C[t]);
+        const double cv = __dmul_rn(n, v);
+        rd.P[t + 1] = make_double2(cv, __dmul_rn(cv, v));
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double p1 = 0.0, p2 = 0.0;
+        rd.P[0] = make_double2(0.0, 0.0);
+        constexpr int kAhead = 16;                         // the loads do not wait for the chain of additions
+        int t = 1;
+        if (m >= kAhead) {
+            double2 nxt[kAhead];
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) nxt[i] = rd.P[1 + i];
+            for (; t + 2 * kAhead - 1 <= m; t += kAhead) {
+                double2 now[kAhead];
+#pragma unroll
+                for (int i = 0; i < kAhead; ++i) { now[i] = nxt[i]; nxt[i] = rd.P[t + kAhead + i]; }
+#pragma unroll
+                for (int i = 0; i < kAhead; ++i) {
+                    p1 = __dadd_rn(p1, now[i].x); p2 = __dadd_rn(p2, now[i].y);
+                    rd.P[t + i] = make_double2(p1, p2);
+                }
+            }
+        }
+        for (; t <= m; ++t) {
+            const double2 v = rd.P[t];
+            p1 = __dadd_rn(p1, v.x); p2 = __dadd_rn(p2, v.y);
+            rd.P[t] = make_double2(p1, p2);
+        }
+    }
+}
+
+// Where element i of an array of doubles lies.  The lanes of a warp read at strides of one, two or four elements
+// (neighbouring nodes' candidates); permuted like this all three touch every bank pair equally often.
+__device__ __forceinline__ int at(int i) { return i ^ ((i >> 4) & 3); }
+
+struct Dp {
+    const double *P1, *P2;
+    const int *C;             // null: all values are distinct, C[t] = t
+    const double *recip;
+    double margin;            // twice the error bound of an estimate
+
+    __device__ __forceinline__ int count(int t) const { return C ? C[t] : t; }
+    __device__ __forceinline__ double exact(const double *prev, int t, double p1, double p2, int cm) const {
+        const double d1 = __dsub_rn(p1, P1[at(t)]), d2 = __dsub_rn(p2, P2[at(t)]);
+        const double q = __ddiv_rn(__dmul_rn(d1, d1), (double)(cm - count(t)));
+        const double seg = __dsub_rn(d2, q);
+        return prev ? __dadd_rn(prev[at(t)], seg) : seg;
+    }
+    // the same with the reciprocal of the count rounded first
+    __device__ __forceinline__ double estimate(const double *prev, int t, double p1, double p2, int cm) const {
+        const int i = at(t);
+        const double d1 = __dsub_rn(p1, P1[i]), d2 = __dsub_rn(p2, P2[i]);
+        const double q = __dmul_rn(__dmul_rn(d1, d1), recip[at(cm - count(t))]);
+        return __dadd_rn(prev[i], __dsub_rn(d2, q));
+    }
+    // first minimum of prev[t] + cost(t, mid) over t = t0 + first, t0 + first + step, ... <= t1; kAhead estimates at a
+    // time hide each other's latency
+    template <int kAhead>
+    __device__ __forceinline__ void scan(const double *prev, int t0, int t1, int first, int step, int mid, double &best, int &bt) const {
+        const double p1 = P1[at(mid)], p2 = P2[at(mid)];
+        const int cm = count(mid);
+        double low = __longlong_as_double(0x7ff0000000000000LL), limit = low;
+        int pos = -1;
+        bool several = false;             // more than one candidate may be the minimum
+        for (int tb = t0 + first; tb <= t1; tb += kAhead * step) {
+            double e[kAhead];
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) e[i] = estimate(prev, min(tb + i * step, t1), p1, p2, cm);
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                const int t = tb + i * step;
+                if (t > t1) break;
+                const double a = e[i];
+                if (a < low) {
+                    several = pos >= 0 && !(__dadd_rn(a, margin) < low);
+                    low = a; pos = t; limit = __dadd_rn(a, margin);
+                } else if (!(a > limit)) {    // (also when something is not a number)
+                    several = true;
+                }
+            }
+        }
+        best = DBL_MAX;
+        bt = 0x7fffffff;
+        if (several) {
+            for (int t = t0 + first; t <= t1; t += step)
+                if (!(estimate(prev, t, p1, p2, cm) > limit)) {
+                    const double c = exact(prev, t, p1, p2, cm);
+                    if (c < best) { best = c; bt = t; }
+                }
+        } else if (pos >= 0) {
+            const double c = exact(prev, pos, p1, p2, cm);
+            if (c < best) { best = c; bt = pos; }
+        }
+    }
+};
+
+__device__ __forceinline__ void take_first_min(double &best, int &bt, double ob, int ot) {
+    if (ob < best || (ob == best && ot < bt)) { best = ob; bt = ot; }
+}
+
+// kAllShared: every array lies in shared memory (the compiler then knows the address space)
+template <int kThreads, bool kAllShared>
+__global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__restrict__ W, int row0, int rows, int K, int g,
+                                                              uint8_t *__restrict__ qw, const __half *__restrict__ scales,
+                                                              __half *__restrict__ codebook, const unsigned char *__restrict__ row_ws,
+                                                              unsigned char *__restrict__ cta_ws, const __grid_constant__ Layout L) {
+    constexpr int kWarps = kThreads / 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_zero, s_breaks[kClasses + 1];
+    __shared__ float s_upper[kClasses];                // largest value of each class
+    // ranges that all warps share: a level's long nodes, the pieces of their ranges and the pieces' results.  A range is
+    // long from 16 candidates per lane of its group and 1/64 of the row, a piece at least 1/64 of the row, and a level's
+    // ranges add up to at most twice the row, so that neither array overflows (what did would be scanned by its group)
+    constexpr int kWide = kThreads / 4, kPieces = kThreads / 2;
+    struct Wide { int first, count, mid, t0; };
+    struct Piece { int t0, t1, mid; };
+    __shared__ Wide s_wide[kWide];
+    __shared__ Piece s_piece[kPieces];
+    __shared__ double s_best[kPieces];
+    __shared__ int s_bt[kPieces];
+    __shared__ int s_count[2][2];                      // long nodes, pieces; by parity of the level, as warps leave a level without any at different times
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned char *slice = cta_ws + (size_t)blockIdx.x * L.cta_bytes;
+    auto array = [&](int a) -> unsigned char * {
+        if (kAllShared) return smem_raw + L.off[a];
+        return ((L.shared >> a) & 1u) ? smem_raw + L.off[a] : slice + L.off[a];
+    };
+    double *P1 = reinterpret_cast<double *>(array(kP1)), *P2 = reinterpret_cast<double *>(array(kP2));
+    double *prev = reinterpret_cast<double *>(array(kPrev)), *cur = reinterpret_cast<double *>(array(kCur));
+    int *C = reinterpret_cast<int *>(array(kCount));
+    unsigned short *arg = reinterpret_cast<unsigned short *>(array(kArg));
+    double *recip = reinterpret_cast<double *>(array(kRecip));
+    unsigned short *arg_all = reinterpret_cast<unsigned short *>(slice);          // [class][K + 1]
     const int G = g ? K / g : 0;
     const int stride_b = jq_row_stride_codes(K) >> 1;
 
-    for (int row = blockIdx.x; row < N; row += gridDim.x) {
+    for (int i = tid; i <= K; i += kThreads) recip[at(i)] = i ? __ddiv_rn(1.0, (double)i) : 0.0;
+
+    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+        const int row = row0 + r;
         const float *wr = W + (size_t)row * K;
-        // ---- 1. scales and normalised values
-        if (g) {
-            for (int gi = warp; gi < G; gi += kWarps) {
-                float amax = 0.f;
-                for (int k = lane; k < g; k += 32) amax = fmaxf(amax, fabsf(wr[gi * g + k]));
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-                __half hs = __float2half_rn(amax);
-                float s = __half2float(hs);
-                if (amax == 0.f || s == 0.f || isinf(s) || isnan(s)) { hs = __float2half_rn(1.0f); s = 1.0f; }
-                if (lane == 0) scales[(size_t)row * G + gi] = hs;
-                for (int k = lane; k < g; k += 32) sv[gi * g + k] = __fdiv_rn(wr[gi * g + k], s);
-            }
-        } else {
-            for (int k = tid; k < K; k += kThreads) sv[k] = wr[k];
-        }
-        for (int k = K + tid; k < npad; k += kThreads) sv[k] = __int_as_float(0x7f800000);  // +inf padding sorts last
-        __syncthreads();
-        // ---- 2. bitonic sort, ascending
-        for (int size = 2; size <= npad; size <<= 1) {
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                for (int i = tid; i < npad / 2; i += kThreads) {
-                    const int lo = 2 * i - (i & (stride - 1));
-                    const int hi = lo + stride;
-                    const bool up = (lo & size) == 0;
-                    const float a = sv[lo], b = sv[hi];
-                    if ((a > b) == up) { sv[lo] = b; sv[hi] = a; }
-                }
-                __syncthreads();
-            }
-        }
-        // ---- 3. run-length compression of sv[0..K) into (uv, cnt)
-        {
-            // each thread owns a contiguous slice; head = first element of a run
-            const int per = (K + kThreads - 1) / kThreads;
-            const int b0 = min(tid * per, K), b1 = min(b0 + per, K);
-            int heads = 0;
-            for (int i = b0; i < b1; ++i) heads += (i == 0 || sv[i] != sv[i - 1]) ? 1 : 0;
-            // block exclusive scan of heads
-            int inc = heads;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { int t = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += t; }
-            if (lane == 31) s_scan[warp] = inc;
-            __syncthreads();
-            if (warp == 0) {
-                int v = lane < kWarps ? s_scan[lane] : 0, vi = v;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) { int t = __shfl_up_sync(0xffffffffu, vi, o); if (lane >= o) vi += t; }
-                if (lane < kWarps) s_scan[lane] = vi - v;
-                if (lane == kWarps - 1) s_scan[kWarps] = vi;
-            }
-            __syncthreads();
-            int pos = s_scan[warp] + inc - heads;   // index of this slice's first head
-            if (tid == 0) s_m = s_scan[kWarps];
-            // heads write their value; run lengths follow from the next head's position
-            for (int i = b0; i < b1; ++i) {
-                if (i == 0 || sv[i] != sv[i - 1]) {
-                    w.uv[pos] = (double)sv[i] + 0.0;   // -0.0 and +0.0 are one value: +0.0
-                    w.cnt[pos] = i;                     // start index for now
-                    ++pos;
-                }
-            }
-            __syncthreads();
-            const int m = s_m;
-            for (int t = tid; t < m; t += kThreads) {
-                const int start = w.cnt[t];
-                const int next = t + 1 < m ? w.cnt[t + 1] : K;
-                // cannot overwrite cnt[t] before the neighbour read it: stash in prev (as int bits are not needed yet)
-                w.prev[t] = (double)(next - start);
-            }
-            __syncthreads();
-            for (int t = tid; t < m; t += kThreads) w.cnt[t] = (int)w.prev[t];
-            __syncthreads();
-        }
-        const int m = s_m;
+        const RowData rd = row_data(const_cast<unsigned char *>(row_ws) + (size_t)r * row_bytes(K), K);
+        const int m = *rd.m;
         const int ke = m < kClasses ? m : kClasses;
-        // ---- 4. sequential float64 prefix sums
-        if (tid == 0) {
-            double p1 = 0.0, p2 = 0.0, c = 0.0;
-            w.P1[0] = 0.0; w.P2[0] = 0.0; w.C[0] = 0.0;
-#pragma unroll 4
-            for (int t = 0; t < m; ++t) {
-                const double v = w.uv[t], n = (double)w.cnt[t];
-                const double cv = __dmul_rn(n, v);
-                const double cvv = __dmul_rn(cv, v);
-                p1 = __dadd_rn(p1, cv); p2 = __dadd_rn(p2, cvv); c = __dadd_rn(c, n);
-                w.P1[t + 1] = p1; w.P2[t + 1] = p2; w.C[t + 1] = c;
-            }
-            s_ke = ke;
+        for (int i = tid; i <= m; i += kThreads) {
+            const double2 p = rd.P[i];
+            P1[at(i)] = p.x;
+            P2[at(i)] = p.y;
+            C[i] = rd.C[i];
         }
         __syncthreads();
-        // ---- 5. dynamic programme
-        for (int i = tid; i <= m; i += kThreads) { w.prev[i] = i >= 1 ? seg_cost(w, 0, i) : DBL_MAX; w.cur[i] = DBL_MAX; }
+        // ---- 5. dynamic programme.  An estimate differs from the exact cost by a few roundings of terms that are at
+        // most the row's sum of squares: 2^-49 of it, with room to spare 2^-46
+        const Dp dp{P1, P2, m == K ? nullptr : C, recip, P2[at(m)] * 0x1p-45};
+        for (int i = tid; i <= m; i += kThreads) prev[at(i)] = i >= 1 ? dp.exact(nullptr, 0, P1[at(i)], P2[at(i)], dp.count(i)) : DBL_MAX;
         __syncthreads();
-        double *prev = w.prev, *cur = w.cur;
+        int parity = 0;
+        if (tid < 4) s_count[tid >> 1][tid & 1] = 0;
+        __syncthreads();
         for (int j = 2; j <= ke; ++j) {
-            for (int i = tid; i <= m; i += kThreads) cur[i] = DBL_MAX;
-            if (tid == 0) {
-                w.nodes[0][0] = (j == ke) ? Node{m, m, j - 1, m - 1} : Node{j, m, j - 1, m - 1};
-                s_nn[0] = 1; s_nn[1] = 0;
-            }
-            __syncthreads();
-            int buf = 0;
-            while (true) {
-                const Node *in = w.nodes[buf];
-                Node *out = w.nodes[buf ^ 1];
-                const int nn = s_nn[buf];
-                for (int q = warp; q < nn; q += kWarps) {
-                    const Node nd = in[q];   // never empty: only non-empty intervals are queued
-                    const int mid = (nd.lo + nd.hi) >> 1;
-                    const int t0 = max(nd.olo, j - 1), t1 = min(mid - 1, nd.ohi);
+            unsigned short *out_arg = arg_all + (size_t)j * (K + 1);
+            auto write = [&](int mid, double best, int bt) {
+                cur[at(mid)] = best;
+                arg[mid] = (unsigned short)bt;
+                out_arg[mid] = (unsigned short)bt;
+            };
+            const int root = j == ke ? m : j, piece_len = max(128, m / 64);
+            for (int level = 0; (1 << level) <= m - root + 1; ++level, parity ^= 1) {
+                const int nodes = 1 << level, width = nodes <= kWarps ? 32 : max(kThreads >> level, 1);   // lanes per node
+                const int long_range = max(16 * width, m / 64);
+                const int in_group = lane & (width - 1), leader = lane - in_group;
+                for (int base = 0; base < nodes; base += kThreads / width) {
+                    const int node = base + tid / width;
+                    int l = root, h = m;
+                    for (int b = level - 1; b >= 0 && l <= h; --b) {
+                        const int mid = (l + h) >> 1;
+                        if ((node >> b) & 1) l = mid + 1; else h = mid - 1;
+                    }
+                    const bool live = node < nodes && l <= h;
+                    const int mid = (l + h) >> 1;
+                    int t0 = 0, t1 = -1;
+                    if (live) {
+                        t0 = max(l == root ? j - 1 : (int)arg[l - 1], j - 1);
+                        t1 = min(mid - 1, h == m ? m - 1 : (int)arg[h + 1]);
+                    }
+                    int shared_out = 0;
+                    if (t1 - t0 >= long_range && in_group == 0) {
+                        const int n = (t1 - t0) / piece_len + 1;
+                        const int slot = atomicAdd(&s_count[parity][0], 1), first = atomicAdd(&s_count[parity][1], n);
+                        shared_out = slot < kWide && first + n <= kPieces;
+                        if (slot < kWide) s_wide[slot] = Wide{first, shared_out ? n : 0, mid, t0};
+                        for (int i = 0; i < n && first + i < kPieces; ++i) {
+                            const int a = t0 + i * piece_len;
+                            s_piece[first + i] = shared_out ? Piece{a, min(t1, a + piece_len - 1), mid} : Piece{1, 0, mid};
+                        }
+                    }
+                    shared_out = __shfl_sync(0xffffffffu, shared_out, leader);
                     double best = DBL_MAX;
                     int bt = 0x7fffffff;
-                    for (int t = t0 + lane; t <= t1; t += 32) {
-                        const double c = __dadd_rn(prev[t], seg_cost(w, t, mid));
-                        if (c < best) { best = c; bt = t; }   // ascending t per lane: first minimum of the lane
+                    if (live && !shared_out) {
+                        if (width >= 16) dp.scan<4>(prev, t0, t1, in_group, width, mid, best, bt);
+                        else dp.scan<2>(prev, t0, t1, in_group, width, mid, best, bt);
                     }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                        const int ot = __shfl_xor_sync(0xffffffffu, bt, o);
-                        if (ob < best || (ob == best && ot < bt)) { best = ob; bt = ot; }
-                    }
-                    if (bt == 0x7fffffff) bt = t0;            // empty range or all DBL_MAX: the host keeps t0
-                    if (lane == 0) {
-                        cur[mid] = best;
-                        w.arg[(size_t)j * (m + 1) + mid] = bt;
-                        if (nd.lo <= mid - 1) out[atomicAdd(&s_nn[buf ^ 1], 1)] = Node{nd.lo, mid - 1, nd.olo, bt};
-                        if (mid + 1 <= nd.hi) out[atomicAdd(&s_nn[buf ^ 1], 1)] = Node{mid + 1, nd.hi, bt, nd.ohi};
-                    }
+                    __syncwarp();
+                    for (int o = width >> 1; o > 0; o >>= 1)
+                        take_first_min(best, bt, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, bt, o));
+                    // (an empty range or all DBL_MAX: the host keeps t0)
+                    if (live && !shared_out && in_group == 0) write(mid, best, bt == 0x7fffffff ? t0 : bt);
                 }
                 __syncthreads();
-                const int next = s_nn[buf ^ 1];
+                const int n_wide = min(s_count[parity][0], kWide), n_pieces = min(s_count[parity][1], kPieces);
+                if (n_wide == 0) continue;             // (the same for all threads)
+                for (int c = warp; c < n_pieces; c += kWarps) {
+                    const Piece pc = s_piece[c];
+                    double best;
+                    int bt;
+                    dp.scan<4>(prev, pc.t0, pc.t1, lane, 32, pc.mid, best, bt);
+                    __syncwarp();
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1)
+                        take_first_min(best, bt, __shfl_xor_sync(0xffffffffu, best, o), __shfl_xor_sync(0xffffffffu, bt, o));
+                    if (lane == 0) { s_best[c] = best; s_bt[c] = bt; }
+                }
                 __syncthreads();
-                if (tid == 0) s_nn[buf] = 0;   // becomes the "next" counter after the swap
-                buf ^= 1;
+                if (tid < n_wide) {
+                    const Wide wd = s_wide[tid];
+                    double best = DBL_MAX;
+                    int bt = 0x7fffffff;
+                    for (int i = 0; i < wd.count; ++i) take_first_min(best, bt, s_best[wd.first + i], s_bt[wd.first + i]);
+                    if (wd.count) write(wd.mid, best, bt == 0x7fffffff ? wd.t0 : bt);
+                }
+                if (tid < 2) s_count[parity][tid] = 0;
                 __syncthreads();
-                if (next == 0) break;
             }
             double *tswap = prev; prev = cur; cur = tswap;
-            __syncthreads();
         }
         // ---- 6. back-track, codebook, class upper bounds
         if (tid == 0) {
             s_breaks[ke] = m;
-            for (int j = ke; j >= 2; --j) s_breaks[j - 1] = w.arg[(size_t)j * (m + 1) + s_breaks[j]];
+            for (int j = ke; j >= 2; --j) s_breaks[j - 1] = arg_all[(size_t)j * (K + 1) + s_breaks[j]];
             s_breaks[0] = 0;
             // index of the distinct value 0.0 (m if the row has no exact zero)
             int lo = 0, hi = m;
             while (lo < hi) {
                 const int mid = (lo + hi) >> 1;
-                if (w.uv[mid] < 0.0) lo = mid + 1; else hi = mid;
+                if (rd.uv[mid] < 0.0f) lo = mid + 1; else hi = mid;
             }
-            s_zero = (lo < m && w.uv[lo] == 0.0) ? lo : m;
+            s_zero = (lo < m && rd.uv[lo] == 0.0f) ? lo : m;
         }
         __syncthreads();
         if (tid < kClasses) {
             const int c = tid < ke ? tid : ke - 1;
             const int a = s_breaks[c], b = s_breaks[c + 1];
-            double mean = __ddiv_rn(__dsub_rn(w.P1[b], w.P1[a]), __dsub_rn(w.C[b], w.C[a]));
+            double mean = __ddiv_rn(__dsub_rn(P1[at(b)], P1[at(a)]), (double)(C[b] - C[a]));
             if (s_zero >= a && s_zero < b) mean = 0.0;   // the class holding an exact zero is pinned to 0 (as the host packer)
             codebook[(size_t)row * kClasses + tid] = __double2half(mean);
-            s_upper[tid] = tid < ke ? (float)w.uv[b - 1] : __int_as_float(0x7f800000);
+            s_upper[tid] = tid < ke ? rd.uv[b - 1] : __int_as_float(0x7f800000);
         }
         __syncthreads();
         // codes: class = number of class upper bounds below the value
@@ -281,9 +434,14 @@ __global__ void __launch_bounds__(kThreads, 1) pack_gf4_kernel(const float *__re
 
 static int next_pow2(int v) { int p = 1; while (p < v) p <<= 1; return p; }
 
+// CTAs of the second kernel per SM: short rows leave room for more of them, with fewer threads each
+static int jenks_threads(int K) { return K <= 1024 ? 256 : (K <= 2048 ? 512 : 1024); }
+static int jenks_ctas(int K) { return jq_sm_count() * (1024 / jenks_threads(K)); }
+static jqg::Layout jenks_layout(int K) { return jqg::make_layout(K, jqg::kSharedLimit / (1024 / jenks_threads(K))); }
+
 extern "C" size_t jq_pack_gf4_workspace_bytes(int K) {
     if (K <= 0) return 0;
-    return jqg::ws_bytes_per_cta(next_pow2(K)) * (size_t)jq_sm_count();
+    return jqg::row_bytes(K) * (size_t)(jq_sm_count() * jqg::kRowsPerSm) + jenks_layout(K).cta_bytes * (size_t)jenks_ctas(K);
 }
 
 extern "C" int jq_pack_gf4(const float *W, int N, int K, int g, void *qweight, void *scales, void *codebook,
@@ -292,17 +450,31 @@ extern "C" int jq_pack_gf4(const float *W, int N, int K, int g, void *qweight, v
     if (N <= 0 || K <= 0 || g < 0 || (g && (g % 32 || K % g))) return JQ_ERR_BAD_SHAPE;
     if (g && !scales) return JQ_ERR_NULL_PTR;
     const int npad = next_pow2(K);
-    const size_t smem = (size_t)npad * sizeof(float);
-    if (smem > 200 * 1024) return JQ_ERR_UNSUPPORTED;   // rows longer than 51200 values
+    const size_t sort_smem = (size_t)npad * sizeof(float);
+    if (sort_smem > 200 * 1024) return JQ_ERR_UNSUPPORTED;   // rows longer than 32768 values
     if (workspace_bytes < jq_pack_gf4_workspace_bytes(K)) return JQ_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) || !jq_aligned16(qweight) || (reinterpret_cast<uintptr_t>(W) & 3u))
         return JQ_ERR_BAD_ALIGN;
-    auto kern = jqg::pack_gf4_kernel;
-    JQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int grid = jq_sm_count();
-    if (grid > N) grid = N;
-    kern<<<grid, jqg::kThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-        W, N, K, g, reinterpret_cast<uint8_t *>(qweight), reinterpret_cast<__half *>(scales),
-        reinterpret_cast<__half *>(codebook), reinterpret_cast<unsigned char *>(workspace), npad);
+    const jqg::Layout L = jenks_layout(K);
+    const bool all_shared = L.shared == (1u << jqg::kArrays) - 1u;
+    const int threads = jenks_threads(K);
+    auto kern = threads == 256 ? (all_shared ? jqg::jenks_rows_kernel<256, true> : jqg::jenks_rows_kernel<256, false>)
+              : threads == 512 ? (all_shared ? jqg::jenks_rows_kernel<512, true> : jqg::jenks_rows_kernel<512, false>)
+                               : (all_shared ? jqg::jenks_rows_kernel<1024, true> : jqg::jenks_rows_kernel<1024, false>);
+    JQ_CUDA_TRY(cudaFuncSetAttribute(jqg::sort_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem));
+    JQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.shared_bytes));
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    const int chunk = jq_sm_count() * jqg::kRowsPerSm;
+    unsigned char *row_ws = reinterpret_cast<unsigned char *>(workspace);
+    unsigned char *cta_ws = row_ws + jqg::row_bytes(K) * (size_t)chunk;
+    for (int row0 = 0; row0 < N; row0 += chunk) {
+        const int rows = N - row0 < chunk ? N - row0 : chunk;
+        jqg::sort_rows_kernel<<<rows, jqg::kSortThreads, sort_smem, st>>>(W, row0, N, K, g, reinterpret_cast<__half *>(scales),
+                                                                          row_ws, npad);
+        const int grid = rows < jenks_ctas(K) ? rows : jenks_ctas(K);
+        kern<<<grid, threads, L.shared_bytes, st>>>(W, row0, rows, K, g, reinterpret_cast<uint8_t *>(qweight),
+                                                    reinterpret_cast<const __half *>(scales), reinterpret_cast<__half *>(codebook),
+                                                    row_ws, cta_ws, L);
+    }
     return jq_launch_status();
 }
