@@ -7,39 +7,52 @@ namespace jq {
 __constant__ float kE2M1[16] = {0.f, 0.5f, 1.f, 1.5f, 2.f, 3.f, 4.f, 6.f,
                                 -0.f, -0.5f, -1.f, -1.5f, -2.f, -3.f, -4.f, -6.f};
 
-// One thread per 32-bit word (8 codes).  Rows of the packed matrix are
-// stride/8 words; the dense output has no padding.
+// A warp turns 1024 consecutive codes of one row into fp32, 128 per step: lane l holds codes 4 l .. 4 l + 3 of a step, so
+// that the warp's 16-byte stores cover 512 consecutive bytes (the kernel is bound by writing the dense matrix, eight
+// times the bytes it reads).  The 16 values of the row's table sit in the lanes and are looked up with shuffles.
+// Rows of the packed matrix are padded to 32 codes; the dense output has no padding, so rows that are not a multiple of
+// four floats, or start off a 16-byte boundary, are stored element by element.
+constexpr int kDequantSteps = 8;
 template <int FMT>
-__global__ void __launch_bounds__(256) dequant_kernel(const uint32_t *__restrict__ qw, const __half *__restrict__ scales,
+__global__ void __launch_bounds__(256) dequant_kernel(const uint8_t *__restrict__ qw, const __half *__restrict__ scales,
                                                        const __half *__restrict__ codebook, float *__restrict__ out,
                                                        int N, int K, int g) {
-    const int words_per_row = jq_row_stride_codes(K) >> 3;
-    const long long total = (long long)N * words_per_row;
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const int n = (int)(idx / words_per_row), wi = (int)(idx % words_per_row);
-        const int k0 = wi * 8;
-        if (k0 >= K) continue;
-        const uint32_t word = qw[idx];
-        float s = 1.f;
-        if (g) s = __half2float(scales[(size_t)n * (K / g) + k0 / g]);  // g % 32 == 0: one group per word
-        float v[8];
+    const int lane = threadIdx.x & 31;
+    const int per_row = (K + 128 * kDequantSteps - 1) / (128 * kDequantSteps);
+    const long long units = (long long)N * per_row;
+    const int row_bytes = jq_row_stride_codes(K) >> 1, G = g ? K / g : 0;
+    const bool vec = (K & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+    for (long long u = blockIdx.x * 8LL + (threadIdx.x >> 5); u < units; u += gridDim.x * 8LL) {
+        const int n = (int)(u / per_row), k0 = (int)(u - (long long)n * per_row) * (128 * kDequantSteps) + lane * 4;
+        const uint8_t *row = qw + (size_t)n * row_bytes;
+        uint32_t w[kDequantSteps];
+        float s[kDequantSteps];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t c = (word >> (4 * j)) & 0xfu;
-            float t;
-            if (FMT == JQ_FMT_E2M1) t = kE2M1[c];
-            else t = __half2float(codebook[(size_t)n * 16 + c]);
-            v[j] = g ? __fmul_rn(t, s) : t;
+        for (int i = 0; i < kDequantSteps; ++i) {
+            const int k = k0 + 128 * i;
+            w[i] = k < K ? *reinterpret_cast<const unsigned short *>(row + (k >> 1)) : 0u;
+            s[i] = (g && k < K) ? __half2float(scales[(size_t)n * G + k / g]) : 1.f;   // g % 32 == 0: one group per 4 codes
         }
-        float *o = out + (size_t)n * K + k0;
-        if (k0 + 8 <= K && ((reinterpret_cast<uintptr_t>(o) & 15u) == 0)) {
-            reinterpret_cast<float4 *>(o)[0] = make_float4(v[0], v[1], v[2], v[3]);
-            reinterpret_cast<float4 *>(o)[1] = make_float4(v[4], v[5], v[6], v[7]);
-        } else {
+        float entry;
+        if (FMT == JQ_FMT_E2M1) entry = kE2M1[lane & 15];
+        else entry = __half2float(codebook[(size_t)n * 16 + (lane & 15)]);
+        float *o = out + (size_t)n * K;
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (k0 + j < K) o[j] = v[j];
+        for (int i = 0; i < kDequantSteps; ++i) {
+            const int k = k0 + 128 * i;
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float t = __shfl_sync(0xffffffffu, entry, (w[i] >> (4 * j)) & 0xfu);
+                v[j] = g ? __fmul_rn(t, s[i]) : t;
+            }
+            if (vec) {
+                if (k < K) __stcs(reinterpret_cast<float4 *>(o + k), make_float4(v[0], v[1], v[2], v[3]));
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (k + j < K) o[k + j] = v[j];
+            }
         }
     }
 }
@@ -74,20 +87,15 @@ static int dequant_common(int fmt, const void *qw, const void *scales, const voi
     if (g && !scales) return JQ_ERR_NULL_PTR;
     if (!jq_aligned16(qw)) return JQ_ERR_BAD_ALIGN;
     if (reinterpret_cast<uintptr_t>(out) & 3u) return JQ_ERR_BAD_ALIGN;
-    const long long total = (long long)N * (jq_row_stride_codes(K) >> 3);
-    long long blocks = (total + 255) / 256;
-    const long long cap = (long long)jq_sm_count() * 16;
+    const long long units = (long long)N * ((K + 128 * kDequantSteps - 1) / (128 * kDequantSteps));
+    long long blocks = (units + 7) / 8;
+    const long long cap = 0x7fffffff;                  // one unit per warp: blocks that retire one by one keep loads and stores of different units overlapped
     if (blocks > cap) blocks = cap;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (fmt == JQ_FMT_E2M1)
-        dequant_kernel<JQ_FMT_E2M1><<<(int)blocks, 256, 0, st>>>(reinterpret_cast<const uint32_t *>(qw),
-                                                                 reinterpret_cast<const __half *>(scales), nullptr, out,
-                                                                 N, K, g);
-    else
-        dequant_kernel<JQ_FMT_GF4><<<(int)blocks, 256, 0, st>>>(reinterpret_cast<const uint32_t *>(qw),
-                                                                reinterpret_cast<const __half *>(scales),
-                                                                reinterpret_cast<const __half *>(codebook), out, N, K,
-                                                                g);
+    const uint8_t *q = reinterpret_cast<const uint8_t *>(qw);
+    const __half *sc = reinterpret_cast<const __half *>(scales), *cb = reinterpret_cast<const __half *>(codebook);
+    if (fmt == JQ_FMT_E2M1) dequant_kernel<JQ_FMT_E2M1><<<(int)blocks, 256, 0, st>>>(q, sc, nullptr, out, N, K, g);
+    else dequant_kernel<JQ_FMT_GF4><<<(int)blocks, 256, 0, st>>>(q, sc, cb, out, N, K, g);
     return jq_launch_status();
 }
 
