@@ -25,8 +25,13 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
 
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    """Handle of the current device's current stream."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def _addr(t: Optional[torch.Tensor]) -> Optional[int]:
+    return None if t is None else t.data_ptr()
 
 
 def _need_cuda(*ts):
@@ -130,7 +135,8 @@ def _workspace(device, nbytes: int, kind: str = "gemv") -> torch.Tensor:
     stream are ordered, so consecutive calls may share it; another stream gets
     its own.  The family with a status word at offset 0 ("ta") never shares
     a buffer with the split-K partial sums, and starts zeroed."""
-    key = (device, torch.cuda.current_stream(device).cuda_stream, kind)
+    index = torch._C._cuda_getDevice() if device.index is None else device.index
+    key = (index, torch._C._cuda_getCurrentRawStream(index), kind)
     cache = _ws_cache()
     t = cache.get(key)
     if t is None or t.numel() < nbytes:
@@ -154,10 +160,8 @@ def check_status(raise_on_error: bool = True) -> int:
     leaves JQ_ERR_TIMEOUT there and returns early with its outputs partly
     written; every later call keeps the word until it is read here."""
     lib = _lib.load()
-    dev = torch.device("cuda", torch.cuda.current_device())
-    stream = torch.cuda.current_stream(dev).cuda_stream
     worst = 0
-    ws = _ws_cache().get((dev, stream, "ta"))
+    ws = _ws_cache().get((torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream, "ta"))
     if ws is not None:
         worst = min(worst, lib.jq_ta_status(_ptr(ws), 1, _stream()))
     if worst and raise_on_error:
@@ -165,23 +169,30 @@ def check_status(raise_on_error: bool = True) -> int:
     return worst
 
 
+_ta_workspace_bytes = {}       # (K, rows) -> bytes
+
+
 def _linear_rows_ta(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y):
     """Through the TMA-fed kernels, at most ta_max_batch rows per pass."""
     lib = _lib.load()
     Bt = x2.shape[0]
-    MAX_TA_BATCH = ta_max_batch(fmt_id)
-    prob = _lib.jq_problem()
-    prob.K = K
+    most = ta_max_batch(fmt_id)
     with _on(x2.device):
         stream = _stream()
-        for b0 in range(0, Bt, MAX_TA_BATCH):
-            b1 = min(Bt, b0 + MAX_TA_BATCH)
-            wsb = lib.jq_ta_workspace_bytes(ctypes.byref(prob), 1, b1 - b0)
+        for b0 in range(0, Bt, most):
+            b1 = min(Bt, b0 + most)
+            wsb = _ta_workspace_bytes.get((K, b1 - b0))
+            if wsb is None:
+                prob = _lib.jq_problem()
+                prob.K = K
+                wsb = _ta_workspace_bytes[(K, b1 - b0)] = lib.jq_ta_workspace_bytes(ctypes.byref(prob), 1, b1 - b0)
             ws = _workspace(x2.device, wsb, "ta")
-            xs, ys = (x2, y) if Bt <= MAX_TA_BATCH else (x2[b0:b1], y[b0:b1])
-            st = lib.jq_gemm_ta(fmt_id, _ptr(qweight), _ptr(scales), _ptr(codebook), _ptr(xs), _ptr(bias),
-                                _ptr(ys), N, K, b1 - b0, g, had, _DT[x2.dtype], _DT[y.dtype], _ptr(ws), ws.numel(), stream)
-            _lib.check(st, "jq_gemm_ta")
+            xs, ys = (x2, y) if Bt <= most else (x2[b0:b1], y[b0:b1])
+            st = lib.jq_gemm_ta(fmt_id, _addr(qweight), _addr(scales), _addr(codebook), xs.data_ptr(), _addr(bias),
+                                ys.data_ptr(), N, K, b1 - b0, g, had, _DT[x2.dtype], _DT[y.dtype], ws.data_ptr(), ws.numel(),
+                                stream)
+            if st:
+                _lib.check(st, "jq_gemm_ta")
     if _checked:
         check_status()
     return y
@@ -192,9 +203,9 @@ def _rows_scratch(device, nbytes: int):
     fits into it as it is, an allocation of the call's own otherwise.  The status word is the buffer's."""
     ws = _workspace(device, 1024, "ta")
     if ws.numel() >= 1024 + nbytes:
-        return None, ctypes.c_void_p(ws.data_ptr() + 1024), ws.numel() - 1024, _ptr(ws)
+        return None, ws.data_ptr() + 1024, ws.numel() - 1024, ws.data_ptr()
     own = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    return own, _ptr(own), nbytes, _ptr(ws)
+    return own, own.data_ptr(), nbytes, ws.data_ptr()
 
 
 def _linear_many_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y):
@@ -206,9 +217,11 @@ def _linear_many_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had,
             b1 = min(rows, b0 + part)
             xs, ys = (x2, y) if rows <= part else (x2[b0:b1], y[b0:b1])
             own, scratch, size, status = _rows_scratch(x2.device, lib.jq_gemm_rows_scratch_bytes(fmt_id, N, K, b1 - b0, g))
-            st = lib.jq_gemm_rows(fmt_id, _ptr(qweight), _ptr(scales), _ptr(codebook), _ptr(xs), _ptr(bias), _ptr(ys), N, K,
-                                  b1 - b0, g, had, _DT[x2.dtype], _DT[y.dtype], scratch, size, status, _stream())
-            _lib.check(st, "jq_gemm_rows")
+            st = lib.jq_gemm_rows(fmt_id, _addr(qweight), _addr(scales), _addr(codebook), xs.data_ptr(), _addr(bias),
+                                  ys.data_ptr(), N, K, b1 - b0, g, had, _DT[x2.dtype], _DT[y.dtype], scratch, size, status,
+                                  _stream())
+            if st:
+                _lib.check(st, "jq_gemm_rows")
             del own
     if _checked:
         check_status()
@@ -261,7 +274,7 @@ _NO_SWITCH = _NoDeviceSwitch()
 
 def _on(device):
     """Device guard that costs nothing when the tensor's device is already current."""
-    return _NO_SWITCH if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+    return _NO_SWITCH if device.index == torch._C._cuda_getDevice() else torch.cuda.device(device)
 
 
 def _linear_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, out_id=-1):
@@ -273,7 +286,7 @@ def _linear_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, out_
     if ta_eligible(fmt_id, K, g, Bt) and _ta_aligned(qweight, scales, codebook):
         return _linear_rows_ta(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y)
     xd, yd = _DT[x2.dtype], _DT[y.dtype]
-    qw_p, sc_p, cb_p, bias_p = _ptr(qweight), _ptr(scales), _ptr(codebook), _ptr(bias)
+    qw_p, sc_p, cb_p, bias_p = _addr(qweight), _addr(scales), _addr(codebook), _addr(bias)
     with _on(x2.device):
         stream = _stream()
         for b0 in range(0, Bt, MAX_GEMV_BATCH):
@@ -289,10 +302,10 @@ def _linear_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, out_
             def call(ws_t):
                 nb = ws_t.numel() if ws_t is not None else 0
                 if fmt_id == _lib.JQ_FMT_E2M1:
-                    return lib.jq_gemv_e2m1(qw_p, sc_p, _ptr(xs), bias_p, _ptr(ys), N, K,
-                                            b1 - b0, g, had, xd, yd, _ptr(ws_t), nb, stream)
-                return lib.jq_gemv_gf4(qw_p, sc_p, cb_p, _ptr(xs), bias_p, _ptr(ys),
-                                       N, K, b1 - b0, g, had, xd, yd, _ptr(ws_t), nb, stream)
+                    return lib.jq_gemv_e2m1(qw_p, sc_p, xs.data_ptr(), bias_p, ys.data_ptr(), N, K,
+                                            b1 - b0, g, had, xd, yd, _addr(ws_t), nb, stream)
+                return lib.jq_gemv_gf4(qw_p, sc_p, cb_p, xs.data_ptr(), bias_p, ys.data_ptr(),
+                                       N, K, b1 - b0, g, had, xd, yd, _addr(ws_t), nb, stream)
 
             st = call(ws)
             if st == -6 and ws is not None:   # workspace too small for this group size: sub-batch path
@@ -332,12 +345,13 @@ def linear(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor] = Non
         # through the dispatcher so that tracing sees one opaque op with a fake implementation
         return torch.ops.jq.linear(x, pw.qweight, pw.scales, pw.codebook, bias, pw.spec.fmt_id, pw.N, pw.K,
                                    pw.spec.group_size, pw.spec.had_block, out_id)
-    x2 = x.reshape(-1, pw.K)
+    flat = x.dim() == 2
+    x2 = x if flat else x.reshape(-1, pw.K)
     if not x2.is_contiguous():
         x2 = x2.contiguous()
     y = _linear_rows(x2, pw.qweight, pw.scales, pw.codebook, bias, pw.spec.fmt_id, pw.N, pw.K, pw.spec.group_size,
                      pw.spec.had_block, out_id)
-    return y.reshape(*x.shape[:-1], pw.N)
+    return y if flat else y.reshape(*x.shape[:-1], pw.N)
 
 
 class GroupedGemv:
