@@ -14,8 +14,11 @@
 // Tensor memory: three accumulators of 128 columns in rotation + two operand slots of 64.
 //
 // What bounds it: at NT = 256 a 128-code group is 1024 clocks of tensor pipe; decoding it takes about 670 clocks of the
-// ALU pipe (GF4, 21 operations per 8 codes) and the folding 256 issue slots per scheduler, both beside the MMAs.  A
-// pair table in shared memory (as in gemm_ta.cu) would save ALU work, but its lookups, the 64 KB of activations
+// ALU pipe (GF4, 21 operations per 8 codes) and the folding 256 issue slots per scheduler, both beside the MMAs.  Measured,
+// the one decode warp of a scheduler is bound by the latency of its own chain, not by either pipe (ALU 32 %, tensor 38 %
+// busy): 11008 x 4096 GF4, 2048 rows: 249 us (745 TFLOP/s; passes of 16 rows took 2848), 8192 x 8192 E2M1, 777 rows: 148 us
+// (705 TFLOP/s; 639).  Two decode warps per scheduler with tiles of 192 rows, which is what the registers allow, took 277 and
+// 185 us.  A pair table in shared memory (as in gemm_ta.cu) would save ALU work, but its lookups, the 64 KB of activations
 // per group that land in shared memory and the MMA's own reads together exceed the shared-memory bandwidth.
 //
 // A call with few tiles splits K over the CTAs of a cluster (up to 8); the partial sums meet through distributed
@@ -188,11 +191,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const __grid_con
                 for (int gi = 0; gi < 2; ++gi) {
                     const int g = 2 * step + gi;
                     if (g >= p.G) break;
-                    if (handed >= 2) {      // the slot's previous group has been multiplied
-                        ok = __all_sync(0xffffffffu, mbar_wait(afree(a_slot), a_par ^ 1, err));
-                        if (!ok) break;
-                        tc_fence_after();
-                    }
                     uint4 w4[4];
 #pragma unroll
                     for (int part = 0; part < 4; ++part) w4[part] = lds128(slot + (((gi * 4 + part) << 4) ^ lkey));
@@ -231,11 +229,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const __grid_con
                         }
                     };
                     // the decode of the next 32 codes is issued before the previous 16 pairs are stored; a group is
-                    // handed to the issuer only once the next group's first lookups are under way
+                    // handed to the issuer only once the next group's first lookups are under way, but before the wait
+                    // for that group's slot (with the wait in front, decoding and multiplying took turns)
                     uint32_t va[16], vb[16];
                     decode16(0, va);
                     decode16(1, vb);
                     hand_over();
+                    if (handed >= 2) {      // the slot's previous group has been multiplied
+                        ok = __all_sync(0xffffffffu, mbar_wait(afree(a_slot), a_par ^ 1, err));
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
                     tmem_st16(a_t, va);
                     decode16(2, va);
                     tmem_st16(a_t + 16, vb);

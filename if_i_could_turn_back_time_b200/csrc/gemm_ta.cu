@@ -390,14 +390,6 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
 #pragma unroll
                 for (int gi = 0; gi < 2; ++gi) {
                     const uint2 sc4 = gi ? make_uint2(sc_cur.z, sc_cur.w) : make_uint2(sc_cur.x, sc_cur.y);
-                    // the slot is free once the MMAs of the group that used it last are done
-                    if (t_next >= (uint32_t)kRing) {
-                        const uint32_t t = t_next - kRing, n = t >> 1;     // group t was its issuer's n-th
-                        ok = __all_sync(0xffffffffu, mbar_wait(dbar(h + 2 * (t & 1), n % C::kAccBufs), (n / C::kAccBufs) & 1, err));
-                        if (!ok) break;
-                        tc_fence_after();
-                    }
-                    ++t_next;
                     const uint32_t a_t = lane_t + (h * kRing + slot) * 64;
                     uint4 w4[4];
 #pragma unroll
@@ -434,11 +426,19 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                     };
                     // the decode of the next 32 codes is issued before the previous 16 pairs are stored, and the
                     // previous group is handed to the MMA issuer only once this group's first lookups are under way
-                    // (its tensor-memory stores have had that long to land)
+                    // (its tensor-memory stores have had that long to land), and before the wait for this group's slot
                     uint32_t va[16], vb[16];
                     decode16(0, va);
                     decode16(1, vb);
                     hand_over();
+                    // the slot is free once the MMAs of the group that used it last are done
+                    if (t_next >= (uint32_t)kRing) {
+                        const uint32_t t = t_next - kRing, n = t >> 1;     // group t was its issuer's n-th
+                        ok = __all_sync(0xffffffffu, mbar_wait(dbar(h + 2 * (t & 1), n % C::kAccBufs), (n / C::kAccBufs) & 1, err));
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
+                    ++t_next;
                     tmem_st16(a_t, va);
                     decode16(2, va);
                     tmem_st16(a_t + 16, vb);
@@ -1035,12 +1035,8 @@ static bool ta_shape_ok(int fmt, int N, int K, int g, int had) {
 }
 
 // batch 1 runs on the CUDA cores when the prepared activation of one problem fits its shared-memory buffer
-// (K up to 12288); from two rows on the tensor-memory kernel is faster (decode7b: 1800 against 1090 tokens/s)
-#ifdef JQ_NO_LUT
-static bool ta_use_lut(int B, int maxK) { return false; }
-#else
+// (K up to 12288); on the 7B-shaped step 931 us against 1114 on the tensor-memory kernel, which takes over from two rows
 static bool ta_use_lut(int B, int maxK) { return B == 1 && (size_t)maxK * 2 <= (size_t)LutSmem::kXBytes; }
-#endif
 
 extern "C" size_t jq_ta_workspace_bytes(const jq_problem *ph, int n, int B) {
     if (!ph || n <= 0 || B < 1 || B > 64) return 0;

@@ -25,18 +25,23 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
+// The same, suspended by the hardware for up to about a microsecond: a waiting warp that polls takes issue slots (some
+// ten instructions every 50 clocks) from the decode warps beside it.
+__device__ __forceinline__ bool mbar_try_suspended(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok) : "r"(bar), "r"(parity), "r"(1000u) : "memory");
+    return ok != 0;
+}
 // Bounded wait: false (and the CTA-wide error flag raised) when it gives up, after kSpinLimit polls or
 // about 0.25 s of SM clock, whichever comes first; also false as soon as another thread has raised the flag.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *err) {
     if (mbar_try(bar, parity)) return true;
     const long long t0 = clock64();
     for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        if (mbar_try(bar, parity)) return true;
+        if (mbar_try_suspended(bar, parity)) return true;
         if (*err) return false;
-        if (i > 8192) {
-            __nanosleep(64);
-            if (clock64() - t0 > 500000000LL) break;
-        }
+        if ((i & 63) == 63 && clock64() - t0 > 500000000LL) break;
     }
     *err = JQ_ERR_TIMEOUT;
     return false;
