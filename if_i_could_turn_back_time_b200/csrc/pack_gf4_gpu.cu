@@ -24,7 +24,7 @@
 // first (6 operations), and only a thread's candidates within the estimate's error bound of its smallest are computed
 // exactly, normally one.  The ranges of a level add up to K, but one node's can be most of it (weights with outliers): left
 // to the node's own lanes, the longest range set the pace.  4096 x 4096: 92.7 ms with queues of nodes in global memory, one
-// warp per node; 26 ms with a static tree of warps and lanes; see jq_pack_gf4 for the present figure.
+// warp per node; 27.8 ms like this.  (Doubles permuted against bank conflicts: 30.8 ms, the index arithmetic costs more.)
 #include "common.cuh"
 #include <cfloat>
 
@@ -64,7 +64,7 @@ struct Layout {
     size_t shared_bytes, cta_bytes;
 };
 __host__ inline Layout make_layout(int K, size_t shared_limit) {
-    const size_t m1 = (size_t)K + 1, d = sizeof(double) * ((m1 + 15) / 16 * 16);     // (doubles are stored permuted in blocks of 16)
+    const size_t m1 = (size_t)K + 1, d = sizeof(double) * m1;
     const size_t bytes[kArrays] = {d, d, d, d, d, sizeof(unsigned short) * m1, sizeof(int) * m1};
     Layout L{};
     L.cta_bytes = up256((kClasses + 1) * sizeof(unsigned short) * m1);    // the arguments of all classes, for the back-track
@@ -177,10 +177,6 @@ __global__ void __launch_bounds__(kSortThreads) sort_rows_kernel(const float *__
     }
 }
 
-// Where element i of an array of doubles lies.  The lanes of a warp read at strides of one, two or four elements
-// (neighbouring nodes' candidates); permuted like this all three touch every bank pair equally often.
-__device__ __forceinline__ int at(int i) { return i ^ ((i >> 4) & 3); }
-
 struct Dp {
     const double *P1, *P2;
     const int *C;             // null: all values are distinct, C[t] = t
@@ -189,23 +185,23 @@ struct Dp {
 
     __device__ __forceinline__ int count(int t) const { return C ? C[t] : t; }
     __device__ __forceinline__ double exact(const double *prev, int t, double p1, double p2, int cm) const {
-        const double d1 = __dsub_rn(p1, P1[at(t)]), d2 = __dsub_rn(p2, P2[at(t)]);
+        const double d1 = __dsub_rn(p1, P1[t]), d2 = __dsub_rn(p2, P2[t]);
         const double q = __ddiv_rn(__dmul_rn(d1, d1), (double)(cm - count(t)));
         const double seg = __dsub_rn(d2, q);
-        return prev ? __dadd_rn(prev[at(t)], seg) : seg;
+        return prev ? __dadd_rn(prev[t], seg) : seg;
     }
     // the same with the reciprocal of the count rounded first
     __device__ __forceinline__ double estimate(const double *prev, int t, double p1, double p2, int cm) const {
-        const int i = at(t);
+        const int i = t;
         const double d1 = __dsub_rn(p1, P1[i]), d2 = __dsub_rn(p2, P2[i]);
-        const double q = __dmul_rn(__dmul_rn(d1, d1), recip[at(cm - count(t))]);
+        const double q = __dmul_rn(__dmul_rn(d1, d1), recip[(cm - count(t))]);
         return __dadd_rn(prev[i], __dsub_rn(d2, q));
     }
     // first minimum of prev[t] + cost(t, mid) over t = t0 + first, t0 + first + step, ... <= t1; kAhead estimates at a
     // time hide each other's latency
     template <int kAhead>
     __device__ __forceinline__ void scan(const double *prev, int t0, int t1, int first, int step, int mid, double &best, int &bt) const {
-        const double p1 = P1[at(mid)], p2 = P2[at(mid)];
+        const double p1 = P1[mid], p2 = P2[mid];
         const int cm = count(mid);
         double low = __longlong_as_double(0x7ff0000000000000LL), limit = low;
         int pos = -1;
@@ -257,7 +253,7 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
     __shared__ int s_zero, s_breaks[kClasses + 1];
     __shared__ float s_upper[kClasses];                // largest value of each class
     // ranges that all warps share: a level's long nodes, the pieces of their ranges and the pieces' results.  A range is
-    // long from 16 candidates per lane of its group and 1/64 of the row, a piece at least 1/64 of the row, and a level's
+    // long from 32 candidates per lane of its group and 1/128 of the row, a piece at least 1/64 of the row, and a level's
     // ranges add up to at most twice the row, so that neither array overflows (what did would be scanned by its group)
     constexpr int kWide = kThreads / 4, kPieces = kThreads / 2;
     struct Wide { int first, count, mid, t0; };
@@ -282,7 +278,7 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
     const int G = g ? K / g : 0;
     const int stride_b = jq_row_stride_codes(K) >> 1;
 
-    for (int i = tid; i <= K; i += kThreads) recip[at(i)] = i ? __ddiv_rn(1.0, (double)i) : 0.0;
+    for (int i = tid; i <= K; i += kThreads) recip[i] = i ? __ddiv_rn(1.0, (double)i) : 0.0;
 
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
         const int row = row0 + r;
@@ -292,15 +288,15 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
         const int ke = m < kClasses ? m : kClasses;
         for (int i = tid; i <= m; i += kThreads) {
             const double2 p = rd.P[i];
-            P1[at(i)] = p.x;
-            P2[at(i)] = p.y;
+            P1[i] = p.x;
+            P2[i] = p.y;
             C[i] = rd.C[i];
         }
         __syncthreads();
         // ---- 5. dynamic programme.  An estimate differs from the exact cost by a few roundings of terms that are at
         // most the row's sum of squares: 2^-49 of it, with room to spare 2^-46
-        const Dp dp{P1, P2, m == K ? nullptr : C, recip, P2[at(m)] * 0x1p-45};
-        for (int i = tid; i <= m; i += kThreads) prev[at(i)] = i >= 1 ? dp.exact(nullptr, 0, P1[at(i)], P2[at(i)], dp.count(i)) : DBL_MAX;
+        const Dp dp{P1, P2, m == K ? nullptr : C, recip, P2[m] * 0x1p-45};
+        for (int i = tid; i <= m; i += kThreads) prev[i] = i >= 1 ? dp.exact(nullptr, 0, P1[i], P2[i], dp.count(i)) : DBL_MAX;
         __syncthreads();
         int parity = 0;
         if (tid < 4) s_count[tid >> 1][tid & 1] = 0;
@@ -308,14 +304,14 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
         for (int j = 2; j <= ke; ++j) {
             unsigned short *out_arg = arg_all + (size_t)j * (K + 1);
             auto write = [&](int mid, double best, int bt) {
-                cur[at(mid)] = best;
+                cur[mid] = best;
                 arg[mid] = (unsigned short)bt;
                 out_arg[mid] = (unsigned short)bt;
             };
             const int root = j == ke ? m : j, piece_len = max(128, m / 64);
             for (int level = 0; (1 << level) <= m - root + 1; ++level, parity ^= 1) {
                 const int nodes = 1 << level, width = nodes <= kWarps ? 32 : max(kThreads >> level, 1);   // lanes per node
-                const int long_range = max(16 * width, m / 64);
+                const int long_range = max(32 * width, m / 128);
                 const int in_group = lane & (width - 1), leader = lane - in_group;
                 for (int base = 0; base < nodes; base += kThreads / width) {
                     const int node = base + tid / width;
@@ -346,8 +342,8 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
                     double best = DBL_MAX;
                     int bt = 0x7fffffff;
                     if (live && !shared_out) {
-                        if (width >= 16) dp.scan<4>(prev, t0, t1, in_group, width, mid, best, bt);
-                        else dp.scan<2>(prev, t0, t1, in_group, width, mid, best, bt);
+                        if (width >= 8) dp.scan<4>(prev, t0, t1, in_group, width, mid, best, bt);
+                        else dp.scan<1>(prev, t0, t1, in_group, width, mid, best, bt);
                     }
                     __syncwarp();
                     for (int o = width >> 1; o > 0; o >>= 1)
@@ -399,7 +395,7 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
         if (tid < kClasses) {
             const int c = tid < ke ? tid : ke - 1;
             const int a = s_breaks[c], b = s_breaks[c + 1];
-            double mean = __ddiv_rn(__dsub_rn(P1[at(b)], P1[at(a)]), (double)(C[b] - C[a]));
+            double mean = __ddiv_rn(__dsub_rn(P1[b], P1[a]), (double)(C[b] - C[a]));
             if (s_zero >= a && s_zero < b) mean = 0.0;   // the class holding an exact zero is pinned to 0 (as the host packer)
             codebook[(size_t)row * kClasses + tid] = __double2half(mean);
             s_upper[tid] = tid < ke ? rd.uv[b - 1] : __int_as_float(0x7f800000);
