@@ -80,7 +80,8 @@ def test_many_rows_in_parts_and_from_a_cuda_graph(monkeypatch):
 
 @pytest.mark.parametrize("cin,cout,k,stride,pad,dilation,hw,batch,dtype", [
     (3, 8, 3, 1, 1, 1, (9, 11), 2, torch.float32), (16, 130, 5, 2, 2, 1, (17, 8), 3, torch.float16),
-    (48, 24, 1, 1, 0, 1, (7, 7), 5, torch.bfloat16), (20, 40, (3, 2), (2, 1), (0, 3), (2, 3), (14, 13), 2, torch.float32)])
+    (48, 24, 1, 1, 0, 1, (7, 7), 5, torch.bfloat16), (20, 40, (3, 2), (2, 1), (0, 3), (2, 3), (14, 13), 2, torch.float32),
+    (96, 16, 3, 1, 1, 1, (6, 7), 2, torch.float32)])          # fields too long for shared memory
 def test_convolution_gathers_receptive_fields(cin, cout, k, stride, pad, dilation, hw, batch, dtype):
     """Against float64 conv2d on the dequantised weight; contiguous, channels-last and sliced images give the same bits."""
     torch.manual_seed(cin)
