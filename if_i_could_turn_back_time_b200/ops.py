@@ -103,8 +103,9 @@ MAX_ROWS_SCRATCH = 256 << 20      # bytes of prepared activation a many-row call
 
 def many_rows(fmt_id: int, K: int, g: int, batch: int) -> bool:
     """Calls that the many-row kernel takes: more rows than one pass of the kernels for small batches.  Those read the
-    weights once per pass (16 rows for GF4, 64 for E2M1 in 32-code groups, 8 for the shapes that only the row loops
-    take), the many-row kernel decodes them once per 256 rows."""
+    weights once per pass (64 rows; 8 for the shapes that only the row loops take), the many-row kernel decodes them
+    once per 256 rows.  GF4 goes there from 17 rows, where the tensor-memory kernel has to give up its pair tables;
+    the row loops keep 9 to 16 rows, two passes."""
     if fmt_id == _lib.JQ_FMT_E2M1 and ta_eligible(fmt_id, K, g, batch):
         return batch > ta_max_batch(fmt_id)
     return batch > 16
@@ -433,8 +434,8 @@ class GroupedGemv:
                      and _ta_aligned(w.qweight, w.scales, w.codebook) for w in weights)
         if use_ta:
             MAX_TA_BATCH = ta_max_batch(spec0.fmt_id)
-            # through the TMA-fed kernels: one plan (and workspace) per sub-batch of at most 16 (GF4) or 64 (E2M1)
-            # rows; a run is one activation-preparation launch plus one persistent launch per sub-batch
+            # through the TMA-fed kernels: one plan (and workspace) per sub-batch of at most 64 rows;
+            # a run is one activation-preparation launch plus one persistent launch per sub-batch
             with torch.cuda.device(self.device):
                 for b0 in range(0, batch, MAX_TA_BATCH):
                     nb = min(MAX_TA_BATCH, batch - b0)

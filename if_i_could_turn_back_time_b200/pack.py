@@ -68,7 +68,7 @@ def _pack_e2m1_cuda(W: torch.Tensor, spec: QuantSpec, rotate: bool) -> PackedWei
 
 
 def _pack_gf4_cuda(W: torch.Tensor, spec: QuantSpec, rotate: bool) -> PackedWeight:
-    """GF4 quantisation on the GPU: one CTA per row runs the same exact
+    """GF4 quantisation on the GPU: runs the same exact
     16-class Jenks dynamic programme as the host packer, bit for bit."""
     import ctypes
     lib = _lib.load()

@@ -310,8 +310,8 @@ int jq_jenks2_break(const float *sorted, long long n, double *var_or_null, doubl
 int jq_pack_e2m1(const float *W, int N, int K, int g, void *qweight, void *scales,
                  jq_stream_t stream);
 
-/* GF4 packer on the device (per-row 16-class Jenks natural breaks, one CTA per
- * row), bit-identical to jq_pack_gf4_host; rows up to 51200 values.  scales
+/* GF4 packer on the device (per-row 16-class Jenks natural breaks; rows are
+ * sorted by one kernel and classified by another), bit-identical to jq_pack_gf4_host; rows up to 51200 values.  scales
  * may be NULL when g == 0.  workspace: jq_pack_gf4_workspace_bytes(K) bytes. */
 size_t jq_pack_gf4_workspace_bytes(int K);
 int jq_pack_gf4(const float *W, int N, int K, int g, void *qweight, void *scales_or_null,
