@@ -11,8 +11,8 @@
 //   * GF4: a byte (two codes) indexes the row's 256-entry table of fp16 pairs,
 //     built once per tile in a shared-memory column that only this lane's bank
 //     serves (one conflict-free 32-bit lookup per two codes, the address formed
-//     by one dp4a), for up to 16 rows and three words of four, otherwise the
-//     row's codebook in registers through byte permutes; E2M1: cvt.rn.f16x2.e2m1x2 per byte, times the group's fp16
+//     by one dp4a); above 16 rows the row's codebook in registers, through byte
+//     permutes; E2M1: cvt.rn.f16x2.e2m1x2 per byte, times the group's fp16
 //     scale in fp16x2;
 //   * the fp16 values go to tensor memory with tcgen05.st as the A operand
 //     (M = 128 rows, K = 16 per instruction) of tcgen05.mma kind::f16; the B
@@ -27,8 +27,8 @@
 //     scales into the fp16 weights (one rounding per weight).
 // The multiply-accumulate work thus costs the CUDA cores nothing, whatever the
 // batch (up to 64 columns per pass), and the lookups are halved.  7B-shaped GF4
-// stack, 8 rows: 1167 us with decoding, folding and outputs in the same threads,
-// 1074 us with the roles below.
+// stack, 8 rows: 1162 us with decoding, folding and outputs in the same threads,
+// 1034 us with the roles below.
 //
 // Every wait on an mbarrier is bounded: on expiry the CTA raises a status word
 // in the workspace, all roles leave their loops, tensor memory is freed and
@@ -128,10 +128,11 @@ __global__ void __launch_bounds__(kPrepThreads) ta_prepare_kernel(const TaProble
 // accumulators of NB columns per issuer.
 //
 // The decode threads bound the kernel, so everything else is kept off them.  (When they also folded the accumulators,
-// exchanged the halves' sums and wrote the outputs, they were decoding for 60 % of a tile.)  GF4 up to 16 rows: the
-// shared-memory pipe takes 5 wavefronts per 8 codes of 32 rows with every byte looked up in the pair table; one word of
-// four goes through byte permutes on the ALU instead (tc.cuh, Codebook), which has room.  From 17 rows on there is no
-// shared memory for tables beside the activation rings and all words go through the permutes.
+// exchanged the halves' sums and wrote the outputs, they were decoding for 60 % of a tile.)  GF4 up to 16 rows looks
+// every byte up in the pair table; sending words through byte permutes on the ALU instead (tc.cuh, Codebook) to relieve
+// the shared-memory pipe costs more issue slots than it saves (7B-shaped step, 8 rows: none 1050 us, one word of four
+// 1086, two 1200).  From 17 rows on there is no shared memory for tables beside the activation rings, and all words go
+// through the permutes.
 //
 // A row's sum is formed in four parts of K (one, for short rows and for 33 rows and more), each in group order, added in
 // part order.  A single call with few tiles lets the CTAs of a cluster take the parts; the partial sums meet in
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             const uint4 *srow = reinterpret_cast<const uint4 *>(p.scales + (size_t)row * p.lds);
             uint4 sc_nxt = make_uint4(0, 0, 0, 0);
             if (!kGf4 && s_lo + h < s_hi) sc_nxt = __ldg(srow + s_lo + h);
-            if constexpr (kGf4) book.set(cb0, cb1);
+            if constexpr (kGf4 && !C::kTable) book.set(cb0, cb1);
             if constexpr (C::kTable) {
                 // ---- the pair table of this row (this thread fills the entries whose second code is in its half)
                 if (!(ok = quarter_sync())) break;      // both warps are done with the previous tile's lookups
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                         for (int wi = 0; wi < 4; ++wi) {
                             const uint32_t w = wi == 0 ? w4[part].x : (wi == 1 ? w4[part].y : (wi == 2 ? w4[part].z : w4[part].w));
                             if constexpr (kGf4) {
-                                if (C::kTable && wi < 3) {
+                                if (C::kTable) {
 #pragma unroll
                                     for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = lds32(dp4a_u(w, 0x80u << (8 * bj), tcol));
                                 } else {

@@ -215,10 +215,9 @@ int jq_gemv_grouped_peers(const jq_problem *problems_dev, const void *plan_host,
  * swizzle), a decode thread owns one weight row of a 128-row tile.
  *   GF4: a byte of packed codes indexes a 256-entry table of fp16 pairs that is
  *        built per tile in shared memory, one bank column per weight row, so
- *        two codes cost one conflict-free lookup (part of the codes, and all
- *        of them for B > 16, are looked up in registers instead).  Every weight
- *        and every scale stays exact; only the fp32 summation order differs
- *        from jq_gemv_gf4.
+ *        two codes cost one conflict-free lookup (B > 16: lookups in
+ *        registers instead).  Every weight and every scale stays exact; only
+ *        the fp32 summation order differs from jq_gemv_gf4.
  *        B == 1 (K <= 12288): the decode threads also multiply (fma.rn.f32.f16,
  *        fp32 accumulation), reading the prepared activation by broadcast
  *        shared-memory loads.  Otherwise the fp16 values go to tensor memory
