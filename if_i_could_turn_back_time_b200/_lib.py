@@ -56,8 +56,8 @@ _SIGNATURES = {
     "jq_gemm_rows_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
     "jq_gemm_rows": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                              c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p]),
-    "jq_conv_rows": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                             c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p]),
+    "jq_conv_rows": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                             c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p]),
     "jq_ta_status": (c_int, [c_void_p, c_int, c_void_p]),
     "jq_selftest_bounded_wait": (c_int, [c_void_p, ctypes.c_uint, c_void_p]),
     "jq_grouped_plan_bytes": (c_size_t, [c_int]),

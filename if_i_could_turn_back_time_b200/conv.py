@@ -85,7 +85,7 @@ class JenksQuantConv2d(nn.Conv2d):
         if (x.is_cuda and x.dtype in ops._DT and packed.spec.had_block == 0 and ho > 0 and wo > 0
                 and ops.many_rows(packed.spec.fmt_id, packed.K, packed.spec.group_size, B * ho * wo)
                 and not torch.compiler.is_compiling()):
-            return ops.conv2d(x, packed, self.bias, self.kernel_size, self.stride, self.padding, self.dilation, (ho, wo))
+            return ops.conv2d(x, packed, self.bias, self.kernel_size, self.stride, self.padding, self.dilation)
         cols = F.unfold(x, self.kernel_size, self.dilation, self.padding, self.stride)   # [B, I*kh*kw, L]
         rows = cols.transpose(1, 2).reshape(B * ho * wo, -1).contiguous()
         y = ops.linear(rows, packed, self.bias)                                       # [B*L, O]

@@ -745,8 +745,8 @@ extern "C" int jq_gemm_rows(int fmt, const void *qweight, const void *scales, co
 }
 
 extern "C" int jq_conv_rows(int fmt, const void *qweight, const void *scales, const void *codebook, const void *x,
-                            const float *bias, void *y, const jq_conv *c, int O, int g, int x_dtype, int y_dtype, void *scratch,
-                            size_t scratch_size, int *status, jq_stream_t stream) {
+                            const float *bias, void *y, const jq_conv *c, int O, int K, int rows, int g, int x_dtype, int y_dtype,
+                            void *scratch, size_t scratch_size, int *status, jq_stream_t stream) {
     if (!x || !c) return JQ_ERR_NULL_PTR;
     if (x_dtype < 0 || x_dtype > 2) return JQ_ERR_BAD_DTYPE;
     if (c->batch <= 0 || c->channels <= 0 || c->height <= 0 || c->width <= 0 || c->kernel_h <= 0 || c->kernel_w <= 0 ||
@@ -754,14 +754,16 @@ extern "C" int jq_conv_rows(int fmt, const void *qweight, const void *scales, co
         return JQ_ERR_BAD_SHAPE;
     const long long ho = ((long long)c->height + 2 * c->pad_h - (long long)c->dilation_h * (c->kernel_h - 1) - 1) / c->stride_h + 1;
     const long long wo = ((long long)c->width + 2 * c->pad_w - (long long)c->dilation_w * (c->kernel_w - 1) - 1) / c->stride_w + 1;
-    const long long T = ho * wo * c->batch, K = (long long)c->channels * c->kernel_h * c->kernel_w;
-    if (ho <= 0 || wo <= 0 || T > 0x3fffffffLL || K > 0x3fffffffLL) return JQ_ERR_BAD_SHAPE;
+    const long long most = 0x3fffffff, taps = (long long)c->kernel_h * c->kernel_w;
+    if (ho <= 0 || wo <= 0 || ho > most || wo > most || ho * wo > most || taps > most || rows > most) return JQ_ERR_BAD_SHAPE;
+    // the weights' row stride and scales per row follow from K, the extent of y from rows
+    if (ho * wo * c->batch != rows || taps * c->channels != K) return JQ_ERR_BAD_SHAPE;
     ConvArgs a{};
-    a.x = x; a.T = (int)T; a.K = (int)K; a.x_dtype = x_dtype;
+    a.x = x; a.T = rows; a.K = K; a.x_dtype = x_dtype;
     a.C = c->channels; a.H = c->height; a.W = c->width; a.kh = c->kernel_h; a.kw = c->kernel_w;
     a.sh = c->stride_h; a.sw = c->stride_w; a.ph = c->pad_h; a.pw = c->pad_w; a.dh = c->dilation_h; a.dw = c->dilation_w;
     a.wo = (int)wo; a.L = (int)(ho * wo);
     a.sb = c->stride_x[0]; a.sc = c->stride_x[1]; a.sr = c->stride_x[2]; a.sx = c->stride_x[3];
-    return launch(fmt, qweight, scales, codebook, bias, y, O, (int)K, (int)T, g, y_dtype, scratch, scratch_size, status,
+    return launch(fmt, qweight, scales, codebook, bias, y, O, K, rows, g, y_dtype, scratch, scratch_size, status,
                   reinterpret_cast<cudaStream_t>(stream), nullptr, &a);
 }

@@ -229,18 +229,31 @@ def _linear_many_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had,
     return y
 
 
-def conv2d(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor], kernel_size, stride, padding, dilation,
-           out_hw) -> torch.Tensor:
+def conv2d(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor], kernel_size, stride, padding,
+           dilation) -> torch.Tensor:
     """The receptive fields of x [B, C, H, W] times the packed [O, C*kh*kw] matrix -> [B, O, ho, wo] (channels-last
     strides): the fields are gathered by the preparation kernel, there is no unfolded copy."""
+    if x.dim() != 4:
+        raise RuntimeError(f"x has {x.dim()} dimensions, a convolution takes [B, C, H, W]")
+    if x.dtype not in _DT:
+        raise RuntimeError(f"unsupported activation dtype {x.dtype}")
+    B, C, H, W = x.shape
+    geo = [int(v) for pair in (kernel_size, stride, padding, dilation) for v in pair]
+    kh, kw, stride_h, stride_w, pad_h, pad_w, dil_h, dil_w = geo
+    if C * kh * kw != pw.K:
+        raise RuntimeError(f"x has {C} channels: fields of {C * kh * kw} values, packed weight has K={pw.K}")
+    if pw.spec.had_block:
+        raise RuntimeError("a rotated weight needs the fields laid out for the linear operator")
+    ho = (H + 2 * pad_h - dil_h * (kh - 1) - 1) // stride_h + 1
+    wo = (W + 2 * pad_w - dil_w * (kw - 1) - 1) // stride_w + 1
+    if ho <= 0 or wo <= 0:
+        raise RuntimeError(f"an image of {H} x {W} leaves no output position")
     lib = _lib.load()
     _need_cuda(x, pw.qweight, pw.scales, pw.codebook, bias)
     if bias is not None and bias.dtype != torch.float32:
         bias = bias.float()
-    B, C, H, W = x.shape
-    L = out_hw[0] * out_hw[1]
+    L = ho * wo
     y = torch.empty((B * L, pw.N), dtype=x.dtype, device=x.device)
-    geo = [int(v) for pair in (kernel_size, stride, padding, dilation) for v in pair]
     part = max(1, MAX_ROWS_SCRATCH // ((pw.K + 127) // 128 * 256) // L)          # images at once
     with _on(x.device):
         for b0 in range(0, B, part):
@@ -250,13 +263,13 @@ def conv2d(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor], kern
             own, scratch, size, status = _rows_scratch(
                 x.device, lib.jq_gemm_rows_scratch_bytes(pw.spec.fmt_id, pw.N, pw.K, (b1 - b0) * L, pw.spec.group_size))
             st = lib.jq_conv_rows(pw.spec.fmt_id, _ptr(pw.qweight), _ptr(pw.scales), _ptr(pw.codebook), _ptr(xs), _ptr(bias),
-                                  _ptr(ys), ctypes.byref(c), pw.N, pw.spec.group_size, _DT[x.dtype], _DT[y.dtype], scratch, size,
-                                  status, _stream())
+                                  _ptr(ys), ctypes.byref(c), pw.N, pw.K, ys.shape[0], pw.spec.group_size, _DT[x.dtype],
+                                  _DT[y.dtype], scratch, size, status, _stream())
             _lib.check(st, "jq_conv_rows")
             del own
     if _checked:
         check_status()
-    return y.view(B, out_hw[0], out_hw[1], pw.N).permute(0, 3, 1, 2)
+    return y.view(B, ho, wo, pw.N).permute(0, 3, 1, 2)
 
 
 _wsb_cache = {}

@@ -279,15 +279,16 @@ int jq_gemm_rows(int fmt, const void *qweight, const void *scales_or_null, const
 /* A convolution as the same product: the packed matrix is [O, channels * kernel_h * kernel_w], the activation rows are
  * the receptive fields of the output positions, gathered from the image x (zeros outside it) by the preparation
  * kernel without an unfolded copy; y is [batch * out_h * out_w, O] row-major.  Replaces the F.conv2d of
- * Quantization_Experiments/layers.py:48-97 (groups = 1).  Scratch as for jq_gemm_rows with B = batch * out_h * out_w. */
+ * Quantization_Experiments/layers.py:48-97 (groups = 1).  K is the packed matrix's row length and rows the number of rows
+ * of y: the image's geometry has to give both (JQ_ERR_BAD_SHAPE otherwise).  Scratch as for jq_gemm_rows with B = rows. */
 typedef struct jq_conv {
     int32_t batch, channels, height, width;
     int32_t kernel_h, kernel_w, stride_h, stride_w, pad_h, pad_w, dilation_h, dilation_w;
     int64_t stride_x[4];   /* elements between images, channels, rows and columns of x */
 } jq_conv;
 int jq_conv_rows(int fmt, const void *qweight, const void *scales_or_null, const void *codebook_or_null, const void *x,
-                 const float *bias_or_null, void *y, const jq_conv *conv, int O, int g, int x_dtype, int y_dtype,
-                 void *scratch, size_t scratch_bytes, int *status_dev, jq_stream_t stream);
+                 const float *bias_or_null, void *y, const jq_conv *conv, int O, int K, int rows, int g, int x_dtype,
+                 int y_dtype, void *scratch, size_t scratch_bytes, int *status_dev, jq_stream_t stream);
 
 /* Bytes of caller-provided device scratch an op needs for these sizes. */
 size_t jq_workspace_bytes(int op, int N, int K, int B);

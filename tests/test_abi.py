@@ -72,3 +72,20 @@ def test_host_packer_argument_checks():
     assert lib.jq_pack_e2m1_host(W.ctypes.data, 2, 64, 48, q.ctypes.data, s.ctypes.data, 1) == -2
     assert lib.jq_pack_gf4_host(W.ctypes.data, 2, 64, 32, q.ctypes.data, None, s.ctypes.data, 1) == -1
     assert lib.jq_rotate_weights_host(W.ctypes.data, 2, 64, 128, 1) == -2
+
+
+def test_convolution_geometry_has_to_match_the_packed_matrix():
+    """jq_conv_rows takes the row length of the packed matrix and the rows of y; an image that does not give them is
+    refused before anything is launched."""
+    lib = _lib.load()
+    buf = np.zeros(4096, dtype=np.uint8)
+    p = (buf.ctypes.data + 255) // 256 * 256
+
+    def call(channels, K, rows, batch=2, g=0):
+        c = _lib.jq_conv(batch, channels, 9, 7, 3, 3, 1, 1, 1, 1, 1, 1, (ctypes.c_int64 * 4)(channels * 63, 63, 7, 1))
+        return lib.jq_conv_rows(_lib.JQ_FMT_GF4, p, p, p, p, None, p, ctypes.byref(c), 8, K, rows, g, 0, 0, p, 256, p, None)
+
+    assert call(4, 36, 126) == -6                      # the shapes agree: only the scratch is too small
+    assert call(3, 36, 126) == -2 and call(5, 36, 126) == -2
+    assert call(64, 512, 126, g=64) == -2 and call(32, 576, 126, g=64) == -2
+    assert call(4, 36, 125) == -2 and call(4, 36, 63) == -2 and call(4, 36, 126, batch=1) == -2

@@ -97,3 +97,14 @@ def test_convolution_gathers_receptive_fields(cin, cout, k, stride, pad, dilatio
     wide[:, 1:, 1:-1, 2:-1] = x
     assert torch.equal(q(wide[:, 1:, 1:-1, 2:-1]), y)
     assert ops.check_status(raise_on_error=False) == 0
+
+
+@pytest.mark.parametrize("fmt,g", [("gf4", 0), ("gf4", 32)])
+def test_convolution_refuses_other_channel_counts(fmt, g):
+    """From the module's forward, as torch.nn.Conv2d does; the refusal is the host's, nothing is launched."""
+    q = jq.JenksQuantConv2d(torch.nn.Conv2d(32, 8, 3, padding=1), 4, fmt=fmt, group_size=g).to(DEV)
+    q.commit()
+    for channels in (31, 33, 64):
+        with pytest.raises(RuntimeError, match=f"{channels} channels"):
+            q(torch.randn(2, channels, 9, 9, device=DEV))
+    assert q(torch.randn(2, 32, 9, 9, device=DEV)).shape == (2, 8, 9, 9)

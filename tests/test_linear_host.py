@@ -131,3 +131,12 @@ def test_grouped_plan_partitions_the_row_space_evenly():
     arr[3].qweight += 8
     st = lib.jq_grouped_plan(_lib.JQ_FMT_E2M1, ctypes.byref(arr), n, 1, plan.ctypes.data, plan.nbytes)
     assert st != 0 and "align" in _lib.strerror(st)
+
+
+@pytest.mark.parametrize("fmt,g", [("gf4", 0), ("gf4", 32)])
+@pytest.mark.parametrize("shape", [(2, 31, 9, 9), (2, 33, 9, 9), (2, 64, 9, 9), (32, 9, 9)])
+def test_convolution_refuses_an_image_that_is_not_the_layers(fmt, g, shape):
+    """The check comes before the devices are looked at, so that it needs no GPU."""
+    q = jq.JenksQuantConv2d(nn.Conv2d(32, 4, 3, padding=1), 4, fmt=fmt, group_size=g)
+    with pytest.raises(RuntimeError, match="channels|dimensions"):
+        jq.ops.conv2d(torch.randn(*shape), q.packed, q.bias, q.kernel_size, q.stride, q.padding, q.dilation)
