@@ -266,7 +266,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const __grid_con
         int buf = p.halves == 2 ? h : 0;
         uint32_t par = 0;
         float acc[128];
-        pdl_wait();                                // the prepared activation's row factors are read below
+        // The prepared activation's row factors are read below: with plain loads, as the preparation kernel may still be
+        // writing them while this one starts, and a read-only load (__ldg) need not stay behind the wait.
+        pdl_wait();
         bool ok = true;
         for (int tile = tile_lo; tile < p.tiles; tile += tile_stride) {
             const int n = (tile % p.rt) * kTileM + r, tt = tile / p.rt;
@@ -317,13 +319,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const __grid_con
                     if (t >= p.T) break;
                     float v = 0.f;
                     for (int k = 0; k < p.split; ++k) v += ld_cluster_f32(xring + (uint32_t)c * (kTileM * 4) + r * 4, k);
-                    if (ok && n < p.N) jq::store_out(p.y, (size_t)t * p.N + n, fmaf(v, __ldg(p.xscale + t), bias), p.y_dtype);
+                    if (ok && n < p.N) jq::store_out(p.y, (size_t)t * p.N + n, fmaf(v, p.xscale[t], bias), p.y_dtype);
                 }
                 cluster_sync();
             } else if (ok) {
                 float xs[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) xs[i] = (t0 + i * 32 + lane < p.T) ? __ldg(p.xscale + t0 + i * 32 + lane) : 0.f;
+                for (int i = 0; i < 4; ++i) xs[i] = (t0 + i * 32 + lane < p.T) ? p.xscale[t0 + i * 32 + lane] : 0.f;
                 if (p.y_dtype == JQ_F32) store_tile<float>(p, acc, xs, bias, n, t0, cols);
                 else if (p.y_dtype == JQ_F16) store_tile<__half>(p, acc, xs, bias, n, t0, cols);
                 else store_tile<__nv_bfloat16>(p, acc, xs, bias, n, t0, cols);

@@ -89,3 +89,16 @@ def test_convolution_geometry_has_to_match_the_packed_matrix():
     assert call(3, 36, 126) == -2 and call(5, 36, 126) == -2
     assert call(64, 512, 126, g=64) == -2 and call(32, 576, 126, g=64) == -2
     assert call(4, 36, 125) == -2 and call(4, 36, 63) == -2 and call(4, 36, 126, batch=1) == -2
+
+
+def test_prepared_activations_are_not_read_through_the_read_only_path():
+    """The main kernels start while the kernel that prepares the activation still runs (griddepcontrol.wait orders them);
+    read-only loads are for data that nothing writes during the kernel: weights, scales, codebooks, bias."""
+    csrc = os.path.join(ROOT, "if_i_could_turn_back_time_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        text = open(os.path.join(csrc, name)).read()
+        if "pdl_wait()" not in text:
+            continue
+        for load in re.findall(r"__ld(?:g|cg|cs|lu|cv)\s*\(([^;]*)", text):
+            assert not re.search(r"\b(?:xscale|xp|xprep)\b", load.split(")")[0]), f"{name}: {load}"
+        assert not re.search(r"const\s+\w+\s*\*\s*__restrict__\s+(?:xscale|xp|xprep)\b", text), name
