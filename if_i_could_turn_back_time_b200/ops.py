@@ -112,6 +112,7 @@ def many_rows(fmt_id: int, K: int, g: int, batch: int) -> bool:
 
 
 _tls = threading.local()   # every host thread has its own scratch buffers: calls from different threads never share one
+_captured = {}             # address -> buffer that a graph capture has used: the graph replays into it, so it is never freed
 _checked = False
 
 
@@ -135,7 +136,10 @@ def _workspace(device, nbytes: int, kind: str = "gemv") -> torch.Tensor:
     """Grow-only scratch per (device, stream, kernel family): calls on one
     stream are ordered, so consecutive calls may share it; another stream gets
     its own.  The family with a status word at offset 0 ("ta") never shares
-    a buffer with the split-K partial sums, and starts zeroed."""
+    a buffer with the split-K partial sums, and starts zeroed.  A buffer that a
+    captured call has used stays alive when a larger one takes its place or its
+    thread ends; the successor is at least twice as large, so that what a
+    stream keeps is at most its newest buffer's size."""
     index = torch._C._cuda_getDevice() if device.index is None else device.index
     key = (index, torch._C._cuda_getCurrentRawStream(index), kind)
     cache = _ws_cache()
@@ -143,8 +147,11 @@ def _workspace(device, nbytes: int, kind: str = "gemv") -> torch.Tensor:
     if t is None or t.numel() < nbytes:
         if t is not None and kind != "gemv" and check_status(raise_on_error=False):
             raise RuntimeError("a device-side wait gave up in an earlier call (status word raised)")
-        t = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+        least = 2 * t.numel() if t is not None and t.data_ptr() in _captured else 1 << 20
+        t = torch.zeros(max(nbytes, least), dtype=torch.uint8, device=device)
         cache[key] = t
+    if torch.cuda.is_current_stream_capturing():
+        _captured[t.data_ptr()] = t
     return t
 
 

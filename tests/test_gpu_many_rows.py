@@ -108,3 +108,41 @@ def test_convolution_refuses_other_channel_counts(fmt, g):
         with pytest.raises(RuntimeError, match=f"{channels} channels"):
             q(torch.randn(2, channels, 9, 9, device=DEV))
     assert q(torch.randn(2, 32, 9, 9, device=DEV)).shape == (2, 8, 9, 9)
+
+
+def test_captured_calls_survive_a_larger_call_on_their_stream():
+    """Between capture and replay a call that needs more scratch replaces the stream's buffer, and other tensors are
+    allocated and filled: the replay still gives the right results and leaves the others alone."""
+    gen = torch.Generator("cpu").manual_seed(4)
+    flat = jq.pack_weight(_weights(130, 700, 8), jq.QuantSpec("gf4", 0, 0)).to(DEV)
+    grouped = jq.pack_weight(_weights(192, 1024, 9), jq.QuantSpec("gf4", 128, 128)).to(DEV)
+    wide = jq.pack_weight(_weights(64, 11008, 10).to(DEV), jq.QuantSpec("e2m1", 32, 0))
+    conv = jq.JenksQuantConv2d(torch.nn.Conv2d(16, 24, 3), 4).to(DEV)
+    conv.commit()
+    xs = [torch.randn(40, 700, generator=gen).to(DEV), torch.randn(12, 1024, generator=gen).bfloat16().to(DEV),
+          torch.randn(2, 16, 9, 9, generator=gen).to(DEV)]
+    calls = [lambda x: ops.linear(x, flat), lambda x: ops.linear(x, grouped), conv]
+    x_wide = torch.randn(64, 11008, generator=gen).bfloat16().to(DEV)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        for call, x in zip(calls, xs):
+            call(x)
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        ys = [call(x) for call, x in zip(calls, xs)]
+    with torch.cuda.stream(stream):
+        ops.linear(x_wide, wide)
+        fill = [torch.full((1 << 20,), 7, dtype=torch.uint8, device=DEV) for _ in range(8)]
+    stream.synchronize()
+    for _ in range(2):
+        for x in xs:
+            x.copy_(torch.randn(x.shape, generator=gen))
+        graph.replay()
+        torch.cuda.synchronize()
+        for call, x, y in zip(calls, xs, ys):
+            assert torch.equal(y, call(x))
+        assert all(bool((f == 7).all()) for f in fill)
+    with torch.cuda.stream(stream):
+        assert ops.check_status(raise_on_error=False) == 0

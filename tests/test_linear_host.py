@@ -140,3 +140,34 @@ def test_convolution_refuses_an_image_that_is_not_the_layers(fmt, g, shape):
     q = jq.JenksQuantConv2d(nn.Conv2d(32, 4, 3, padding=1), 4, fmt=fmt, group_size=g)
     with pytest.raises(RuntimeError, match="channels|dimensions"):
         jq.ops.conv2d(torch.randn(*shape), q.packed, q.bias, q.kernel_size, q.stride, q.padding, q.dilation)
+
+
+@pytest.fixture
+def scratch(monkeypatch):
+    """ops' scratch buffers on the CPU: one device, one stream, and a switch that says whether a graph is being captured."""
+    import threading
+    from if_i_could_turn_back_time_b200 import ops
+    state = {"capturing": False}
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 0, raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 7, raising=False)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state["capturing"])
+    monkeypatch.setattr(ops, "check_status", lambda raise_on_error=True: 0)
+    monkeypatch.setattr(ops, "_tls", threading.local())
+    monkeypatch.setattr(ops, "_captured", {}, raising=False)
+    return ops, state
+
+
+@pytest.mark.parametrize("kind", ["ta", "gemv"])
+def test_a_scratch_buffer_that_a_graph_holds_is_not_freed(scratch, kind):
+    import weakref
+    ops, state = scratch
+    cpu = torch.device("cpu")
+    plain = weakref.ref(ops._workspace(cpu, 1024, kind))
+    held = weakref.ref(ops._workspace(cpu, 3 << 20, kind))
+    assert plain() is None                              # nothing but eager calls used it
+    state["capturing"] = True
+    assert ops._workspace(cpu, 1024, kind) is held()
+    state["capturing"] = False
+    largest = ops._workspace(cpu, 4 << 20, kind)
+    assert held() is not None and largest is not held()
+    assert largest.numel() >= 2 * held().numel()        # what is kept stays below the buffer in use
