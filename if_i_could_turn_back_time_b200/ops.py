@@ -208,9 +208,10 @@ def _linear_rows_ta(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y
 
 def _rows_scratch(device, nbytes: int):
     """(scratch pointer, size, status word) of a many-row call: the thread's "ta" buffer when the prepared activation
-    fits into it as it is, an allocation of the call's own otherwise.  The status word is the buffer's."""
+    fits into it as it is, an allocation of the call's own otherwise, and always while a graph is captured (from the
+    graph's pool: graphs that were captured on one stream may replay on several).  The status word is the buffer's."""
     ws = _workspace(device, 1024, "ta")
-    if ws.numel() >= 1024 + nbytes:
+    if ws.numel() >= 1024 + nbytes and not torch.cuda.is_current_stream_capturing():
         return None, ws.data_ptr() + 1024, ws.numel() - 1024, ws.data_ptr()
     own = torch.empty(nbytes, dtype=torch.uint8, device=device)
     return own, own.data_ptr(), nbytes, ws.data_ptr()

@@ -171,3 +171,13 @@ def test_a_scratch_buffer_that_a_graph_holds_is_not_freed(scratch, kind):
     largest = ops._workspace(cpu, 4 << 20, kind)
     assert held() is not None and largest is not held()
     assert largest.numel() >= 2 * held().numel()        # what is kept stays below the buffer in use
+
+
+def test_captured_many_row_calls_have_scratch_of_their_own(scratch):
+    ops, state = scratch
+    cpu = torch.device("cpu")
+    own, ptr, size, status = ops._rows_scratch(cpu, 4096)
+    assert own is None and ptr == status + 1024 and size >= 4096
+    state["capturing"] = True
+    own, ptr, size, captured_status = ops._rows_scratch(cpu, 4096)
+    assert own is not None and ptr == own.data_ptr() and size == own.numel() == 4096 and captured_status == status
