@@ -69,6 +69,7 @@ _SIGNATURES = {
     "jq_jenks2_break": (c_int, [c_void_p, ctypes.c_longlong, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "jq_pack_e2m1": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "jq_pack_gf4_workspace_bytes": (c_size_t, [c_int]),
+    "jq_pack_gf4_workspace_bytes_rows": (c_size_t, [c_int, c_int]),
     "jq_pack_gf4": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "jq_pack_e2m1_host": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int]),
     "jq_pack_gf4_host": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int]),

@@ -32,9 +32,12 @@ namespace jqg {
 
 constexpr int kClasses = 16;
 constexpr int kSortThreads = 256;
-constexpr int kRowsPerSm = 8;             // rows of a chunk per SM
+constexpr int kRowsPerSm = 8;             // rows of a chunk per SM, at most
+// Workspace per SM: 152 bytes per value of a row padded to a power of two.  With eight rows per SM whatever their length it
+// was 1.3 GB for rows of 32768 values.
+constexpr size_t kSmBudget = 152;
 
-__host__ __device__ inline size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+__host__ __device__ inline size_t up16(size_t v) { return (v + 15) / 16 * 16; }
 
 // a chunk row's slice of the workspace, written by the first kernel
 struct RowData {
@@ -44,12 +47,16 @@ struct RowData {
     int *m;              // how many
 };
 __host__ __device__ inline size_t row_bytes(int K) {
-    return up256(sizeof(double2) * ((size_t)K + 1)) + up256(sizeof(int) * ((size_t)K + 1)) + up256(sizeof(float) * (size_t)K + 8);
+    return sizeof(double2) * ((size_t)K + 1) + up16(sizeof(int) * ((size_t)K + 1)) + up16(sizeof(float) * (size_t)K + 8);
 }
+// The second kernel reads P and C of its row first; their place then takes the split arguments of ten classes.  The
+// other five classes' have a place of their own.
+constexpr int kArgsInRow = (sizeof(double2) + sizeof(int)) / sizeof(unsigned short);
+constexpr int kArgsBeside = kClasses - 1 - kArgsInRow;
 __device__ inline RowData row_data(unsigned char *base, int K) {
     RowData r;
-    r.P = reinterpret_cast<double2 *>(base); base += up256(sizeof(double2) * ((size_t)K + 1));
-    r.C = reinterpret_cast<int *>(base); base += up256(sizeof(int) * ((size_t)K + 1));
+    r.P = reinterpret_cast<double2 *>(base); base += sizeof(double2) * ((size_t)K + 1);
+    r.C = reinterpret_cast<int *>(base); base += up16(sizeof(int) * ((size_t)K + 1));
     r.m = reinterpret_cast<int *>(base);
     r.uv = reinterpret_cast<float *>(base) + 2;
     return r;
@@ -67,11 +74,11 @@ __host__ inline Layout make_layout(int K, size_t shared_limit) {
     const size_t m1 = (size_t)K + 1, d = sizeof(double) * m1;
     const size_t bytes[kArrays] = {d, d, d, d, d, sizeof(unsigned short) * m1, sizeof(int) * m1};
     Layout L{};
-    L.cta_bytes = up256((kClasses + 1) * sizeof(unsigned short) * m1);    // the arguments of all classes, for the back-track
+    L.cta_bytes = up16(kArgsBeside * sizeof(unsigned short) * m1);
     for (int a = 0; a < kArrays; ++a) {
-        const size_t b = (bytes[a] + 15) / 16 * 16;
+        const size_t b = up16(bytes[a]);
         if (L.shared_bytes + b <= shared_limit) { L.shared |= 1u << a; L.off[a] = L.shared_bytes; L.shared_bytes += b; }
-        else { L.off[a] = L.cta_bytes; L.cta_bytes += up256(b); }
+        else { L.off[a] = L.cta_bytes; L.cta_bytes += b; }
     }
     return L;
 }
@@ -246,8 +253,8 @@ __device__ __forceinline__ void take_first_min(double &best, int &bt, double ob,
 template <int kThreads, bool kAllShared>
 __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__restrict__ W, int row0, int rows, int K, int g,
                                                               uint8_t *__restrict__ qw, const __half *__restrict__ scales,
-                                                              __half *__restrict__ codebook, const unsigned char *__restrict__ row_ws,
-                                                              unsigned char *__restrict__ cta_ws, const __grid_constant__ Layout L) {
+                                                              __half *__restrict__ codebook, unsigned char *row_ws,
+                                                              unsigned char *cta_ws, const __grid_constant__ Layout L) {
     constexpr int kWarps = kThreads / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_zero, s_breaks[kClasses + 1];
@@ -274,7 +281,6 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
     int *C = reinterpret_cast<int *>(array(kCount));
     unsigned short *arg = reinterpret_cast<unsigned short *>(array(kArg));
     double *recip = reinterpret_cast<double *>(array(kRecip));
-    unsigned short *arg_all = reinterpret_cast<unsigned short *>(slice);          // [class][K + 1]
     const int G = g ? K / g : 0;
     const int stride_b = jq_row_stride_codes(K) >> 1;
 
@@ -283,7 +289,12 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
         const int row = row0 + r;
         const float *wr = W + (size_t)row * K;
-        const RowData rd = row_data(const_cast<unsigned char *>(row_ws) + (size_t)r * row_bytes(K), K);
+        const RowData rd = row_data(row_ws + (size_t)r * row_bytes(K), K);
+        // the split arguments of class j = 2 .. 16, for the back-track
+        auto args_of = [&](int j) {
+            return j - 2 < kArgsInRow ? reinterpret_cast<unsigned short *>(rd.P) + (size_t)(j - 2) * (K + 1)
+                                      : reinterpret_cast<unsigned short *>(slice) + (size_t)(j - 2 - kArgsInRow) * (K + 1);
+        };
         const int m = *rd.m;
         const int ke = m < kClasses ? m : kClasses;
         for (int i = tid; i <= m; i += kThreads) {
@@ -302,7 +313,7 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
         if (tid < 4) s_count[tid >> 1][tid & 1] = 0;
         __syncthreads();
         for (int j = 2; j <= ke; ++j) {
-            unsigned short *out_arg = arg_all + (size_t)j * (K + 1);
+            unsigned short *out_arg = args_of(j);
             auto write = [&](int mid, double best, int bt) {
                 cur[mid] = best;
                 arg[mid] = (unsigned short)bt;
@@ -381,7 +392,7 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
         // ---- 6. back-track, codebook, class upper bounds
         if (tid == 0) {
             s_breaks[ke] = m;
-            for (int j = ke; j >= 2; --j) s_breaks[j - 1] = arg_all[(size_t)j * (K + 1) + s_breaks[j]];
+            for (int j = ke; j >= 2; --j) s_breaks[j - 1] = args_of(j)[s_breaks[j]];
             s_breaks[0] = 0;
             // index of the distinct value 0.0 (m if the row has no exact zero)
             int lo = 0, hi = m;
@@ -432,13 +443,30 @@ static int next_pow2(int v) { int p = 1; while (p < v) p <<= 1; return p; }
 
 // CTAs of the second kernel per SM: short rows leave room for more of them, with fewer threads each
 static int jenks_threads(int K) { return K <= 1024 ? 256 : (K <= 2048 ? 512 : 1024); }
-static int jenks_ctas(int K) { return jq_sm_count() * (1024 / jenks_threads(K)); }
-static jqg::Layout jenks_layout(int K) { return jqg::make_layout(K, jqg::kSharedLimit / (1024 / jenks_threads(K))); }
+static int jenks_ctas_per_sm(int K) { return 1024 / jenks_threads(K); }
+static jqg::Layout jenks_layout(int K) { return jqg::make_layout(K, jqg::kSharedLimit / jenks_ctas_per_sm(K)); }
 
-extern "C" size_t jq_pack_gf4_workspace_bytes(int K) {
-    if (K <= 0) return 0;
-    return jqg::row_bytes(K) * (size_t)(jq_sm_count() * jqg::kRowsPerSm) + jenks_layout(K).cta_bytes * (size_t)jenks_ctas(K);
+// Rows of a chunk: as many per SM as the budget holds beside the second kernel's slices, a multiple of its CTAs; and the
+// CTAs that have work.
+struct Chunk { int rows, ctas; };
+static Chunk pack_chunk(int N, int K) {
+    const int per_sm = jenks_ctas_per_sm(K), sms = jq_sm_count();
+    const size_t budget = jqg::kSmBudget * (size_t)next_pow2(K), slices = jenks_layout(K).cta_bytes * (size_t)per_sm;
+    size_t rows = budget > slices ? (budget - slices) / jqg::row_bytes(K) : 0;
+    if (rows > (size_t)jqg::kRowsPerSm) rows = jqg::kRowsPerSm;
+    rows = rows / per_sm * per_sm;
+    if (rows < (size_t)per_sm) rows = per_sm;
+    const long long chunk = (long long)rows * sms, ctas = (long long)per_sm * sms;
+    return Chunk{(int)(N < chunk ? N : chunk), (int)(N < ctas ? N : ctas)};
 }
+
+extern "C" size_t jq_pack_gf4_workspace_bytes_rows(int N, int K) {
+    if (N <= 0 || K <= 0) return 0;
+    const Chunk c = pack_chunk(N, K);
+    return jqg::row_bytes(K) * (size_t)c.rows + jenks_layout(K).cta_bytes * (size_t)c.ctas;
+}
+
+extern "C" size_t jq_pack_gf4_workspace_bytes(int K) { return jq_pack_gf4_workspace_bytes_rows(0x7fffffff, K); }
 
 extern "C" int jq_pack_gf4(const float *W, int N, int K, int g, void *qweight, void *scales, void *codebook,
                            void *workspace, size_t workspace_bytes, jq_stream_t stream) {
@@ -448,7 +476,7 @@ extern "C" int jq_pack_gf4(const float *W, int N, int K, int g, void *qweight, v
     const int npad = next_pow2(K);
     const size_t sort_smem = (size_t)npad * sizeof(float);
     if (sort_smem > 200 * 1024) return JQ_ERR_UNSUPPORTED;   // rows longer than 32768 values
-    if (workspace_bytes < jq_pack_gf4_workspace_bytes(K)) return JQ_ERR_WORKSPACE;
+    if (workspace_bytes < jq_pack_gf4_workspace_bytes_rows(N, K)) return JQ_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) || !jq_aligned16(qweight) || (reinterpret_cast<uintptr_t>(W) & 3u))
         return JQ_ERR_BAD_ALIGN;
     const jqg::Layout L = jenks_layout(K);
@@ -460,14 +488,14 @@ extern "C" int jq_pack_gf4(const float *W, int N, int K, int g, void *qweight, v
     JQ_CUDA_TRY(cudaFuncSetAttribute(jqg::sort_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem));
     JQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.shared_bytes));
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const int chunk = jq_sm_count() * jqg::kRowsPerSm;
+    const Chunk chunk = pack_chunk(N, K);
     unsigned char *row_ws = reinterpret_cast<unsigned char *>(workspace);
-    unsigned char *cta_ws = row_ws + jqg::row_bytes(K) * (size_t)chunk;
-    for (int row0 = 0; row0 < N; row0 += chunk) {
-        const int rows = N - row0 < chunk ? N - row0 : chunk;
+    unsigned char *cta_ws = row_ws + jqg::row_bytes(K) * (size_t)chunk.rows;
+    for (int row0 = 0; row0 < N; row0 += chunk.rows) {
+        const int rows = N - row0 < chunk.rows ? N - row0 : chunk.rows;
         jqg::sort_rows_kernel<<<rows, jqg::kSortThreads, sort_smem, st>>>(W, row0, N, K, g, reinterpret_cast<__half *>(scales),
                                                                           row_ws, npad);
-        const int grid = rows < jenks_ctas(K) ? rows : jenks_ctas(K);
+        const int grid = rows < chunk.ctas ? rows : chunk.ctas;
         kern<<<grid, threads, L.shared_bytes, st>>>(W, row0, rows, K, g, reinterpret_cast<uint8_t *>(qweight),
                                                     reinterpret_cast<const __half *>(scales), reinterpret_cast<__half *>(codebook),
                                                     row_ws, cta_ws, L);

@@ -87,7 +87,7 @@ def _pack_gf4_cuda(W: torch.Tensor, spec: QuantSpec, rotate: bool) -> PackedWeig
     cb = torch.empty((N, 16), dtype=torch.float16, device=W.device)
     P = lambda t: None if t is None else ctypes.c_void_p(t.data_ptr())
     with torch.cuda.device(W.device):
-        wsb = lib.jq_pack_gf4_workspace_bytes(K)
+        wsb = lib.jq_pack_gf4_workspace_bytes_rows(N, K)
         ws = torch.empty(wsb, dtype=torch.uint8, device=W.device)
         st = lib.jq_pack_gf4(P(Wf), N, K, g, P(q), P(s), P(cb), P(ws), wsb,
                              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))

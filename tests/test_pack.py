@@ -173,3 +173,17 @@ def test_a_few_zeros_per_row_stay_zero(g):
     w_hat = _host_dequant(pw)
     assert (W == 0).sum() > 20 and np.all(w_hat[W == 0] == 0)
     assert np.all(np.diff(cb.astype(np.float32), axis=1) >= 0)
+
+
+@pytest.mark.parametrize("K", [1, 16, 96, 784, 1024, 1025, 2048, 4096, 4864, 8192, 11008, 16385, 28672, 32768])
+def test_device_packer_scratch_is_bounded_and_grows_with_the_rows(K):
+    """Ten rows pay for ten rows; any number of rows needs at most 152 bytes per SM and value of a padded row (and a little
+    for the shortest rows)."""
+    from if_i_could_turn_back_time_b200 import _lib
+    lib = _lib.load()
+    npad = 1 << (K - 1).bit_length()
+    most, sms = lib.jq_pack_gf4_workspace_bytes(K), 148
+    assert 0 < most <= sms * (152 * npad + 512)
+    sizes = [lib.jq_pack_gf4_workspace_bytes_rows(n, K) for n in (1, 10, 300, 5000, 1 << 30)]
+    assert sizes == sorted(sizes) and sizes[-1] == most
+    assert sizes[1] <= 10 * (80 * K + 512)
