@@ -7,8 +7,8 @@
 //     2. bitonic sort of u (padded with +inf to a power of two);
 //     3. run-length compression to distinct values and their start indices (= the prefix sums of the multiplicities);
 //     4. float64 prefix sums, sequential in index order (the summation order is part of the format contract: codebooks
-//        must come out bit-identical).  A chain of K dependent additions by one thread: the other CTAs of the SM fill
-//        the time.
+//        must come out bit-identical).  A chain of K dependent additions, some 44 clocks each: the other CTAs of the SM
+//        fill the time.
 //   jenks_rows_kernel, one CTA per SM:
 //     5. the dynamic programme over 16 classes in its divide-and-conquer form (the left-most optimal split is monotone
 //        in the prefix length), with the host's candidates and tie rule.  The recursion [lo, hi] -> mid,
@@ -31,7 +31,6 @@
 namespace jqg {
 
 constexpr int kClasses = 16;
-constexpr int kSortThreads = 256;
 constexpr int kRowsPerSm = 8;             // rows of a chunk per SM, at most
 // Workspace per SM: 152 bytes per value of a row padded to a power of two.  With eight rows per SM whatever their length it
 // was 1.3 GB for rows of 32768 values.
@@ -84,12 +83,12 @@ __host__ inline Layout make_layout(int K, size_t shared_limit) {
 }
 constexpr size_t kSharedLimit = 200 * 1024;       // of the second kernel's CTAs on an SM together (besides their static arrays)
 
-__global__ void __launch_bounds__(kSortThreads) sort_rows_kernel(const float *__restrict__ W, int row0, int N, int K, int g,
-                                                                 __half *__restrict__ scales, unsigned char *__restrict__ ws,
-                                                                 int npad) {
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads) sort_rows_kernel(const float *__restrict__ W, int row0, int N, int K, int g,
+                                                             __half *__restrict__ scales, unsigned char *__restrict__ ws, int npad) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float *sv = reinterpret_cast<float *>(smem_raw);   // npad floats: the row being sorted
-    constexpr int kWarps = kSortThreads / 32;
+    constexpr int kWarps = kThreads / 32;
     __shared__ int s_scan[kWarps + 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row = row0 + blockIdx.x;
@@ -110,14 +109,14 @@ __global__ void __launch_bounds__(kSortThreads) sort_rows_kernel(const float *__
             for (int k = lane; k < g; k += 32) sv[gi * g + k] = __fdiv_rn(wr[gi * g + k], s);
         }
     } else {
-        for (int k = tid; k < K; k += kSortThreads) sv[k] = wr[k];
+        for (int k = tid; k < K; k += kThreads) sv[k] = wr[k];
     }
-    for (int k = K + tid; k < npad; k += kSortThreads) sv[k] = __int_as_float(0x7f800000);  // +inf padding sorts last
+    for (int k = K + tid; k < npad; k += kThreads) sv[k] = __int_as_float(0x7f800000);  // +inf padding sorts last
     __syncthreads();
     // ---- 2. bitonic sort, ascending
     for (int size = 2; size <= npad; size <<= 1) {
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = tid; i < npad / 2; i += kSortThreads) {
+            for (int i = tid; i < npad / 2; i += kThreads) {
                 const int lo = 2 * i - (i & (stride - 1));
                 const int hi = lo + stride;
                 const bool up = (lo & size) == 0;
@@ -129,7 +128,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_rows_kernel(const float *__
     }
     // ---- 3. run-length compression of sv[0..K): a warp's 32 consecutive elements at a time
     int base = 0;                                          // distinct values so far
-    for (int c0 = 0; c0 < K; c0 += kSortThreads) {
+    for (int c0 = 0; c0 < K; c0 += kThreads) {
         const int i = c0 + tid;
         const bool head = i < K && (i == 0 || sv[i] != sv[i - 1]);
         const unsigned mask = __ballot_sync(0xffffffffu, head);
@@ -150,36 +149,27 @@ __global__ void __launch_bounds__(kSortThreads) sort_rows_kernel(const float *__
     if (tid == 0) { rd.C[m] = K; *rd.m = m; }
     __syncthreads();
     // ---- 4. the terms, then their sequential float64 prefix sums
-    for (int t = tid; t < m; t += kSortThreads) {
+    for (int t = tid; t < m; t += kThreads) {
         const double v = (double)rd.uv[t], n = (double)(rd.C[t + 1] - rd.C[t]);
         const double cv = __dmul_rn(n, v);
         rd.P[t + 1] = make_double2(cv, __dmul_rn(cv, v));
     }
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0) {        // every lane carries the chain of additions along and keeps the sums of its own element
         double p1 = 0.0, p2 = 0.0;
-        rd.P[0] = make_double2(0.0, 0.0);
-        constexpr int kAhead = 16;                         // the loads do not wait for the chain of additions
-        int t = 1;
-        if (m >= kAhead) {
-            double2 nxt[kAhead];
+        if (lane == 0) rd.P[0] = make_double2(0.0, 0.0);
+        double2 nxt = lane < m ? rd.P[1 + lane] : make_double2(0.0, 0.0);
+        for (int t0 = 0; t0 < m; t0 += 32) {
+            const double2 now = nxt;
+            double2 sums = now;
+            if (t0 + 32 + lane < m) nxt = rd.P[t0 + 33 + lane];
 #pragma unroll
-            for (int i = 0; i < kAhead; ++i) nxt[i] = rd.P[1 + i];
-            for (; t + 2 * kAhead - 1 <= m; t += kAhead) {
-                double2 now[kAhead];
-#pragma unroll
-                for (int i = 0; i < kAhead; ++i) { now[i] = nxt[i]; nxt[i] = rd.P[t + kAhead + i]; }
-#pragma unroll
-                for (int i = 0; i < kAhead; ++i) {
-                    p1 = __dadd_rn(p1, now[i].x); p2 = __dadd_rn(p2, now[i].y);
-                    rd.P[t + i] = make_double2(p1, p2);
-                }
+            for (int i = 0; i < 32; ++i) {
+                p1 = __dadd_rn(p1, __shfl_sync(0xffffffffu, now.x, i));
+                p2 = __dadd_rn(p2, __shfl_sync(0xffffffffu, now.y, i));
+                if (i == lane) sums = make_double2(p1, p2);
             }
-        }
-        for (; t <= m; ++t) {
-            const double2 v = rd.P[t];
-            p1 = __dadd_rn(p1, v.x); p2 = __dadd_rn(p2, v.y);
-            rd.P[t] = make_double2(p1, p2);
+            if (t0 + lane < m) rd.P[t0 + 1 + lane] = sums;
         }
     }
 }
@@ -276,15 +266,11 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
         if (kAllShared) return smem_raw + L.off[a];
         return ((L.shared >> a) & 1u) ? smem_raw + L.off[a] : slice + L.off[a];
     };
-    double *P1 = reinterpret_cast<double *>(array(kP1)), *P2 = reinterpret_cast<double *>(array(kP2));
-    double *prev = reinterpret_cast<double *>(array(kPrev)), *cur = reinterpret_cast<double *>(array(kCur));
-    int *C = reinterpret_cast<int *>(array(kCount));
-    unsigned short *arg = reinterpret_cast<unsigned short *>(array(kArg));
-    double *recip = reinterpret_cast<double *>(array(kRecip));
+    double *const table = reinterpret_cast<double *>(array(kRecip));
     const int G = g ? K / g : 0;
     const int stride_b = jq_row_stride_codes(K) >> 1;
 
-    for (int i = tid; i <= K; i += kThreads) recip[i] = i ? __ddiv_rn(1.0, (double)i) : 0.0;
+    for (int i = tid; i <= K; i += kThreads) table[i] = i ? __ddiv_rn(1.0, (double)i) : 0.0;
 
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
         const int row = row0 + r;
@@ -297,6 +283,12 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
         };
         const int m = *rd.m;
         const int ke = m < kClasses ? m : kClasses;
+        auto classify = [&](unsigned char *at_P1, unsigned char *at_P2, unsigned char *at_prev, unsigned char *at_cur,
+                            unsigned char *at_C, unsigned char *at_arg, const double *recip) __attribute__((always_inline)) {
+        double *P1 = reinterpret_cast<double *>(at_P1), *P2 = reinterpret_cast<double *>(at_P2);
+        double *prev = reinterpret_cast<double *>(at_prev), *cur = reinterpret_cast<double *>(at_cur);
+        int *C = reinterpret_cast<int *>(at_C);
+        unsigned short *arg = reinterpret_cast<unsigned short *>(at_arg);
         for (int i = tid; i <= m; i += kThreads) {
             const double2 p = rd.P[i];
             P1[i] = p.x;
@@ -332,6 +324,7 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
                         if ((node >> b) & 1) l = mid + 1; else h = mid - 1;
                     }
                     const bool live = node < nodes && l <= h;
+                    if (!__any_sync(0xffffffffu, live)) continue;
                     const int mid = (l + h) >> 1;
                     int t0 = 0, t1 = -1;
                     if (live) {
@@ -434,6 +427,26 @@ __global__ void __launch_bounds__(kThreads) jenks_rows_kernel(const float *__res
             reinterpret_cast<uint32_t *>(qw + (size_t)row * stride_b)[wi] = word;
         }
         __syncthreads();
+        };
+        if (!kAllShared) {
+            // The layout is for rows of K distinct values.  A row of fewer may fit in shared memory after all, reciprocals
+            // and all: the walk down a tree is then not a chain of L2 latencies (1000 x 8192, about 550 distinct values a
+            // row: 4.8 -> 3.1 ms).  The code is there twice so that the compiler knows which arrays are in shared memory
+            // (with pointers chosen per row, rows of many values took 11 % longer).
+            const size_t room = ((L.shared >> kRecip) & 1u) ? L.off[kRecip] : L.shared_bytes;
+            const size_t d = sizeof(double) * ((m + 2) & ~1), used = up16(4 * d + d / 2 + d / 4);
+            if (used <= room) {
+                const double *recip = table;
+                if (room == L.shared_bytes && used + sizeof(double) * ((size_t)K + 1) <= room) {
+                    double *copy = reinterpret_cast<double *>(smem_raw + used);
+                    for (int i = tid; i <= K; i += kThreads) copy[i] = table[i];
+                    recip = copy;
+                }
+                classify(smem_raw, smem_raw + d, smem_raw + 2 * d, smem_raw + 3 * d, smem_raw + 4 * d, smem_raw + 4 * d + d / 2, recip);
+                continue;
+            }
+        }
+        classify(array(kP1), array(kP2), array(kPrev), array(kCur), array(kCount), array(kArg), table);
     }
 }
 
@@ -485,16 +498,20 @@ extern "C" int jq_pack_gf4(const float *W, int N, int K, int g, void *qweight, v
     auto kern = threads == 256 ? (all_shared ? jqg::jenks_rows_kernel<256, true> : jqg::jenks_rows_kernel<256, false>)
               : threads == 512 ? (all_shared ? jqg::jenks_rows_kernel<512, true> : jqg::jenks_rows_kernel<512, false>)
                                : (all_shared ? jqg::jenks_rows_kernel<1024, true> : jqg::jenks_rows_kernel<1024, false>);
-    JQ_CUDA_TRY(cudaFuncSetAttribute(jqg::sort_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem));
     JQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.shared_bytes));
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const Chunk chunk = pack_chunk(N, K);
+    // 256 threads per row while several rows share an SM (the sequential sums of one run beside the sorting of others); 1024
+    // for rows that have an SM to themselves, for want of rows or (from 16385 values) of shared memory for a second: 148 rows
+    // of 11008 with 560 distinct values 182 -> 127 us, 300 of 28672 1176 -> 754
+    const int sort_threads = chunk.rows <= jq_sm_count() || sort_smem > 64 * 1024 ? 1024 : 256;
+    auto sort = sort_threads == 1024 ? jqg::sort_rows_kernel<1024> : jqg::sort_rows_kernel<256>;
+    JQ_CUDA_TRY(cudaFuncSetAttribute(sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem));
     unsigned char *row_ws = reinterpret_cast<unsigned char *>(workspace);
     unsigned char *cta_ws = row_ws + jqg::row_bytes(K) * (size_t)chunk.rows;
     for (int row0 = 0; row0 < N; row0 += chunk.rows) {
         const int rows = N - row0 < chunk.rows ? N - row0 : chunk.rows;
-        jqg::sort_rows_kernel<<<rows, jqg::kSortThreads, sort_smem, st>>>(W, row0, N, K, g, reinterpret_cast<__half *>(scales),
-                                                                          row_ws, npad);
+        sort<<<rows, sort_threads, sort_smem, st>>>(W, row0, N, K, g, reinterpret_cast<__half *>(scales), row_ws, npad);
         const int grid = rows < chunk.ctas ? rows : chunk.ctas;
         kern<<<grid, threads, L.shared_bytes, st>>>(W, row0, rows, K, g, reinterpret_cast<uint8_t *>(qweight),
                                                     reinterpret_cast<const __half *>(scales), reinterpret_cast<__half *>(codebook),
