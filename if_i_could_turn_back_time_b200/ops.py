@@ -102,15 +102,27 @@ MAX_ROWS_SCRATCH = 256 << 20      # bytes of prepared activation a many-row call
 
 
 def many_rows(fmt_id: int, K: int, g: int, batch: int) -> bool:
-    """Calls that the many-row kernel takes: more rows than one pass of the kernels for small batches.  Those read the
-    weights once per pass (64 rows; 8 for the shapes that only the row loops take), the many-row kernel decodes them
-    once per 256 rows.  GF4 goes there from 17 rows, where the tensor-memory kernel has to give up its pair tables;
-    the row loops keep 9 to 16 rows, two passes."""
-    if fmt_id == _lib.JQ_FMT_E2M1 and ta_eligible(fmt_id, K, g, batch):
-        return batch > ta_max_batch(fmt_id)
+    """Calls that the many-row kernel takes: more rows than the kernels for small batches take well.  Those read the
+    weights once per pass (8 rows for the shapes that only the row loops take, which keep 9 to 16 rows, two passes), the
+    many-row kernel decodes them once per 256 rows.
+
+    GF4 on the tensor-memory kernel's shapes: up to 32 rows that kernel is the faster one everywhere, from 33 rows it
+    depends on the matrix, as it no longer splits a row over CTAs.  Device time of a call in us, tensor-memory kernel /
+    many-row kernel (two to four passes of 16 rows, the only kernel there was before):
+
+        rows   1024 x 1024           4096 x 4096           11008 x 4096          4096 x 11008          28672 x 8192
+        17     10.5 / 11.6 (16.1)    13.6 / 20.6 (29.8)    22.0 / 40.4 (35.9)    22.5 / 43.0 (61.4)    75.7 / 142 (119)
+        32     10.5 / 11.7 (18.9)    15.0 / 20.5 (37.8)    22.1 / 40.9 (38.0)    25.0 / 43.1 (83.6)    76.9 / 142 (130)
+        48     11.8 / 11.8 (28.0)    23.3 / 24.4 (56.5)    23.8 / 41.4 (57.0)    52.5 / 46.1 (125)     81.1 / 144 (196)
+        64     12.3 / 12.1 (37.5)    23.3 / 24.5 (75.5)    25.7 / 41.6 (75.7)    52.8 / 46.2 (167)     81.6 / 144 (260)"""
+    if ta_eligible(fmt_id, K, g, batch):
+        return batch > (32 if fmt_id == _lib.JQ_FMT_GF4 else ta_max_batch(fmt_id))
     return batch > 16
 
 
+# Smallest scratch buffer of a kernel family.  "ta": one pass of 64 rows of up to 32000 codes, so that calls on a stream
+# that has made one, in a graph capture too, do not need a larger one.
+_LEAST_SCRATCH = {"ta": 4 << 20, "gemv": 1 << 20}
 _tls = threading.local()   # every host thread has its own scratch buffers: calls from different threads never share one
 _captured = {}             # address -> buffer that a graph capture has used: the graph replays into it, so it is never freed
 _checked = False
@@ -147,7 +159,7 @@ def _workspace(device, nbytes: int, kind: str = "gemv") -> torch.Tensor:
     if t is None or t.numel() < nbytes:
         if t is not None and kind != "gemv" and check_status(raise_on_error=False):
             raise RuntimeError("a device-side wait gave up in an earlier call (status word raised)")
-        least = 2 * t.numel() if t is not None and t.data_ptr() in _captured else 1 << 20
+        least = 2 * t.numel() if t is not None and t.data_ptr() in _captured else _LEAST_SCRATCH[kind]
         t = torch.zeros(max(nbytes, least), dtype=torch.uint8, device=device)
         cache[key] = t
     if torch.cuda.is_current_stream_capturing():
@@ -305,8 +317,11 @@ def _linear_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, out_
     y = torch.empty((Bt, N), dtype=_OUT[out_id] or x2.dtype, device=x2.device)
     if many_rows(fmt_id, K, g, Bt):
         return _linear_many_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y)
-    if ta_eligible(fmt_id, K, g, Bt) and _ta_aligned(qweight, scales, codebook):
-        return _linear_rows_ta(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y)
+    if ta_eligible(fmt_id, K, g, Bt):
+        if _ta_aligned(qweight, scales, codebook):
+            return _linear_rows_ta(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y)
+        if fmt_id == _lib.JQ_FMT_GF4 and Bt > 16:       # scales off a 16-byte boundary, which the many-row kernel takes
+            return _linear_many_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y)
     xd, yd = _DT[x2.dtype], _DT[y.dtype]
     qw_p, sc_p, cb_p, bias_p = _addr(qweight), _addr(scales), _addr(codebook), _addr(bias)
     with _on(x2.device):

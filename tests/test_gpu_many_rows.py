@@ -116,13 +116,13 @@ def test_captured_calls_survive_a_larger_call_on_their_stream():
     gen = torch.Generator("cpu").manual_seed(4)
     flat = jq.pack_weight(_weights(130, 700, 8), jq.QuantSpec("gf4", 0, 0)).to(DEV)
     grouped = jq.pack_weight(_weights(192, 1024, 9), jq.QuantSpec("gf4", 128, 128)).to(DEV)
-    wide = jq.pack_weight(_weights(64, 11008, 10).to(DEV), jq.QuantSpec("e2m1", 32, 0))
+    wide = jq.pack_weight(_weights(64, 34048, 10).to(DEV), jq.QuantSpec("e2m1", 32, 0))
     conv = jq.JenksQuantConv2d(torch.nn.Conv2d(16, 24, 3), 4).to(DEV)
     conv.commit()
     xs = [torch.randn(40, 700, generator=gen).to(DEV), torch.randn(12, 1024, generator=gen).bfloat16().to(DEV),
           torch.randn(2, 16, 9, 9, generator=gen).to(DEV)]
     calls = [lambda x: ops.linear(x, flat), lambda x: ops.linear(x, grouped), conv]
-    x_wide = torch.randn(64, 11008, generator=gen).bfloat16().to(DEV)
+    x_wide = torch.randn(64, 34048, generator=gen).bfloat16().to(DEV)
     stream = torch.cuda.Stream()
     stream.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(stream):
@@ -134,7 +134,7 @@ def test_captured_calls_survive_a_larger_call_on_their_stream():
         ys = [call(x) for call, x in zip(calls, xs)]
     with torch.cuda.stream(stream):
         ops.linear(x_wide, wide)
-        fill = [torch.full((1 << 20,), 7, dtype=torch.uint8, device=DEV) for _ in range(8)]
+        fill = [torch.full((4 << 20,), 7, dtype=torch.uint8, device=DEV) for _ in range(4)]
     stream.synchronize()
     for _ in range(2):
         for x in xs:

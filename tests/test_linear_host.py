@@ -163,12 +163,12 @@ def test_a_scratch_buffer_that_a_graph_holds_is_not_freed(scratch, kind):
     ops, state = scratch
     cpu = torch.device("cpu")
     plain = weakref.ref(ops._workspace(cpu, 1024, kind))
-    held = weakref.ref(ops._workspace(cpu, 3 << 20, kind))
+    held = weakref.ref(ops._workspace(cpu, 6 << 20, kind))
     assert plain() is None                              # nothing but eager calls used it
     state["capturing"] = True
     assert ops._workspace(cpu, 1024, kind) is held()
     state["capturing"] = False
-    largest = ops._workspace(cpu, 4 << 20, kind)
+    largest = ops._workspace(cpu, 7 << 20, kind)
     assert held() is not None and largest is not held()
     assert largest.numel() >= 2 * held().numel()        # what is kept stays below the buffer in use
 
@@ -181,3 +181,24 @@ def test_captured_many_row_calls_have_scratch_of_their_own(scratch):
     state["capturing"] = True
     own, ptr, size, captured_status = ops._rows_scratch(cpu, 4096)
     assert own is not None and ptr == own.data_ptr() and size == own.numel() == 4096 and captured_status == status
+
+
+def test_routes_of_calls_with_several_rows():
+    """GF4 on the tensor-memory kernel's shapes leaves it at 33 rows, E2M1 at 65, everything else the row loops at 17."""
+    from if_i_could_turn_back_time_b200 import _lib, ops
+    gf4, e2m1 = _lib.JQ_FMT_GF4, _lib.JQ_FMT_E2M1
+    for fmt, K, g, last in [(gf4, 4096, 128, 32), (gf4, 512, 256, 32), (gf4, 4096, 64, 16), (gf4, 784, 0, 16), (gf4, 384, 128, 16),
+                            (e2m1, 4096, 32, 64), (e2m1, 4096, 64, 16), (e2m1, 1152, 32, 16)]:
+        assert [ops.many_rows(fmt, K, g, b) for b in (1, last, last + 1, 4096)] == [False, False, True, True]
+
+
+def test_calls_of_up_to_64_rows_fit_in_the_first_scratch_buffer(scratch):
+    """A call in a graph capture cannot replace the stream's buffer (its status word would have to be read first)."""
+    import ctypes
+    from if_i_could_turn_back_time_b200 import _lib
+    ops, _ = scratch
+    prob = _lib.jq_problem()
+    prob.K = 28672
+    need = _lib.load().jq_ta_workspace_bytes(ctypes.byref(prob), 1, 64)
+    first = ops._workspace(torch.device("cpu"), 1024, "ta")
+    assert ops._workspace(torch.device("cpu"), need, "ta") is first
