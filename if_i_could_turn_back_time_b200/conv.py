@@ -7,8 +7,9 @@ built from an ``nn.Conv2d`` with ``(conv_module, bitwidth=4, mask=None)``,
 ``commit()``.  The weight ``[O, I, kh, kw]`` is packed as the matrix
 ``[O, I*kh*kw]`` and the convolution runs as an implicit GEMM: the many-row
 kernel's preparation step gathers the receptive fields from the image.  With a
-rotation, or for a handful of output positions, ``F.unfold`` lays the fields
-out and the linear operator does the multiply.  groups must be 1.
+rotation, for a handful of output positions, or for long fields at few
+positions (``ops.conv_gathers``), ``F.unfold`` lays the fields out and the
+linear operator does the multiply.  groups must be 1.
 """
 from __future__ import annotations
 
@@ -83,7 +84,7 @@ class JenksQuantConv2d(nn.Conv2d):
         wo = (W + 2 * self.padding[1] - self.dilation[1] * (kw - 1) - 1) // self.stride[1] + 1
         packed = self.packed
         if (x.is_cuda and x.dtype in ops._DT and packed.spec.had_block == 0 and ho > 0 and wo > 0
-                and ops.many_rows(packed.spec.fmt_id, packed.K, packed.spec.group_size, B * ho * wo)
+                and ops.conv_gathers(packed.spec.fmt_id, packed.K, packed.spec.group_size, B * ho * wo)
                 and not torch.compiler.is_compiling()):
             return ops.conv2d(x, packed, self.bias, self.kernel_size, self.stride, self.padding, self.dilation)
         cols = F.unfold(x, self.kernel_size, self.dilation, self.padding, self.stride)   # [B, I*kh*kw, L]

@@ -202,3 +202,13 @@ def test_calls_of_up_to_64_rows_fit_in_the_first_scratch_buffer(scratch):
     need = _lib.load().jq_ta_workspace_bytes(ctypes.byref(prob), 1, 64)
     first = ops._workspace(torch.device("cpu"), 1024, "ta")
     assert ops._workspace(torch.device("cpu"), need, "ta") is first
+
+
+def test_long_fields_at_few_positions_are_unfolded():
+    from if_i_could_turn_back_time_b200 import _lib, ops
+    gf4, e2m1 = _lib.JQ_FMT_GF4, _lib.JQ_FMT_E2M1
+    assert [ops.conv_gathers(gf4, 576, 0, p) for p in (1, 16, 17, 4096)] == [False, False, True, True]
+    assert [ops.conv_gathers(gf4, 1024, 128, p) for p in (16, 17)] == [False, True]
+    assert [ops.conv_gathers(e2m1, 1024, 32, p) for p in (64, 65)] == [False, True]
+    assert [ops.conv_gathers(gf4, 4608, 0, p) for p in (17, 32, 2048, 2049)] == [False, False, False, True]
+    assert [ops.conv_gathers(gf4, K, 0, 100) for K in (1536, 1537)] == [True, False]
