@@ -146,3 +146,56 @@ def test_captured_calls_survive_a_larger_call_on_their_stream():
         assert all(bool((f == 7).all()) for f in fill)
     with torch.cuda.stream(stream):
         assert ops.check_status(raise_on_error=False) == 0
+
+
+@pytest.mark.parametrize("fmt,g,rows", [("gf4", 128, 24), ("gf4", 128, 70), ("e2m1", 32, 40), ("e2m1", 32, 65), ("e2m1", 32, 130)])
+def test_scales_off_a_16_byte_boundary(fmt, g, rows):
+    """The tensor-memory kernel reads scales in 16-byte pieces: such a view goes to the row loops or to the many-row kernel,
+    which then keeps E2M1 weights exact at a shape where it would have folded the scales."""
+    pw = jq.pack_weight(_weights(140, 1024, 11), jq.QuantSpec(fmt, g, 0))
+    dev = pw.to(DEV)
+    room = torch.zeros(dev.scales.numel() + 8, dtype=dev.scales.dtype, device=DEV)
+    off = room[1:1 + dev.scales.numel()].view(dev.scales.shape)
+    off.copy_(dev.scales)
+    assert off.data_ptr() % 16 == 2
+    shifted = jq.PackedWeight(dev.spec, dev.N, dev.K, dev.qweight, off, dev.codebook)
+    x = torch.randn(rows, 1024, generator=torch.Generator("cpu").manual_seed(rows)).bfloat16()
+    y = ops.linear(x.to(DEV), shifted, out_dtype=torch.float32).cpu().numpy()
+    w = ops.dequantize(dev).cpu().double().numpy()
+    # 11 bits of the activation, 1024 products summed in fp32; no rounding of the weights
+    exact = x.double().numpy() @ w.T
+    assert np.abs(y - exact).max() <= 1e-3 * np.abs(exact).max()
+    assert formats.rel_err(y, ops.linear(x.to(DEV), dev, out_dtype=torch.float32).cpu().numpy()) <= 1e-3
+    assert ops.check_status(raise_on_error=False) == 0
+
+
+@pytest.mark.parametrize("fmt,K,g,had", [("gf4", 700, 0, 0), ("gf4", 1024, 128, 0), ("e2m1", 1024, 32, 0), ("e2m1", 1152, 64, 128)])
+def test_rows_that_are_not_finite_stay_among_themselves(fmt, K, g, had):
+    """A row with an infinity or a NaN gives no finite output (every product with it is one of these, or the sum is); the
+    rows beside it are what they are without it."""
+    spec = jq.QuantSpec(fmt, g, had)
+    pw = jq.pack_weight(_weights(130, K, 12), spec).to(DEV)
+    x = torch.randn(80, K, generator=torch.Generator("cpu").manual_seed(7)).to(DEV)
+    clean = ops.linear(x, pw)
+    bad = [0, 31, 32, 79]
+    for i, v in zip(bad, (float("nan"), float("inf"), float("-inf"), float("nan"))):
+        x[i, (i * 37) % K] = v
+    y = ops.linear(x, pw)
+    good = [i for i in range(80) if i not in bad]
+    assert torch.equal(y[good], clean[good])
+    assert not torch.isfinite(y[[0, 79]]).any()
+    hit = ops.dequantize(pw)[:, [(31 * 37) % K, (32 * 37) % K]] != 0
+    if not had:
+        assert not torch.isfinite(y[31][hit[:, 0]]).any() and not torch.isfinite(y[32][hit[:, 1]]).any()
+
+
+def test_convolution_with_group_scales():
+    """Groups of 64 and 96 values of the unfolded field, gathered and unfolded, against float64 conv2d."""
+    for cin, k, g, fmt in ((64, 3, 64, "gf4"), (32, 3, 96, "e2m1"), (256, 3, 128, "gf4")):
+        torch.manual_seed(cin)
+        q = jq.JenksQuantConv2d(torch.nn.Conv2d(cin, 20, k, padding=1), 4, fmt=fmt, group_size=g).to(DEV)
+        assert q.spec.group_size == g
+        x = torch.randn(2, cin, 7, 9, device=DEV)
+        y = q(x)
+        ref = torch.nn.functional.conv2d(x.double(), q.dequantized_weight().double(), q.bias.double(), padding=1)
+        assert (y.double() - ref).abs().max() <= TOL * ref.abs().max()
