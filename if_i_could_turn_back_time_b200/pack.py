@@ -41,6 +41,9 @@ class PackedWeight:
         return sum(t.numel() * t.element_size() for t in (self.qweight, self.scales, self.codebook) if t is not None)
 
 
+GF4_DEVICE_MAX_K = 32768       # longest row of the GF4 packer on the GPU: it sorts a row, padded to a power of two, in shared memory
+
+
 def _gpu_packable(W: torch.Tensor, spec: QuantSpec) -> bool:
     pg = spec.group_size // 32
     return W.shape[1] % 32 == 0 and 1 <= pg <= 32 and pg & (pg - 1) == 0 and W.shape[1] % spec.group_size == 0
@@ -102,7 +105,7 @@ def pack_weight(W: torch.Tensor, spec: QuantSpec, threads: int = 0, rotate: bool
     lib = _lib.load()
     if W.is_cuda and spec.fmt == "e2m1" and _gpu_packable(W, spec):
         return _pack_e2m1_cuda(W, spec, rotate)
-    if W.is_cuda and spec.fmt == "gf4" and W.shape[1] <= 51200:
+    if W.is_cuda and spec.fmt == "gf4" and W.shape[1] <= GF4_DEVICE_MAX_K:
         return _pack_gf4_cuda(W, spec, rotate)
     Wf = W.detach().to("cpu", torch.float32).contiguous().clone()
     N, K = Wf.shape

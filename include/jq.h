@@ -311,7 +311,7 @@ int jq_pack_e2m1(const float *W, int N, int K, int g, void *qweight, void *scale
                  jq_stream_t stream);
 
 /* GF4 packer on the device (per-row 16-class Jenks natural breaks; rows are
- * sorted by one kernel and classified by another), bit-identical to jq_pack_gf4_host; rows up to 51200 values.  scales
+ * sorted by one kernel and classified by another), bit-identical to jq_pack_gf4_host; rows up to 32768 values.  scales
  * may be NULL when g == 0.  workspace: jq_pack_gf4_workspace_bytes_rows(N, K) bytes, which grow with N up to
  * jq_pack_gf4_workspace_bytes(K), enough for any number of rows (about 152 bytes per SM and value of a row padded to a
  * power of two). */

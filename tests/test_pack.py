@@ -187,3 +187,25 @@ def test_device_packer_scratch_is_bounded_and_grows_with_the_rows(K):
     sizes = [lib.jq_pack_gf4_workspace_bytes_rows(n, K) for n in (1, 10, 300, 5000, 1 << 30)]
     assert sizes == sorted(sizes) and sizes[-1] == most
     assert sizes[1] <= 10 * (80 * K + 512)
+
+
+@pytest.mark.parametrize("K", [32767, 32768, 32769, 51200])
+def test_rows_too_long_for_the_device_packer_go_to_the_host_packer(monkeypatch, K):
+    from if_i_could_turn_back_time_b200 import _lib, pack
+
+    class OnDevice(torch.Tensor):
+        is_cuda = property(lambda self: True)
+
+    seen = []
+    monkeypatch.setattr(pack, "_pack_gf4_cuda", lambda W, spec, rotate: seen.append(W.shape[1]))
+    W = torch.round(torch.randn(1, K, generator=torch.Generator().manual_seed(K)) * 4) / 4
+    spec = jq.QuantSpec("gf4", 0, 0)
+    got = jq.pack_weight(W.as_subclass(OnDevice), spec)
+    lib, one = _lib.load(), 256
+    refused = lib.jq_pack_gf4(one, 1, K, 0, one, None, one, one, 0, None)      # the entry's own limit, before it looks at the scratch
+    if K <= 32768:
+        assert seen == [K] and refused == -6
+    else:
+        assert not seen and refused == -5
+        want = jq.pack_weight(W, spec)
+        assert torch.equal(got.qweight, want.qweight) and torch.equal(got.codebook, want.codebook)
