@@ -272,6 +272,7 @@ def conv2d(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor], kern
     _need_cuda(x, pw.qweight, pw.scales, pw.codebook, bias)
     if bias is not None and bias.dtype != torch.float32:
         bias = bias.float()
+    x = x.resolve_neg()        # (the imaginary part of a conjugate is a view whose sign is not in memory)
     L = ho * wo
     y = torch.empty((B * L, pw.N), dtype=x.dtype, device=x.device)
     part = max(1, MAX_ROWS_SCRATCH // ((pw.K + 127) // 128 * 256) // L)          # images at once

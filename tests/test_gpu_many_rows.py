@@ -199,3 +199,10 @@ def test_convolution_with_group_scales():
         y = q(x)
         ref = torch.nn.functional.conv2d(x.double(), q.dequantized_weight().double(), q.bias.double(), padding=1)
         assert (y.double() - ref).abs().max() <= TOL * ref.abs().max()
+
+
+def test_convolution_of_a_lazily_negated_image():
+    q = jq.JenksQuantConv2d(torch.nn.Conv2d(6, 8, 3, padding=1), 4).to(DEV)
+    x = torch.randn(2, 6, 9, 9, dtype=torch.complex64, device=DEV).conj().imag
+    assert x.is_neg()
+    assert torch.equal(q(x), q(x + 0.0))
