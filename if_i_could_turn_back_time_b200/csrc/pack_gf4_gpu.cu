@@ -203,7 +203,9 @@ struct Dp {
         double low = __longlong_as_double(0x7ff0000000000000LL), limit = low;
         int pos = -1;
         bool several = false;             // more than one candidate may be the minimum
-        for (int tb = t0 + first; tb <= t1; tb += kAhead * step) {
+        const bool one_each = kAhead > 1 && t1 - t0 < step;        // a candidate per lane needs no estimate
+        if (one_each && t0 + first <= t1) pos = t0 + first;
+        for (int tb = one_each ? t1 + 1 : t0 + first; tb <= t1; tb += kAhead * step) {
             double e[kAhead];
 #pragma unroll
             for (int i = 0; i < kAhead; ++i) e[i] = estimate(prev, min(tb + i * step, t1), p1, p2, cm);
