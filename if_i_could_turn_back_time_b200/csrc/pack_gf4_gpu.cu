@@ -189,10 +189,9 @@ struct Dp {
     }
     // the same with the reciprocal of the count rounded first
     __device__ __forceinline__ double estimate(const double *prev, int t, double p1, double p2, int cm) const {
-        const int i = t;
-        const double d1 = __dsub_rn(p1, P1[i]), d2 = __dsub_rn(p2, P2[i]);
-        const double q = __dmul_rn(__dmul_rn(d1, d1), recip[(cm - count(t))]);
-        return __dadd_rn(prev[i], __dsub_rn(d2, q));
+        const double d1 = __dsub_rn(p1, P1[t]), d2 = __dsub_rn(p2, P2[t]);
+        const double q = __dmul_rn(__dmul_rn(d1, d1), recip[cm - count(t)]);
+        return __dadd_rn(prev[t], __dsub_rn(d2, q));
     }
     // first minimum of prev[t] + cost(t, mid) over t = t0 + first, t0 + first + step, ... <= t1; kAhead estimates at a
     // time hide each other's latency
