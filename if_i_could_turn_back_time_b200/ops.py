@@ -144,6 +144,12 @@ def set_checked(on: bool) -> None:
     _checked = bool(on)
 
 
+def _capturing(stream: int) -> bool:
+    """Whether a graph is being captured on the current stream.  The legacy default stream (0) cannot be captured, and
+    calls on it save the 0.4 us that asking takes."""
+    return stream != 0 and torch.cuda.is_current_stream_capturing()
+
+
 def _workspace(device, nbytes: int, kind: str = "gemv") -> torch.Tensor:
     """Grow-only scratch per (device, stream, kernel family): calls on one
     stream are ordered, so consecutive calls may share it; another stream gets
@@ -162,7 +168,7 @@ def _workspace(device, nbytes: int, kind: str = "gemv") -> torch.Tensor:
         least = 2 * t.numel() if t is not None and t.data_ptr() in _captured else _LEAST_SCRATCH[kind]
         t = torch.zeros(max(nbytes, least), dtype=torch.uint8, device=device)
         cache[key] = t
-    if torch.cuda.is_current_stream_capturing():
+    if _capturing(key[1]):
         _captured[t.data_ptr()] = t
     return t
 
@@ -223,7 +229,7 @@ def _rows_scratch(device, nbytes: int):
     fits into it as it is, an allocation of the call's own otherwise, and always while a graph is captured (from the
     graph's pool: graphs that were captured on one stream may replay on several).  The status word is the buffer's."""
     ws = _workspace(device, 1024, "ta")
-    if ws.numel() >= 1024 + nbytes and not torch.cuda.is_current_stream_capturing():
+    if ws.numel() >= 1024 + nbytes and not _capturing(_stream()):
         return None, ws.data_ptr() + 1024, ws.numel() - 1024, ws.data_ptr()
     own = torch.empty(nbytes, dtype=torch.uint8, device=device)
     return own, own.data_ptr(), nbytes, ws.data_ptr()
