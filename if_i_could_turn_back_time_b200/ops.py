@@ -120,9 +120,9 @@ def many_rows(fmt_id: int, K: int, g: int, batch: int) -> bool:
     return batch > 16
 
 
-# Smallest scratch buffer of a kernel family.  "ta": one pass of 64 rows of up to 32000 codes, so that calls on a stream
+# Smallest scratch buffer of a kernel family, 1 MB if not named here.  "ta": one pass of 64 rows of up to 32000 codes, so that calls on a stream
 # that has made one, in a graph capture too, do not need a larger one.
-_LEAST_SCRATCH = {"ta": 4 << 20, "gemv": 1 << 20}
+_LEAST_SCRATCH = {"ta": 4 << 20}
 _tls = threading.local()   # every host thread has its own scratch buffers: calls from different threads never share one
 _captured = {}             # address -> buffer that a graph capture has used: the graph replays into it, so it is never freed
 _checked = False
@@ -165,7 +165,7 @@ def _workspace(device, nbytes: int, kind: str = "gemv") -> torch.Tensor:
     if t is None or t.numel() < nbytes:
         if t is not None and kind != "gemv" and check_status(raise_on_error=False):
             raise RuntimeError("a device-side wait gave up in an earlier call (status word raised)")
-        least = 2 * t.numel() if t is not None and t.data_ptr() in _captured else _LEAST_SCRATCH[kind]
+        least = 2 * t.numel() if t is not None and t.data_ptr() in _captured else _LEAST_SCRATCH.get(kind, 1 << 20)
         t = torch.zeros(max(nbytes, least), dtype=torch.uint8, device=device)
         cache[key] = t
     if _capturing(key[1]):
