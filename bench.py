@@ -51,8 +51,8 @@ PARITY_GATE = 1e-3
 # algorithmic bytes.
 DRAM_TRAFFIC_RATIO = {
     "gf4_lut2_kernel": (377.961216 + 5.431552) / 378.101760,
-    "gemm_ta_kernel<gf4>": (380.471808 + 8.067328) / 385.351680,
-    "gemm_ta_kernel<e2m1>": (621.232640 + 6.949376) / 612.368384,
+    "gemm_ta_kernel<gf4>": (379.913984 + 7.676416) / 385.351680,
+    "gemm_ta_kernel<e2m1>": (621.605632 + 6.630912) / 612.368384,
     "gemv_grouped_kernel": 608.581888 / 604.504064,      # E2M1; GF4 reaches this kernel only for ungrouped or short rows
 }
 

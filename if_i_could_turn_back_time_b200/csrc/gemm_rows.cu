@@ -1,5 +1,5 @@
 // Packed 4-bit weights x many activation rows (prompts, evaluation batches, convolutions) on the 5th-generation
-// tensor cores (sm_100a): every weight is decoded once per 256 activation rows instead of once per 16.
+// tensor cores (sm_100a): every weight is decoded once per 256 activation rows.
 //
 // A CTA computes a tile of 128 weight rows x NT <= 256 activation rows ("tokens"), D = W . X^T:
 //   * warps 0-3 decode: thread = weight row = tensor-memory lane.  The packed codes of a warp's 32 rows arrive by TMA
@@ -15,11 +15,12 @@
 //
 // What bounds it: at NT = 256 a 128-code group is 1024 clocks of tensor pipe; decoding it takes about 670 clocks of the
 // ALU pipe (GF4, 21 operations per 8 codes) and the folding 256 issue slots per scheduler, both beside the MMAs.  Measured,
-// the one decode warp of a scheduler is bound by the latency of its own chain, not by either pipe (ALU 32 %, tensor 38 %
-// busy): 11008 x 4096 GF4, 2048 rows: 249 us (745 TFLOP/s; passes of 16 rows took 2848), 8192 x 8192 E2M1, 777 rows: 148 us
-// (705 TFLOP/s; 639).  Two decode warps per scheduler with tiles of 192 rows, which is what the registers allow, took 277 and
-// 185 us.  A pair table in shared memory (as in gemm_ta.cu) would save ALU work, but its lookups, the 64 KB of activations
-// per group that land in shared memory and the MMA's own reads together exceed the shared-memory bandwidth.
+// the one decode warp of a scheduler is bound by the latency of its own chain, not by a pipe:
+//   11008 x 4096 GF4, 2048 rows:  247 us, 749 TFLOP/s (passes of 16 rows took 2868); ALU 38 %, tensor 46 %, issue 40 % busy
+//   8192 x 8192 E2M1, 777 rows:   149 us, 701 TFLOP/s (passes of 64 rows took 646);  ALU 14 %, tensor 51 %, issue 31 %
+// Two decode warps per scheduler with tiles of 192 rows, which is what the registers allow, took 277 and 185 us.  A pair
+// table in shared memory (as in gemm_ta.cu) would save ALU work, but its lookups, the 64 KB of activations per group that
+// land in shared memory and the MMA's own reads together exceed the shared-memory bandwidth.
 //
 // A call with few tiles splits K over the CTAs of a cluster (up to 8); the partial sums meet through distributed
 // shared memory and are added in rank order.
@@ -522,7 +523,8 @@ __global__ void __launch_bounds__(256) rows_prepare_kernel(const __grid_constant
 // lane = output position, so loads of one tap and stores of one 8-code piece are consecutive over the warp.  Bound by the
 // index arithmetic of the gathering, so a block that can keep its 32 fields in shared memory (96 KB: K up to 768, two
 // blocks per SM) gathers once; longer ones gather again for the second pass.  64 -> 128 channels, 3x3, 16 images of 32 x 32,
-// the whole call: 57 us gathering twice, 41 us gathering once.
+// the whole call: 57 us gathering twice, 41 us gathering once.  Its time grows with K, not with the positions, until the
+// blocks fill the chip (K = 4608: 159 us for 25 to 784 positions): long fields at few positions are not for this kernel.
 constexpr int kFieldBytes = 96 * 1024;
 struct ConvArgs {
     const void *x;             // element (b, c, h, w) at b sb + c sc + h sr + w sx

@@ -70,7 +70,7 @@ struct PeerInfo {
 // One block per (problem, batch row): x -> (x 2^-e) -> block Hadamard -> fp16, written as
 // [8-code piece][batch row][8 halves].  Copied to shared memory as it is, this is the K-major operand
 // layout of the MMA with a piece stride of 16 B bytes: row n of piece c sits at (c B + n) 16 bytes.  The MMA
-// always reads 16 rows; rows >= B are whatever follows (the next pieces), and their accumulator columns
+// reads 16, 32 or 64 rows; rows >= B are whatever follows (the next pieces), and their accumulator columns
 // are never read.
 // The second pass is a chain of load -> rotate -> store per 128-element block and warp, and its latency is what a
 // decode step waits for before the main kernel can start.  With one or two batch rows there are few blocks: 32 warps
@@ -688,9 +688,11 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
 // activation values, which they read as broadcast 16-byte shared-memory loads (one wavefront per eight
 // codes) from the prepared activation of the whole problem, and a looked-up pair feeds two
 // fma.rn.f32.f16 (fp16 x fp16 exact, fp32 accumulation).  Per 128-code group the partial sum is scaled by
-// the group's fp16 scale in fp32.  At batch 1 this costs about 2.2 instructions and 0.75 shared-memory
-// wavefronts per code, where one 16-bit lookup per code costs 1.2 wavefronts; the tensor pipe, whose
-// K = 16 instructions have a floor of about 45 clocks whatever the batch, is not involved.
+// the group's fp16 scale in fp32.  At batch 1 the loop costs about 2.2 instructions and 0.75 shared-memory
+// wavefronts per code of a warp, where one 16-bit lookup per code costs 1.2 wavefronts; a whole launch 1.17
+// (tables, partial sums and syncs 0.25, global loads 0.17, most of them the scales' 2-byte loads), with the
+// LSU data pipe 74 % busy (11008 x 4096, 122 us for 16); the tensor pipe, whose K = 16 instructions have a
+// floor of about 45 clocks whatever the batch, is not involved.
 // Per code a lane receives 2 bytes of looked-up pairs, 0.5 of packed weights and 2 of activations through
 // the shared-memory pipe (128 bytes per clock and SM).  A variant whose lanes carry two rows each and read
 // the activations once for both (8 warps instead of 16, same tables and ring) was slower: 950 against 1022

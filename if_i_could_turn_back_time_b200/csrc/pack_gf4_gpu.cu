@@ -23,8 +23,10 @@
 // row.  A candidate's cost has a division (some 20 float64 operations); it is estimated with a table of reciprocals
 // first (6 operations), and only a thread's candidates within the estimate's error bound of its smallest are computed
 // exactly, normally one.  The ranges of a level add up to K, but one node's can be most of it (weights with outliers): left
-// to the node's own lanes, the longest range set the pace.  4096 x 4096: 92.7 ms with queues of nodes in global memory, one
-// warp per node; 27.8 ms like this.  (Doubles permuted against bank conflicts: 30.8 ms, the index arithmetic costs more.)
+// to the node's own lanes, the longest range set the pace.  Measured: issue slots 54 %, float64 pipe 17 % busy, waits at
+// the level barriers the top stall.  4096 x 4096: 92.3 ms with queues of nodes in global memory, one warp per node; 26.9 ms
+// like this.  (Doubles permuted against bank conflicts: 30.8 ms, the index arithmetic costs more.  Costs compared as
+// integers in the reductions over lanes: 0 to 3 % slower.)
 #include "common.cuh"
 #include <cfloat>
 
