@@ -3,9 +3,9 @@
 //
 // One persistent CTA per SM works through 128-row tiles of the weight matrices.
 // A decode thread owns one weight row of the tile (= one tensor-memory lane)
-// and one half of the 256-code steps of that row:
-//   * the packed codes of a warp's 32 rows arrive by TMA (cp.async.bulk.tensor,
-//     one 32-row x 128-byte box per step with the 128-byte swizzle, completion
+// and every fourth 128-code group of that row:
+//   * the packed codes of the tile arrive by TMA (cp.async.bulk.tensor, one
+//     128-row x 128-byte box per 256 codes with the 128-byte swizzle, completion
 //     counted on an mbarrier), so that every lane reads its own row without
 //     bank conflicts;
 //   * GF4: a byte (two codes) indexes the row's 256-entry table of fp16 pairs,
@@ -17,18 +17,15 @@
 //   * the fp16 values go to tensor memory with tcgen05.st as the A operand
 //     (M = 128 rows, K = 16 per instruction) of tcgen05.mma kind::f16; the B
 //     operand is the prepared activation (rotated, normalised by a power of
-//     two, fp16, in the K-major core-matrix layout) that each MMA-issuing
-//     warp streams from global memory into a ring of its own, one 128-code
-//     chunk per bulk copy;
+//     two, fp16, in the K-major core-matrix layout), streamed from global
+//     memory, one 128-code chunk per bulk copy;
 //   * every 128-code group has an fp32 accumulator in tensor memory; fold
 //     threads read it back with tcgen05.ld and, for GF4, apply the group's fp16
 //     scale in fp32, so every product and every scale stays exact (the results
 //     differ from the FMA kernels only in summation order).  E2M1 folds its
 //     scales into the fp16 weights (one rounding per weight).
 // The multiply-accumulate work thus costs the CUDA cores nothing, whatever the
-// batch (up to 64 columns per pass), and the lookups are halved.  7B-shaped GF4
-// stack, 8 rows: 1162 us with decoding, folding and outputs in the same threads,
-// 1034 us with the roles below.
+// batch (up to 64 columns per pass), and the lookups are halved.
 //
 // Every wait on an mbarrier is bounded: on expiry the CTA raises a status word
 // in the workspace, all roles leave their loops, tensor memory is freed and
@@ -38,10 +35,8 @@
 
 namespace jqta {
 
-constexpr int kDecodeWarps = 8;              // warps 0-3: first half of the steps, warps 4-7: second half
 constexpr int kTileM = 128;
-constexpr int kWStage = 32 * 128;            // bytes of a weight stage: 32 rows x 128 bytes (256 codes), swizzled by TMA
-constexpr int kXMaxStages = 8;               // stages of an MMA issuer's activation ring, at most
+constexpr int kWStage = kTileM * 128;        // bytes of a weight stage: 128 rows x 128 bytes (256 codes), swizzled by TMA
 constexpr int kTabBytes = 4 * 256 * 128;     // GF4, up to 16 rows: 256 entries x 32 lanes x 4 bytes per 32-row quarter
 constexpr int kHeaderBytes = 1024;           // workspace: int status
 
@@ -117,63 +112,58 @@ __global__ void __launch_bounds__(kPrepThreads) ta_prepare_kernel(const TaProble
 }
 
 // ---- main kernel --------------------------------------------------------------------
-// Roles of a CTA (16 warps): warps 0-7 decode (warp = 32-row quarter q of the tile x half h of the 256-code
-// steps of a row: step sg belongs to half sg & 1); warps 8-11 fold (thread = row): they read every 128-code group's
-// accumulator back, add it, times the group's scale, to the row's fp32 sums, and write the outputs; warps
-// 12-15 issue MMAs (two issuers per half: a thread cannot issue a tcgen05.mma more often than every 50 clocks, threads
-// of different warps can) and stream the prepared activation of their own groups; warp 15 also owns the tensor-memory
-// allocation.
+// Roles of a CTA (24 warps): warps 0-15 decode (warp = 32-row quarter q of the tile x phase ph: the CTA's 128-code groups are
+// numbered through, phase ph takes groups t = ph, ph + 4, ...); warps 16-19 fold (thread = row): they read every group's
+// accumulator back, add it, times the group's scale, to the row's fp32 sums, and write the outputs; warps 20 and 21 issue
+// the MMAs of the even and the odd groups (two issuers reach 14 clocks per MMA of 16 columns, one 27); warp 22 streams the
+// prepared activation, warp 23 the packed rows, and owns the tensor memory.
 //
-// Tensor-memory columns: kRing slots per half of 64 columns each for the A operand (one 128-code group) and kAccBufs
-// accumulators of NB columns per issuer.
+// Tensor-memory columns: kSlots operand slots of 64 columns (one 128-code group each, group t in slot t mod kSlots) and
+// kAccs accumulators of NB columns (group t in t mod kAccs).  An activation stage belongs to the operand slot of its group.
 //
-// The decode threads bound the kernel, so everything else is kept off them.  (When they also folded the accumulators,
-// exchanged the halves' sums and wrote the outputs, they were decoding for 60 % of a tile.)  GF4 up to 16 rows looks
-// every byte up in the pair table; sending words through byte permutes on the ALU instead (tc.cuh, Codebook) to relieve
-// the shared-memory pipe costs more issue slots than it saves (7B-shaped step, 8 rows: none 1050 us, one word of four
-// 1086, two 1200).  From 17 rows on there is no shared memory for tables beside the activation rings, and all words go
-// through the permutes.
+// What bounds it: neither a pipe nor the decode warps alone.  7B-shaped GF4 step, 8 rows (70B-shaped E2M1, 7 layers, 16 rows),
+// 8 decode warps before: 1053 us (889); now 969 (876).  With the lookups left out 801 (778), with one MMA of eight 857 (811),
+// without folding no change; nothing but the barriers, the loads and a quarter of the stores 720 (725).  Barrier operations
+// are a large part of what is left (a ready wait with its vote takes 105 clocks, an elected arrival 50 to 70): operand slots of
+// half a group, which are busy for a shorter time, were slower (953 against 928 us on one GPU), one issuer and one slot per
+// phase too (939).
+// GF4 up to 16 rows looks every byte up in the pair table.  From 17 rows on there is no shared memory for tables beside the
+// activation stages, and all words go through byte permutes.
 //
 // A row's sum is formed in four parts of K (one, for short rows and for 33 rows and more), each in group order, added in
 // part order.  A single call with few tiles lets the CTAs of a cluster take the parts; the partial sums meet in
 // distributed shared memory and are added in the same order, so the result does not depend on the split.
-constexpr int kTaThreads = 16 * 32;
+constexpr int kTaThreads = 24 * 32;
+constexpr int kSlots = 6;
 constexpr int kPartMinSteps = 8;                                    // 256-code steps from which a row is summed in parts
 template <int FMT, int NB>
 struct Cols {
     static constexpr bool kTable = FMT == JQ_FMT_GF4 && NB == 16;   // pair tables in shared memory
-    static constexpr int kRing = NB == 16 ? 3 : 2;                  // groups a half may have in flight
-    static constexpr int kAccBufs = NB == 64 ? 1 : 2;               // accumulators of an issuer
-    static constexpr int kAcc = 2 * kRing * 64;                     // accumulator b of issuer i at kAcc + (i * kAccBufs + b) * NB
+    static constexpr int kAcc = kSlots * 64;                        // first column of the accumulators
+    static constexpr int kAccs = 128 / NB;
+    static constexpr int kPer = NB == 64 ? 1 : 2;                   // accumulators that are handed over together
+    static constexpr int kAccBars = kAccs / kPer;
     static constexpr int kParts = NB == 64 ? 1 : 4;
-    static_assert(kAcc + 4 * kAccBufs * NB <= 512, "tensor memory");
-    // one barrier per accumulator says that a group's MMAs are done, to the fold threads and to the decode threads that
-    // wait for the group's slot; before a slot's next group is written, no later group can have used the accumulator
-    static_assert(2 * kAccBufs >= kRing, "the barrier would be a phase ahead");
+    // registers of a fold thread, of an issue / load thread; the decode threads have 72: 61440 in all, what 768 threads
+    // start with at 80
+    static constexpr int kFoldRegs = NB == 16 ? 112 : (NB == 32 ? 128 : 136), kAuxRegs = NB == 16 ? 80 : (NB == 32 ? 64 : 56);
+    static_assert(512 * 72 + 128 * (kFoldRegs + kAuxRegs) <= 80 * kTaThreads, "registers");
+    static_assert(kAcc + kAccs * NB <= 512, "tensor memory");
 };
 
-template <bool TABLE>
+template <bool TABLE, int NB>
 struct Smem {
     static constexpr int kTab = 0;
     static constexpr int kWRing = TABLE ? kTabBytes : 0;
-    static constexpr int kSW = 2;       // stages of a decode warp's weight ring (four did not change anything: the ring is not what the decode threads wait for)
-    static constexpr int kXRing = kWRing + kDecodeWarps * kSW * kWStage;
-    static constexpr int kXBytes = TABLE ? 32 * 1024 : 152 * 1024;  // without tables: two stages of 64 batch rows per issuer
-    static constexpr int kBars = kXRing + kXBytes + 512;            // + what the MMA reads past the last chunk (rows >= B)
-    static constexpr int kNumBars = kDecodeWarps * kSW + 6 + 2 * 8 + 4 * kXMaxStages + 4;   // weights, A full, accumulator full/free, x full per issuer, quarter sync
+    static constexpr int kWs = TABLE ? 4 : (NB == 64 ? 6 : 8);      // weight stages (even: a decode warp takes every other one)
+    static constexpr int kXRing = kWRing + kWs * kWStage;
+    static constexpr int kXStage = 256 * NB;                        // one group of up to NB rows
+    static constexpr int kBars = kXRing + kSlots * kXStage;
+    static constexpr int kNumBars = 2 * 8 + 3 * kSlots + 2 * 8 + 4;
     static constexpr int kBytes = kBars + kNumBars * 8 + 1024;      // + slack for the 1 KB alignment of the base (TMA swizzle)
     static constexpr int kExch = TABLE ? kTab : kXRing;             // K split: partial sums, once nothing else uses the region
     static_assert(kBytes <= 227 * 1024, "shared memory");
-};
-
-// geometry of an issuer's activation ring for a batch of B rows: a stage is one group (128 codes), 256 B bytes
-struct XGeom {
-    int chunk, ring, nstages;
-    __host__ __device__ XGeom(int B, int ring_bytes) {
-        chunk = 256 * B;
-        ring = ring_bytes;
-        nstages = ring_bytes / chunk < kXMaxStages ? ring_bytes / chunk : kXMaxStages;
-    }
+    static_assert(NB == 64 || TABLE || 2 * NB * 512 <= kSlots * kXStage, "exchange");
 };
 
 // first step of part i of a row of nsteps 256-code steps
@@ -186,40 +176,33 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                                                                 const int *tile_start, const int *cta_first,
                                                                 int B, int y_dtype, PeerInfo peers, int split, int *status) {
     using C = Cols<FMT, NB>;
-    using S = Smem<C::kTable>;
+    using S = Smem<C::kTable, NB>;
     constexpr bool kGf4 = FMT == JQ_FMT_GF4;
-    constexpr int kRing = C::kRing;
-    constexpr int kSW = S::kSW;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint32_t s_tmem;
     __shared__ int s_err;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (uniform for the compiler)
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bars = sbase + S::kBars;
-    constexpr int kB0 = kDecodeWarps * kSW;
-    auto wbar = [&](int w, int s) { return bars + 8u * (w * kSW + s); };
-    auto abar = [&](int h, int s) { return bars + 8u * (kB0 + h * 3 + s); };                  // operand slot written
-    auto dbar = [&](int iss, int b) { return bars + 8u * (kB0 + 6 + iss * 2 + b); };          // accumulator complete: a group's MMAs are done
-    auto ebar = [&](int iss, int b) { return bars + 8u * (kB0 + 14 + iss * 2 + b); };         // accumulator folded
-    auto xbar = [&](int iss, int s) { return bars + 8u * (kB0 + 22 + iss * kXMaxStages + s); };   // issuer's stage filled
-    auto qbar = [&](int q) { return bars + 8u * (kB0 + 22 + 4 * kXMaxStages + q); };
+    auto wfull = [&](int s) { return bars + 8u * s; };                                  // packed rows of a step landed
+    auto wempty = [&](int s) { return bars + 8u * (8 + s); };                           // and read by the eight warps
+    auto afull = [&](int s) { return bars + 8u * (16 + s); };                           // operand slot written
+    auto sfree = [&](int s) { return bars + 8u * (16 + kSlots + s); };                  // its MMAs are done (activation stage too)
+    auto xfull = [&](int s) { return bars + 8u * (16 + 2 * kSlots + s); };              // activation stage landed
+    auto dfull = [&](int a) { return bars + 8u * (16 + 3 * kSlots + a); };              // accumulators complete
+    auto dfree = [&](int a) { return bars + 8u * (24 + 3 * kSlots + a); };              // accumulators read
+    auto qbar = [&](int q) { return bars + 8u * (32 + 3 * kSlots + q); };
     volatile int *err = &s_err;
-    const XGeom xg(B, S::kXBytes / 4);
 
     if (tid == 0) {
         s_err = 0;
-        for (int w = 0; w < kDecodeWarps; ++w)
-            for (int s = 0; s < kSW; ++s) mbar_init(wbar(w, s), 1);     // one arrive.expect_tx per fill
-        for (int h = 0; h < 2; ++h)
-            for (int s = 0; s < 3; ++s) mbar_init(abar(h, s), 128);     // the 128 decode threads of the half
-        for (int i = 0; i < 4; ++i)
-            for (int b = 0; b < 2; ++b) { mbar_init(dbar(i, b), 1); mbar_init(ebar(i, b), 128); }
-        for (int i = 0; i < 4; ++i)
-            for (int s = 0; s < kXMaxStages; ++s) mbar_init(xbar(i, s), 1);
-        for (int q = 0; q < 4; ++q) mbar_init(qbar(q), 64);             // the two warps that share a quarter of the rows
+        for (int s = 0; s < S::kWs; ++s) { mbar_init(wfull(s), 1); mbar_init(wempty(s), 8); }
+        for (int s = 0; s < kSlots; ++s) { mbar_init(afull(s), 4); mbar_init(sfree(s), 1); mbar_init(xfull(s), 1); }
+        for (int a = 0; a < C::kAccBars; ++a) { mbar_init(dfull(a), C::kPer); mbar_init(dfree(a), 4); }
+        for (int q = 0; q < 4; ++q) mbar_init(qbar(q), 4);             // the warps that share a quarter of the rows
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 15) {
+    if (warp == 23) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -262,55 +245,21 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
         p = probs[pi];
         t_end = tile_start[pi + 1];
     };
+    auto warp_wait = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)); };
+    auto warp_arrive = [&](uint32_t bar) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar);
+    };
 
-    if (warp < kDecodeWarps) {
-        // =============================== decode threads ===============================
-        if constexpr (NB > 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");     // 256 x 112 + 128 x 184 + 128 x 96 of 65536 registers
-        const int q = warp & 3, h = warp >> 2;
+    if (warp < 16) {
+        // =============================== decode warps ===============================
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+        const int q = warp & 3, ph = warp >> 2, gi = ph & 1;
         const int r = q * 32 + lane;                       // row of the tile = tensor-memory lane
         const uint32_t lane_t = tmem + ((uint32_t)(q * 32) << 16);
         const uint32_t tcol = sbase + S::kTab + q * (256 * 128) + lane * 4;   // pair table: entry e of this row at tcol + 128 e
-        const uint32_t wring = sbase + S::kWRing + warp * (kSW * kWStage);     // + stage * kWStage; 1 KB aligned
-        // 16-byte piece c of this lane's row sits at piece c ^ (lane & 7) of the row (128-byte swizzle)
-        const uint32_t lrow = lane * 128, lkey = (lane & 7) << 4;
-
-        // ---- producer side of the weight ring: the (tile, step) whose box is requested next
-        int i_tile = tile_lo, i_pi = 0, i_tend = -1, i_j = 0, i_n = 0, i_x = 0, i_x0 = 0, i_y = 0, i_tile0 = 0, i_steps = 0, i_stage = 0;
-        const void *i_map = nullptr;
-        auto i_open = [&]() {
-            while (i_tile < tile_hi) {
-                if (i_tile >= i_tend) {
-                    TaProblem p;
-                    problem_at(i_pi, i_tend, i_tile, p);
-                    const int ns = p.K >> 8, lo = step_lo(ns);
-                    i_steps = (step_hi(ns) - lo - h + 1) >> 1;
-                    i_x0 = (lo + h) * 128;
-                    i_tile0 = p.tile0;
-                    i_map = nprob ? &maps[i_pi] : &single_map;
-                }
-                i_n = i_steps;
-                i_x = i_x0;
-                i_y = (i_tile - i_tile0) * kTileM + q * 32;     // rows past N read as zeros
-                i_j = 0;
-                if (i_n > 0) return;
-                ++i_tile;
-            }
-        };
-        auto issue = [&]() {
-            if (i_tile < tile_hi) {
-                if (lane == 0) {
-                    const uint32_t bar = wbar(warp, i_stage);
-                    mbar_expect_tx(bar, kWStage);
-                    tma_2d_g2s(wring + i_stage * kWStage, i_map, i_x, i_y, bar);
-                }
-                i_x += 256;
-                if (++i_j == i_n) { ++i_tile; i_open(); }
-            }
-            i_stage = (i_stage + 1 == kSW) ? 0 : i_stage + 1;
-        };
-        i_open();
-#pragma unroll
-        for (int s = 0; s < kSW; ++s) issue();
+        // this row's 64 bytes of the group: 16-byte piece c of a row sits at piece c ^ (row & 7) (128-byte swizzle)
+        const uint32_t wrow = sbase + S::kWRing + r * 128, wkey = (lane & 7) << 4;
 
         // ---- per-row side data one tile ahead: GF4 codebook row
         int f_pi = 0, f_tend = -1, f_tile0 = 0, f_N = 1;
@@ -330,50 +279,50 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             }
         };
 
-        // ---- consumer state
-        int w_stage = 0, slot = 0, pend_slot = -1;   // pend_slot: its tensor-memory stores are issued but not yet handed over
-        uint32_t w_par = 0;
-        uint32_t t_next = 0;                         // groups this half has decoded so far
-        uint32_t qcount = 0;                         // quarter syncs so far
+        // The CTA's steps are numbered through: step c is in weight stage c mod kWs, its groups are t = 2 c and 2 c + 1.
+        // This warp takes the steps of its parity.
+        int skip = ph >> 1;                          // steps of other warps before this warp's next one (0 or 1)
+        int w_stage = ph >> 1, slot = ph;            // slot of group ph: ph < kSlots
+        uint32_t w_par = 0, s_par = 1;               // (the first use of a slot finds it free)
+        uint32_t q_par = 0;
         Codebook book;
-        auto hand_over = [&]() {
-            if (pend_slot >= 0) {
-                tmem_wait_st();
-                tc_fence_before();
-                mbar_arrive(abar(h, pend_slot));
-                pend_slot = -1;
-            }
-        };
         auto quarter_sync = [&]() -> bool {
-            mbar_arrive(qbar(q));
-            const bool ok = mbar_wait(qbar(q), qcount & 1, err);
-            ++qcount;
+            warp_arrive(qbar(q));
+            const bool ok = warp_wait(qbar(q), q_par);
+            q_par ^= 1;
             return ok;
         };
 
         int c_pi = 0, c_tend = -1;
-        TaProblem p = single;
+        int K = single.K, N = single.N, lds = single.lds, tile0 = 0;
+        const __half *scales = single.scales;
         fetch_codebook(tile_lo);
         bool ok = true;
         for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
-            if (tile >= c_tend) problem_at(c_pi, c_tend, tile, p);
-            const int s_lo = step_lo(p.K >> 8), s_hi = step_hi(p.K >> 8);
-            // E2M1: eight fp16 scales (16 bytes) per 256-code step of the row, a step ahead
-            const int row = min((tile - p.tile0) * kTileM + r, p.N - 1);
-            const uint4 *srow = reinterpret_cast<const uint4 *>(p.scales + (size_t)row * p.lds);
-            uint4 sc_nxt = make_uint4(0, 0, 0, 0);
-            if (!kGf4 && s_lo + h < s_hi) sc_nxt = __ldg(srow + s_lo + h);
+            if (tile >= c_tend) {
+                TaProblem p;
+                problem_at(c_pi, c_tend, tile, p);
+                K = p.K; N = p.N; lds = p.lds; tile0 = p.tile0; scales = p.scales;
+            }
+            const int s_lo = step_lo(K >> 8), s_hi = step_hi(K >> 8);
+            const int s_first = s_lo + skip;
+            skip = (skip + s_hi - s_lo) & 1;         // (s_hi > s_lo)
+            // E2M1: four fp16 scales (8 bytes) per group, one group of this warp ahead
+            const int row = min((tile - tile0) * kTileM + r, N - 1);
+            const uint2 *srow = reinterpret_cast<const uint2 *>(scales + (size_t)row * lds) + gi;
+            uint2 sc_nxt = make_uint2(0, 0);
+            if (!kGf4 && s_first < s_hi) sc_nxt = __ldg(srow + 2 * s_first);
             if constexpr (kGf4 && !C::kTable) book.set(cb0, cb1);
             if constexpr (C::kTable) {
-                // ---- the pair table of this row (this thread fills the entries whose second code is in its half)
-                if (!(ok = quarter_sync())) break;      // both warps are done with the previous tile's lookups
+                // ---- the pair table of this row (this thread fills the entries whose second code is 4 ph .. 4 ph + 3)
+                if (!(ok = quarter_sync())) break;      // the four warps are done with the previous tile's lookups
                 const uint32_t c[8] = {cb0.x, cb0.y, cb0.z, cb0.w, cb1.x, cb1.y, cb1.z, cb1.w};
-                uint32_t ch[4];
+                uint32_t ch[2] = {c[0], c[1]};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) ch[i] = h ? c[4 + i] : c[i];
-                const uint32_t tb = tcol + h * (128 * 128);
+                for (int i = 1; i < 4; ++i) { ch[0] = ph == i ? c[2 * i] : ch[0]; ch[1] = ph == i ? c[2 * i + 1] : ch[1]; }
+                const uint32_t tb = tcol + ph * (64 * 128);
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
+                for (int i = 0; i < 4; ++i)
 #pragma unroll
                     for (int lo = 0; lo < 16; ++lo) {
                         const uint32_t e = __byte_perm(c[lo >> 1], ch[i >> 1],
@@ -383,88 +332,74 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             }
             fetch_codebook(tile + 1);
             if constexpr (C::kTable) { if (!(ok = quarter_sync())) break; }
-            for (int sg = s_lo + h; sg < s_hi; sg += 2) {
-                ok = __all_sync(0xffffffffu, mbar_wait(wbar(warp, w_stage), w_par, err));
-                if (!ok) break;
-                const uint32_t src = wring + w_stage * kWStage + lrow;
-                if (++w_stage == kSW) { w_stage = 0; w_par ^= 1; }
-                const uint4 sc_cur = sc_nxt;
-                if (!kGf4 && sg + 2 < s_hi) sc_nxt = __ldg(srow + sg + 2);
+            for (int sg = s_first; sg < s_hi; sg += 2) {
+                if (!(ok = warp_wait(wfull(w_stage), w_par))) break;
+                const uint32_t src = wrow + w_stage * kWStage;
+                const uint2 sc4 = sc_nxt;
+                if (!kGf4 && sg + 2 < s_hi) sc_nxt = __ldg(srow + 2 * (sg + 2));
+                const uint32_t a_t = lane_t + slot * 64;
+                uint4 w4[4];
 #pragma unroll
-                for (int gi = 0; gi < 2; ++gi) {
-                    const uint2 sc4 = gi ? make_uint2(sc_cur.z, sc_cur.w) : make_uint2(sc_cur.x, sc_cur.y);
-                    const uint32_t a_t = lane_t + (h * kRing + slot) * 64;
-                    uint4 w4[4];
+                for (int part = 0; part < 4; ++part) w4[part] = lds128(src + ((uint32_t)((gi * 4 + part) << 4) ^ wkey));
+                // 32 codes (four words) -> 16 fp16 pairs
+                auto decode16 = [&](int part, uint32_t (&v)[16]) {
 #pragma unroll
-                    for (int part = 0; part < 4; ++part) w4[part] = lds128(src + (((gi * 4 + part) << 4) ^ lkey));
-                    // 32 codes (four words) -> 16 fp16 pairs
-                    auto decode16 = [&](int part, uint32_t (&v)[16]) {
+                    for (int wi = 0; wi < 4; ++wi) {
+                        const uint32_t w = wi == 0 ? w4[part].x : (wi == 1 ? w4[part].y : (wi == 2 ? w4[part].z : w4[part].w));
+                        if constexpr (kGf4) {
+                            if (C::kTable) {
 #pragma unroll
-                        for (int wi = 0; wi < 4; ++wi) {
-                            const uint32_t w = wi == 0 ? w4[part].x : (wi == 1 ? w4[part].y : (wi == 2 ? w4[part].z : w4[part].w));
-                            if constexpr (kGf4) {
-                                if (C::kTable) {
-#pragma unroll
-                                    for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = lds32(dp4a_u(w, 0x80u << (8 * bj), tcol));
-                                } else {
-                                    uint32_t hh[4];
-                                    book.look_up8(w, hh);
-#pragma unroll
-                                    for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = hh[bj];
-                                }
+                                for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = lds32(dp4a_u(w, 0x80u << (8 * bj), tcol));
                             } else {
-                                // E2M1: the group scale folded into the fp16 weight (one rounding per weight)
-                                const uint32_t pr = part < 2 ? sc4.x : sc4.y;
-                                const uint32_t s2 = prmt(pr, pr, (part & 1) ? 0x3232 : 0x1010);
                                 uint32_t hh[4];
-                                asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %4;\n"
-                                    "  cvt.rn.f16x2.e2m1x2 %0, b0; cvt.rn.f16x2.e2m1x2 %1, b1;\n"
-                                    "  cvt.rn.f16x2.e2m1x2 %2, b2; cvt.rn.f16x2.e2m1x2 %3, b3; }"
-                                    : "=r"(hh[0]), "=r"(hh[1]), "=r"(hh[2]), "=r"(hh[3]) : "r"(w));
+                                book.look_up8(w, hh);
 #pragma unroll
-                                for (int bj = 0; bj < 4; ++bj)
-                                    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(v[wi * 4 + bj]) : "r"(hh[bj]), "r"(s2));
+                                for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = hh[bj];
                             }
+                        } else {
+                            // E2M1: the group scale folded into the fp16 weight (one rounding per weight)
+                            const uint32_t pr = part < 2 ? sc4.x : sc4.y;
+                            const uint32_t s2 = prmt(pr, pr, (part & 1) ? 0x3232 : 0x1010);
+                            uint32_t hh[4];
+                            asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %4;\n"
+                                "  cvt.rn.f16x2.e2m1x2 %0, b0; cvt.rn.f16x2.e2m1x2 %1, b1;\n"
+                                "  cvt.rn.f16x2.e2m1x2 %2, b2; cvt.rn.f16x2.e2m1x2 %3, b3; }"
+                                : "=r"(hh[0]), "=r"(hh[1]), "=r"(hh[2]), "=r"(hh[3]) : "r"(w));
+#pragma unroll
+                            for (int bj = 0; bj < 4; ++bj)
+                                asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(v[wi * 4 + bj]) : "r"(hh[bj]), "r"(s2));
                         }
-                    };
-                    // the decode of the next 32 codes is issued before the previous 16 pairs are stored, and the
-                    // previous group is handed to the MMA issuer only once this group's first lookups are under way
-                    // (its tensor-memory stores have had that long to land), and before the wait for this group's slot
-                    uint32_t va[16], vb[16];
-                    decode16(0, va);
-                    decode16(1, vb);
-                    hand_over();
-                    // the slot is free once the MMAs of the group that used it last are done
-                    if (t_next >= (uint32_t)kRing) {
-                        const uint32_t t = t_next - kRing, n = t >> 1;     // group t was its issuer's n-th
-                        ok = __all_sync(0xffffffffu, mbar_wait(dbar(h + 2 * (t & 1), n % C::kAccBufs), (n / C::kAccBufs) & 1, err));
-                        if (!ok) break;
-                        tc_fence_after();
                     }
-                    ++t_next;
-                    tmem_st16(a_t, va);
-                    decode16(2, va);
-                    tmem_st16(a_t + 16, vb);
-                    decode16(3, vb);
-                    tmem_st16(a_t + 32, va);
-                    tmem_st16(a_t + 48, vb);
-                    pend_slot = slot;
-                    if (++slot == kRing) slot = 0;
-                }
-                if (!ok) break;
-                __syncwarp();                           // every lane has read its row of the stage
-                fence_async_smem();
-                issue();                                // refill the stage just read
+                };
+                // half of the group is decoded before the wait for its slot, the rest while the first pairs are being stored;
+                // handed over at once (kept until the next group's first lookups are under way, which spares a wait for the
+                // stores, a slot is held for longer: 1022 against 953 us for the 7B-shaped GF4 step with 8 rows)
+                uint32_t va[16], vb[16];
+                decode16(0, va);
+                decode16(1, vb);
+                if (!(ok = warp_wait(sfree(slot), s_par))) break;
+                tc_fence_after();
+                tmem_st16(a_t, va);
+                decode16(2, va);
+                tmem_st16(a_t + 16, vb);
+                decode16(3, vb);
+                tmem_st16(a_t + 32, va);
+                tmem_st16(a_t + 48, vb);
+                warp_arrive(wempty(w_stage));
+                tmem_wait_st();
+                tc_fence_before();
+                warp_arrive(afull(slot));
+                if ((slot += 4) >= kSlots) { slot -= kSlots; s_par ^= 1; }
+                if ((w_stage += 2) >= S::kWs) { w_stage -= S::kWs; w_par ^= 1; }
             }
-            hand_over();
         }
         if (split > 1) { __syncwarp(); cluster_sync(); cluster_sync(); }
-    } else if (warp < 12) {
+    } else if (warp < 20) {
         // =============================== fold threads ===============================
-        if constexpr (NB > 16) asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kFoldRegs));
         const int r = tid & 127;
         const uint32_t lane_t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::kAcc;
-        uint32_t counts = 0;                        // steps of each half so far, modulo 4 (two bits each)
+        uint32_t buf = 0, par = 0;                  // accumulators of the next step (or group) and their phase
         int c_pi = 0, c_tend = -1;
         TaProblem p = single;
         pdl_wait();                                 // the row factors of the prepared activation are read below
@@ -475,6 +410,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             const int nsteps = p.K >> 8, parts = parts_of(nsteps), s_lo = step_lo(nsteps), s_hi = step_hi(nsteps);
             const unsigned short *srow = reinterpret_cast<const unsigned short *>(p.scales) + (size_t)row * p.lds;
             const int gshift = kGf4 ? 31 - __clz(p.g >> 7) : 0;   // GF4: log2 of the 128-code groups per scale
+            const bool word = gshift == 0 && ((size_t)p.scales & 3) == 0;
             float xs[(NB + 31) / 32];
 #pragma unroll
             for (int i = 0; i < (NB + 31) / 32; ++i) xs[i] = (lane + 32 * i < B) ? p.xscale[lane + 32 * i] : 0.f;
@@ -485,31 +421,43 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             const uint32_t exch = sbase + S::kExch + r * 4;
             int part = split > 1 ? C::kParts / split * rank : 0, part_end = part_step(nsteps, parts, part + 1);
             bool first = true;
-            unsigned short raw0 = 0, raw1 = 0;
+            // the two scales of a step, a step ahead; in 128-code groups they are one aligned word (K is a multiple of 256)
+            uint32_t raw = 0;
             auto load_scales = [&](int sg) {
-                if (kGf4) { raw0 = __ldg(srow + ((2 * sg) >> gshift)); raw1 = __ldg(srow + ((2 * sg + 1) >> gshift)); }
+                if (kGf4) {
+                    if (word) raw = __ldg(reinterpret_cast<const unsigned int *>(srow + 2 * sg));
+                    else raw = __ldg(srow + ((2 * sg) >> gshift)) | (uint32_t)__ldg(srow + ((2 * sg + 1) >> gshift)) << 16;
+                }
             };
             load_scales(s_lo);
             for (int sg = s_lo; sg < s_hi && ok; ++sg) {
-                const int h = (sg - s_lo) & 1;
-                const uint32_t cnt = (counts >> (2 * h)) & 3;
-                const uint32_t buf = C::kAccBufs == 2 ? cnt & 1 : 0, par = C::kAccBufs == 2 ? cnt >> 1 : cnt & 1;
-                const float sc[2] = {__half2float(__ushort_as_half(raw0)), __half2float(__ushort_as_half(raw1))};
+                const float sc[2] = {__half2float(__ushort_as_half((unsigned short)raw)),
+                                     __half2float(__ushort_as_half((unsigned short)(raw >> 16)))};
                 if (sg + 1 < s_hi) load_scales(sg + 1);
-#pragma unroll
-                for (int gi = 0; gi < 2; ++gi) {
-                    const int iss = h + 2 * gi;
-                    ok = __all_sync(0xffffffffu, mbar_wait(dbar(iss, buf), par, err));
-                    if (!ok) break;
+                if constexpr (NB == 16) {
+                    // both groups of the step at once: the way from the barrier through tensor memory to the release is a
+                    // chain of latencies
+                    if (!(ok = warp_wait(dfull(buf), par))) break;
                     tc_fence_after();
-                    const uint32_t d_t = lane_t + (iss * C::kAccBufs + buf) * NB;
-                    if constexpr (NB == 16) {
-                        uint32_t d[16];
-                        tmem_ld16(d_t, d);
-                        tmem_wait_ld();
+                    uint32_t d0[16], d1[16];
+                    tmem_ld16(lane_t + buf * 2 * NB, d0);
+                    tmem_ld16(lane_t + buf * 2 * NB + NB, d1);
+                    tmem_wait_ld();
+                    tc_fence_before();
+                    warp_arrive(dfree(buf));
 #pragma unroll
-                        for (int i = 0; i < 16; i += 2) fma2(acc[i], acc[i + 1], d[i], d[i + 1], kGf4 ? sc[gi] : 1.f);
-                    } else {
+                    for (int i = 0; i < 16; i += 2) fma2(acc[i], acc[i + 1], d0[i], d0[i + 1], kGf4 ? sc[0] : 1.f);
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) fma2(acc[i], acc[i + 1], d1[i], d1[i + 1], kGf4 ? sc[1] : 1.f);
+                    if (++buf == (uint32_t)C::kAccBars) { buf = 0; par ^= 1; }
+                } else {
+#pragma unroll
+                    for (int gi = 0; gi < 2; ++gi) {
+                        if (gi == 0 || C::kPer == 1) {
+                            if (!(ok = warp_wait(dfull(buf), par))) break;
+                            tc_fence_after();
+                        }
+                        const uint32_t d_t = lane_t + (buf * C::kPer + (C::kPer == 2 ? gi : 0)) * NB;
 #pragma unroll
                         for (int c = 0; c < NB; c += 32) {
                             uint32_t d[32];
@@ -518,12 +466,14 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
 #pragma unroll
                             for (int i = 0; i < 32; i += 2) fma2(acc[c + i], acc[c + i + 1], d[i], d[i + 1], kGf4 ? sc[gi] : 1.f);
                         }
+                        if (gi == 1 || C::kPer == 1) {
+                            tc_fence_before();
+                            warp_arrive(dfree(buf));
+                            if (++buf == (uint32_t)C::kAccBars) { buf = 0; par ^= 1; }
+                        }
                     }
-                    tc_fence_before();
-                    mbar_arrive(ebar(iss, buf));
                 }
                 if (!ok) break;
-                counts = (counts & ~(3u << (2 * h))) | (((cnt + 1) & 3) << (2 * h));
                 if (C::kParts > 1 && sg + 1 == part_end) {      // a part of the row's sum is complete
                     if (split > 1) {        // at most two per CTA: the first waits in `total`, the second stays in `acc`
                         if (first) {
@@ -544,7 +494,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             }
             if constexpr (C::kParts > 1) {
                 if (split > 1) {
-                    // every group of this CTA has been folded: nothing reads the tables or the activation rings any more.
+                    // every group of this CTA has been folded: nothing reads the tables or the activation stages any more.
                     // Each CTA leaves its parts in its shared memory; rank k writes columns k, k + split, ...
                     const int per = C::kParts / split;
 #pragma unroll
@@ -579,94 +529,83 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             }
         }
     } else {
-        // =============================== MMA issuers ===============================
-        // Warps 12, 13: half 0, 1; warps 14, 15: the second issuer per half.  A half's groups alternate between its
-        // issuers (the first group of every 256-code step to one, the second to the other).
-        // Every issuer owns a ring of activation stages (one 128-code group each) that it fills itself, so the
-        // only things it ever waits for are the decode and fold threads and its own earlier work.
-        if constexpr (NB > 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
-        const int h = (warp - 12) & 1, sub = (warp - 12) >> 1, iss = warp - 12;
-        // (the warps run converged, see mma_f16_ts)
-        {
+        if constexpr (C::kAuxRegs < 80) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kAuxRegs));
+        // walk of this CTA's tiles: (tile, its problem, the range of its steps)
+        int pi = 0, t_end = -1, lo = 0, hi = 0;
+        TaProblem p = single;
+        auto open = [&](int tile) {
+            if (tile >= t_end) {
+                problem_at(pi, t_end, tile, p);
+                lo = step_lo(p.K >> 8);
+                hi = step_hi(p.K >> 8);
+            }
+        };
+        bool ok = true;
+        if (warp < 22) {
+            // =============================== MMA issuers ===============================
+            // (the warps run converged, see mma_f16_ts; slots, accumulators and parities are carried along instead of being
+            // divided out of counters, and the operand descriptor is formed once per group)
             const uint32_t elected = elect_one();
-            auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)); };
             constexpr uint32_t idesc = idesc_f16(kTileM, NB);
             const uint32_t lbo = (uint32_t)B * 16;
-            const uint32_t ring = sbase + S::kXRing + iss * xg.ring;
-            // two walks over the same sequence of groups: the loads run ahead of the MMAs
-            struct Walk { int tile, pi, t_end, lo, hi, sg; const unsigned char *xp; };
-            auto open_tile = [&](Walk &w) {
-                while (w.tile < tile_hi) {
-                    if (w.tile >= w.t_end) {
-                        TaProblem p;
-                        problem_at(w.pi, w.t_end, w.tile, p);
-                        w.lo = step_lo(p.K >> 8);
-                        w.hi = step_hi(p.K >> 8);
-                        w.xp = reinterpret_cast<const unsigned char *>(p.xprep);
-                    }
-                    w.sg = w.lo + h;
-                    if (w.sg < w.hi) return;
-                    ++w.tile;
-                }
-            };
-            auto advance = [&](Walk &w) {
-                w.sg += 2;
-                if (w.sg >= w.hi) { ++w.tile; open_tile(w); }
-            };
-            Walk ld = {tile_lo, 0, -1, 0, 0, 0, nullptr};
-            open_tile(ld);
-            Walk mm = ld;
-            // An issuer shares its scheduler with two decode warps, so every instruction of this loop costs several clocks:
-            // ring positions and parities are carried along instead of being divided out of counters, and the operand
-            // descriptor is formed once per group.
-            uint32_t ld_s = 0;                          // stage the next load goes to
-            auto load_next = [&]() {
-                if (ld.tile < tile_hi) {
-                    const int G = 2 * ld.sg + sub;
-                    if (elected) {
-                        mbar_expect_tx(xbar(iss, ld_s), xg.chunk);
-                        bulk_g2s(ring + ld_s * xg.chunk, ld.xp + (size_t)G * xg.chunk, xg.chunk, xbar(iss, ld_s));
-                    }
-                    __syncwarp();
-                    advance(ld);
-                }
-                ld_s = (ld_s + 1 == (uint32_t)xg.nstages) ? 0 : ld_s + 1;
-            };
-            pdl_wait();
-            for (int i = 0; i < xg.nstages; ++i) load_next();
-            bool ok = true;
-            uint32_t cs = 0, cpar = 0;                  // stage and phase parity of the group being multiplied
-            uint32_t slot = (uint32_t)sub % kRing, spar = 0;   // A slot of this issuer's next group (the half's group count t = 2 n + sub)
-            uint32_t db = 0, dpar = 1;                  // accumulator (the first round finds it free)
-            const bool tight = xg.nstages <= C::kAccBufs;
             const uint32_t desc_step = (2 * lbo) >> 4;  // descriptor address field per K = 16 slice
-            for (uint32_t n = 0; mm.tile < tile_hi && ok; ++n) {
-                // a ring with no more stages than accumulators refills the previous group's stage once its MMAs are done
-                if (tight && n > 0) {
-                    if (!(ok = wait(dbar(iss, (n - 1) % C::kAccBufs), ((n - 1) / C::kAccBufs) & 1))) break;
-                    load_next();
-                }
-                // the accumulator's last group has been folded, so its MMAs have read their activation stage: refill that
-                if (!(ok = wait(ebar(iss, db), dpar))) break;
-                if (!tight && n >= (uint32_t)C::kAccBufs) load_next();
-                if (!(ok = wait(xbar(iss, cs), cpar))) break;
-                if (!(ok = wait(abar(h, slot), spar))) break;
-                tc_fence_after();
-                const uint32_t a_t = tmem + (h * kRing + slot) * 64;
-                const uint32_t d_t = tmem + C::kAcc + (iss * C::kAccBufs + db) * NB;
-                const uint64_t desc0 = smem_desc(ring + cs * xg.chunk, lbo, 128);
+            uint32_t slot = warp - 20, s_par = 0, acc = C::kPer == 2 ? 0 : warp - 20, d_par = 1;   // (the first use of an accumulator finds it free)
+            for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
+                open(tile);
+                for (int sg = lo; sg < hi; ++sg) {
+                    if (!(ok = warp_wait(dfree(acc), d_par) && warp_wait(xfull(slot), s_par) && warp_wait(afull(slot), s_par))) break;
+                    tc_fence_after();
+                    const uint32_t a_t = tmem + slot * 64;
+                    const uint32_t d_t = tmem + C::kAcc + (C::kPer == 2 ? 2 * acc + warp - 20 : acc) * NB;
+                    const uint64_t desc0 = smem_desc(sbase + S::kXRing + slot * S::kXStage, lbo, 128);
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    mma_f16_ts(elected, d_t, a_t + 8 * i, desc0 + (uint64_t)(i * desc_step), idesc, i > 0);
-                mma_commit(elected, dbar(iss, db));
-                if (++cs == (uint32_t)xg.nstages) { cs = 0; cpar ^= 1; }
-                if (++db == (uint32_t)C::kAccBufs) { db = 0; dpar ^= 1; }
-                slot += 2;
-                if (slot >= (uint32_t)kRing) { slot -= kRing; spar ^= 1; }
-                advance(mm);
+                    for (int i = 0; i < 8; ++i)
+                        mma_f16_ts(elected, d_t, a_t + 8 * i, desc0 + (uint64_t)(i * desc_step), idesc, i > 0);
+                    mma_commit(elected, sfree(slot));
+                    mma_commit(elected, dfull(acc));
+                    if ((slot += 2) >= (uint32_t)kSlots) { slot -= kSlots; s_par ^= 1; }
+                    if ((acc += 2 / C::kPer) >= (uint32_t)C::kAccBars) { acc -= C::kAccBars; d_par ^= 1; }
+                }
+            }
+        } else if (warp == 22 && lane == 0) {
+            // =============================== activation loader ===============================
+            const uint32_t chunk = 256 * B;
+            uint32_t slot = 0, par = 1;                 // (the first use of a stage finds it free)
+            pdl_wait();
+            for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
+                open(tile);
+                const unsigned char *src = reinterpret_cast<const unsigned char *>(p.xprep) + (size_t)(2 * lo) * chunk;
+                for (int g = 2 * lo; g < 2 * hi; ++g, src += chunk) {
+                    if (!(ok = mbar_wait(sfree(slot), par, err))) break;
+                    mbar_expect_tx(xfull(slot), chunk);
+                    bulk_g2s(sbase + S::kXRing + slot * S::kXStage, src, chunk, xfull(slot));
+                    if (++slot == (uint32_t)kSlots) { slot = 0; par ^= 1; }
+                }
+            }
+        } else if (warp == 23 && lane == 0) {
+            // =============================== weight loader ===============================
+            uint32_t stage = 0, par = 1;
+            for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
+                open(tile);
+                const void *map = nprob ? &maps[pi] : &single_map;
+                const int row0 = (tile - p.tile0) * kTileM;     // rows past N read as zeros
+                if (split == 1) {
+                    // the tile's scales are read in small pieces a step or two ahead, which hides the L2's latency but not
+                    // the memory's: they are one piece of memory (rows of lds scales), fetched into the L2 by one instruction
+                    const size_t a = (size_t)(p.scales + (size_t)row0 * p.lds) & ~(size_t)15;
+                    const uint32_t bytes = (uint32_t)min(kTileM, p.N - row0) * (uint32_t)p.lds * 2u & ~15u;
+                    if (bytes) l2_prefetch(reinterpret_cast<const void *>(a), bytes);
+                }
+                for (int sg = lo; sg < hi; ++sg) {
+                    if (!(ok = mbar_wait(wempty(stage), par, err))) break;
+                    mbar_expect_tx(wfull(stage), kWStage);
+                    tma_2d_g2s(sbase + S::kWRing + stage * kWStage, map, sg * 128, row0, wfull(stage));
+                    if (++stage == (uint32_t)S::kWs) { stage = 0; par ^= 1; }
+                }
             }
         }
-        if (split > 1) { __syncwarp(); cluster_sync(); cluster_sync(); }
+        __syncwarp();
+        if (split > 1) { cluster_sync(); cluster_sync(); }
     }
 
     // ---- teardown
@@ -676,7 +615,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
     tc_fence_before();
     __syncthreads();
     if (tid == 0 && s_err) atomicExch(status, s_err);
-    if (warp == 15) {
+    if (warp == 23) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }
@@ -702,7 +641,7 @@ constexpr int kLutTileM = 32 * kLutQuarters;
 constexpr int kLutSplit = 8;                         // warps that share a row set, each taking every 8th 256-code step
 constexpr int kLutWarps = kLutQuarters * kLutSplit;
 constexpr int kLutThreads = kLutWarps * 32;
-constexpr int kLutStage = kWStage;                   // a weight stage: 32 rows x 128 bytes (two 128-code groups), 128-byte swizzle
+constexpr int kLutStage = 32 * 128;                   // a weight stage: 32 rows x 128 bytes (two 128-code groups), 128-byte swizzle
 constexpr int kLutSW = 2;                            // stages per warp (16 warps x 2 x 4 KB: this TMA pattern streams at 6.5 TB/s when
                                                      // nothing else limits it; 64-byte boxes four deep reached only 4.3 TB/s)
 struct LutSmem {
@@ -1001,10 +940,13 @@ using namespace jqta;
 // largest K, 0, 0, 0],
 // tile_start[n + 1], cta_first[grid + 1], padding to 64 bytes, TaProblem[n], padding to 64 bytes, CUtensorMap[n]
 static const int kTaMagic = 0x4a515441;
-// fixed time per tile / per problem of the partition's cost model, in codes of one row.  Swept on the 7B-shaped
+// fixed time per tile / per problem of the partition's cost model, in codes of one row, for gf4_lut2_kernel.  Swept on the 7B-shaped
 // GF4 step (us per step on one GPU / for an eighth of it): bytes only 940 / 150.5; 384, 2048: 921.5 / 143.0;
 // 768, 4096: 910.1 / 141.3; 1408, 6144: 900.1 / 140.1; 2304, 8192: 943.3 / 143.9.
-static const double kTileCost = 1408, kProblemCost = 6144;
+static const double kLutTileCost = 1408, kLutProblemCost = 6144;
+// The same for the tensor-memory kernel, whose loads and decode warps run across tile boundaries.  7B-shaped GF4 step with 8
+// rows / 70B-shaped E2M1 with 16: 1408, 6144: 923 / 846 us; 700, 3000: 900 / 794; 300, 3000: 901 / 778; 0, 0: 907 / 817.
+static const double kTaTileCost = 400, kTaProblemCost = 3000;
 static const int kTaHeader = 12;
 
 // MMA N
@@ -1013,15 +955,15 @@ static int ta_cols(int B) { return B <= 16 ? 16 : (B <= 32 ? 32 : (B <= 64 ? 64 
 static bool ta_use_lut(int B, int maxK);
 static size_t ta_align(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Tensor map over the packed rows of one matrix: bytes [N rows][ldw], boxes of 32 rows x 128 bytes with the
+// Tensor map over the packed rows of one matrix: bytes [N rows][ldw], boxes of rows x 128 bytes with the
 // 128-byte swizzle; rows past N read as zeros.  The driver entry point is looked up once (no link-time
 // dependency on the driver library).
-static int ta_encode_map(CUtensorMap *out, const void *qw, int N, int ldw) {
+static int ta_encode_map(CUtensorMap *out, const void *qw, int N, int ldw, int rows) {
     ta_encode_fn enc = ta_encoder();
     if (!enc) return JQ_ERR_UNSUPPORTED;
     const cuuint64_t dims[2] = {(cuuint64_t)ldw, (cuuint64_t)N};
     const cuuint64_t strides[1] = {(cuuint64_t)ldw};
-    const cuuint32_t box[2] = {128, 32};
+    const cuuint32_t box[2] = {128, (cuuint32_t)rows};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(qw), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1101,18 +1043,19 @@ extern "C" int jq_ta_plan(int fmt, const jq_problem *ph, int n, int B, void *wor
     for (int i = 0; i < n; ++i) maxK = ph[i].K > maxK ? ph[i].K : maxK;
     const bool lut = fmt == JQ_FMT_GF4 && ta_use_lut(B, maxK);
     const int tile_m = lut ? kLutTileM : kTileM;
+    const double tile_cost = lut ? kLutTileCost : kTaTileCost, problem_cost = lut ? kLutProblemCost : kTaProblemCost;
     tile_start[0] = 0;
     for (int i = 0; i < n; ++i) {
         int st = ta_fill_problem(tp[i], fmt, ph[i], reinterpret_cast<unsigned char *>(workspace_dev), off, B);
         if (st) return st;
         CUtensorMap tm;
-        st = ta_encode_map(&tm, ph[i].qweight, ph[i].N, ph[i].K >> 1);
+        st = ta_encode_map(&tm, ph[i].qweight, ph[i].N, ph[i].K >> 1, lut ? 32 : kTileM);
         if (st) return st;
         memcpy(maps + (size_t)i * sizeof(CUtensorMap), &tm, sizeof(CUtensorMap));
         const int tiles = (ph[i].N + tile_m - 1) / tile_m;
         tp[i].tile0 = tile_start[i];
         tile_start[i + 1] = tile_start[i] + tiles;
-        total += (double)tiles * (ph[i].K + kTileCost) + kProblemCost;
+        total += (double)tiles * (ph[i].K + tile_cost) + problem_cost;
     }
     // contiguous tile ranges of (nearly) equal cost: cut where the running cost passes c * total / grid.  A tile
     // costs its packed bytes plus a fixed part (table build, two syncs, outputs), a problem's first tile also the
@@ -1122,7 +1065,7 @@ extern "C" int jq_ta_plan(int fmt, const jq_problem *ph, int n, int B, void *wor
     cta_first[0] = 0;
     for (int i = 0; i < n; ++i)
         for (int t = tile_start[i]; t < tile_start[i + 1]; ++t) {
-            const double c = ph[i].K + kTileCost + (t == tile_start[i] ? kProblemCost : 0);
+            const double c = ph[i].K + tile_cost + (t == tile_start[i] ? problem_cost : 0);
             while (cta + 1 < grid && acc + 0.5 * c >= total * (cta + 1) / grid) cta_first[++cta] = t;
             acc += c;
         }
@@ -1161,7 +1104,7 @@ static int ta_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, co
     if (s) return s;
     auto kern = gemm_ta_kernel<FMT, NB>;
     using C = Cols<FMT, NB>;
-    constexpr int smem = Smem<C::kTable>::kBytes;
+    constexpr int smem = Smem<C::kTable, NB>::kBytes;
     // A single matrix with few tiles: 4 or 2 CTAs take parts of every row (N = 4096 is 32 tiles for 148 SMs)
     int split = 1;
     if (!nprob && C::kParts == 4 && (single.K >> 8) >= kPartMinSteps)
@@ -1255,13 +1198,14 @@ extern "C" int jq_gemm_ta(int fmt, const void *qweight, const void *scales, cons
     int st = ta_fill_problem(t, fmt, p, reinterpret_cast<unsigned char *>(workspace), off, B);
     if (st) return st;
     CUtensorMap tm;
-    st = ta_encode_map(&tm, qweight, N, K >> 1);
+    const bool lut = fmt == JQ_FMT_GF4 && ta_use_lut(B, K);
+    st = ta_encode_map(&tm, qweight, N, K >> 1, lut ? 32 : kTileM);
     if (st) return st;
     jqta::PeerInfo peers;
     peers.n = 1;
     for (int i = 0; i < 8; ++i) peers.delta[i] = 0;
     int grid = jq_sm_count();
-    const int tile_m = (fmt == JQ_FMT_GF4 && ta_use_lut(B, K)) ? kLutTileM : kTileM;
+    const int tile_m = lut ? kLutTileM : kTileM;
     const int tiles = (N + tile_m - 1) / tile_m;
     if (grid > tiles) grid = tiles;
     return ta_dispatch(fmt, ta_cols(B), K, nullptr, nullptr, t, tm, 0, nullptr, nullptr, grid, B, x_dtype, y_dtype, peers,

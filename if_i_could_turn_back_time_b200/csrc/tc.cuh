@@ -56,6 +56,10 @@ __device__ __forceinline__ void tma_2d_g2s(uint32_t dst, const void *tmap, int x
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar) : "memory");
 }
+// a hint: memory that will be read soon, into the L2 (16-byte aligned, a multiple of 16 bytes)
+__device__ __forceinline__ void l2_prefetch(const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // K-major operand in shared memory without swizzle: 8 rows x 16 bytes are contiguous; lbo = bytes between

@@ -39,3 +39,33 @@ def test_single_calls_groups_and_row_shards_agree(fmt, g, B, N, K):
         assert torch.equal(ops.linear(x.to(DEV).float(), half(1)), y[:, N // 2:2 * (N // 2)])
     else:
         assert (ops.linear(x.to(DEV).float(), pw) - grp.ys[0]).abs().max() <= 3e-6 * grp.ys[0].abs().max()
+
+
+@pytest.mark.parametrize("fmt,g,B", [("gf4", 128, 3), ("gf4", 256, 16), ("gf4", 128, 20), ("gf4", 128, 64), ("e2m1", 32, 16), ("e2m1", 32, 40)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_tiles_of_odd_step_counts_and_scales_off_a_word(fmt, g, B, shift):
+    """Rows of 3 and 5 steps, several tiles per CTA: the warps' turns, the weight stages, the operand slots and the
+    accumulators all run across tile boundaries out of step.  GF4 scales may start at any 2-byte boundary."""
+    import ctypes
+    from if_i_could_turn_back_time_b200 import _lib
+    spec = jq.QuantSpec(fmt, g, 0)
+    gen = torch.Generator("cpu").manual_seed(B)
+    packed = [jq.pack_weight(_weights(N, K, N + K).to(DEV), spec) for N, K in ((20000, 768), (9000, 1280), (18950, 768))]
+    grp = ops.GroupedGemv(packed, B, torch.float32)
+    for x in grp.xs:
+        x.copy_(torch.randn(x.shape, generator=gen))
+    grp.run()
+    assert grp.status() == 0 and grp._ta
+    for w, x, y in zip(packed, grp.xs, grp.ys):
+        # (fp16 rounding of the activation, 2^-12 of a term, and of value x scale for E2M1; sums of at most 1280 terms)
+        ref = x.double() @ ops.dequantize(w).double().t()
+        assert (y - ref).abs().max() <= 1e-3 * ref.abs().max()
+    if fmt == "gf4" and shift:
+        w, x = packed[1], grp.xs[1]
+        raw = torch.empty(w.scales.numel() + 1, dtype=torch.float16, device=DEV)
+        raw[1:] = w.scales.reshape(-1)
+        y, ws = torch.empty_like(grp.ys[1]), torch.zeros(4 << 20, dtype=torch.uint8, device=DEV)
+        p = lambda t, off=0: ctypes.c_void_p(t.data_ptr() + off)
+        _lib.check(_lib.load().jq_gemm_ta(w.spec.fmt_id, p(w.qweight), p(raw, 2), p(w.codebook), p(x), None, p(y), w.N, w.K, B, g, 0,
+                                          _lib.JQ_F32, _lib.JQ_F32, p(ws), ws.numel(), ops._stream()), "jq_gemm_ta")
+        assert torch.equal(y, grp.ys[1])
