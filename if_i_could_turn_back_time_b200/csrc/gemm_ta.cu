@@ -662,14 +662,17 @@ __device__ __forceinline__ void fma_pair(float &acc0, float &acc1, uint32_t w, u
         : "+f"(acc0), "+f"(acc1) : "r"(w), "r"(x));
 }
 
-template <int B>
+// kOwn: a single call, which prepares its activation itself (a kernel of its own, as the grouped one gets 0.7 % slower with that
+// code in it)
+template <int B, bool kOwn>
 __global__ void __launch_bounds__(kLutThreads, 1) gf4_lut2_kernel(const TaProblem *probs, const CUtensorMap *maps,
                                                                   const __grid_constant__ TaProblem single,
                                                                   const __grid_constant__ CUtensorMap single_map,
                                                                   int nprob, const int *tile_start, const int *cta_first,
-                                                                  int y_dtype, PeerInfo peers, int *status) {
+                                                                  int x_dtype, int y_dtype, PeerInfo peers, int *status) {
     using S = LutSmem;
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ float s_max[kLutWarps];
     __shared__ int s_err;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -813,7 +816,48 @@ __global__ void __launch_bounds__(kLutThreads, 1) gf4_lut2_kernel(const TaProble
     int c_pi = 0, c_tend = -1, x_pi = -1;
     TaProblem p = single;
     fetch_codebook(tile_lo);
-    pdl_wait();                     // from here on the prepared activation and its row factors are read
+    float own_scale = 0.f;
+    if constexpr (kOwn) {
+        // in every CTA, as ta_prepare_kernel does (same operations, same bits): a launch in front of this one and the way
+        // through memory cost more than the few hundred elements per warp (4096 x 4096: 15.9 -> 13.5 us per call)
+        static_assert(B == 1, "one row");
+        constexpr int kMost = (S::kXBytes / 2 / 128 + kLutWarps - 1) / kLutWarps;     // blocks of 128 elements per warp
+        float v[kMost][4], m = 0.f;
+#pragma unroll
+        for (int i = 0; i < kMost; ++i) {
+            const int k0 = (warp + i * kLutWarps) * 128 + lane * 4;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[i][j] = k0 < p.K ? jq::load_act(p.x, (size_t)k0 + j, x_dtype) : 0.f;
+                m = fmaxf(m, fabsf(v[i][j]));
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) s_max[warp] = m;
+        __syncthreads();
+        m = s_max[0];
+#pragma unroll
+        for (int w = 1; w < kLutWarps; ++w) m = fmaxf(m, s_max[w]);
+        const int ex = act_exponent(m, p.had != 0);
+        own_scale = __uint_as_float((uint32_t)(127 + ex) << 23);
+        const float down = __uint_as_float((uint32_t)(127 - ex) << 23);
+#pragma unroll
+        for (int i = 0; i < kMost; ++i) {
+            const int blk = warp + i * kLutWarps;
+            if (blk * 128 < p.K) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[i][j] *= down;
+                if (p.had) jq::fwht128_warp(v[i], lane);
+                const __half2 h01 = __floats2half2_rn(v[i][0], v[i][1]), h23 = __floats2half2_rn(v[i][2], v[i][3]);
+                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(xs_u + (blk * 128 + lane * 4) * 2),
+                             "r"(*reinterpret_cast<const uint32_t *>(&h01)), "r"(*reinterpret_cast<const uint32_t *>(&h23)) : "memory");
+            }
+        }
+        __syncthreads();
+        x_pi = 0;
+    }
+    if (!kOwn) pdl_wait();          // from here on the prepared activation and its row factors are read
     bool ok = true;
     int tparity = 0;
     for (int tile = tile_lo; tile < tile_hi && ok; ++tile, tparity ^= 1) {
@@ -860,7 +904,7 @@ __global__ void __launch_bounds__(kLutThreads, 1) gf4_lut2_kernel(const TaProble
 #pragma unroll
         for (int b = 0; b < B; ++b) {
             acc[b] = 0.f;
-            xsc[b] = p.xscale[b];                                    // in flight during the tile, needed at its end
+            xsc[b] = kOwn ? own_scale : p.xscale[b];                // in flight during the tile, needed at its end
         }
         const float bias = (p.bias && row_raw < p.N) ? p.bias[row_raw] : 0.f;
         const int nsteps = ((p.K >> 8) - h + kLutSplit - 1) / kLutSplit;
@@ -1122,20 +1166,21 @@ template <int B>
 static int lut2_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, const TaProblem &single,
                        const CUtensorMap &single_map, int nprob, const int *tile_start, const int *cta_first, int grid,
                        int x_dtype, int y_dtype, const jqta::PeerInfo &peers, int *status, cudaStream_t st) {
-    const int nblk = (nprob ? nprob : 1) * B;
-    if (B <= 2) ta_prepare_kernel<1024><<<nblk, 1024, 0, st>>>(probs_dev, single, B, x_dtype);
-    else ta_prepare_kernel<256><<<nblk, 256, 0, st>>>(probs_dev, single, B, x_dtype);
-    int s = jq_launch_status();
-    if (s) return s;
-    auto kern = gf4_lut2_kernel<B>;
+    if (nprob) {
+        ta_prepare_kernel<1024><<<nprob * B, 1024, 0, st>>>(probs_dev, single, B, x_dtype);
+        const int s = jq_launch_status();
+        if (s) return s;
+    }
+    auto kern = nprob ? gf4_lut2_kernel<B, false> : gf4_lut2_kernel<B, true>;
     constexpr int smem = LutSmem::kBytes;
     static_assert(smem <= 227 * 1024, "shared memory");
     JQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     ta_pdl_config(cfg, attr, grid, kLutThreads, smem, 1, st);
-    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, probs_dev, maps_dev, single, single_map, nprob, tile_start, cta_first, y_dtype,
-                                   peers, status));
+    if (!nprob) cfg.numAttrs = 0;      // the activation is read from the start: after everything in front of it
+    JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, probs_dev, maps_dev, single, single_map, nprob, tile_start, cta_first, x_dtype,
+                                   y_dtype, peers, status));
     return jq_launch_status();
 }
 

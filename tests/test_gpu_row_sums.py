@@ -69,3 +69,25 @@ def test_tiles_of_odd_step_counts_and_scales_off_a_word(fmt, g, B, shift):
         _lib.check(_lib.load().jq_gemm_ta(w.spec.fmt_id, p(w.qweight), p(raw, 2), p(w.codebook), p(x), None, p(y), w.N, w.K, B, g, 0,
                                           _lib.JQ_F32, _lib.JQ_F32, p(ws), ws.numel(), ops._stream()), "jq_gemm_ta")
         assert torch.equal(y, grp.ys[1])
+
+
+@pytest.mark.parametrize("K", [512, 2304, 4096, 12288])
+@pytest.mark.parametrize("had,dtype", [(0, torch.float32), (128, torch.float16), (128, torch.bfloat16)])
+def test_one_row_prepared_in_the_kernel_or_in_front_of_it(K, had, dtype):
+    """A single call of one row prepares its activation itself, a grouped launch reads one that a kernel of its own has
+    prepared: the same bits, for the shortest and longest rows, blocks that do not divide over the warps, a row of zeros, one
+    with an infinity and one that starts off a vector boundary."""
+    pw = jq.pack_weight(_weights(200, K, K).to(DEV), jq.QuantSpec("gf4", 128, had))
+    gen = torch.Generator("cpu").manual_seed(K)
+    grp = ops.GroupedGemv([pw], 1, dtype)
+    raw = torch.zeros(K + 1, dtype=dtype, device=DEV)
+    for scale in (1.0, 1e-3, 0.0, float("inf")):
+        row = torch.randn(1, K, generator=gen)
+        row[0, 0] *= scale if scale == float("inf") else 1.0
+        raw[1:] = (row * (1.0 if scale == float("inf") else scale))[0].to(dtype).to(DEV)
+        x = raw[1:].view(1, K)
+        grp.xs[0].copy_(x)
+        grp.run()
+        y = ops.linear(x, pw)
+        assert torch.equal(y.view(torch.uint8), grp.ys[0].view(torch.uint8))
+    assert grp.status() == 0 and ops.check_status(raise_on_error=False) == 0
