@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include <atomic>
 #include "../../include/jq.h"
 
 #define JQ_SM_COUNT_FALLBACK 148
@@ -22,6 +23,19 @@ static inline int jq_launch_status() {
 }
 
 static inline bool jq_aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+// Dynamic shared memory of a kernel raised to `bytes`, once per device (asking for it costs a call about a microsecond).
+// `done` has a bit per device and belongs to this kernel and size.
+static inline cudaError_t jq_allow_smem(const void *kernel, int bytes, std::atomic<unsigned long long> &done) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    const cudaError_t s = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (s == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+    return s;
+}
 
 // Number of SMs of the current device (cached per device id).
 int jq_sm_count();

@@ -599,7 +599,7 @@ struct Shape { int NT, halves, HN, ntt, split; };
 
 // Tokens per tile and CTAs per tile, by a cost in SM clocks: a wave of tiles costs its 128-code groups (the slowest of
 // multiplying, decoding and folding) plus a fixed part (first stage's latency, outputs; with a K split also the exchange).
-static Shape choose_shape(int mode, int N, int T, int G, int unit, int sms) {
+static Shape search_shape(int mode, int N, int T, int G, int unit, int sms) {
     const int rt = (N + kTileM - 1) / kTileM, steps = (G + 1) / 2;
     const double decode = mode == kGf4 ? 700 : 450;
     Shape best{};
@@ -627,6 +627,19 @@ static Shape choose_shape(int mode, int N, int T, int G, int unit, int sms) {
         }
     }
     return best;
+}
+
+// The search takes some microseconds, three times per call (the scratch of both forms, and the launch): a thread keeps its
+// last answers.
+static Shape choose_shape(int mode, int N, int T, int G, int unit, int sms) {
+    struct Entry { int mode, N, T, G, unit, sms; Shape shape; };
+    constexpr unsigned kEntries = 64;
+    static thread_local Entry kept[kEntries] = {};
+    unsigned h = (unsigned)N * 0x9E3779B1u ^ (unsigned)T * 0x85EBCA77u ^ (unsigned)G * 0xC2B2AE3Du ^ (unsigned)(mode * 1024 + unit) * 0x27D4EB2Fu;
+    Entry &e = kept[(h >> 16) % kEntries];
+    if (e.N != N || e.T != T || e.G != G || e.mode != mode || e.unit != unit || e.sms != sms)
+        e = Entry{mode, N, T, G, unit, sms, search_shape(mode, N, T, G, unit, sms)};
+    return e.shape;
 }
 
 static int fold_unit(int g) { return (g == 0 || g % 128 == 0) ? 128 : (g % 64 == 0 ? 64 : 32); }
@@ -687,7 +700,8 @@ static int launch(int fmt, const void *qw, const void *scales, const void *codeb
         return JQ_ERR_CUDA_BASE - (int)cudaErrorInvalidValue;
 
     auto kern = mode == kGf4 ? gemm_rows_kernel<kGf4> : (mode == kE2m1 ? gemm_rows_kernel<kE2m1> : gemm_rows_kernel<kE2m1Folded>);
-    JQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    static std::atomic<unsigned long long> done[3], conv_done;
+    JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(kern), kSmemBytes, done[mode]));
     if (lin) {
         lin->xp = xp; lin->xscale = xscale; lin->G = G; lin->NT = s.NT;
         rows_prepare_kernel<<<(T + 1) / 2, 256, 0, st>>>(*lin);
@@ -695,7 +709,7 @@ static int launch(int fmt, const void *qw, const void *scales, const void *codeb
         conv->xp = xp; conv->xscale = xscale; conv->G = G; conv->NT = s.NT;
         const int bytes = (K + 7) / 8 * 8 * 32 * (int)sizeof(float);
         conv->keep = K <= kFieldBytes / 128 && bytes <= kFieldBytes;
-        if (conv->keep) JQ_CUDA_TRY(cudaFuncSetAttribute(conv_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFieldBytes));
+        if (conv->keep) JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(conv_prepare_kernel), kFieldBytes, conv_done));
         conv_prepare_kernel<<<(T + 31) / 32, 256, conv->keep ? bytes : 0, st>>>(*conv);
     }
     int rc = jq_launch_status();

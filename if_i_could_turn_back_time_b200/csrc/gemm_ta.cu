@@ -1153,7 +1153,8 @@ static int ta_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, co
     int split = 1;
     if (!nprob && C::kParts == 4 && (single.K >> 8) >= kPartMinSteps)
         split = grid * 4 <= jq_sm_count() ? 4 : (grid * 2 <= jq_sm_count() ? 2 : 1);
-    JQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    static std::atomic<unsigned long long> done{0};
+    JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(kern), smem, done));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     ta_pdl_config(cfg, attr, grid * split, kTaThreads, smem, split, st);
@@ -1174,7 +1175,8 @@ static int lut2_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, 
     auto kern = nprob ? gf4_lut2_kernel<B, false> : gf4_lut2_kernel<B, true>;
     constexpr int smem = LutSmem::kBytes;
     static_assert(smem <= 227 * 1024, "shared memory");
-    JQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    static std::atomic<unsigned long long> done[2];
+    JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(kern), smem, done[nprob ? 0 : 1]));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     ta_pdl_config(cfg, attr, grid, kLutThreads, smem, 1, st);

@@ -61,7 +61,8 @@ class JenksQuantLinear(nn.Linear):
     def packed(self) -> PackedWeight:
         if self.qweight is None:
             self._pack()
-        return PackedWeight(self.spec, self.out_features, self.in_features, self.qweight, self.scales, self.codebook)
+        b = self._buffers             # (a module's look-up of a buffer as an attribute tries two other places first)
+        return PackedWeight(self.spec, self.out_features, self.in_features, b["qweight"], b["scales"], b["codebook"])
 
     def _pack(self) -> None:
         dense = self._parameters["weight"]

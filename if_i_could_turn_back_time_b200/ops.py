@@ -235,6 +235,20 @@ def _rows_scratch(device, nbytes: int):
     return own, own.data_ptr(), nbytes, ws.data_ptr()
 
 
+_rows_scratch_bytes = {}       # (device, format, N, K, rows, group size) -> bytes
+
+
+def _many_rows_scratch_bytes(lib, *key) -> int:
+    """Scratch of a many-row call on the current device; the library searches for the call's tile shape to know it."""
+    key = (torch._C._cuda_getDevice(), *key)
+    n = _rows_scratch_bytes.get(key)
+    if n is None:
+        if len(_rows_scratch_bytes) >= 4096:
+            _rows_scratch_bytes.clear()
+        n = _rows_scratch_bytes[key] = lib.jq_gemm_rows_scratch_bytes(*key[1:])
+    return n
+
+
 def _linear_many_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had, y):
     lib = _lib.load()
     rows = x2.shape[0]
@@ -243,7 +257,7 @@ def _linear_many_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had,
         for b0 in range(0, rows, part):
             b1 = min(rows, b0 + part)
             xs, ys = (x2, y) if rows <= part else (x2[b0:b1], y[b0:b1])
-            own, scratch, size, status = _rows_scratch(x2.device, lib.jq_gemm_rows_scratch_bytes(fmt_id, N, K, b1 - b0, g))
+            own, scratch, size, status = _rows_scratch(x2.device, _many_rows_scratch_bytes(lib, fmt_id, N, K, b1 - b0, g))
             st = lib.jq_gemm_rows(fmt_id, _addr(qweight), _addr(scales), _addr(codebook), xs.data_ptr(), _addr(bias),
                                   ys.data_ptr(), N, K, b1 - b0, g, had, _DT[x2.dtype], _DT[y.dtype], scratch, size, status,
                                   _stream())
@@ -253,6 +267,9 @@ def _linear_many_rows(x2, qweight, scales, codebook, bias, fmt_id, N, K, g, had,
     if _checked:
         check_status()
     return y
+
+
+_Strides = ctypes.c_int64 * 4
 
 
 def conv2d(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor], kernel_size, stride, padding,
@@ -285,14 +302,15 @@ def conv2d(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor], kern
     with _on(x.device):
         for b0 in range(0, B, part):
             b1 = min(B, b0 + part)
-            xs, ys = x[b0:b1], y[b0 * L:b1 * L]
-            c = _lib.jq_conv(b1 - b0, C, H, W, *geo, (ctypes.c_int64 * 4)(*x.stride()))
-            own, scratch, size, status = _rows_scratch(
-                x.device, lib.jq_gemm_rows_scratch_bytes(pw.spec.fmt_id, pw.N, pw.K, (b1 - b0) * L, pw.spec.group_size))
-            st = lib.jq_conv_rows(pw.spec.fmt_id, _ptr(pw.qweight), _ptr(pw.scales), _ptr(pw.codebook), _ptr(xs), _ptr(bias),
-                                  _ptr(ys), ctypes.byref(c), pw.N, pw.K, ys.shape[0], pw.spec.group_size, _DT[x.dtype],
-                                  _DT[y.dtype], scratch, size, status, _stream())
-            _lib.check(st, "jq_conv_rows")
+            rows, fmt_id, g = (b1 - b0) * L, pw.spec.fmt_id, pw.spec.group_size
+            xs, ys = (x, y) if b1 - b0 == B else (x[b0:b1], y[b0 * L:b1 * L])
+            c = _lib.jq_conv(b1 - b0, C, H, W, *geo, _Strides(*x.stride()))
+            own, scratch, size, status = _rows_scratch(x.device, _many_rows_scratch_bytes(lib, fmt_id, pw.N, pw.K, rows, g))
+            st = lib.jq_conv_rows(fmt_id, _addr(pw.qweight), _addr(pw.scales), _addr(pw.codebook), xs.data_ptr(), _addr(bias),
+                                  ys.data_ptr(), ctypes.byref(c), pw.N, pw.K, rows, g, _DT[x.dtype], _DT[y.dtype], scratch, size,
+                                  status, _stream())
+            if st:
+                _lib.check(st, "jq_conv_rows")
             del own
     if _checked:
         check_status()
