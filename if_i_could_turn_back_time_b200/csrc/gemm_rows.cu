@@ -521,10 +521,12 @@ __global__ void __launch_bounds__(256) rows_prepare_kernel(const __grid_constant
 
 // Convolution: the receptive fields are gathered straight from the image into the same layout (no unfolded copy).
 // lane = output position, so loads of one tap and stores of one 8-code piece are consecutive over the warp.  Bound by the
-// index arithmetic of the gathering, so a block that can keep its 32 fields in shared memory (96 KB: K up to 768, two
-// blocks per SM) gathers once; longer ones gather again for the second pass.  64 -> 128 channels, 3x3, 16 images of 32 x 32,
-// the whole call: 57 us gathering twice, 41 us gathering once.  Its time grows with K, not with the positions, until the
-// blocks fill the chip (K = 4608: 159 us for 25 to 784 positions): long fields at few positions are not for this kernel.
+// instructions between the loads, so a block that can keep its 32 fields in shared memory (96 KB: K up to 768) gathers once;
+// longer ones gather again for the second pass.  64 -> 128 channels, 3x3, 16 images of 32 x 32, the whole call: 56 us gathering
+// twice, 40 us gathering once, 30 us with addresses formed by additions; loading from a valid place under every condition, so
+// that the loads need not wait for one another, was slower (44 us).  Time grows with K, not with the positions, until the
+// blocks fill the chip, so few blocks have more warps: 128 -> 128 channels, 3x3, 8 images of 14 x 14 (49 blocks): 49 us before,
+// 32 with 8 warps a block, 26 with 32.
 constexpr int kFieldBytes = 96 * 1024;
 struct ConvArgs {
     const void *x;             // element (b, c, h, w) at b sb + c sc + h sr + w sx
@@ -536,31 +538,45 @@ struct ConvArgs {
     int keep;                  // the block's fields fit in shared memory
 };
 
-__global__ void __launch_bounds__(256) conv_prepare_kernel(const __grid_constant__ ConvArgs p) {
-    __shared__ float red[8][32];
+template <class T, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32) conv_prepare_kernel(const __grid_constant__ ConvArgs p) {
+    __shared__ float red[kWarps][32];
     extern __shared__ __align__(16) float fields[];    // [pieces * 8][32], or empty
     pdl_launch_dependents();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // (uniform for the compiler: so is the walk over the taps)
     const int t = blockIdx.x * 32 + lane;
     const bool live = t < p.T;
     const int b = live ? t / p.L : 0, l = live ? t - b * p.L : 0;
     const int y0 = (l / p.wo) * p.sh - p.ph, x0 = (l % p.wo) * p.sw - p.pw;
-    const long long img = b * p.sb;
+    const T *const at0 = reinterpret_cast<const T *>(p.x) + (b * p.sb + y0 * p.sr + x0 * p.sx);   // (not read from there where out of range)
     const int taps = p.kh * p.kw;
     const int pieces = p.G * 16;
-    // walk of one piece's eight codes: k -> (channel, tap row, tap column)
+    // Walk of one piece's eight codes: k -> (channel, tap row, tap column).  Position and address go along by additions (three
+    // products of 64 bits per code were most of this kernel's time).
+    const long long to_x = p.dw * p.sx, to_y = p.dh * p.sr - p.kw * to_x, to_c = p.sc - p.kh * (p.dh * p.sr);
+    const int back_x = p.kw * p.dw, back_y = p.kh * p.dh;
     auto gather = [&](int piece, float (&v)[8]) {
-        int k = piece * 8, c = k / taps, r = k - c * taps, ky = r / p.kw, kx = r - ky * p.kw;
+        const int k = piece * 8, c = k / taps, r = k - c * taps;
+        int ky = r / p.kw, kx = r - ky * p.kw;
+        int yy = y0 + ky * p.dh, xx = x0 + kx * p.dw;
+        const T *at = at0 + (c * p.sc + (long long)(ky * p.dh) * p.sr + (long long)(kx * p.dw) * p.sx);
+        const int left = live ? p.K - k : 0;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const int yy = y0 + ky * p.dh, xx = x0 + kx * p.dw;
-            v[e] = (live && k + e < p.K && yy >= 0 && yy < p.H && xx >= 0 && xx < p.W)
-                       ? jq::load_act(p.x, (size_t)(img + c * p.sc + yy * p.sr + xx * p.sx), p.x_dtype) : 0.f;
-            if (++kx == p.kw) { kx = 0; if (++ky == p.kh) { ky = 0; ++c; } }
+            v[e] = (e < left && (unsigned)yy < (unsigned)p.H && (unsigned)xx < (unsigned)p.W) ? (float)*at : 0.f;
+            at += to_x;
+            xx += p.dw;
+            if (++kx == p.kw) {
+                kx = 0;
+                xx -= back_x;
+                yy += p.dh;
+                at += to_y;
+                if (++ky == p.kh) { ky = 0; yy -= back_y; at += to_c; }
+            }
         }
     };
     float m = 0.f;
-    for (int piece = warp; piece * 8 < p.K; piece += 8) {
+    for (int piece = warp; piece * 8 < p.K; piece += kWarps) {
         float v[8];
         gather(piece, v);
 #pragma unroll
@@ -572,11 +588,11 @@ __global__ void __launch_bounds__(256) conv_prepare_kernel(const __grid_constant
     red[warp][lane] = m;
     __syncthreads();
 #pragma unroll
-    for (int w = 0; w < 8; ++w) m = fmaxf(m, red[w][lane]);
+    for (int w = 0; w < kWarps; ++w) m = fmaxf(m, red[w][lane]);
     const int ex = act_exponent(m, false);
     const float down = __uint_as_float((uint32_t)(127 - ex) << 23);
     if (warp == 0 && live) p.xscale[t] = __uint_as_float((uint32_t)(127 + ex) << 23);
-    for (int piece = warp; piece < pieces; piece += 8) {
+    for (int piece = warp; piece < pieces; piece += kWarps) {
         float v[8];
         if (p.keep) {
 #pragma unroll
@@ -700,7 +716,7 @@ static int launch(int fmt, const void *qw, const void *scales, const void *codeb
         return JQ_ERR_CUDA_BASE - (int)cudaErrorInvalidValue;
 
     auto kern = mode == kGf4 ? gemm_rows_kernel<kGf4> : (mode == kE2m1 ? gemm_rows_kernel<kE2m1> : gemm_rows_kernel<kE2m1Folded>);
-    static std::atomic<unsigned long long> done[3], conv_done;
+    static std::atomic<unsigned long long> done[3], conv_done[9];
     JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(kern), kSmemBytes, done[mode]));
     if (lin) {
         lin->xp = xp; lin->xscale = xscale; lin->G = G; lin->NT = s.NT;
@@ -709,8 +725,15 @@ static int launch(int fmt, const void *qw, const void *scales, const void *codeb
         conv->xp = xp; conv->xscale = xscale; conv->G = G; conv->NT = s.NT;
         const int bytes = (K + 7) / 8 * 8 * 32 * (int)sizeof(float);
         conv->keep = K <= kFieldBytes / 128 && bytes <= kFieldBytes;
-        if (conv->keep) JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(conv_prepare_kernel), kFieldBytes, conv_done));
-        conv_prepare_kernel<<<(T + 31) / 32, 256, conv->keep ? bytes : 0, st>>>(*conv);
+        // A block's time is its warps' walks along 32 fields: with few blocks, more warps share them
+        const int blocks = (T + 31) / 32, more = blocks <= sms ? 2 : (blocks <= 2 * sms ? 1 : 0);
+        void (*const kernels[3][3])(const ConvArgs) = {
+            {conv_prepare_kernel<float, 8>, conv_prepare_kernel<float, 16>, conv_prepare_kernel<float, 32>},
+            {conv_prepare_kernel<__half, 8>, conv_prepare_kernel<__half, 16>, conv_prepare_kernel<__half, 32>},
+            {conv_prepare_kernel<__nv_bfloat16, 8>, conv_prepare_kernel<__nv_bfloat16, 16>, conv_prepare_kernel<__nv_bfloat16, 32>}};
+        auto gather = kernels[conv->x_dtype][more];
+        if (conv->keep) JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(gather), kFieldBytes, conv_done[conv->x_dtype * 3 + more]));
+        gather<<<blocks, 256 << more, conv->keep ? bytes : 0, st>>>(*conv);
     }
     int rc = jq_launch_status();
     if (rc) return rc;

@@ -320,14 +320,15 @@ def conv2d(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor], kern
 def conv_gathers(fmt_id: int, K: int, g: int, positions: int) -> bool:
     """Convolutions whose fields the preparation kernel gathers (the others are unfolded first): the output positions that
     the many-row kernel is for, and fields of up to 1536 values or more than 2048 positions.  A block gathers 32 positions and
-    walks along the whole field, so that long fields at few positions leave most of the chip idle.  Calls in us, gathered /
-    unfolded, one to four images:
+    walks along the whole field, so that long fields at few positions leave most of the chip idle.  Device time of calls with
+    3 x 3 kernels in us, gathered / unfolded (which also has five more launches):
 
         positions   K = 1152       K = 2304       K = 4608       K = 9216
-        25          49 / 59        87 / 54        160 / 62       308 / 53
-        196         54 / 55        84 / 72        159 / 56       301 / 56
-        784         51 / 70        88 / 70        164 / 81       311 / 120
-        3136        57 / 81        96 / 118       172 / 189      --"""
+        25          22 / 19        33 / 21        56 / 25        102 / 32
+        196         22 / 21        33 / 24        57 / 31        103 / 46
+        784         24 / 29        35 / 38        59 / 55        105 / 94
+        1568        27 / 40        40 / 60        63 / 92        110 / 167
+        3136        30 / 63        44 / 104       68 / 169       115 / 325"""
     few = ta_max_batch(fmt_id) if fmt_id == _lib.JQ_FMT_E2M1 and ta_eligible(fmt_id, K, g, positions) else 16
     return positions > few and (K <= 1536 or positions > 2048)
 

@@ -206,3 +206,18 @@ def test_convolution_of_a_lazily_negated_image():
     x = torch.randn(2, 6, 9, 9, dtype=torch.complex64, device=DEV).conj().imag
     assert x.is_neg()
     assert torch.equal(q(x), q(x + 0.0))
+
+
+@pytest.mark.parametrize("positions", [31, 4736, 4737, 9472, 9473])
+@pytest.mark.parametrize("cin,dtype", [(4, torch.float32), (88, torch.float16)])       # fields kept in shared memory, or not
+def test_convolution_gathered_by_more_or_fewer_warps(positions, cin, dtype):
+    """Up to 148 blocks of 32 positions, up to 296 and beyond have 32, 16 and 8 warps each: row 1 of a two-row image whose
+    kernel reaches over both edges, against float64 conv2d."""
+    torch.manual_seed(cin)
+    q = jq.JenksQuantConv2d(torch.nn.Conv2d(cin, 12, 3, stride=(2, 1), padding=1), 4).to(DEV)
+    x = torch.randn(1, cin, 2, positions, device=DEV).to(dtype)
+    y = ops.conv2d(x, q.packed, q.bias, q.kernel_size, q.stride, q.padding, q.dilation)
+    ref = torch.nn.functional.conv2d(x.double(), q.dequantized_weight().double(), q.bias.double(), (2, 1), 1)
+    assert y.shape == ref.shape == (1, 12, 1, positions)
+    limit = TOL + (2.0 ** -11 if dtype == torch.float16 else 0)
+    assert (y.double() - ref).abs().max() <= limit * ref.abs().max()
