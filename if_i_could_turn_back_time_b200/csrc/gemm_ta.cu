@@ -127,8 +127,7 @@ __global__ void __launch_bounds__(kPrepThreads) ta_prepare_kernel(const TaProble
 // are a large part of what is left (a ready wait with its vote takes 105 clocks, an elected arrival 50 to 70): operand slots of
 // half a group, which are busy for a shorter time, were slower (953 against 928 us on one GPU), one issuer and one slot per
 // phase too (939).
-// GF4 up to 16 rows looks every byte up in the pair table.  From 17 rows on there is no shared memory for tables beside the
-// activation stages, and all words go through byte permutes.
+// GF4 looks every byte up in the pair table.  Up to 16 rows; more are for the kernel below.
 //
 // A row's sum is formed in four parts of K (one, for short rows and for 33 rows and more), each in group order, added in
 // part order.  A single call with few tiles lets the CTAs of a cluster take the parts; the partial sums meet in
@@ -136,26 +135,20 @@ __global__ void __launch_bounds__(kPrepThreads) ta_prepare_kernel(const TaProble
 constexpr int kTaThreads = 24 * 32;
 constexpr int kSlots = 6;
 constexpr int kPartMinSteps = 8;                                    // 256-code steps from which a row is summed in parts
-template <int FMT, int NB>
-struct Cols {
-    static constexpr bool kTable = FMT == JQ_FMT_GF4 && NB == 16;   // pair tables in shared memory
-    static constexpr int kAcc = kSlots * 64;                        // first column of the accumulators
-    static constexpr int kAccs = 128 / NB;
-    static constexpr int kPer = NB == 64 ? 1 : 2;                   // accumulators that are handed over together
-    static constexpr int kAccBars = kAccs / kPer;
-    static constexpr int kParts = NB == 64 ? 1 : 4;
-    // registers of a fold thread, of an issue / load thread; the decode threads have 72: 61440 in all, what 768 threads
-    // start with at 80
-    static constexpr int kFoldRegs = NB == 16 ? 112 : (NB == 32 ? 128 : 136), kAuxRegs = NB == 16 ? 80 : (NB == 32 ? 64 : 56);
-    static_assert(512 * 72 + 128 * (kFoldRegs + kAuxRegs) <= 80 * kTaThreads, "registers");
-    static_assert(kAcc + kAccs * NB <= 512, "tensor memory");
-};
+constexpr int NB = 16;                                              // columns of an MMA
+constexpr int kAcc = kSlots * 64;                                   // first column of the accumulators
+constexpr int kAccs = 128 / NB, kAccBars = kAccs / 2;               // the two of a step are handed over together
+constexpr int kParts = 4;
+// registers of a fold thread; the decode threads have 72 and the others 80: 61440 in all, what 768 threads start with at 80
+constexpr int kFoldRegs = 112;
+static_assert(512 * 72 + 128 * (kFoldRegs + 80) <= 80 * kTaThreads, "registers");
+static_assert(kAcc + kAccs * NB <= 512, "tensor memory");
 
-template <bool TABLE, int NB>
+template <bool TABLE>
 struct Smem {
     static constexpr int kTab = 0;
     static constexpr int kWRing = TABLE ? kTabBytes : 0;
-    static constexpr int kWs = TABLE ? 4 : (NB == 64 ? 6 : 8);      // weight stages (even: a decode warp takes every other one)
+    static constexpr int kWs = TABLE ? 4 : 8;                       // weight stages (even: a decode warp takes every other one)
     static constexpr int kXRing = kWRing + kWs * kWStage;
     static constexpr int kXStage = 256 * NB;                        // one group of up to NB rows
     static constexpr int kBars = kXRing + kSlots * kXStage;
@@ -163,21 +156,20 @@ struct Smem {
     static constexpr int kBytes = kBars + kNumBars * 8 + 1024;      // + slack for the 1 KB alignment of the base (TMA swizzle)
     static constexpr int kExch = TABLE ? kTab : kXRing;             // K split: partial sums, once nothing else uses the region
     static_assert(kBytes <= 227 * 1024, "shared memory");
-    static_assert(NB == 64 || TABLE || 2 * NB * 512 <= kSlots * kXStage, "exchange");
+    static_assert(TABLE || 2 * NB * 512 <= kSlots * kXStage, "exchange");
 };
 
 // first step of part i of a row of nsteps 256-code steps
 __host__ __device__ inline int part_step(int nsteps, int parts, int i) { return nsteps * i / parts; }
 
-template <int FMT, int NB>
+template <int FMT>
 __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem *probs, const CUtensorMap *maps,
                                                                 const __grid_constant__ TaProblem single,
                                                                 const __grid_constant__ CUtensorMap single_map, int nprob,
                                                                 const int *tile_start, const int *cta_first,
                                                                 int B, int y_dtype, PeerInfo peers, int split, int *status) {
-    using C = Cols<FMT, NB>;
-    using S = Smem<C::kTable, NB>;
-    constexpr bool kGf4 = FMT == JQ_FMT_GF4;
+    constexpr bool kGf4 = FMT == JQ_FMT_GF4;                        // with pair tables in shared memory
+    using S = Smem<kGf4>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint32_t s_tmem;
     __shared__ int s_err;
@@ -198,7 +190,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
         s_err = 0;
         for (int s = 0; s < S::kWs; ++s) { mbar_init(wfull(s), 1); mbar_init(wempty(s), 8); }
         for (int s = 0; s < kSlots; ++s) { mbar_init(afull(s), 4); mbar_init(sfree(s), 1); mbar_init(xfull(s), 1); }
-        for (int a = 0; a < C::kAccBars; ++a) { mbar_init(dfull(a), C::kPer); mbar_init(dfree(a), 4); }
+        for (int a = 0; a < kAccBars; ++a) { mbar_init(dfull(a), 2); mbar_init(dfree(a), 4); }
         for (int q = 0; q < 4; ++q) mbar_init(qbar(q), 4);             // the warps that share a quarter of the rows
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -223,9 +215,9 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
         tile_hi = cta_first[blockIdx.x + 1];
     }
     // parts of a row's sum, and the steps [lo, hi) of a row that this CTA works on
-    auto parts_of = [&](int nsteps) { return nsteps >= kPartMinSteps ? C::kParts : 1; };
-    auto step_lo = [&](int nsteps) { return split > 1 ? part_step(nsteps, C::kParts, C::kParts / split * rank) : 0; };
-    auto step_hi = [&](int nsteps) { return split > 1 ? part_step(nsteps, C::kParts, C::kParts / split * (rank + 1)) : nsteps; };
+    auto parts_of = [&](int nsteps) { return nsteps >= kPartMinSteps ? kParts : 1; };
+    auto step_lo = [&](int nsteps) { return split > 1 ? part_step(nsteps, kParts, kParts / split * rank) : 0; };
+    auto step_hi = [&](int nsteps) { return split > 1 ? part_step(nsteps, kParts, kParts / split * (rank + 1)) : nsteps; };
     // Problems change rarely along a CTA's tile sequence: every walker keeps what it needs of its current
     // problem in registers and goes back to global memory only for a tile beyond that problem's last one.
     auto problem_at = [&](int &pi, int &t_end, int tile, TaProblem &p) {
@@ -285,7 +277,6 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
         int w_stage = ph >> 1, slot = ph;            // slot of group ph: ph < kSlots
         uint32_t w_par = 0, s_par = 1;               // (the first use of a slot finds it free)
         uint32_t q_par = 0;
-        Codebook book;
         auto quarter_sync = [&]() -> bool {
             warp_arrive(qbar(q));
             const bool ok = warp_wait(qbar(q), q_par);
@@ -312,8 +303,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             const uint2 *srow = reinterpret_cast<const uint2 *>(scales + (size_t)row * lds) + gi;
             uint2 sc_nxt = make_uint2(0, 0);
             if (!kGf4 && s_first < s_hi) sc_nxt = __ldg(srow + 2 * s_first);
-            if constexpr (kGf4 && !C::kTable) book.set(cb0, cb1);
-            if constexpr (C::kTable) {
+            if constexpr (kGf4) {
                 // ---- the pair table of this row (this thread fills the entries whose second code is 4 ph .. 4 ph + 3)
                 if (!(ok = quarter_sync())) break;      // the four warps are done with the previous tile's lookups
                 const uint32_t c[8] = {cb0.x, cb0.y, cb0.z, cb0.w, cb1.x, cb1.y, cb1.z, cb1.w};
@@ -331,7 +321,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                     }
             }
             fetch_codebook(tile + 1);
-            if constexpr (C::kTable) { if (!(ok = quarter_sync())) break; }
+            if constexpr (kGf4) { if (!(ok = quarter_sync())) break; }
             for (int sg = s_first; sg < s_hi; sg += 2) {
                 if (!(ok = warp_wait(wfull(w_stage), w_par))) break;
                 const uint32_t src = wrow + w_stage * kWStage;
@@ -347,15 +337,8 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                     for (int wi = 0; wi < 4; ++wi) {
                         const uint32_t w = wi == 0 ? w4[part].x : (wi == 1 ? w4[part].y : (wi == 2 ? w4[part].z : w4[part].w));
                         if constexpr (kGf4) {
-                            if (C::kTable) {
 #pragma unroll
-                                for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = lds32(dp4a_u(w, 0x80u << (8 * bj), tcol));
-                            } else {
-                                uint32_t hh[4];
-                                book.look_up8(w, hh);
-#pragma unroll
-                                for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = hh[bj];
-                            }
+                            for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = lds32(dp4a_u(w, 0x80u << (8 * bj), tcol));
                         } else {
                             // E2M1: the group scale folded into the fp16 weight (one rounding per weight)
                             const uint32_t pr = part < 2 ? sc4.x : sc4.y;
@@ -396,9 +379,9 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
         if (split > 1) { __syncwarp(); cluster_sync(); cluster_sync(); }
     } else if (warp < 20) {
         // =============================== fold threads ===============================
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kFoldRegs));
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFoldRegs));
         const int r = tid & 127;
-        const uint32_t lane_t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::kAcc;
+        const uint32_t lane_t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + kAcc;
         uint32_t buf = 0, par = 0;                  // accumulators of the next step (or group) and their phase
         int c_pi = 0, c_tend = -1;
         TaProblem p = single;
@@ -411,15 +394,13 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             const unsigned short *srow = reinterpret_cast<const unsigned short *>(p.scales) + (size_t)row * p.lds;
             const int gshift = kGf4 ? 31 - __clz(p.g >> 7) : 0;   // GF4: log2 of the 128-code groups per scale
             const bool word = gshift == 0 && ((size_t)p.scales & 3) == 0;
-            float xs[(NB + 31) / 32];
-#pragma unroll
-            for (int i = 0; i < (NB + 31) / 32; ++i) xs[i] = (lane + 32 * i < B) ? p.xscale[lane + 32 * i] : 0.f;
+            const float xs = lane < B ? p.xscale[lane] : 0.f;
             const float bias = (p.bias && row_raw < p.N) ? p.bias[row_raw] : 0.f;
-            float acc[NB], total[C::kParts > 1 ? NB : 1];
+            float acc[NB], total[NB];
 #pragma unroll
             for (int b = 0; b < NB; ++b) acc[b] = 0.f;
             const uint32_t exch = sbase + S::kExch + r * 4;
-            int part = split > 1 ? C::kParts / split * rank : 0, part_end = part_step(nsteps, parts, part + 1);
+            int part = split > 1 ? kParts / split * rank : 0, part_end = part_step(nsteps, parts, part + 1);
             bool first = true;
             // the two scales of a step, a step ahead; in 128-code groups they are one aligned word (K is a multiple of 256)
             uint32_t raw = 0;
@@ -434,47 +415,23 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                 const float sc[2] = {__half2float(__ushort_as_half((unsigned short)raw)),
                                      __half2float(__ushort_as_half((unsigned short)(raw >> 16)))};
                 if (sg + 1 < s_hi) load_scales(sg + 1);
-                if constexpr (NB == 16) {
-                    // both groups of the step at once: the way from the barrier through tensor memory to the release is a
-                    // chain of latencies
-                    if (!(ok = warp_wait(dfull(buf), par))) break;
-                    tc_fence_after();
-                    uint32_t d0[16], d1[16];
-                    tmem_ld16(lane_t + buf * 2 * NB, d0);
-                    tmem_ld16(lane_t + buf * 2 * NB + NB, d1);
-                    tmem_wait_ld();
-                    tc_fence_before();
-                    warp_arrive(dfree(buf));
+                // both groups of the step at once: the way from the barrier through tensor memory to the release is a
+                // chain of latencies
+                if (!(ok = warp_wait(dfull(buf), par))) break;
+                tc_fence_after();
+                uint32_t d0[16], d1[16];
+                tmem_ld16(lane_t + buf * 2 * NB, d0);
+                tmem_ld16(lane_t + buf * 2 * NB + NB, d1);
+                tmem_wait_ld();
+                tc_fence_before();
+                warp_arrive(dfree(buf));
 #pragma unroll
-                    for (int i = 0; i < 16; i += 2) fma2(acc[i], acc[i + 1], d0[i], d0[i + 1], kGf4 ? sc[0] : 1.f);
+                for (int i = 0; i < 16; i += 2) fma2(acc[i], acc[i + 1], d0[i], d0[i + 1], kGf4 ? sc[0] : 1.f);
 #pragma unroll
-                    for (int i = 0; i < 16; i += 2) fma2(acc[i], acc[i + 1], d1[i], d1[i + 1], kGf4 ? sc[1] : 1.f);
-                    if (++buf == (uint32_t)C::kAccBars) { buf = 0; par ^= 1; }
-                } else {
-#pragma unroll
-                    for (int gi = 0; gi < 2; ++gi) {
-                        if (gi == 0 || C::kPer == 1) {
-                            if (!(ok = warp_wait(dfull(buf), par))) break;
-                            tc_fence_after();
-                        }
-                        const uint32_t d_t = lane_t + (buf * C::kPer + (C::kPer == 2 ? gi : 0)) * NB;
-#pragma unroll
-                        for (int c = 0; c < NB; c += 32) {
-                            uint32_t d[32];
-                            tmem_ld32(d_t + c, d);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int i = 0; i < 32; i += 2) fma2(acc[c + i], acc[c + i + 1], d[i], d[i + 1], kGf4 ? sc[gi] : 1.f);
-                        }
-                        if (gi == 1 || C::kPer == 1) {
-                            tc_fence_before();
-                            warp_arrive(dfree(buf));
-                            if (++buf == (uint32_t)C::kAccBars) { buf = 0; par ^= 1; }
-                        }
-                    }
-                }
+                for (int i = 0; i < 16; i += 2) fma2(acc[i], acc[i + 1], d1[i], d1[i + 1], kGf4 ? sc[1] : 1.f);
+                if (++buf == (uint32_t)kAccBars) { buf = 0; par ^= 1; }
                 if (!ok) break;
-                if (C::kParts > 1 && sg + 1 == part_end) {      // a part of the row's sum is complete
+                if (sg + 1 == part_end) {      // a part of the row's sum is complete
                     if (split > 1) {        // at most two per CTA: the first waits in `total`, the second stays in `acc`
                         if (first) {
 #pragma unroll
@@ -492,32 +449,29 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                     part_end = part_step(nsteps, parts, part + 1);
                 }
             }
-            if constexpr (C::kParts > 1) {
-                if (split > 1) {
-                    // every group of this CTA has been folded: nothing reads the tables or the activation stages any more.
-                    // Each CTA leaves its parts in its shared memory; rank k writes columns k, k + split, ...
-                    const int per = C::kParts / split;
+            if (split > 1) {
+                // every group of this CTA has been folded: nothing reads the tables or the activation stages any more.
+                // Each CTA leaves its parts in its shared memory; rank k writes columns k, k + split, ...
+                const int per = kParts / split;
 #pragma unroll
-                    for (int b = 0; b < NB; ++b) {
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(exch + b * 512), "f"(total[b]) : "memory");
-                        if (per == 2) asm volatile("st.shared.f32 [%0], %1;" ::"r"(exch + (NB + b) * 512), "f"(acc[b]) : "memory");
-                    }
-                    cluster_sync();
-                    for (int b = rank; b < B; b += split) {
-                        float v = ld_cluster_f32(exch + b * 512, 0);
-                        for (int i = 1; i < C::kParts; ++i) v += ld_cluster_f32(exch + ((i % per) * NB + b) * 512, i / per);
-                        if (ok && row_raw < p.N) jq::store_out(p.y, (size_t)b * p.ldy + row_raw, fmaf(v, p.xscale[b], bias), y_dtype);
-                    }
-                    cluster_sync();
-                    break;
+                for (int b = 0; b < NB; ++b) {
+                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(exch + b * 512), "f"(total[b]) : "memory");
+                    if (per == 2) asm volatile("st.shared.f32 [%0], %1;" ::"r"(exch + (NB + b) * 512), "f"(acc[b]) : "memory");
                 }
+                cluster_sync();
+                for (int b = rank; b < B; b += split) {
+                    float v = ld_cluster_f32(exch + b * 512, 0);
+                    for (int i = 1; i < kParts; ++i) v += ld_cluster_f32(exch + ((i % per) * NB + b) * 512, i / per);
+                    if (ok && row_raw < p.N) jq::store_out(p.y, (size_t)b * p.ldy + row_raw, fmaf(v, p.xscale[b], bias), y_dtype);
+                }
+                cluster_sync();
+                break;
             }
             if (!ok) break;
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
-                const float xs_b = __shfl_sync(0xffffffffu, xs[b >> 5], b & 31);
-                const float v = C::kParts > 1 ? total[C::kParts > 1 ? b : 0] : acc[b];
-                acc[b] = fmaf(v, xs_b, bias);
+                const float xs_b = __shfl_sync(0xffffffffu, xs, b);
+                acc[b] = fmaf(total[b], xs_b, bias);
             }
             if (row_raw < p.N) {
                 for (int cpy = 0; cpy < peers.n; ++cpy) {
@@ -529,7 +483,6 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             }
         }
     } else {
-        if constexpr (C::kAuxRegs < 80) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kAuxRegs));
         // walk of this CTA's tiles: (tile, its problem, the range of its steps)
         int pi = 0, t_end = -1, lo = 0, hi = 0;
         TaProblem p = single;
@@ -549,14 +502,14 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
             constexpr uint32_t idesc = idesc_f16(kTileM, NB);
             const uint32_t lbo = (uint32_t)B * 16;
             const uint32_t desc_step = (2 * lbo) >> 4;  // descriptor address field per K = 16 slice
-            uint32_t slot = warp - 20, s_par = 0, acc = C::kPer == 2 ? 0 : warp - 20, d_par = 1;   // (the first use of an accumulator finds it free)
+            uint32_t slot = warp - 20, s_par = 0, acc = 0, d_par = 1;   // (the first use of an accumulator finds it free)
             for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
                 open(tile);
                 for (int sg = lo; sg < hi; ++sg) {
                     if (!(ok = warp_wait(dfree(acc), d_par) && warp_wait(xfull(slot), s_par) && warp_wait(afull(slot), s_par))) break;
                     tc_fence_after();
                     const uint32_t a_t = tmem + slot * 64;
-                    const uint32_t d_t = tmem + C::kAcc + (C::kPer == 2 ? 2 * acc + warp - 20 : acc) * NB;
+                    const uint32_t d_t = tmem + kAcc + (2 * acc + warp - 20) * NB;
                     const uint64_t desc0 = smem_desc(sbase + S::kXRing + slot * S::kXStage, lbo, 128);
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
@@ -564,7 +517,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                     mma_commit(elected, sfree(slot));
                     mma_commit(elected, dfull(acc));
                     if ((slot += 2) >= (uint32_t)kSlots) { slot -= kSlots; s_par ^= 1; }
-                    if ((acc += 2 / C::kPer) >= (uint32_t)C::kAccBars) { acc -= C::kAccBars; d_par ^= 1; }
+                    if (++acc == (uint32_t)kAccBars) { acc = 0; d_par ^= 1; }
                 }
             }
         } else if (warp == 22 && lane == 0) {
@@ -620,6 +573,520 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }
 }
+
+// ---- 17 to 64 rows --------------------------------------------------------------------
+// With 32 or 64 columns the folding of the accumulators weighs as much as the decoding, and a kernel of fewer warps is ahead:
+// the kernel above took 83 us for 28672 x 8192 E2M1 with 64 rows, this one 54; 17.0 and 14.8 for 11008 x 4096 with 24; 316 and
+// 285 for a step of eight 8B-shaped layers with 24 rows.
+// Roles of a CTA (16 warps): warps 0-7 decode (warp = 32-row quarter q of the tile x half h of the 256-code
+// steps of a row: step sg belongs to half sg & 1); warps 8-11 fold (thread = row); warps 12-15 issue MMAs (two issuers per half)
+// and stream the prepared activation of their own groups; warp 15 also owns the tensor-memory allocation.
+//
+// Tensor-memory columns: two slots per half of 64 columns each for the A operand (one 128-code group) and kAccBufs
+// accumulators of NB columns per issuer.  GF4 words go through byte permutes: there is no shared memory for tables beside the
+// activation rings.
+namespace wide {
+
+constexpr int kDecodeWarps = 8;              // warps 0-3: first half of the steps, warps 4-7: second half
+constexpr int kWStage = 32 * 128;            // bytes of a weight stage: 32 rows x 128 bytes (256 codes), swizzled by TMA
+constexpr int kXMaxStages = 8;               // stages of an MMA issuer's activation ring, at most
+constexpr int kTaThreads = 16 * 32;
+template <int FMT, int NB>
+struct Cols {
+    static constexpr int kRing = 2;                                 // groups a half may have in flight
+    static constexpr int kAccBufs = NB == 64 ? 1 : 2;               // accumulators of an issuer
+    static constexpr int kAcc = 2 * kRing * 64;                     // accumulator b of issuer i at kAcc + (i * kAccBufs + b) * NB
+    static constexpr int kParts = NB == 64 ? 1 : 4;
+    static_assert(kAcc + 4 * kAccBufs * NB <= 512, "tensor memory");
+    // one barrier per accumulator says that a group's MMAs are done, to the fold threads and to the decode threads that
+    // wait for the group's slot; before a slot's next group is written, no later group can have used the accumulator
+    static_assert(2 * kAccBufs >= kRing, "the barrier would be a phase ahead");
+};
+
+struct Smem {
+    static constexpr int kWRing = 0;
+    static constexpr int kSW = 2;       // stages of a decode warp's weight ring (four did not change anything: the ring is not what the decode threads wait for)
+    static constexpr int kXRing = kWRing + kDecodeWarps * kSW * kWStage;
+    static constexpr int kXBytes = 152 * 1024;                      // two stages of 64 batch rows per issuer
+    static constexpr int kBars = kXRing + kXBytes + 512;            // + what the MMA reads past the last chunk (rows >= B)
+    static constexpr int kNumBars = kDecodeWarps * kSW + 6 + 2 * 8 + 4 * kXMaxStages;   // weights, A full, accumulator full/free, x full per issuer
+    static constexpr int kBytes = kBars + kNumBars * 8 + 1024;      // + slack for the 1 KB alignment of the base (TMA swizzle)
+    static constexpr int kExch = kXRing;                            // K split: partial sums, once nothing else uses the region
+    static_assert(kBytes <= 227 * 1024, "shared memory");
+};
+
+// geometry of an issuer's activation ring for a batch of B rows: a stage is one group (128 codes), 256 B bytes
+struct XGeom {
+    int chunk, ring, nstages;
+    __host__ __device__ XGeom(int B, int ring_bytes) {
+        chunk = 256 * B;
+        ring = ring_bytes;
+        nstages = ring_bytes / chunk < kXMaxStages ? ring_bytes / chunk : kXMaxStages;
+    }
+};
+
+template <int FMT, int NB>
+__global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_wide_kernel(const TaProblem *probs, const CUtensorMap *maps,
+                                                                const __grid_constant__ TaProblem single,
+                                                                const __grid_constant__ CUtensorMap single_map, int nprob,
+                                                                const int *tile_start, const int *cta_first,
+                                                                int B, int y_dtype, PeerInfo peers, int split, int *status) {
+    using C = Cols<FMT, NB>;
+    using S = Smem;
+    constexpr bool kGf4 = FMT == JQ_FMT_GF4;
+    constexpr int kRing = C::kRing;
+    constexpr int kSW = S::kSW;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_err;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // (uniform for the compiler)
+    const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t bars = sbase + S::kBars;
+    constexpr int kB0 = kDecodeWarps * kSW;
+    auto wbar = [&](int w, int s) { return bars + 8u * (w * kSW + s); };
+    auto abar = [&](int h, int s) { return bars + 8u * (kB0 + h * 3 + s); };                  // operand slot written
+    auto dbar = [&](int iss, int b) { return bars + 8u * (kB0 + 6 + iss * 2 + b); };          // accumulator complete: a group's MMAs are done
+    auto ebar = [&](int iss, int b) { return bars + 8u * (kB0 + 14 + iss * 2 + b); };         // accumulator folded
+    auto xbar = [&](int iss, int s) { return bars + 8u * (kB0 + 22 + iss * kXMaxStages + s); };   // issuer's stage filled
+    volatile int *err = &s_err;
+    const XGeom xg(B, S::kXBytes / 4);
+
+    if (tid == 0) {
+        s_err = 0;
+        for (int w = 0; w < kDecodeWarps; ++w)
+            for (int s = 0; s < kSW; ++s) mbar_init(wbar(w, s), 1);     // one arrive.expect_tx per fill
+        for (int h = 0; h < 2; ++h)
+            for (int s = 0; s < 3; ++s) mbar_init(abar(h, s), 128);     // the 128 decode threads of the half
+        for (int i = 0; i < 4; ++i)
+            for (int b = 0; b < 2; ++b) { mbar_init(dbar(i, b), 1); mbar_init(ebar(i, b), 128); }
+        for (int i = 0; i < 4; ++i)
+            for (int s = 0; s < kXMaxStages; ++s) mbar_init(xbar(i, s), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 15) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
+
+    // this CTA's tiles
+    int tile_lo, tile_hi, rank = 0;
+    if (nprob == 0) {   // one problem, passed by value: an even split of its tiles; with a K split one tile per cluster
+        const int nt = (single.N + kTileM - 1) / kTileM, n_cl = gridDim.x / split, cl = blockIdx.x / split;
+        rank = blockIdx.x - cl * split;
+        tile_lo = (int)((long long)nt * cl / n_cl);
+        tile_hi = (int)((long long)nt * (cl + 1) / n_cl);
+    } else {
+        tile_lo = cta_first[blockIdx.x];
+        tile_hi = cta_first[blockIdx.x + 1];
+    }
+    // parts of a row's sum, and the steps [lo, hi) of a row that this CTA works on
+    auto parts_of = [&](int nsteps) { return nsteps >= kPartMinSteps ? C::kParts : 1; };
+    auto step_lo = [&](int nsteps) { return split > 1 ? part_step(nsteps, C::kParts, C::kParts / split * rank) : 0; };
+    auto step_hi = [&](int nsteps) { return split > 1 ? part_step(nsteps, C::kParts, C::kParts / split * (rank + 1)) : nsteps; };
+    // Problems change rarely along a CTA's tile sequence: every walker keeps what it needs of its current
+    // problem in registers and goes back to global memory only for a tile beyond that problem's last one.
+    auto problem_at = [&](int &pi, int &t_end, int tile, TaProblem &p) {
+        if (nprob == 0) { p = single; t_end = 0x7fffffff; return; }
+        if (t_end < 0) {
+            // first look-up of a walker: bisect (a step's list can hold hundreds of problems, and a scan from the
+            // first one is a chain of dependent global loads, 0.2 us each, in front of the last CTAs' first tile)
+            int lo = 0, hi = nprob - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (tile_start[mid] <= tile) lo = mid; else hi = mid - 1;
+            }
+            pi = lo;
+        } else {
+            while (pi + 1 < nprob && tile_start[pi + 1] <= tile) ++pi;
+        }
+        p = probs[pi];
+        t_end = tile_start[pi + 1];
+    };
+
+    if (warp < kDecodeWarps) {
+        // =============================== decode threads ===============================
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");     // 256 x 112 + 128 x 184 + 128 x 96 of 65536 registers
+        const int q = warp & 3, h = warp >> 2;
+        const int r = q * 32 + lane;                       // row of the tile = tensor-memory lane
+        const uint32_t lane_t = tmem + ((uint32_t)(q * 32) << 16);
+        const uint32_t wring = sbase + S::kWRing + warp * (kSW * kWStage);     // + stage * kWStage; 1 KB aligned
+        // 16-byte piece c of this lane's row sits at piece c ^ (lane & 7) of the row (128-byte swizzle)
+        const uint32_t lrow = lane * 128, lkey = (lane & 7) << 4;
+
+        // ---- producer side of the weight ring: the (tile, step) whose box is requested next
+        int i_tile = tile_lo, i_pi = 0, i_tend = -1, i_j = 0, i_n = 0, i_x = 0, i_x0 = 0, i_y = 0, i_tile0 = 0, i_steps = 0, i_stage = 0;
+        const void *i_map = nullptr;
+        auto i_open = [&]() {
+            while (i_tile < tile_hi) {
+                if (i_tile >= i_tend) {
+                    TaProblem p;
+                    problem_at(i_pi, i_tend, i_tile, p);
+                    const int ns = p.K >> 8, lo = step_lo(ns);
+                    i_steps = (step_hi(ns) - lo - h + 1) >> 1;
+                    i_x0 = (lo + h) * 128;
+                    i_tile0 = p.tile0;
+                    i_map = nprob ? &maps[i_pi] : &single_map;
+                }
+                i_n = i_steps;
+                i_x = i_x0;
+                i_y = (i_tile - i_tile0) * kTileM + q * 32;     // rows past N read as zeros
+                i_j = 0;
+                if (i_n > 0) return;
+                ++i_tile;
+            }
+        };
+        auto issue = [&]() {
+            if (i_tile < tile_hi) {
+                if (lane == 0) {
+                    const uint32_t bar = wbar(warp, i_stage);
+                    mbar_expect_tx(bar, kWStage);
+                    tma_2d_g2s(wring + i_stage * kWStage, i_map, i_x, i_y, bar);
+                }
+                i_x += 256;
+                if (++i_j == i_n) { ++i_tile; i_open(); }
+            }
+            i_stage = (i_stage + 1 == kSW) ? 0 : i_stage + 1;
+        };
+        i_open();
+#pragma unroll
+        for (int s = 0; s < kSW; ++s) issue();
+
+        // ---- per-row side data one tile ahead: GF4 codebook row
+        int f_pi = 0, f_tend = -1, f_tile0 = 0, f_N = 1;
+        const __half *f_cb = nullptr;
+        uint4 cb0 = make_uint4(0, 0, 0, 0), cb1 = cb0;
+        auto fetch_codebook = [&](int tile) {
+            if (kGf4 && tile < tile_hi) {
+                if (tile >= f_tend) {
+                    TaProblem p;
+                    problem_at(f_pi, f_tend, tile, p);
+                    f_tile0 = p.tile0; f_N = p.N; f_cb = p.codebook;
+                }
+                const int row = min((tile - f_tile0) * kTileM + r, f_N - 1);
+                const uint4 *src = reinterpret_cast<const uint4 *>(f_cb + (size_t)row * 16);
+                cb0 = __ldg(src);
+                cb1 = __ldg(src + 1);
+            }
+        };
+
+        // ---- consumer state
+        int w_stage = 0, slot = 0, pend_slot = -1;   // pend_slot: its tensor-memory stores are issued but not yet handed over
+        uint32_t w_par = 0;
+        uint32_t t_next = 0;                         // groups this half has decoded so far
+        Codebook book;
+        auto hand_over = [&]() {
+            if (pend_slot >= 0) {
+                tmem_wait_st();
+                tc_fence_before();
+                mbar_arrive(abar(h, pend_slot));
+                pend_slot = -1;
+            }
+        };
+        int c_pi = 0, c_tend = -1;
+        TaProblem p = single;
+        fetch_codebook(tile_lo);
+        bool ok = true;
+        for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
+            if (tile >= c_tend) problem_at(c_pi, c_tend, tile, p);
+            const int s_lo = step_lo(p.K >> 8), s_hi = step_hi(p.K >> 8);
+            // E2M1: eight fp16 scales (16 bytes) per 256-code step of the row, a step ahead
+            const int row = min((tile - p.tile0) * kTileM + r, p.N - 1);
+            const uint4 *srow = reinterpret_cast<const uint4 *>(p.scales + (size_t)row * p.lds);
+            uint4 sc_nxt = make_uint4(0, 0, 0, 0);
+            if (!kGf4 && s_lo + h < s_hi) sc_nxt = __ldg(srow + s_lo + h);
+            if constexpr (kGf4) book.set(cb0, cb1);
+            fetch_codebook(tile + 1);
+            for (int sg = s_lo + h; sg < s_hi; sg += 2) {
+                ok = __all_sync(0xffffffffu, mbar_wait(wbar(warp, w_stage), w_par, err));
+                if (!ok) break;
+                const uint32_t src = wring + w_stage * kWStage + lrow;
+                if (++w_stage == kSW) { w_stage = 0; w_par ^= 1; }
+                const uint4 sc_cur = sc_nxt;
+                if (!kGf4 && sg + 2 < s_hi) sc_nxt = __ldg(srow + sg + 2);
+#pragma unroll
+                for (int gi = 0; gi < 2; ++gi) {
+                    const uint2 sc4 = gi ? make_uint2(sc_cur.z, sc_cur.w) : make_uint2(sc_cur.x, sc_cur.y);
+                    const uint32_t a_t = lane_t + (h * kRing + slot) * 64;
+                    uint4 w4[4];
+#pragma unroll
+                    for (int part = 0; part < 4; ++part) w4[part] = lds128(src + (((gi * 4 + part) << 4) ^ lkey));
+                    // 32 codes (four words) -> 16 fp16 pairs
+                    auto decode16 = [&](int part, uint32_t (&v)[16]) {
+#pragma unroll
+                        for (int wi = 0; wi < 4; ++wi) {
+                            const uint32_t w = wi == 0 ? w4[part].x : (wi == 1 ? w4[part].y : (wi == 2 ? w4[part].z : w4[part].w));
+                            if constexpr (kGf4) {
+                                uint32_t hh[4];
+                                book.look_up8(w, hh);
+#pragma unroll
+                                for (int bj = 0; bj < 4; ++bj) v[wi * 4 + bj] = hh[bj];
+                            } else {
+                                // E2M1: the group scale folded into the fp16 weight (one rounding per weight)
+                                const uint32_t pr = part < 2 ? sc4.x : sc4.y;
+                                const uint32_t s2 = prmt(pr, pr, (part & 1) ? 0x3232 : 0x1010);
+                                uint32_t hh[4];
+                                asm("{ .reg .b8 b0, b1, b2, b3; mov.b32 {b0, b1, b2, b3}, %4;\n"
+                                    "  cvt.rn.f16x2.e2m1x2 %0, b0; cvt.rn.f16x2.e2m1x2 %1, b1;\n"
+                                    "  cvt.rn.f16x2.e2m1x2 %2, b2; cvt.rn.f16x2.e2m1x2 %3, b3; }"
+                                    : "=r"(hh[0]), "=r"(hh[1]), "=r"(hh[2]), "=r"(hh[3]) : "r"(w));
+#pragma unroll
+                                for (int bj = 0; bj < 4; ++bj)
+                                    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(v[wi * 4 + bj]) : "r"(hh[bj]), "r"(s2));
+                            }
+                        }
+                    };
+                    // the decode of the next 32 codes is issued before the previous 16 pairs are stored, and the
+                    // previous group is handed to the MMA issuer only once this group's first lookups are under way
+                    // (its tensor-memory stores have had that long to land), and before the wait for this group's slot
+                    uint32_t va[16], vb[16];
+                    decode16(0, va);
+                    decode16(1, vb);
+                    hand_over();
+                    // the slot is free once the MMAs of the group that used it last are done
+                    if (t_next >= (uint32_t)kRing) {
+                        const uint32_t t = t_next - kRing, n = t >> 1;     // group t was its issuer's n-th
+                        ok = __all_sync(0xffffffffu, mbar_wait(dbar(h + 2 * (t & 1), n % C::kAccBufs), (n / C::kAccBufs) & 1, err));
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
+                    ++t_next;
+                    tmem_st16(a_t, va);
+                    decode16(2, va);
+                    tmem_st16(a_t + 16, vb);
+                    decode16(3, vb);
+                    tmem_st16(a_t + 32, va);
+                    tmem_st16(a_t + 48, vb);
+                    pend_slot = slot;
+                    if (++slot == kRing) slot = 0;
+                }
+                if (!ok) break;
+                __syncwarp();                           // every lane has read its row of the stage
+                fence_async_smem();
+                issue();                                // refill the stage just read
+            }
+            hand_over();
+        }
+        if (split > 1) { __syncwarp(); cluster_sync(); cluster_sync(); }
+    } else if (warp < 12) {
+        // =============================== fold threads ===============================
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+        const int r = tid & 127;
+        const uint32_t lane_t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::kAcc;
+        uint32_t counts = 0;                        // steps of each half so far, modulo 4 (two bits each)
+        int c_pi = 0, c_tend = -1;
+        TaProblem p = single;
+        pdl_wait();                                 // the row factors of the prepared activation are read below
+        bool ok = true;
+        for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
+            if (tile >= c_tend) problem_at(c_pi, c_tend, tile, p);
+            const int row_raw = (tile - p.tile0) * kTileM + r, row = min(row_raw, p.N - 1);
+            const int nsteps = p.K >> 8, parts = parts_of(nsteps), s_lo = step_lo(nsteps), s_hi = step_hi(nsteps);
+            const unsigned short *srow = reinterpret_cast<const unsigned short *>(p.scales) + (size_t)row * p.lds;
+            const int gshift = kGf4 ? 31 - __clz(p.g >> 7) : 0;   // GF4: log2 of the 128-code groups per scale
+            float xs[(NB + 31) / 32];
+#pragma unroll
+            for (int i = 0; i < (NB + 31) / 32; ++i) xs[i] = (lane + 32 * i < B) ? p.xscale[lane + 32 * i] : 0.f;
+            const float bias = (p.bias && row_raw < p.N) ? p.bias[row_raw] : 0.f;
+            float acc[NB], total[C::kParts > 1 ? NB : 1];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) acc[b] = 0.f;
+            const uint32_t exch = sbase + S::kExch + r * 4;
+            int part = split > 1 ? C::kParts / split * rank : 0, part_end = part_step(nsteps, parts, part + 1);
+            bool first = true;
+            unsigned short raw0 = 0, raw1 = 0;
+            auto load_scales = [&](int sg) {
+                if (kGf4) { raw0 = __ldg(srow + ((2 * sg) >> gshift)); raw1 = __ldg(srow + ((2 * sg + 1) >> gshift)); }
+            };
+            load_scales(s_lo);
+            for (int sg = s_lo; sg < s_hi && ok; ++sg) {
+                const int h = (sg - s_lo) & 1;
+                const uint32_t cnt = (counts >> (2 * h)) & 3;
+                const uint32_t buf = C::kAccBufs == 2 ? cnt & 1 : 0, par = C::kAccBufs == 2 ? cnt >> 1 : cnt & 1;
+                const float sc[2] = {__half2float(__ushort_as_half(raw0)), __half2float(__ushort_as_half(raw1))};
+                if (sg + 1 < s_hi) load_scales(sg + 1);
+#pragma unroll
+                for (int gi = 0; gi < 2; ++gi) {
+                    const int iss = h + 2 * gi;
+                    ok = __all_sync(0xffffffffu, mbar_wait(dbar(iss, buf), par, err));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t d_t = lane_t + (iss * C::kAccBufs + buf) * NB;
+#pragma unroll
+                    for (int c = 0; c < NB; c += 32) {
+                        uint32_t d[32];
+                        tmem_ld32(d_t + c, d);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 32; i += 2) fma2(acc[c + i], acc[c + i + 1], d[i], d[i + 1], kGf4 ? sc[gi] : 1.f);
+                    }
+                    tc_fence_before();
+                    mbar_arrive(ebar(iss, buf));
+                }
+                if (!ok) break;
+                counts = (counts & ~(3u << (2 * h))) | (((cnt + 1) & 3) << (2 * h));
+                if (C::kParts > 1 && sg + 1 == part_end) {      // a part of the row's sum is complete
+                    if (split > 1) {        // at most two per CTA: the first waits in `total`, the second stays in `acc`
+                        if (first) {
+#pragma unroll
+                            for (int b = 0; b < NB; ++b) { total[b] = acc[b]; acc[b] = 0.f; }
+                        }
+                    } else {
+#pragma unroll
+                        for (int b = 0; b < NB; ++b) {
+                            total[b] = first ? acc[b] : total[b] + acc[b];
+                            acc[b] = 0.f;
+                        }
+                    }
+                    first = false;
+                    ++part;
+                    part_end = part_step(nsteps, parts, part + 1);
+                }
+            }
+            if constexpr (C::kParts > 1) {
+                if (split > 1) {
+                    // every group of this CTA has been folded: nothing reads the tables or the activation rings any more.
+                    // Each CTA leaves its parts in its shared memory; rank k writes columns k, k + split, ...
+                    const int per = C::kParts / split;
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(exch + b * 512), "f"(total[b]) : "memory");
+                        if (per == 2) asm volatile("st.shared.f32 [%0], %1;" ::"r"(exch + (NB + b) * 512), "f"(acc[b]) : "memory");
+                    }
+                    cluster_sync();
+                    for (int b = rank; b < B; b += split) {
+                        float v = ld_cluster_f32(exch + b * 512, 0);
+                        for (int i = 1; i < C::kParts; ++i) v += ld_cluster_f32(exch + ((i % per) * NB + b) * 512, i / per);
+                        if (ok && row_raw < p.N) jq::store_out(p.y, (size_t)b * p.ldy + row_raw, fmaf(v, p.xscale[b], bias), y_dtype);
+                    }
+                    cluster_sync();
+                    break;
+                }
+            }
+            if (!ok) break;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const float xs_b = __shfl_sync(0xffffffffu, xs[b >> 5], b & 31);
+                const float v = C::kParts > 1 ? total[C::kParts > 1 ? b : 0] : acc[b];
+                acc[b] = fmaf(v, xs_b, bias);
+            }
+            if (row_raw < p.N) {
+                for (int cpy = 0; cpy < peers.n; ++cpy) {
+                    char *yb = reinterpret_cast<char *>(p.y) + jq::peer_offset(peers.delta, cpy);
+#pragma unroll
+                    for (int b = 0; b < NB; ++b)
+                        if (b < B) jq::store_out(yb, (size_t)b * p.ldy + row_raw, acc[b], y_dtype);
+                }
+            }
+        }
+    } else {
+        // =============================== MMA issuers ===============================
+        // Warps 12, 13: half 0, 1; warps 14, 15: the second issuer per half.  A half's groups alternate between its
+        // issuers (the first group of every 256-code step to one, the second to the other).
+        // Every issuer owns a ring of activation stages (one 128-code group each) that it fills itself, so the
+        // only things it ever waits for are the decode and fold threads and its own earlier work.
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+        const int h = (warp - 12) & 1, sub = (warp - 12) >> 1, iss = warp - 12;
+        // (the warps run converged, see mma_f16_ts)
+        {
+            const uint32_t elected = elect_one();
+            auto wait = [&](uint32_t bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)); };
+            constexpr uint32_t idesc = idesc_f16(kTileM, NB);
+            const uint32_t lbo = (uint32_t)B * 16;
+            const uint32_t ring = sbase + S::kXRing + iss * xg.ring;
+            // two walks over the same sequence of groups: the loads run ahead of the MMAs
+            struct Walk { int tile, pi, t_end, lo, hi, sg; const unsigned char *xp; };
+            auto open_tile = [&](Walk &w) {
+                while (w.tile < tile_hi) {
+                    if (w.tile >= w.t_end) {
+                        TaProblem p;
+                        problem_at(w.pi, w.t_end, w.tile, p);
+                        w.lo = step_lo(p.K >> 8);
+                        w.hi = step_hi(p.K >> 8);
+                        w.xp = reinterpret_cast<const unsigned char *>(p.xprep);
+                    }
+                    w.sg = w.lo + h;
+                    if (w.sg < w.hi) return;
+                    ++w.tile;
+                }
+            };
+            auto advance = [&](Walk &w) {
+                w.sg += 2;
+                if (w.sg >= w.hi) { ++w.tile; open_tile(w); }
+            };
+            Walk ld = {tile_lo, 0, -1, 0, 0, 0, nullptr};
+            open_tile(ld);
+            Walk mm = ld;
+            // An issuer shares its scheduler with two decode warps, so every instruction of this loop costs several clocks:
+            // ring positions and parities are carried along instead of being divided out of counters, and the operand
+            // descriptor is formed once per group.
+            uint32_t ld_s = 0;                          // stage the next load goes to
+            auto load_next = [&]() {
+                if (ld.tile < tile_hi) {
+                    const int G = 2 * ld.sg + sub;
+                    if (elected) {
+                        mbar_expect_tx(xbar(iss, ld_s), xg.chunk);
+                        bulk_g2s(ring + ld_s * xg.chunk, ld.xp + (size_t)G * xg.chunk, xg.chunk, xbar(iss, ld_s));
+                    }
+                    __syncwarp();
+                    advance(ld);
+                }
+                ld_s = (ld_s + 1 == (uint32_t)xg.nstages) ? 0 : ld_s + 1;
+            };
+            pdl_wait();
+            for (int i = 0; i < xg.nstages; ++i) load_next();
+            bool ok = true;
+            uint32_t cs = 0, cpar = 0;                  // stage and phase parity of the group being multiplied
+            uint32_t slot = (uint32_t)sub % kRing, spar = 0;   // A slot of this issuer's next group (the half's group count t = 2 n + sub)
+            uint32_t db = 0, dpar = 1;                  // accumulator (the first round finds it free)
+            const bool tight = xg.nstages <= C::kAccBufs;
+            const uint32_t desc_step = (2 * lbo) >> 4;  // descriptor address field per K = 16 slice
+            for (uint32_t n = 0; mm.tile < tile_hi && ok; ++n) {
+                // a ring with no more stages than accumulators refills the previous group's stage once its MMAs are done
+                if (tight && n > 0) {
+                    if (!(ok = wait(dbar(iss, (n - 1) % C::kAccBufs), ((n - 1) / C::kAccBufs) & 1))) break;
+                    load_next();
+                }
+                // the accumulator's last group has been folded, so its MMAs have read their activation stage: refill that
+                if (!(ok = wait(ebar(iss, db), dpar))) break;
+                if (!tight && n >= (uint32_t)C::kAccBufs) load_next();
+                if (!(ok = wait(xbar(iss, cs), cpar))) break;
+                if (!(ok = wait(abar(h, slot), spar))) break;
+                tc_fence_after();
+                const uint32_t a_t = tmem + (h * kRing + slot) * 64;
+                const uint32_t d_t = tmem + C::kAcc + (iss * C::kAccBufs + db) * NB;
+                const uint64_t desc0 = smem_desc(ring + cs * xg.chunk, lbo, 128);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    mma_f16_ts(elected, d_t, a_t + 8 * i, desc0 + (uint64_t)(i * desc_step), idesc, i > 0);
+                mma_commit(elected, dbar(iss, db));
+                if (++cs == (uint32_t)xg.nstages) { cs = 0; cpar ^= 1; }
+                if (++db == (uint32_t)C::kAccBufs) { db = 0; dpar ^= 1; }
+                slot += 2;
+                if (slot >= (uint32_t)kRing) { slot -= kRing; spar ^= 1; }
+                advance(mm);
+            }
+        }
+        if (split > 1) { __syncwarp(); cluster_sync(); cluster_sync(); }
+    }
+
+    // ---- teardown
+    if (*err) {   // a wait gave up: let the copies still in flight land before the CTA's shared memory goes away
+        for (int i = 0; i < 400; ++i) __nanosleep(256);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0 && s_err) atomicExch(status, s_err);
+    if (warp == 15) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+}  // namespace wide
 
 // ---- GF4, batch 1 on the CUDA cores (the template also covers two rows, where the tensor-memory kernel is faster) ----
 // Same tiles, same TMA weight ring, same per-row pair tables as the tensor-memory kernel above, but the
@@ -1093,7 +1560,7 @@ extern "C" int jq_ta_plan(int fmt, const jq_problem *ph, int n, int B, void *wor
         int st = ta_fill_problem(tp[i], fmt, ph[i], reinterpret_cast<unsigned char *>(workspace_dev), off, B);
         if (st) return st;
         CUtensorMap tm;
-        st = ta_encode_map(&tm, ph[i].qweight, ph[i].N, ph[i].K >> 1, lut ? 32 : kTileM);
+        st = ta_encode_map(&tm, ph[i].qweight, ph[i].N, ph[i].K >> 1, (lut || B > NB) ? 32 : kTileM);
         if (st) return st;
         memcpy(maps + (size_t)i * sizeof(CUtensorMap), &tm, sizeof(CUtensorMap));
         const int tiles = (ph[i].N + tile_m - 1) / tile_m;
@@ -1136,7 +1603,7 @@ static void ta_pdl_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2
     cfg.numAttrs = cluster > 1 ? 2 : 1;
 }
 
-template <int FMT, int NB>
+template <int FMT, int COLS>
 static int ta_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, const TaProblem &single,
                      const CUtensorMap &single_map, int nprob, const int *tile_start,
                      const int *cta_first, int grid, int B, int x_dtype, int y_dtype, const jqta::PeerInfo &peers,
@@ -1146,18 +1613,28 @@ static int ta_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, co
     else ta_prepare_kernel<256><<<nblk, 256, 0, st>>>(probs_dev, single, B, x_dtype);
     int s = jq_launch_status();
     if (s) return s;
-    auto kern = gemm_ta_kernel<FMT, NB>;
-    using C = Cols<FMT, NB>;
-    constexpr int smem = Smem<C::kTable, NB>::kBytes;
+    void (*kern)(const TaProblem *, const CUtensorMap *, const TaProblem, const CUtensorMap, int, const int *, const int *, int, int,
+                 jqta::PeerInfo, int, int *);
+    int smem, threads;
+    constexpr int parts = COLS == 64 ? 1 : 4;
+    if constexpr (COLS == NB) {
+        kern = gemm_ta_kernel<FMT>;
+        smem = Smem<FMT == JQ_FMT_GF4>::kBytes;
+        threads = kTaThreads;
+    } else {
+        kern = wide::gemm_ta_wide_kernel<FMT, COLS>;
+        smem = wide::Smem::kBytes;
+        threads = wide::kTaThreads;
+    }
     // A single matrix with few tiles: 4 or 2 CTAs take parts of every row (N = 4096 is 32 tiles for 148 SMs)
     int split = 1;
-    if (!nprob && C::kParts == 4 && (single.K >> 8) >= kPartMinSteps)
+    if (!nprob && parts == 4 && (single.K >> 8) >= kPartMinSteps)
         split = grid * 4 <= jq_sm_count() ? 4 : (grid * 2 <= jq_sm_count() ? 2 : 1);
     static std::atomic<unsigned long long> done{0};
     JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(kern), smem, done));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
-    ta_pdl_config(cfg, attr, grid * split, kTaThreads, smem, split, st);
+    ta_pdl_config(cfg, attr, grid * split, threads, smem, split, st);
     JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, probs_dev, maps_dev, single, single_map, nprob, tile_start, cta_first, B, y_dtype,
                                    peers, split, status));
     return jq_launch_status();
@@ -1246,7 +1723,7 @@ extern "C" int jq_gemm_ta(int fmt, const void *qweight, const void *scales, cons
     if (st) return st;
     CUtensorMap tm;
     const bool lut = fmt == JQ_FMT_GF4 && ta_use_lut(B, K);
-    st = ta_encode_map(&tm, qweight, N, K >> 1, lut ? 32 : kTileM);
+    st = ta_encode_map(&tm, qweight, N, K >> 1, (lut || B > NB) ? 32 : kTileM);
     if (st) return st;
     jqta::PeerInfo peers;
     peers.n = 1;
