@@ -67,22 +67,48 @@ struct PeerInfo {
 // layout of the MMA with a piece stride of 16 B bytes: row n of piece c sits at (c B + n) 16 bytes.  The MMA
 // reads 16, 32 or 64 rows; rows >= B are whatever follows (the next pieces), and their accumulator columns
 // are never read.
-// The second pass is a chain of load -> rotate -> store per 128-element block and warp, and its latency is what a
-// decode step waits for before the main kernel can start.  With one or two batch rows there are few blocks: 32 warps
-// each (K = 11008: 3 rounds instead of 11; 4.5 us less per 7B-shaped step).  With many batch rows 8 warps per block
-// keep more rows resident per SM.
-template <int kPrepThreads>
-__global__ void __launch_bounds__(kPrepThreads) ta_prepare_kernel(const TaProblem *probs, TaProblem single, int B,
-                                                                   int x_dtype) {
-    constexpr int kWarps = kPrepThreads / 32;
+// A thread has the same four elements of every 128 kWarps in both passes (maximum; rotation) and keeps what it has loaded, up
+// to kKeep times four.  The pass is a chain of load -> rotate -> store per warp, and its latency is what a call waits for before
+// the main kernel can start: few blocks (a single call, a decode step of one row) have 32 warps each; with many, 8 warps per
+// block keep more rows resident per SM.
+template <class T> __device__ __forceinline__ float4 load_four(const T *x, bool vec);
+template <> __device__ __forceinline__ float4 load_four<float>(const float *x, bool vec) {
+    return vec ? *reinterpret_cast<const float4 *>(x) : make_float4(x[0], x[1], x[2], x[3]);
+}
+template <> __device__ __forceinline__ float4 load_four<__half>(const __half *x, bool vec) {
+    if (!vec) return make_float4(__half2float(x[0]), __half2float(x[1]), __half2float(x[2]), __half2float(x[3]));
+    const uint2 u = *reinterpret_cast<const uint2 *>(x);
+    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+template <> __device__ __forceinline__ float4 load_four<__nv_bfloat16>(const __nv_bfloat16 *x, bool vec) {
+    if (!vec) return make_float4(__bfloat162float(x[0]), __bfloat162float(x[1]), __bfloat162float(x[2]), __bfloat162float(x[3]));
+    const uint2 u = *reinterpret_cast<const uint2 *>(x);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                       __uint_as_float(u.y & 0xffff0000u));
+}
+template <int kPrepThreads, class T>
+__global__ void __launch_bounds__(kPrepThreads) ta_prepare_kernel(const TaProblem *probs, TaProblem single, int B) {
+    constexpr int kWarps = kPrepThreads / 32, kKeep = 4;
     __shared__ float sred[kWarps];
     __shared__ int sexp;
     pdl_launch_dependents();
     const int pi = blockIdx.x / B, b = blockIdx.x % B;
     const TaProblem p = probs ? probs[pi] : single;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const T *const x = reinterpret_cast<const T *>(p.x) + (size_t)b * p.K;       // (K is a multiple of 256)
+    const bool vec = ((size_t)p.x & (4 * sizeof(T) - 1)) == 0;
+    float4 kept[kKeep];
     float m = 0.f;
-    for (int k = tid; k < p.K; k += kPrepThreads) m = fmaxf(m, fabsf(jq::load_act(p.x, (size_t)b * p.K + k, x_dtype)));
+    auto largest = [&](const float4 &q) { m = fmaxf(m, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w)))); };
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i) {
+        const int k = (tid + i * kPrepThreads) * 4;
+        kept[i] = k < p.K ? load_four(x + k, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i) largest(kept[i]);
+    for (int k = (tid + kKeep * kPrepThreads) * 4; k < p.K; k += kPrepThreads * 4) largest(load_four(x + k, vec));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (lane == 0) sred[warp] = m;
@@ -98,17 +124,18 @@ __global__ void __launch_bounds__(kPrepThreads) ta_prepare_kernel(const TaProble
     }
     __syncthreads();
     const float down = __uint_as_float((uint32_t)(127 - sexp) << 23);
-    for (int blk = warp; blk * 128 < p.K; blk += kWarps) {
-        float v[4];
-        const int k0 = blk * 128 + lane * 4;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = jq::load_act(p.x, (size_t)b * p.K + k0 + j, x_dtype) * down;
+    auto finish = [&](int blk, const float4 &q) {
+        float v[4] = {q.x * down, q.y * down, q.z * down, q.w * down};
         if (p.had) jq::fwht128_warp(v, lane);
         __half2 h01 = __floats2half2_rn(v[0], v[1]), h23 = __floats2half2_rn(v[2], v[3]);
         const size_t off = (((size_t)blk * 16 + (lane >> 1)) * B + b) * 8 + (lane & 1) * 4;
         *reinterpret_cast<uint2 *>(p.xprep + off) =
             make_uint2(*reinterpret_cast<uint32_t *>(&h01), *reinterpret_cast<uint32_t *>(&h23));
-    }
+    };
+#pragma unroll
+    for (int i = 0; i < kKeep; ++i)
+        if ((warp + i * kWarps) * 128 < p.K) finish(warp + i * kWarps, kept[i]);
+    for (int blk = warp + kKeep * kWarps; blk * 128 < p.K; blk += kWarps) finish(blk, load_four(x + blk * 128 + lane * 4, vec));
 }
 
 // ---- main kernel --------------------------------------------------------------------
@@ -1603,15 +1630,25 @@ static void ta_pdl_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2
     cfg.numAttrs = cluster > 1 ? 2 : 1;
 }
 
+static int ta_prepare(const TaProblem *probs_dev, const TaProblem &single, int nblk, int B, int x_dtype, cudaStream_t st) {
+    // up to two blocks of 32 warps per SM.  Single calls, with values loaded one by one by 8 warps before: 4096 x 11008 E2M1, 23
+    // rows, 16.8 -> 14.8 us; 4096 x 14336, 16 rows, 18.0 -> 14.8; the 7B-shaped GF4 step with 8 rows (1792 blocks of 8 warps,
+    // loads of four values) 939 -> 927.
+    const bool wide = nblk <= 2 * jq_sm_count() || B <= 2;
+    void (*const kernels[3][2])(const TaProblem *, TaProblem, int) = {
+        {ta_prepare_kernel<256, float>, ta_prepare_kernel<1024, float>},
+        {ta_prepare_kernel<256, __half>, ta_prepare_kernel<1024, __half>},
+        {ta_prepare_kernel<256, __nv_bfloat16>, ta_prepare_kernel<1024, __nv_bfloat16>}};
+    kernels[x_dtype][wide]<<<nblk, wide ? 1024 : 256, 0, st>>>(probs_dev, single, B);
+    return jq_launch_status();
+}
+
 template <int FMT, int COLS>
 static int ta_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, const TaProblem &single,
                      const CUtensorMap &single_map, int nprob, const int *tile_start,
                      const int *cta_first, int grid, int B, int x_dtype, int y_dtype, const jqta::PeerInfo &peers,
                      int *status, cudaStream_t st) {
-    const int nblk = (nprob ? nprob : 1) * B;
-    if (B <= 2) ta_prepare_kernel<1024><<<nblk, 1024, 0, st>>>(probs_dev, single, B, x_dtype);
-    else ta_prepare_kernel<256><<<nblk, 256, 0, st>>>(probs_dev, single, B, x_dtype);
-    int s = jq_launch_status();
+    const int s = ta_prepare(probs_dev, single, (nprob ? nprob : 1) * B, B, x_dtype, st);
     if (s) return s;
     void (*kern)(const TaProblem *, const CUtensorMap *, const TaProblem, const CUtensorMap, int, const int *, const int *, int, int,
                  jqta::PeerInfo, int, int *);
@@ -1645,8 +1682,7 @@ static int lut2_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, 
                        const CUtensorMap &single_map, int nprob, const int *tile_start, const int *cta_first, int grid,
                        int x_dtype, int y_dtype, const jqta::PeerInfo &peers, int *status, cudaStream_t st) {
     if (nprob) {
-        ta_prepare_kernel<1024><<<nprob * B, 1024, 0, st>>>(probs_dev, single, B, x_dtype);
-        const int s = jq_launch_status();
+        const int s = ta_prepare(probs_dev, single, nprob * B, B, x_dtype, st);
         if (s) return s;
     }
     auto kern = nprob ? gf4_lut2_kernel<B, false> : gf4_lut2_kernel<B, true>;

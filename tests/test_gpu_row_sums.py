@@ -91,3 +91,22 @@ def test_one_row_prepared_in_the_kernel_or_in_front_of_it(K, had, dtype):
         y = ops.linear(x, pw)
         assert torch.equal(y.view(torch.uint8), grp.ys[0].view(torch.uint8))
     assert grp.status() == 0 and ops.check_status(raise_on_error=False) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("K", [512, 4352, 16640])
+def test_activation_prepared_by_wide_and_narrow_blocks(K, dtype):
+    """Few rows are prepared by blocks of 32 warps, the 320 of a large step by blocks of 8, which keep fewer of a row's values
+    between their passes (up to 16384 and 4096): the same bits, also from an activation that starts off a vector boundary."""
+    pw = jq.pack_weight(_weights(40, K, K).to(DEV), jq.QuantSpec("gf4", 128, 128))
+    grp = ops.GroupedGemv([pw] * 40, 8, dtype)
+    gen = torch.Generator("cpu").manual_seed(K)
+    for x in grp.xs:
+        x.copy_(torch.randn(x.shape, generator=gen))
+    grp.run()
+    assert grp.status() == 0
+    for i in (0, 17, 39):
+        raw = torch.zeros(8 * K + 1, dtype=dtype, device=DEV)
+        off = raw[1:].view(8, K)
+        off.copy_(grp.xs[i])
+        assert torch.equal(ops.linear(grp.xs[i], pw), grp.ys[i]) and torch.equal(ops.linear(off, pw), grp.ys[i])
