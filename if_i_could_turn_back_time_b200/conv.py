@@ -21,7 +21,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from .pack import PackedWeight, pack_weight
+from .pack import PackedWeight, pack_weight, packed_tensors
 from .spec import QuantSpec
 
 
@@ -66,8 +66,7 @@ class JenksQuantConv2d(nn.Conv2d):
             pw = pack_weight(W, self.spec, threads=self.threads).to(dense.device)   # on the GPU when the weight is there
             self.qweight, self.scales, self.codebook = pw.qweight, pw.scales, pw.codebook
         kc = self.in_channels * self.kernel_size[0] * self.kernel_size[1]
-        b = self._buffers             # (a module's look-up of a buffer as an attribute tries two other places first)
-        return PackedWeight(self.spec, self.out_channels, kc, b["qweight"], b["scales"], b["codebook"])
+        return PackedWeight(self.spec, self.out_channels, kc, *packed_tensors(self, JenksQuantConv2d))
 
     def weight_quantizer(self) -> torch.Tensor:
         """Dense quantised weight [O, I, kh, kw], as the Conv2d branch of the

@@ -20,7 +20,7 @@ import torch
 import torch.nn as nn
 
 from . import ops
-from .pack import PackedWeight, pack_weight
+from .pack import PackedWeight, pack_weight, packed_tensors
 from .spec import QuantSpec
 
 
@@ -61,8 +61,7 @@ class JenksQuantLinear(nn.Linear):
     def packed(self) -> PackedWeight:
         if self.qweight is None:
             self._pack()
-        b = self._buffers             # (a module's look-up of a buffer as an attribute tries two other places first)
-        return PackedWeight(self.spec, self.out_features, self.in_features, b["qweight"], b["scales"], b["codebook"])
+        return PackedWeight(self.spec, self.out_features, self.in_features, *packed_tensors(self, JenksQuantLinear))
 
     def _pack(self) -> None:
         dense = self._parameters["weight"]

@@ -41,6 +41,17 @@ class PackedWeight:
         return sum(t.numel() * t.element_size() for t in (self.qweight, self.scales, self.codebook) if t is not None)
 
 
+def packed_tensors(layer, plain: type):
+    """qweight, scales and codebook of a quantised layer, as its attributes.  The layer's class without any other on top
+    that has all three as buffers can only answer with those, and looking there takes 0.1 instead of 0.8 us per call;
+    parameters, parametrisations and subclasses are asked for their attributes."""
+    if type(layer) is plain:
+        b = layer._buffers
+        if "qweight" in b and "scales" in b and "codebook" in b:
+            return b["qweight"], b["scales"], b["codebook"]
+    return layer.qweight, layer.scales, layer.codebook
+
+
 GF4_DEVICE_MAX_K = 32768       # longest row of the GF4 packer on the GPU: it sorts a row, padded to a power of two, in shared memory
 
 

@@ -142,6 +142,36 @@ def test_convolution_refuses_an_image_that_is_not_the_layers(fmt, g, shape):
         jq.ops.conv2d(torch.randn(*shape), q.packed, q.bias, q.kernel_size, q.stride, q.padding, q.dilation)
 
 
+@pytest.mark.parametrize("make", [lambda: jq.JenksQuantLinear(nn.Linear(256, 8), 4),
+                                  lambda: jq.JenksQuantConv2d(nn.Conv2d(16, 8, 4), 4, group_size=128)], ids=["linear", "conv"])
+def test_packed_tensors_are_read_as_attributes(make):
+    """A packed tensor that has become a parameter, is computed by a parametrisation or by a property of another class is
+    what `packed` returns, as any other reader of the layer sees it."""
+    class Doubled(nn.Module):
+        def forward(self, t):
+            return t * 2
+
+    layer = make()
+    layer.commit()
+    q, s, c = layer.qweight, layer.scales, layer.codebook
+    assert layer.packed.qweight is q and layer.packed.scales is s and layer.packed.codebook is c
+    layer.qweight = nn.Parameter(q.clone(), requires_grad=False)
+    assert layer.packed.qweight is layer.qweight and torch.equal(layer.packed.qweight, q)
+    assert layer.packed.scales is s and layer.packed.codebook is c
+
+    layer = make()
+    layer.commit()
+    s = layer.scales.clone()
+    nn.utils.parametrize.register_parametrization(layer, "scales", Doubled(), unsafe=True)
+    assert torch.equal(layer.packed.scales, s * 2)
+
+    layer = make()
+    layer.commit()
+    c = layer.codebook.clone()
+    layer.__class__ = type("Other", (type(layer),), {"codebook": property(lambda self: self._buffers["codebook"] + 1)})
+    assert torch.equal(layer.packed.codebook, c + 1)
+
+
 @pytest.fixture
 def scratch(monkeypatch):
     """ops' scratch buffers on the CPU: one device, one stream, and a switch that says whether a graph is being captured."""
