@@ -1677,23 +1677,31 @@ static int ta_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, co
     return jq_launch_status();
 }
 
+// One row whose outputs are written over (part of) its own activation.  Such a call has its activation prepared by a launch in
+// front: where every CTA reads the row itself, another may already be writing to it.
+static bool ta_outputs_on_inputs(const TaProblem &p, int x_dtype, int y_dtype) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(p.x), y = reinterpret_cast<uintptr_t>(p.y);
+    return x < y + (uintptr_t)p.N * (y_dtype == JQ_F32 ? 4 : 2) && y < x + (uintptr_t)p.K * (x_dtype == JQ_F32 ? 4 : 2);
+}
+
 template <int B>
 static int lut2_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, const TaProblem &single,
                        const CUtensorMap &single_map, int nprob, const int *tile_start, const int *cta_first, int grid,
                        int x_dtype, int y_dtype, const jqta::PeerInfo &peers, int *status, cudaStream_t st) {
-    if (nprob) {
-        const int s = ta_prepare(probs_dev, single, nprob * B, B, x_dtype, st);
+    const bool own = !nprob && !ta_outputs_on_inputs(single, x_dtype, y_dtype);
+    if (!own) {
+        const int s = ta_prepare(probs_dev, single, (nprob ? nprob : 1) * B, B, x_dtype, st);
         if (s) return s;
     }
-    auto kern = nprob ? gf4_lut2_kernel<B, false> : gf4_lut2_kernel<B, true>;
+    auto kern = own ? gf4_lut2_kernel<B, true> : gf4_lut2_kernel<B, false>;
     constexpr int smem = LutSmem::kBytes;
     static_assert(smem <= 227 * 1024, "shared memory");
     static std::atomic<unsigned long long> done[2];
-    JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(kern), smem, done[nprob ? 0 : 1]));
+    JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(kern), smem, done[own ? 1 : 0]));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     ta_pdl_config(cfg, attr, grid, kLutThreads, smem, 1, st);
-    if (!nprob) cfg.numAttrs = 0;      // the activation is read from the start: after everything in front of it
+    if (own) cfg.numAttrs = 0;         // the activation is read from the start: after everything in front of it
     JQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, probs_dev, maps_dev, single, single_map, nprob, tile_start, cta_first, x_dtype,
                                    y_dtype, peers, status));
     return jq_launch_status();

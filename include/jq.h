@@ -234,7 +234,10 @@ int jq_gemv_grouped_peers(const jq_problem *problems_dev, const void *plan_host,
  * that are added in order; a single matrix with few tiles spreads the parts over
  * a cluster of CTAs, with the same result.
  * A launch is preceded by a small kernel that rotates, normalises and rounds
- * the activation to fp16 once per problem (not once per CTA).  The workspace
+ * the activation to fp16 once per problem (not once per CTA); in a single call
+ * with B == 1 on the CUDA cores every CTA does that itself and there is one
+ * launch, unless y overlaps x.  Either way all of x is read before anything is
+ * written, so y may lie on it.  The workspace
  * (128-byte aligned, jq_ta_workspace_bytes) holds that prepared activation and
  * a status word at offset 0, which must be zero before the first use and is
  * only ever raised by the kernels: every device-side wait is bounded (2^22

@@ -93,6 +93,35 @@ def test_one_row_prepared_in_the_kernel_or_in_front_of_it(K, had, dtype):
     assert grp.status() == 0 and ops.check_status(raise_on_error=False) == 0
 
 
+@pytest.mark.parametrize("xt,yt", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32),
+                                   (torch.float32, torch.float16)])
+@pytest.mark.parametrize("N,K", [(4096, 4096), (12000, 2048), (200, 12288)])
+def test_one_row_may_be_written_over_its_activation(xt, yt, N, K):
+    """jq_gemm_ta with y on x, and with y reaching over x's first and last element: the bits of the call with y elsewhere (the
+    row is read as a whole before anything is written).  With y right before or right behind x nothing overlaps."""
+    import ctypes
+    from if_i_could_turn_back_time_b200 import _lib
+    pw = jq.pack_weight(_weights(N, K, K).to(DEV), jq.QuantSpec("gf4", 128, 128))
+    lib, dt = _lib.load(), {torch.float32: _lib.JQ_F32, torch.float16: _lib.JQ_F16, torch.bfloat16: _lib.JQ_BF16}
+    p = lambda t, off=0: ctypes.c_void_p(t.data_ptr() + off)
+    ws = torch.zeros(1 << 20, dtype=torch.uint8, device=DEV)
+    xb, yb = K * xt.itemsize, N * yt.itemsize
+    x = torch.randn(1, K, generator=torch.Generator("cpu").manual_seed(N)).to(xt).to(DEV)
+
+    def call(x_ptr, y_ptr):
+        _lib.check(lib.jq_gemm_ta(pw.spec.fmt_id, p(pw.qweight), p(pw.scales), p(pw.codebook), x_ptr, None, y_ptr, N, K, 1, 128, 128,
+                                  dt[xt], dt[yt], p(ws), ws.numel(), ops._stream()), "jq_gemm_ta")
+
+    want = torch.empty(1, N, dtype=yt, device=DEV)
+    call(p(x), p(want))
+    for at in (0, 4 - yb, xb - 4, -yb, xb):                 # byte offset of y from x
+        arena = torch.zeros(xb + 2 * yb, dtype=torch.uint8, device=DEV)
+        arena[yb:yb + xb] = x.view(torch.uint8)[0]
+        call(p(arena, yb), p(arena, yb + at))
+        assert torch.equal(arena[yb + at:2 * yb + at], want.view(torch.uint8)[0])
+    assert lib.jq_ta_status(p(ws), 1, ops._stream()) == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("K", [512, 4352, 16640])
 def test_activation_prepared_by_wide_and_narrow_blocks(K, dtype):
