@@ -1,5 +1,6 @@
 // Version, error text, device queries, workspace sizing.
 #include "common.cuh"
+#include <cuda.h>
 #include <mutex>
 
 int jq_sm_count() {
@@ -15,6 +16,18 @@ int jq_sm_count() {
         cache[dev] = n;
     }
     return cache[dev];
+}
+
+unsigned long long jq_context_id() {
+    typedef CUresult (*get_id_fn)(CUcontext, unsigned long long *);
+    static const get_id_fn get = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        return (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &found) == cudaSuccess &&
+                found == cudaDriverEntryPointSuccess) ? reinterpret_cast<get_id_fn>(p) : nullptr;
+    }();
+    unsigned long long id = 0;
+    return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
 }
 
 extern "C" int jq_version(void) { return JQ_VERSION; }

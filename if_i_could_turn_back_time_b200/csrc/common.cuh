@@ -24,16 +24,19 @@ static inline int jq_launch_status() {
 
 static inline bool jq_aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// Dynamic shared memory of a kernel raised to `bytes`, once per device (asking for it costs a call about a microsecond).
-// `done` has a bit per device and belongs to this kernel and size.
-static inline cudaError_t jq_allow_smem(const void *kernel, int bytes, std::atomic<unsigned long long> &done) {
-    int dev = 0;
-    const cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-    if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+// Number of the calling thread's current CUDA context, from 1 on and never given twice by the driver; 0 if there is none or the
+// driver cannot tell.
+unsigned long long jq_context_id();
+
+// Dynamic shared memory of a kernel raised to `bytes`, once per context (asking for it costs a call about a microsecond).  The
+// limit belongs to the kernel as this context has loaded it: a device that has been reset has a new one, under the same device
+// number.  `done` belongs to this kernel and size; contexts that share one of its places ask in turn.
+typedef std::atomic<unsigned long long> jq_contexts[8];
+static inline cudaError_t jq_allow_smem(const void *kernel, int bytes, jq_contexts &done) {
+    const unsigned long long id = jq_context_id();
+    if (id && done[id & 7].load(std::memory_order_relaxed) == id) return cudaSuccess;
     const cudaError_t s = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (s == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+    if (s == cudaSuccess && id) done[id & 7].store(id, std::memory_order_relaxed);
     return s;
 }
 

@@ -716,7 +716,7 @@ static int launch(int fmt, const void *qw, const void *scales, const void *codeb
         return JQ_ERR_CUDA_BASE - (int)cudaErrorInvalidValue;
 
     auto kern = mode == kGf4 ? gemm_rows_kernel<kGf4> : (mode == kE2m1 ? gemm_rows_kernel<kE2m1> : gemm_rows_kernel<kE2m1Folded>);
-    static std::atomic<unsigned long long> done[3], conv_done[9];
+    static jq_contexts done[3], conv_done[9];
     JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(kern), kSmemBytes, done[mode]));
     if (lin) {
         lin->xp = xp; lin->xscale = xscale; lin->G = G; lin->NT = s.NT;

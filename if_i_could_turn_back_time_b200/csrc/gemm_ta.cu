@@ -1667,7 +1667,7 @@ static int ta_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, co
     int split = 1;
     if (!nprob && parts == 4 && (single.K >> 8) >= kPartMinSteps)
         split = grid * 4 <= jq_sm_count() ? 4 : (grid * 2 <= jq_sm_count() ? 2 : 1);
-    static std::atomic<unsigned long long> done{0};
+    static jq_contexts done;
     JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(kern), smem, done));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
@@ -1696,7 +1696,7 @@ static int lut2_launch(const TaProblem *probs_dev, const CUtensorMap *maps_dev, 
     auto kern = own ? gf4_lut2_kernel<B, true> : gf4_lut2_kernel<B, false>;
     constexpr int smem = LutSmem::kBytes;
     static_assert(smem <= 227 * 1024, "shared memory");
-    static std::atomic<unsigned long long> done[2];
+    static jq_contexts done[2];
     JQ_CUDA_TRY(jq_allow_smem(reinterpret_cast<const void *>(kern), smem, done[own ? 1 : 0]));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
