@@ -1535,28 +1535,27 @@ extern "C" int jq_gemv_grouped_peers(const jq_problem *problems_dev, const void 
 // nor lend a workspace (allocator hooks, fixed-footprint real-time loops): the
 // scratch is this file-scope device array.  In host code the symbol is only a
 // stand-in for the device object, so its device address is fetched once per
-// device with cudaGetSymbolAddress and that pointer is what the kernels get.
+// context with cudaGetSymbolAddress and that pointer is what the kernels get
+// (a device that has been reset has a new context, and the array may lie
+// elsewhere in it).  Contexts that share one of the places fetch it in turn.
 static __device__ __align__(256) unsigned char jq_noalloc_scratch[JQ_NOALLOC_SCRATCH_BYTES];
 
 #include <mutex>
 static int noalloc_scratch_address(void **out) {
-    static void *addr[64];
-    static bool known[64];
+    static struct { unsigned long long context; void *addr; } kept[8];
     static std::mutex mu;
-    int dev = -1;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return JQ_ERR_CUDA_BASE - (int)e;
-    if (dev < 0 || dev >= 64) return JQ_ERR_UNSUPPORTED;
+    const unsigned long long id = jq_context_id();
     std::lock_guard<std::mutex> lk(mu);
-    if (!known[dev]) {
+    if (!id || kept[id & 7].context != id) {
         void *p = nullptr;
-        e = cudaGetSymbolAddress(&p, jq_noalloc_scratch);  // the current device's copy of the array
+        cudaError_t e = cudaGetSymbolAddress(&p, jq_noalloc_scratch);  // the current context's copy of the array
         if (e != cudaSuccess) return JQ_ERR_CUDA_BASE - (int)e;
         if (!p) return JQ_ERR_NULL_PTR;
-        addr[dev] = p;
-        known[dev] = true;
+        *out = p;
+        if (id) { kept[id & 7].context = id; kept[id & 7].addr = p; }
+        return JQ_OK;
     }
-    *out = addr[dev];
+    *out = kept[id & 7].addr;
     return JQ_OK;
 }
 

@@ -137,7 +137,7 @@ int jq_gemv_gf4(const void *qweight, const void *scales_or_null, const void *cod
  * jq_gemv_*.  It has no counterpart in the reference.
  *   - Limit: tiles * B * N * 4 bytes must fit the array, otherwise
  *     JQ_ERR_SCRATCH_LIMIT is returned and nothing is launched.
- *   - The first call on each device looks up the array's device address
+ *   - The first call in each CUDA context looks up the array's device address
  *     (a driver query, not an allocation); make that first call outside any
  *     stream capture.
  *   - All calls on a device share the one array.  Every word a call reads

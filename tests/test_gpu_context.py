@@ -69,3 +69,38 @@ def test_calls_after_the_device_was_reset():
     lib = os.path.join(ROOT, "if_i_could_turn_back_time_b200", "_lib.py")
     r = subprocess.run([sys.executable, "-c", CHILD, lib], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "same", r.stderr[-2000:]
+
+
+NO_ALLOC = CHILD[:CHILD.index("N, K, T = ")] + r"""
+N, K, B = 96, 28672, 8             # more activation than fits in shared memory: partial sums in the library's own array
+rng = np.random.default_rng(2)
+qw = rng.integers(0, 256, (N, K // 2), dtype=np.uint8)
+sc = rng.uniform(0.5, 1, (N, K // 32)).astype(np.float16)
+x = rng.standard_normal((B, K)).astype(np.float32)
+def ok(st):
+    assert st == 0, jq.strerror(st) if st < 0 else st
+def device(a):
+    p = ctypes.c_void_p()
+    ok(rt.cudaMalloc(ctypes.byref(p), a.nbytes))
+    ok(rt.cudaMemcpy(p, a.ctypes.data, a.nbytes, 1))
+    return p
+def call():
+    y = np.zeros((B, N), np.float32)
+    dy = device(y)
+    ok(lib.jq_gemv_noalloc(0, device(qw), device(sc), None, device(x), None, dy, N, K, B, 32, 0, 0, 0, None))
+    ok(rt.cudaMemcpy(y.ctypes.data, dy, y.nbytes, 2))
+    return y
+first = [call(), call()]
+ok(rt.cudaDeviceReset())
+device(np.zeros(64 << 20, np.uint8))      # (the new context's memory is laid out otherwise)
+for y in first + [call(), call()]:
+    assert np.isfinite(y).all() and np.abs(y).max() > 0 and np.array_equal(y, first[0])
+print("same")
+"""
+
+
+def test_calls_without_workspace_after_the_device_was_reset():
+    """The array of the allocation-free entry is looked up again: its address in the first context means nothing in the next."""
+    lib = os.path.join(ROOT, "if_i_could_turn_back_time_b200", "_lib.py")
+    r = subprocess.run([sys.executable, "-c", NO_ALLOC, lib], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "same", r.stderr[-2000:]
