@@ -139,3 +139,29 @@ def test_activation_prepared_by_wide_and_narrow_blocks(K, dtype):
         off = raw[1:].view(8, K)
         off.copy_(grp.xs[i])
         assert torch.equal(ops.linear(grp.xs[i], pw), grp.ys[i]) and torch.equal(ops.linear(off, pw), grp.ys[i])
+
+
+@pytest.mark.parametrize("fmt,g,B", [("gf4", 128, 2), ("gf4", 256, 16), ("gf4", 128, 20), ("gf4", 128, 40), ("e2m1", 32, 9), ("e2m1", 32, 16),
+                                     ("e2m1", 32, 24), ("e2m1", 32, 40)])
+def test_parts_of_odd_step_counts_over_several_tiles(fmt, g, B):
+    """Rows of 9, 3 and 11 steps, two to three tiles per CTA: the four parts of a row's sum begin and end at another stage,
+    slot and accumulator in every tile.  Against 64 bits, and the bits of single calls, whole and by row shards."""
+    spec = jq.QuantSpec(fmt, g, 0)
+    gen = torch.Generator("cpu").manual_seed(B)
+    packed = [jq.pack_weight(_weights(N, K, N + K).to(DEV), spec) for N, K in ((20000, 2304), (18950, 768), (9000, 2816))]
+    grp = ops.GroupedGemv(packed, B, torch.float32)
+    for x in grp.xs:
+        x.copy_(torch.randn(x.shape, generator=gen))
+    grp.run()
+    assert grp.status() == 0 and grp._ta
+    for w, x, y in zip(packed, grp.xs, grp.ys):
+        # (fp16 rounding of the activation, 2^-12 of a term, and of value x scale for E2M1; sums of at most 2816 terms)
+        ref = x.double() @ ops.dequantize(w).double().t()
+        assert (y - ref).abs().max() <= 1e-3 * ref.abs().max()
+        if ops.many_rows(spec.fmt_id, w.K, g, B):
+            continue
+        assert torch.equal(ops.linear(x, w), y)
+        first = w.N // 3 // 64 * 64             # (a shard's tiles start elsewhere; its scales still on a 16-byte boundary)
+        part = w.rows(first, w.N)
+        assert torch.equal(ops.linear(x, part), y[:, first:])
+    assert ops.check_status(raise_on_error=False) == 0
