@@ -1,13 +1,18 @@
 // Packed 4-bit weights x activations on the 5th-generation tensor cores with
 // the decoded weights handed over in tensor memory (tcgen05, sm_100a).
 //
+// Three kernels, by the rows of the activation: gf4_lut2_kernel (GF4, one row, on
+// the CUDA cores: further below), gemm_ta_kernel (up to 16 rows) and
+// wide::gemm_ta_wide_kernel (17 to 64 rows).  What the last two share:
+//
 // One persistent CTA per SM works through 128-row tiles of the weight matrices.
 // A decode thread owns one weight row of the tile (= one tensor-memory lane)
-// and every fourth 128-code group of that row:
+// and every fourth 128-code group of that row (from 17 rows on: every other
+// 256-code step):
 //   * the packed codes of the tile arrive by TMA (cp.async.bulk.tensor, one
-//     128-row x 128-byte box per 256 codes with the 128-byte swizzle, completion
-//     counted on an mbarrier), so that every lane reads its own row without
-//     bank conflicts;
+//     128-row x 128-byte box per 256 codes, from 17 rows on a 32-row box per
+//     warp, with the 128-byte swizzle, completion counted on an mbarrier), so
+//     that every lane reads its own row without bank conflicts;
 //   * GF4: a byte (two codes) indexes the row's 256-entry table of fp16 pairs,
 //     built once per tile in a shared-memory column that only this lane's bank
 //     serves (one conflict-free 32-bit lookup per two codes, the address formed
@@ -25,7 +30,7 @@
 //     differ from the FMA kernels only in summation order).  E2M1 folds its
 //     scales into the fp16 weights (one rounding per weight).
 // The multiply-accumulate work thus costs the CUDA cores nothing, whatever the
-// batch (up to 64 columns per pass), and the lookups are halved.
+// batch (up to 64 columns per pass), and up to 16 rows the lookups are halved.
 //
 // Every wait on an mbarrier is bounded: on expiry the CTA raises a status word
 // in the workspace, all roles leave their loops, tensor memory is freed and
@@ -149,11 +154,11 @@ __global__ void __launch_bounds__(kPrepThreads) ta_prepare_kernel(const TaProble
 // kAccs accumulators of NB columns (group t in t mod kAccs).  An activation stage belongs to the operand slot of its group.
 //
 // What bounds it: neither a pipe nor the decode warps alone.  7B-shaped GF4 step, 8 rows (70B-shaped E2M1, 7 layers, 16 rows),
-// 8 decode warps before: 1053 us (889); now 969 (876).  With the lookups left out 801 (778), with one MMA of eight 857 (811),
-// without folding no change; nothing but the barriers, the loads and a quarter of the stores 720 (725).  Barrier operations
-// are a large part of what is left (a ready wait with its vote takes 105 clocks, an elected arrival 50 to 70): operand slots of
-// half a group, which are busy for a shorter time, were slower (953 against 928 us on one GPU), one issuer and one slot per
-// phase too (939).
+// with 8 decode warps before: 1033 us (879); with this kernel: 949 (861).  Of its time, measured before the partition's costs
+// were set: the lookups 17 % (11), seven MMAs of eight 12 % (7), folding nothing; with nothing but the barriers, the loads and a
+// quarter of the stores it still takes 74 % (83).  Barrier operations are a large part of what is left (a ready wait with its
+// vote takes 105 clocks, an elected arrival 50 to 70): operand slots of half a group, which are busy for a shorter time, were
+// 2.7 % slower, one issuer and one slot per phase 1.2 %.
 // GF4 looks every byte up in the pair table.  Up to 16 rows; more are for the kernel below.
 //
 // A row's sum is formed in four parts of K (one, for short rows and for 33 rows and more), each in group order, added in
@@ -383,7 +388,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_kernel(const TaProblem 
                 };
                 // half of the group is decoded before the wait for its slot, the rest while the first pairs are being stored;
                 // handed over at once (kept until the next group's first lookups are under way, which spares a wait for the
-                // stores, a slot is held for longer: 1022 against 953 us for the 7B-shaped GF4 step with 8 rows)
+                // stores, a slot is held for longer: 7 % slower on the 7B-shaped GF4 step with 8 rows)
                 uint32_t va[16], vb[16];
                 decode16(0, va);
                 decode16(1, vb);
@@ -975,7 +980,7 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_wide_kernel(const TaPro
             }
             if constexpr (C::kParts > 1) {
                 if (split > 1) {
-                    // every group of this CTA has been folded: nothing reads the tables or the activation rings any more.
+                    // every group of this CTA has been folded: nothing reads the activation rings any more.
                     // Each CTA leaves its parts in its shared memory; rank k writes columns k, k + split, ...
                     const int per = C::kParts / split;
 #pragma unroll
@@ -1115,8 +1120,8 @@ __global__ void __launch_bounds__(kTaThreads, 1) gemm_ta_wide_kernel(const TaPro
 
 }  // namespace wide
 
-// ---- GF4, batch 1 on the CUDA cores (the template also covers two rows, where the tensor-memory kernel is faster) ----
-// Same tiles, same TMA weight ring, same per-row pair tables as the tensor-memory kernel above, but the
+// ---- GF4, batch 1 on the CUDA cores (B is 1; sums and partial sums are laid out for two rows) ----
+// Per-row pair tables as in the tensor-memory kernel for up to 16 rows, but tiles of 64 rows, a weight ring per warp, and the
 // multiply-accumulate stays in the decode threads: lane = weight row, so all lanes of a warp need the same
 // activation values, which they read as broadcast 16-byte shared-memory loads (one wavefront per eight
 // codes) from the prepared activation of the whole problem, and a looked-up pair feeds two
@@ -1482,8 +1487,15 @@ static const int kTaMagic = 0x4a515441;
 // GF4 step (us per step on one GPU / for an eighth of it): bytes only 940 / 150.5; 384, 2048: 921.5 / 143.0;
 // 768, 4096: 910.1 / 141.3; 1408, 6144: 900.1 / 140.1; 2304, 8192: 943.3 / 143.9.
 static const double kLutTileCost = 1408, kLutProblemCost = 6144;
-// The same for the tensor-memory kernel, whose loads and decode warps run across tile boundaries.  7B-shaped GF4 step with 8
-// rows / 70B-shaped E2M1 with 16: 1408, 6144: 923 / 846 us; 700, 3000: 900 / 794; 300, 3000: 901 / 778; 0, 0: 907 / 817.
+// The same for the tensor-memory kernels, whose loads and decode warps run across tile boundaries.  Swept in turn on one GPU, us
+// per step, 7B-shaped GF4 (32 layers), 70B-shaped E2M1 (7 layers) and 7B-shaped E2M1 (16 layers):
+//                    GF4, rows 8   24     48     E2M1 70B, rows 16   24    48      E2M1 7B, rows 24   48
+//     1408, 6144          968     1613   2016                  918   971   1216                 522   702
+//      700, 3000          935     1500   1989                  853   913   1166                 507   706
+//      400, 3000          939     1494   2005                  849   908   1198                 511   711
+//      300, 3000          943     1507   2004                  855   914   1193                 512   712
+//        0,    0          957     1517   2009                  851   913   1192                 518   714
+// (runs of one side differ by 1 to 3 % where the power cap holds the clock: all but GF4 with 24 rows)
 static const double kTaTileCost = 400, kTaProblemCost = 3000;
 static const int kTaHeader = 12;
 
@@ -1519,8 +1531,12 @@ static bool ta_shape_ok(int fmt, int N, int K, int g, int had) {
     return fmt == JQ_FMT_E2M1 && g == 32;
 }
 
-// batch 1 runs on the CUDA cores when the prepared activation of one problem fits its shared-memory buffer
-// (K up to 12288); on the 7B-shaped step 931 us against 1114 on the tensor-memory kernel, which takes over from two rows
+// batch 1 runs on the CUDA cores when the prepared activation of one problem fits its shared-memory buffer (K up to 12288).
+// The line is older than the tensor-memory kernel of 24 warps, against whose predecessor this was 931 us to 1114 on the
+// 7B-shaped step.  Now the CUDA cores are ahead for single calls of few tiles, which take one launch instead of two, and behind
+// elsewhere (one row, us, CUDA cores / tensor memory): single calls 1024 x 1024 18.9 / 24.0, 4096 x 4096 14.7 / 17.3, 11008 x 4096
+// 20.9 / 17.6, 4096 x 11008 21.2 / 17.6, 32000 x 4096 32.0 / 28.5; 7B-shaped step 956 / 836.  The two add a row's products in
+// another order, so that moving the line changes last bits of one-row results.
 static bool ta_use_lut(int B, int maxK) { return B == 1 && (size_t)maxK * 2 <= (size_t)LutSmem::kXBytes; }
 
 extern "C" size_t jq_ta_workspace_bytes(const jq_problem *ph, int n, int B) {
@@ -1633,7 +1649,7 @@ static void ta_pdl_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2
 static int ta_prepare(const TaProblem *probs_dev, const TaProblem &single, int nblk, int B, int x_dtype, cudaStream_t st) {
     // up to two blocks of 32 warps per SM.  Single calls, with values loaded one by one by 8 warps before: 4096 x 11008 E2M1, 23
     // rows, 16.8 -> 14.8 us; 4096 x 14336, 16 rows, 18.0 -> 14.8; the 7B-shaped GF4 step with 8 rows (1792 blocks of 8 warps,
-    // loads of four values) 939 -> 927.
+    // loads of four values) 1.3 % less.
     const bool wide = nblk <= 2 * jq_sm_count() || B <= 2;
     void (*const kernels[3][2])(const TaProblem *, TaProblem, int) = {
         {ta_prepare_kernel<256, float>, ta_prepare_kernel<1024, float>},

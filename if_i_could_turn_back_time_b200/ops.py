@@ -320,15 +320,22 @@ def conv2d(x: torch.Tensor, pw: PackedWeight, bias: Optional[torch.Tensor], kern
 def conv_gathers(fmt_id: int, K: int, g: int, positions: int) -> bool:
     """Convolutions whose fields the preparation kernel gathers (the others are unfolded first): the output positions that
     the many-row kernel is for, and fields of up to 1536 values or more than 2048 positions.  A block gathers 32 positions and
-    walks along the whole field, so that long fields at few positions leave most of the chip idle.  Device time of calls with
-    3 x 3 kernels in us, gathered / unfolded (which also has five more launches):
+    walks along the whole field, so that long fields at few positions leave most of the chip idle.
 
-        positions   K = 1152       K = 2304       K = 4608       K = 9216
-        25          22 / 19        33 / 21        56 / 25        102 / 32
-        196         22 / 21        33 / 24        57 / 31        103 / 46
-        784         24 / 29        35 / 38        59 / 55        105 / 94
-        1568        27 / 40        40 / 60        63 / 92        110 / 167
-        3136        30 / 63        44 / 104       68 / 169       115 / 325"""
+    The line of 2048 positions was drawn when the gathering formed its addresses by products and took two to three times as
+    long.  Where it lies now, calls of 1024 to 2048 positions with more than 1536 values are still unfolded although gathering
+    would be faster, and so are 784 positions of 2304 values.  Whole calls of a layer with 3 x 3 kernels and 256 outputs, us,
+    gathered / unfolded (784 positions: four images, 1024 and 2048: images of 16 x 16 and 32 x 32):
+
+        positions   K = 2304       K = 4608       K = 9216
+        196         36 / 53        60 / 52        107 / 57
+        784         42 / 52        66 / 67        112 / 107
+        1024        56 / 89        81 / 103       130 / 157
+        1568        46 / 116       70 / 137       117 / 222
+        2048        46 / 80        72 / 130       142 / 250
+        3136        52 / 124       77 / 197       129 / 355
+
+    On the device alone 196 positions of 2304 values take 33 / 26, and of 1152 values 22 / 21."""
     few = ta_max_batch(fmt_id) if fmt_id == _lib.JQ_FMT_E2M1 and ta_eligible(fmt_id, K, g, positions) else 16
     return positions > few and (K <= 1536 or positions > 2048)
 

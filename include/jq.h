@@ -211,8 +211,10 @@ int jq_gemv_grouped_peers(const jq_problem *problems_dev, const void *plan_host,
  * qweight / codebook / E2M1 scales 16-byte aligned, and
  *   fmt GF4,  group sizes of 128 * 2^k,
  *   fmt E2M1, group size 32,            1 <= B <= 64.
- * The packed rows arrive by 2-D tiled TMA (32-row x 128-byte boxes, 128-byte
- * swizzle), a decode thread owns one weight row of a 128-row tile.
+ * The packed rows arrive by 2-D tiled TMA (boxes of 128 bytes and 128 rows, or
+ * 32 rows for B > 16 and for B == 1 on the CUDA cores; 128-byte swizzle), a
+ * decode thread owns one weight row of a tile of 128 rows (64 on the CUDA
+ * cores).
  *   GF4: a byte of packed codes indexes a 256-entry table of fp16 pairs that is
  *        built per tile in shared memory, one bank column per weight row, so
  *        two codes cost one conflict-free lookup (B > 16: lookups in
@@ -248,7 +250,7 @@ int jq_gemv_grouped_peers(const jq_problem *problems_dev, const void *plan_host,
  * resets it.  Grouped form: jq_ta_plan (host only) validates the problems,
  * creates their tensor maps and writes jq_ta_plan_bytes(n) bytes that the
  * caller copies to the device (64-byte aligned); jq_gemm_ta_grouped enqueues
- * the two launches, with the peer-store all-gather of jq_gemv_grouped_peers
+ * two launches (the preparation always has one here), with the peer-store all-gather of jq_gemv_grouped_peers
  * when npeer > 1.  problems_host[i].K alone is read by jq_ta_workspace_bytes.
  * Unsupported shapes return JQ_ERR_UNSUPPORTED, misaligned pointers
  * JQ_ERR_BAD_ALIGN; nothing is launched then. */
