@@ -50,9 +50,9 @@ PARITY_GATE = 1e-3
 # at batch 1); traffic grows in proportion to the rows processed, so a full launch's traffic is this ratio times its
 # algorithmic bytes.
 DRAM_TRAFFIC_RATIO = {
-    "gf4_lut2_kernel": (377.961216 + 5.431552) / 378.101760,
-    "gemm_ta_kernel<gf4>": (379.913984 + 7.676416) / 385.351680,
-    "gemm_ta_kernel<e2m1>": (621.605632 + 6.630912) / 612.368384,
+    "gf4_lut2_kernel": (377.991936 + 3.914752) / 378.101760,
+    "gemm_ta_kernel<gf4>": (379.895552 + 7.174144) / 385.351680,
+    "gemm_ta_kernel<e2m1>": (631.751168 + 6.501632) / 612.368384,
     "gemv_grouped_kernel": 608.581888 / 604.504064,      # E2M1; GF4 reaches this kernel only for ungrouped or short rows
 }
 
